@@ -350,9 +350,10 @@ __device__ __forceinline__ bool group_may_hit(float4 lo, float4 hi, float3 o, fl
 // spheres, then planes (light planes first); first-tested wins ties.
 // Returns the primitive code (kPrimNone on a miss) with `closest` lowered to
 // its t.
-__device__ __forceinline__ uint32_t scene_analytic(const DScene& S, float3 o, float3 d, float& closest)
+__device__ __noinline__ uint32_t scene_analytic_exact(const DScene& S, float3 o, float3 d, float& closest)
 {
     uint32_t prim = kPrimNone;
+#pragma unroll 1
     for (int i = 0; i < S.n_spheres; i++) {
         float t0;
         if (sphere_hit(S.spheres[i], o, d, t0) && t0 < closest) {
@@ -368,6 +369,7 @@ __device__ __forceinline__ uint32_t scene_analytic(const DScene& S, float3 o, fl
         const float4 lo = S.pgroups[2 * g], hi = S.pgroups[2 * g + 1];
         const int first = __float_as_int(lo.w), count = __float_as_int(hi.w);
         if (count > 1 && !group_may_hit(lo, hi, o, d, rd, closest)) continue;
+#pragma unroll 1
         for (int i = first; i < first + count; i++) {
             float t0;
             if (plane_hit(S.planes[i], o, d, closest, t0) && t0 < closest) {
@@ -377,6 +379,220 @@ __device__ __forceinline__ uint32_t scene_analytic(const DScene& S, float3 o, fl
         }
     }
     return prim;
+}
+
+// ----------------------------------------------------------------- estimates
+// The analytic scene is first traced with plain fused arithmetic and without
+// branches per primitive: axis-aligned rectangles, boxes as three slabs, and
+// spheres, each with a margin around everything the reference's float
+// operations could decide otherwise.  An answer is taken only where the
+// margins leave no doubt (and its t is then computed with the reference's
+// operations); any doubt sends the ray through the exact tests.  So hit ids,
+// t and shadow answers are those of the exact tests.
+//
+// Margins.  With every coordinate, the origin's included, within `reach`,
+// a distance to a plane or slab (and the point a ray meets it at) carries an
+// error of at most 1e-6 reach in these operations and as much in the
+// reference's; flat_pad is 1e-5 reach.  Along the ray an axis-aligned plane's
+// t = (p - o) / d is within 2^-21 of the exact quotient, and a slab's entry
+// lies between those of the slab widened and narrowed by the margin.  A
+// sphere's discriminant carries less than 2e-6 |c - o|^2.  Rays nearly
+// parallel to a plane (which the reference skips below 1e-6) are in doubt.
+//
+// What bounds it: instruction issue.  About 30 instructions a rectangle and 90
+// a box for all lanes of a warp; the exact tests' early rejects left half of
+// the lanes idle (16 to 18 of 32 active) through about 1500 (Cornell box, 18
+// quads).  0.1 % of the rays are in doubt.  24 uneven renders batched, three of
+// them on a mesh: 114.9 -> 108.8 ms.
+struct FlatRay {
+    float3 o, d, rd;
+    bool sure;
+};
+__device__ __forceinline__ FlatRay flat_ray(const DScene& S, float3 o, float3 d)
+{
+    FlatRay r;
+    r.o = o;
+    r.d = d;
+    r.rd = make_float3(rcp_approx(d.x), rcp_approx(d.y), rcp_approx(d.z));
+    // written so that a NaN leaves `sure` false
+    r.sure = fabsf(o.x) < S.flat_reach && fabsf(o.y) < S.flat_reach && fabsf(o.z) < S.flat_reach &&
+             fabsf(f3dot(d, d) - 1.f) < 1e-2f && fabsf(d.x) > 2e-6f && fabsf(d.y) > 2e-6f && fabsf(d.z) > 2e-6f;
+    return r;
+}
+// The ray's components as one axis and the two others in x y z order; next()
+// goes from x over y to z.  (Loops over the axes and the primitives stay
+// loops: unrolled, the code outgrows the instruction cache.)
+struct AxisRay {
+    float ok, rk, oi, di, oj, dj, dk, ri, rj;
+    int axis;
+    __device__ __forceinline__ AxisRay(const FlatRay& r)
+        : ok(r.o.x), rk(r.rd.x), oi(r.o.y), di(r.d.y), oj(r.o.z), dj(r.d.z), dk(r.d.x), ri(r.rd.y), rj(r.rd.z), axis(0)
+    {
+    }
+    __device__ __forceinline__ void next()
+    {
+        // (x; y z) -> (y; x z) -> (z; x y)
+        const bool i = axis == 0;
+        const float o = ok, d = dk, q = rk;
+        ok = i ? oi : oj; dk = i ? di : dj; rk = i ? ri : rj;
+        if (i) { oi = o; di = d; ri = q; }
+        else { oj = o; dj = d; rj = q; }
+        axis++;
+    }
+};
+// t of a rectangle's plane, and by how far the point there lies outside the
+// rectangle (negative: inside).
+__device__ __forceinline__ float rect_excess(const DRect& q, const AxisRay& r, float& t, int& id, int& flags)
+{
+    const float4 a = __ldg(&q.a), b = __ldg(&q.b);
+    t = (a.x - r.ok) * r.rk;
+    id = __float_as_int(a.w);
+    flags = __float_as_int(b.z);
+    return fmaxf(fabsf(fmaf(t, r.di, r.oi) - a.y) - b.x, fabsf(fmaf(t, r.dj, r.oj) - a.z) - b.y);
+}
+struct BoxSpan {
+    float in_p, out_p;   // widened box: entry, exit
+    float in_s;          // narrowed box: entry
+    bool sure;           // enters through one face, away from its edges
+    int axis;            // that face's slab
+    float den;           // and d.n there
+};
+__device__ __forceinline__ void slab_span(float4 nc, float h, float pad, const FlatRay& r, float& den, float& ep, float& es,
+                                          float& xp, float& xs)
+{
+    const float f = fmaf(nc.x, r.o.x, fmaf(nc.y, r.o.y, fmaf(nc.z, r.o.z, -nc.w)));
+    den = fmaf(nc.x, r.d.x, fmaf(nc.y, r.d.y, nc.z * r.d.z));
+    const float inv = rcp_approx(den), ai = fabsf(inv), tc = -f * inv;
+    const float wp = (h + pad) * ai, ws = (h - pad) * ai;
+    ep = tc - wp;
+    es = tc - ws;
+    xp = tc + wp;
+    xs = tc + ws;
+}
+__device__ __forceinline__ BoxSpan box_span(const DBox& B, FlatRay& r)
+{
+    const float4 h = __ldg(&B.h);
+    const float pad = h.w;
+    float den0, den1, den2, p0, p1, p2, s0, s1, s2, xp0, xp1, xp2, xs0, xs1, xs2;
+    slab_span(__ldg(&B.nc[0]), h.x, pad, r, den0, p0, s0, xp0, xs0);
+    slab_span(__ldg(&B.nc[1]), h.y, pad, r, den1, p1, s1, xp1, xs1);
+    slab_span(__ldg(&B.nc[2]), h.z, pad, r, den2, p2, s2, xp2, xs2);
+    r.sure = r.sure && fminf(fminf(fabsf(den0), fabsf(den1)), fabsf(den2)) > 2e-6f;
+    BoxSpan b;
+    b.in_p = fmaxf(fmaxf(p0, p1), p2);
+    b.out_p = fminf(fminf(xp0, xp1), xp2);
+    const float m = fmaxf(s0, s1), second = fmaxf(fminf(s0, s1), fminf(m, s2));
+    b.in_s = fmaxf(m, s2);
+    const bool a2 = s2 > m, a1 = s1 > s0;
+    b.axis = a2 ? 2 : (a1 ? 1 : 0);
+    b.den = a2 ? den2 : (a1 ? den1 : den0);
+    const float ep = a2 ? p2 : (a1 ? p1 : p0);
+    // the entry point lies inside the two other slabs by the margin, and the
+    // ray starts outside the box
+    b.sure = second <= ep && b.in_s <= fminf(fminf(xs0, xs1), xs2) && b.in_p > 1e-4f;
+    return b;
+}
+// A sphere: whether the ray may meet it, surely does, and bounds of t.
+struct SphereSpan {
+    bool may, sure;
+    float lo, hi;
+};
+__device__ __forceinline__ float sqrt_approx(float x)
+{
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ SphereSpan sphere_span(float4 c, const FlatRay& r)
+{
+    const float3 cp = make_float3(c.x - r.o.x, c.y - r.o.y, c.z - r.o.z);
+    const float b = f3dot(r.d, cp), cc = f3dot(cp, cp), out = cc - c.w * c.w, disc = fmaf(b, b, -out);
+    const float pad = 2e-6f * cc + 2e-6f * c.w * c.w;
+    const float far = sqrt_approx(fmaxf(disc + pad, 0.f)) * (1.f + 4e-6f), near = sqrt_approx(fmaxf(disc - pad, 0.f)) * (1.f - 4e-6f);
+    const bool inside = out < 0.f;
+    SphereSpan s;
+    // outside with the centre behind: both roots are negative
+    s.may = disc > -pad && !(out > pad && b <= 0.f);
+    s.sure = disc > pad && fabsf(out) > pad;
+    const float e = 1e-6f * (fabsf(b) + c.w);
+    s.lo = (inside ? b + near : b - far) - e;
+    s.hi = (inside ? b + far : b - near) + e;
+    return s;
+}
+
+// Closest analytic hit where the estimates decide it: returns false in
+// doubt, else sets prim (kPrimNone on a miss) and its exact t in `closest`.
+__device__ __forceinline__ bool flat_closest(const DScene& S, float3 o, float3 d, float& closest, uint32_t& prim)
+{
+    const float inf = __int_as_float(0x7f800000);
+    FlatRay r = flat_ray(S, o, d);
+    const float pad = S.flat_pad;
+    float first = inf, second = inf;  // smallest lower bounds of t
+    int id = -1;                      // plane | -2 - sphere | box face, of `first`
+    bool sure1 = true;
+    auto take = [&](bool may, bool sure, float lo, int code) {
+        const float l = may ? lo : inf;
+        second = fminf(second, fmaxf(first, l));
+        if (l < first) { id = code; sure1 = sure; }
+        first = fminf(first, l);
+    };
+    const DRect* q = S.rects;
+    AxisRay ar(r);
+#pragma unroll 1
+    for (int axis = 0; axis < 3; axis++) {
+        bool met = false;  // an earlier rectangle of the same plane has the point: it wins the tie
+#pragma unroll 1
+        for (const DRect* end = q + S.n_rects[axis]; q < end; q++) {
+            float t;
+            int pid, flags;
+            const float e = rect_excess(*q, ar, t, pid, flags);
+            met = met && (flags & kRectSamePlane);
+            const bool may = e < pad && t > 5e-7f && !met;
+            take(may, e < -pad && t > 2e-6f, t * (1.f - 9.5367431640625e-07f), pid);
+            met = met || may;
+        }
+        ar.next();
+    }
+    constexpr int kBoxCode = 1 << 29;
+#pragma unroll 1
+    for (int i = 0; i < S.n_boxes; i++) {
+        const BoxSpan b = box_span(S.boxes[i], r);
+        take(b.in_p <= b.out_p && b.out_p > 0.f, b.sure, fmaxf(b.in_p, 0.f), kBoxCode | i << 3 | b.axis << 1 | (b.den > 0.f ? 0 : 1));
+    }
+#pragma unroll 1
+    for (int i = 0; i < S.n_spheres; i++) {
+        const SphereSpan s = sphere_span(__ldg(&S.spheres[i].c_r), r);
+        take(s.may, s.sure, fmaxf(s.lo, 0.f), -2 - i);
+    }
+    if (!r.sure || !sure1) return false;
+    prim = kPrimNone;
+    if (id == -1) return true;
+    float t;
+    if (id < -1) {
+        if (!sphere_hit(S.spheres[-2 - id], o, d, t)) return false;
+        prim = kPrimSphere | (uint32_t)(-2 - id);
+    } else {
+        if (id & kBoxCode) {
+            const DBox& B = S.boxes[(id & ~kBoxCode) >> 3];
+            const int4 f = (id & 1) ? B.hi : B.lo;
+            const int a = (id >> 1) & 3;
+            id = a == 0 ? f.x : (a == 1 ? f.y : f.z);
+        }
+        const float4 N4 = S.planes[id].n_emit, po = S.planes[id].o_mat;
+        const float3 N = xyz(N4);
+        t = ex::div(ex::dot(ex::sub3(xyz(po), o), N), ex::dot(d, N));
+        prim = kPrimPlane | (uint32_t)id;
+    }
+    if (!(t < second) || !(t < closest)) return false;
+    closest = t;
+    return true;
+}
+
+__device__ __forceinline__ uint32_t scene_analytic(const DScene& S, float3 o, float3 d, float& closest)
+{
+    uint32_t prim;
+    if (S.flat_ok && flat_closest(S, o, d, closest, prim)) return prim;
+    return scene_analytic_exact(S, o, d, closest);
 }
 
 // Renderer::sceneIntersect: the analytic primitives, then the triangle BVH.
@@ -408,17 +624,18 @@ __device__ __forceinline__ uint32_t scene_closest(const DScene& S, float3 o, flo
 // with emissive triangles is decided here in full), else kShadowWalk with
 // `bound` set for an any-hit walk of the BVH.
 constexpr int kShadowLit = 0, kShadowBlocked = 1, kShadowWalk = 2;
-__device__ __forceinline__ int scene_blocked_analytic(const DScene& S, const DMaterial* mats, float3 o, float3 d,
+template <bool kMesh>
+__device__ __noinline__ int scene_blocked_exact(const DScene& S, const DMaterial* mats, float3 o, float3 d,
                                                       float tmax, double lim, float& bound)
 {
-    if (S.emissive_tris || S.n_emit_spheres < 0 || S.n_emit_planes < 0) {
-        float t = FLT_MAX, hu, hv;
-        const uint32_t prim = scene_closest(S, o, d, tmax, t, hu, hv);
+    if ((kMesh && S.emissive_tris) || S.n_emit_spheres < 0 || S.n_emit_planes < 0) {
+        float t = tmax, hu, hv;
+        const uint32_t prim = kMesh ? scene_closest(S, o, d, tmax, t, hu, hv) : scene_analytic(S, o, d, t);
         if ((prim & kPrimKindMask) == kPrimNone) return kShadowLit;
         const uint32_t kind = prim & kPrimKindMask, pidx = prim & kPrimIndexMask;
         int mi;
         if (kind == kPrimSphere) mi = S.spheres[pidx].mat.x;
-        else if (kind == kPrimPlane) mi = __float_as_int(S.planes[pidx].o_mat.w);
+        else if (!kMesh || kind == kPrimPlane) mi = __float_as_int(S.planes[pidx].o_mat.w);
         else mi = __float_as_int(S.tris[pidx].e1_mat.w);
         if (mats[S.mat_base + mi].flags & kMatEmissive) return kShadowLit;
         return blocks_at(o, d, t, lim) ? kShadowBlocked : kShadowLit;
@@ -432,6 +649,7 @@ __device__ __forceinline__ int scene_blocked_analytic(const DScene& S, const DMa
         float t0;
         if (plane_hit(S.planes[S.emit_planes[k]], o, d, bound, t0) && t0 < bound) bound = t0;
     }
+#pragma unroll 1
     for (int i = 0; i < S.n_spheres; i++) {
         float t0;
         if (sphere_hit(S.spheres[i], o, d, t0) && t0 < bound) {
@@ -444,6 +662,7 @@ __device__ __forceinline__ int scene_blocked_analytic(const DScene& S, const DMa
         const float4 lo = S.sgroups[2 * g], hi = S.sgroups[2 * g + 1];
         const int first = __float_as_int(lo.w), count = __float_as_int(hi.w);
         if (count > 1 && !group_may_hit(lo, hi, o, d, rd, bound)) continue;
+#pragma unroll 1
         for (int i = first; i < first + count; i++) {
             float t0;
             if (plane_hit(S.splanes[i], o, d, bound, t0) && t0 < bound) {
@@ -452,16 +671,102 @@ __device__ __forceinline__ int scene_blocked_analytic(const DScene& S, const DMa
             }
         }
     }
-    return S.n_nodes > 0 ? kShadowWalk : kShadowLit;
+    return kMesh && S.n_nodes > 0 ? kShadowWalk : kShadowLit;
 }
 
-__device__ __forceinline__ bool scene_blocked(const DScene& S, const DMaterial* mats, float3 o, float3 d, float tmax,
-                                              double lim)
+// The analytic shadow query where the estimates decide it, else -1.  `light`
+// receives the plane index of the emissive rectangle that bounds the query
+// (-1: none, the query's end does).
+__device__ __forceinline__ int flat_blocked(const DScene& S, float3 o, float3 d, float tmax, float d2, int& light)
 {
-    float bound = tmax, hu, hv;
-    const int r = scene_blocked_analytic(S, mats, o, d, tmax, lim, bound);
+    const float inf = __int_as_float(0x7f800000);
+    FlatRay r = flat_ray(S, o, d);
+    const float pad = S.flat_pad;
+    float bound = tmax;     // closest emissive hit, or the query's end
+    float may_t = inf;      // no other hit lies in front of this
+    float hit_t = inf;      // one surely lies in front of this
+    light = -1;
+    bool clear = true;      // the bound is beyond doubt
+    const DRect* q = S.rects;
+    AxisRay ar(r);
+#pragma unroll 1
+    for (int axis = 0; axis < 3; axis++) {
+        bool met = false;   // an emissive rectangle of the same plane has the point: the others tie with the bound
+#pragma unroll 1
+        for (const DRect* end = q + S.n_rects[axis]; q < end; q++) {
+            float t;
+            int pid, flags;
+            const float e = rect_excess(*q, ar, t, pid, flags);
+            met = met && (flags & kRectSamePlane);
+            const bool may = e < pad && t > 5e-7f && !met, sure = e < -pad && t > 2e-6f;
+            const bool emissive = flags & kRectEmissive;
+            if (emissive) {
+                clear = clear && (sure || !may);
+                if (may && t < bound) { bound = t; light = pid; }
+                met = may;
+            } else {
+                may_t = fminf(may_t, may ? t : inf);
+                hit_t = fminf(hit_t, may && sure ? t : inf);
+            }
+        }
+        ar.next();
+    }
+#pragma unroll 1
+    for (int i = 0; i < S.n_boxes; i++) {
+        const BoxSpan b = box_span(S.boxes[i], r);
+        const bool may = b.in_p <= b.out_p && b.out_p > 0.f;
+        may_t = fminf(may_t, may ? b.in_p : inf);
+        hit_t = fminf(hit_t, may && b.sure ? b.in_s : inf);
+    }
+#pragma unroll 1
+    for (int i = 0; i < S.n_spheres; i++) {
+        const SphereSpan s = sphere_span(__ldg(&S.spheres[i].c_r), r);
+        if (__ldg(&S.spheres[i].mat).y) clear = clear && !s.may;
+        else {
+            may_t = fminf(may_t, s.may ? s.lo : inf);
+            hit_t = fminf(hit_t, s.may && s.sure ? s.hi : inf);
+        }
+    }
+    if (!r.sure || !clear) return -1;
+    // blocks_at's comparison, with a margin on the squared distance
+    const float dd = f3dot(d, d), lim = d2 - 1e-3f, m = 0.2f * pad * (1.f + d2);
+    if (hit_t < bound * (1.f - 4e-6f) && hit_t * hit_t * dd < lim - m) return kShadowBlocked;
+    // (may_t may be below zero where a box or sphere reaches around the origin)
+    if (may_t > bound * (1.f + 4e-6f) || (may_t > 0.f && may_t * may_t * dd > lim + m)) return kShadowLit;
+    return -1;
+}
+
+// The part of the shadow query before the triangle BVH (see
+// scene_blocked_exact).
+template <bool kMesh>
+__device__ __forceinline__ int scene_blocked_analytic(const DScene& S, const DMaterial* mats, float3 o, float3 d,
+                                                      float d2, float& bound)
+{
+    // a hit beyond the light cannot block: bound the query just past it
+    const float tmax = sqrtf(d2) * 1.0001f + 1e-4f;
+    if (S.flat_ok && !(kMesh && S.emissive_tris)) {
+        int light;
+        const int r = flat_blocked(S, o, d, tmax, d2, light);
+        if (r == kShadowBlocked) return r;
+        if (r == kShadowLit) {
+            if (!kMesh || S.n_nodes <= 0) return r;
+            bound = tmax;
+            if (light >= 0) {
+                const float3 N = xyz(S.planes[light].n_emit), po = xyz(S.planes[light].o_mat);
+                bound = ex::div(ex::dot(ex::sub3(po, o), N), ex::dot(d, N));
+            }
+            return kShadowWalk;
+        }
+    }
+    return scene_blocked_exact<kMesh>(S, mats, o, d, tmax, (double)d2 - 1e-3, bound);
+}
+
+__device__ __forceinline__ bool scene_blocked(const DScene& S, const DMaterial* mats, float3 o, float3 d, float d2)
+{
+    float bound, hu, hv;
+    const int r = scene_blocked_analytic<true>(S, mats, o, d, d2, bound);
     if (r != kShadowWalk) return r == kShadowBlocked;
-    return bvh4_closest<false, true>(S, o, d, bound, hu, hv, nullptr, lim) == -2;
+    return bvh4_closest<false, true>(S, o, d, bound, hu, hv, nullptr, (double)d2 - 1e-3) == -2;
 }
 
 // ----------------------------------------------------------------- spectra

@@ -898,10 +898,8 @@ __global__ void __launch_bounds__(kTraceMaxBlock, kShadowMinBlocks) k_shadow(Eng
         // afterwards, for lit samples, so it holds no registers across it
         const DScene& S = E.scenes[__float_as_int(SQ.c[i].w) >> 16];
         const float d2 = o.w;
-        // a hit beyond the light cannot block: bound the query just past it
-        const float tmax = sqrtf(d2) * 1.0001f + 1e-4f;
         mine++;
-        if (!scene_blocked(S, E.mats, xyz(o), xyz(d), tmax, (double)d2 - 1e-3)) {
+        if (!scene_blocked(S, E.mats, xyz(o), xyz(d), d2)) {
             const float4 c = SQ.c[i];
             const int pixel = __float_as_int(SQ.d[i].w);
             add_xyz(E.reqs[__float_as_int(c.w) & 0xFFFF].accum + (size_t)pixel * 3, make_float3(c.x, c.y, c.z));
@@ -1126,7 +1124,7 @@ __global__ void k_trace_shadow(const DScene* scene, const DMaterial* mats, const
         const float3 o = make_float3(rays[i * 6], rays[i * 6 + 1], rays[i * 6 + 2]);
         const float3 d = make_float3(rays[i * 6 + 3], rays[i * 6 + 4], rays[i * 6 + 5]);
         const float d2 = dist2[i];
-        blocked[i] = scene_blocked(S, mats, o, d, sqrtf(d2) * 1.0001f + 1e-4f, (double)d2 - 1e-3) ? 1 : 0;
+        blocked[i] = scene_blocked(S, mats, o, d, d2) ? 1 : 0;
     }
 }
 

@@ -75,6 +75,21 @@ struct alignas(16) DLight {
     float4 o_mat, u, v, n;  // plane
 };
 
+// Axis-aligned rectangle of the estimate pass (flat_closest, flat_blocked):
+// a = (plane coordinate p, centre on the two other axes in x y z order, plane
+// index (bits)), b = (half extents on those axes, kRect* flags (bits), 0).
+constexpr int kRectEmissive = 1, kRectSamePlane = 2;  // SamePlane: as the rectangle before it in the list
+struct alignas(16) DRect {
+    float4 a, b;
+};
+// Box (six quads that bound a parallelepiped) of the estimate pass: three
+// slabs |n.x - c| <= h, the quads on their low and high sides.
+struct alignas(16) DBox {
+    float4 nc[3];  // unit normal, c
+    float4 h;      // half widths, distance margin
+    int4 lo, hi;   // plane index per slab
+};
+
 struct DScene {
     const DPlane* planes;
     const DSphere* spheres;
@@ -107,6 +122,12 @@ struct DScene {
     int n_emit_spheres, n_emit_planes;
     int emit_spheres[kMaxEmitPrims], emit_planes[kMaxEmitPrims];
     float total_light_area;
+    // Estimate pass: the scene's quads as axis-aligned rectangles (by normal
+    // axis) and boxes.  flat_ok = 0 when some quad is neither.
+    const DRect* rects;
+    const DBox* boxes;
+    int n_rects[3], n_boxes, flat_ok;
+    float flat_pad, flat_reach;  // distance margin; largest |origin coordinate| it holds for
 };
 
 // Request flags
