@@ -49,24 +49,24 @@ sys.path.insert(0, REPO)
 METRIC = "paths/s, batched+served wavefront (64 uneven spectral renders); plain per-request alongside"
 UNIT = "paths/s"
 HBM_FALLBACK = 6650.0
-# DRAM bytes (read + write) per unit of each wavefront kernel, measured with
-# ncu (dram__bytes_read.sum + dram__bytes_write.sum over every launch of one
-# 8-render step, divided by that step's rays / shadow rays; each launch
-# replayed alone with a cold L2; the summary and command are kept in the
-# profiles directory).  Traffic grows in proportion to the units, so a
-# launch's traffic is this figure times its units.
-NCU_DRAM_PER_UNIT = {"extend": 61.0, "shade": 548.7, "shadow": 83.2}
-# Warp instructions per unit (smsp__inst_executed.sum over the same
-# launches, divided by the same units), for the issue-rate roofline below.
-NCU_INST_PER_UNIT = {"extend": 48.25, "shade": 69.57, "shadow": 43.90}
-# Issue-rate side of the same kernels (ncu --set full, one launch each of an
-# 8-render batch with the queue full): the share of issue slots used and the
-# share of a warp's 32 lanes active per instruction.  The plane and triangle
-# tests are dependent IEEE-exact FP32 chains, so these kernels are bound by
-# issue and latency rather than by DRAM.
-NCU_ISSUE = {"extend": {"issue_slots_busy": 0.638, "lanes_active": 16.2 / 32},
-             "shade": {"issue_slots_busy": 0.382, "lanes_active": 23.2 / 32},
-             "shadow": {"issue_slots_busy": 0.573, "lanes_active": 17.6 / 32, "l1_busy": 0.649}}
+# Variants with a triangle mesh: they run in the queue stages (k_extend,
+# k_shade, k_shadow), the others in the whole-path kernel (k_paths).
+MESH_VARIANTS = ("cornell-bunny",)
+# DRAM bytes (read + write) per unit of each kernel, measured with ncu
+# (dram__bytes_read.sum + dram__bytes_write.sum, each launch replayed alone
+# with a cold L2; the summaries and commands are kept in the profiles
+# directory).  Units: rays (path vertices); shadow rays for k_shadow.
+NCU_DRAM_PER_UNIT = {"k_paths": 0.9, "k_extend": 61.0, "k_shade": 548.7, "k_shadow": 83.2}
+# Warp instructions per unit (smsp__inst_executed.sum over the same launches,
+# divided by the same units), for the issue-rate roofline below.
+NCU_INST_PER_UNIT = {"k_paths": 139.6, "k_extend": 48.25, "k_shade": 69.57, "k_shadow": 43.90}
+# Issue-rate side of the same kernels (ncu --set full, one launch each): the
+# share of issue slots used and the share of a warp's 32 lanes active per
+# instruction.
+NCU_ISSUE = {"k_paths": {"issue_slots_busy": 0.503, "lanes_active": 22.8 / 32},
+             "k_extend": {"issue_slots_busy": 0.638, "lanes_active": 16.2 / 32},
+             "k_shade": {"issue_slots_busy": 0.382, "lanes_active": 23.2 / 32},
+             "k_shadow": {"issue_slots_busy": 0.573, "lanes_active": 17.6 / 32, "l1_busy": 0.649}}
 # Algorithmic BVH-fetch bytes per ray of the batched-mesh workload's two
 # scenes: 2 x 24 B of child boxes per internal node processed plus 36 B per
 # leaf triangle tested, counted by the reference's own traversal order
@@ -297,7 +297,7 @@ def matched_run(ctx, sids, stream, a, with_cpu, tune, sm_mhz):
     if not a.no_profile:
         # FP32 roofline of the plane scene: the reference tests all 18 planes
         # for every ray (camera, continuation and shadow rays); a profiled
-        # context times the two trace kernels over the same 64-image batch
+        # context times the whole-path kernel over the same 64-image batch
         pctx = capi.Context(device=ctx.device, profile=True, **tune)
         psid = pctx.load_scene_json(os.path.join(REPO, "tests", "golden", "scenes", "cornell.json"),
                                     os.path.join(REPO, "tests", "golden"))
@@ -308,15 +308,15 @@ def matched_run(ctx, sids, stream, a, with_cpu, tune, sm_mhz):
         ps = pctx.stats()
         pctx.close()
         rays = ps["rays"] + ps["shadow_rays"]
-        t = (ps["stage_ms"]["extend"] + ps["stage_ms"]["shadow"]) / 1e3
+        t = ps["stage_ms"]["other"] / 1e3   # k_paths: the whole of every path
         mhz = sm_mhz or 1965.0
         peak = 148 * 128 * 2 * mhz * 1e6 / 1e12
         ach = rays * 18 * PLANE_TEST_FLOPS / t / 1e12
-        fp32 = {"kernels": "k_extend + k_shadow", "rays": rays, "flops_per_ray": 18 * PLANE_TEST_FLOPS,
+        fp32 = {"kernels": "k_paths", "rays": rays, "flops_per_ray": 18 * PLANE_TEST_FLOPS,
                 "achieved": ach, "unit": "TFLOP/s", "peak": peak, "frac": ach / peak,
                 "peak_basis": f"148 SMs x 128 FP32 lanes x 2 (FMA) x {mhz:.0f} MHz (sampled SM clock)",
                 "flops": f"{PLANE_TEST_FLOPS} per plane test x 18 planes per ray, the reference's per-ray work",
-                "rays_per_s_in_trace_kernels": rays / t}
+                "rays_per_s_in_kernel": rays / t}
     out = {"config": "cornell.json 256x256, depth 4, S=4, hero-4 spectral, Reinhard", "fp32_roofline": fp32,
            "target_rmse": eps, "target": "reference CPU branched s=16 image vs 4096-path converged image",
            "spp_star": spp_star, "gpu_rmse_at_spp_star": err, "paths_per_image": paths,
@@ -632,60 +632,66 @@ def main():
     # ---- per-stage events (profiled pass) for the roofline
     roofline = None
     if not a.no_profile:
+        # Requests on scenes without a mesh run in k_paths, the others in the
+        # queue stages; each kind is profiled by itself.
         tune = {k: st[k] for k in ("queue_capacity", "block_size", "chunk_paths", "regen_every")}
-        pctx = capi.Context(device=local, profile=True, **tune)
-        psids = {v: pctx.load_scene_json(p, data) for v, p in files.items()}
-        ids = [pctx.submit(psids[r["variant"]], d) for r, d in zip(batch, descs)]
-        pctx.run_until_idle()
-        for i in ids:
-            pctx.fetch(i, want_hdr=False, want_rgb=False)
-        ps = pctx.stats()
-        pctx.close()
+        prof = {}
+        for kind, mesh in (("paths", False), ("queue", True)):
+            part = [(r, d) for r, d in zip(batch, descs) if (r["variant"] in MESH_VARIANTS) == mesh]
+            if not part:
+                continue
+            pctx = capi.Context(device=local, profile=True, **tune)
+            psids = {v: pctx.load_scene_json(files[v], data) for v in sorted({r["variant"] for r, _ in part})}
+            ids = [pctx.submit(psids[r["variant"]], d) for r, d in part]
+            pctx.run_until_idle()
+            for i in ids:
+                pctx.fetch(i, want_hdr=False, want_rgb=False)
+            prof[kind] = pctx.stats()
+            pctx.close()
         peak, kind = peaks()
+        mhz = clk.summary().get("sm_mhz") or 1965.0
+        sms = torch.cuda.get_device_properties(local).multi_processor_count
+        issue_peak = sms * 4 * mhz * 1e6
         # algorithmic bytes per unit (queue records, 16-byte words):
         #   extend: ray in (origin, dir, id: 48 B) + hit out (16 B)
         #   shadow: shadow record in (48 B)
         #   shade : spectral path in (o, d, tp, id, XYZ weights: 112 B) + hit in (16 B)
         #           + path out (112 B) + shadow out (48 B each)
-        bytes_stage = {"extend": 64.0 * ps["rays"], "shadow": 48.0 * ps["shadow_rays"],
-                       "shade": 240.0 * ps["rays"] + 48.0 * ps["shadow_rays"]}
-        dom = max(bytes_stage, key=lambda k: ps["stage_ms"][k])
-        t_ms = ps["stage_ms"][dom]
-        n_l = max(1, ps["stage_launches"][dom])
-        achieved = bytes_stage[dom] / (t_ms / 1e3) / 1e9
-        units = ps["shadow_rays"] if dom == "shadow" else ps["rays"]
-        traffic = NCU_DRAM_PER_UNIT[dom] * units / n_l if dom in NCU_DRAM_PER_UNIT else None
-        # every wavefront kernel against the same bound, for the full picture
+        #   paths : the FP64 accumulator read and written once per path (48 B)
         per_kernel = {}
-        for k in bytes_stage:
-            if ps["stage_ms"][k] <= 0:
+        for kind_, stage, name, unit_b in (("paths", "other", "k_paths", None), ("queue", "extend", "k_extend", 64.0),
+                                           ("queue", "shade", "k_shade", 240.0), ("queue", "shadow", "k_shadow", 48.0)):
+            ps = prof.get(kind_)
+            if not ps or ps["stage_ms"][stage] <= 0:
                 continue
-            nk = max(1, ps["stage_launches"][k])
-            gbs = bytes_stage[k] / (ps["stage_ms"][k] / 1e3) / 1e9
-            uk = ps["shadow_rays"] if k == "shadow" else ps["rays"]
-            per_kernel[f"k_{k}"] = {"ms": ps["stage_ms"][k], "achieved_gbs": gbs, "frac_hbm": gbs / peak,
-                                    "ncu_traffic_per_launch": NCU_DRAM_PER_UNIT[k] * uk / nk,
-                                    "algorithmic_bytes_per_launch": bytes_stage[k] / nk}
-        roofline = {"bound": "hbm", "kernel": f"k_{dom}", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                    "frac": achieved / peak, "peak_kind": kind, "traffic": traffic,
+            t, n_l = ps["stage_ms"][stage] / 1e3, max(1, ps["stage_launches"][stage])
+            units = ps["shadow_rays"] if stage == "shadow" else ps["rays"]
+            nbytes = (48.0 * ps["paths"] if name == "k_paths" else unit_b * units +
+                      (48.0 * ps["shadow_rays"] if stage == "shade" else 0.0))
+            inst = NCU_INST_PER_UNIT[name] * units
+            per_kernel[name] = {"ms": t * 1e3, "rays": ps["rays"], "shadow_rays": ps["shadow_rays"],
+                                "achieved_gbs": nbytes / t / 1e9, "frac_hbm": nbytes / t / 1e9 / peak,
+                                "algorithmic_bytes_per_launch": nbytes / n_l,
+                                "ncu_traffic_per_launch": NCU_DRAM_PER_UNIT[name] * units / n_l,
+                                "issue_roofline": {"achieved": inst / t, "peak": issue_peak, "unit": "warp instructions/s",
+                                                   "frac": inst / t / issue_peak,
+                                                   "warp_inst_per_unit": NCU_INST_PER_UNIT[name], "sm_mhz": mhz,
+                                                   "sms": sms}}
+        dom = max(per_kernel, key=lambda k: per_kernel[k]["ms"])
+        dk = per_kernel[dom]
+        dps = prof["paths" if dom == "k_paths" else "queue"]
+        n_l = max(1, dps["stage_launches"]["other" if dom == "k_paths" else dom[2:]])
+        # HBM as the base bound of every kernel; the bound that applies is
+        # instruction issue (issue_roofline: ncu warp instructions per unit x
+        # units over the CUDA-event time, against one warp instruction per
+        # cycle per scheduler at the SM clock sampled during the timed region)
+        roofline = {"bound": "hbm", "kernel": dom, "achieved": dk["achieved_gbs"], "peak": peak, "unit": "GB/s",
+                    "frac": dk["frac_hbm"], "peak_kind": kind, "traffic": dk["ncu_traffic_per_launch"],
                     "traffic_note": "ncu DRAM bytes per unit (8-render capture) x units per launch",
-                    "bytes_per_launch": bytes_stage[dom] / n_l, "ms_per_launch": t_ms / n_l,
-                    "issue": dict(NCU_ISSUE.get(dom, {}), note="ncu, one launch per kernel of an 8-render batch"),
-                    "stage_ms": ps["stage_ms"], "stage_share": {k: v / max(1e-9, sum(ps["stage_ms"].values()))
-                                                                for k, v in ps["stage_ms"].items()},
-                    "per_kernel": per_kernel}
-        # The bound that applies: instruction issue.  The same kernel's warp
-        # instructions (ncu per unit x units) over its CUDA-event time,
-        # against one warp instruction per cycle per scheduler (4 per SM) at
-        # the SM clock sampled during the timed region.
-        if dom in NCU_INST_PER_UNIT:
-            mhz = clk.summary().get("sm_mhz") or 1965.0
-            sms = torch.cuda.get_device_properties(local).multi_processor_count
-            ach = NCU_INST_PER_UNIT[dom] * units / (t_ms / 1e3)
-            pk = sms * 4 * mhz * 1e6
-            roofline["issue_roofline"] = {"achieved": ach, "peak": pk, "unit": "warp instructions/s",
-                                          "frac": ach / pk, "warp_inst_per_unit": NCU_INST_PER_UNIT[dom],
-                                          "sm_mhz": mhz, "sms": sms}
+                    "bytes_per_launch": dk["algorithmic_bytes_per_launch"], "ms_per_launch": dk["ms"] / n_l,
+                    "issue": dict(NCU_ISSUE.get(dom, {}), note="ncu, one launch per kernel"),
+                    "stage_ms": {k: v["stage_ms"] for k, v in prof.items()}, "per_kernel": per_kernel,
+                    "issue_roofline": dk["issue_roofline"]}
 
     # ---- served stream: Poisson arrivals, continuous batching, p50/p99
     serve = None

@@ -95,9 +95,11 @@ typedef struct {
     uint64_t seed;           /* 0 -> 1 */
     int32_t priority;        /* batched / served: pending requests are admitted lowest value
                               * first, in submit order among equals (0 default) */
-    /* plain method only: 0 = one sample per pixel per pass, the reference
-     * wavefront's default (code/Includes/GpuDefaults.h:44-50); 1 = passes
-     * as large as the queue (wavefrontMultiSample) */
+    /* plain method on scenes with a triangle mesh: 0 = one sample per pixel per
+     * pass, the reference wavefront's default
+     * (code/Includes/GpuDefaults.h:44-50); 1 = passes as large as the queue
+     * (wavefrontMultiSample).  Other scenes are traced path by path, without
+     * passes.  The image is the same either way. */
     int32_t multi_sample;
     /* Sample range [sample_begin, sample_end) of `samples` (0, 0 = all).  A
      * render split across GPUs gives each one a range; the HDR images are

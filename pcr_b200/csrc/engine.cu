@@ -9,7 +9,7 @@
 #include <tuple>
 
 #include "bvh_build.h"
-#include "kernels.cuh"
+#include "paths.cuh"
 #include "scene.h"
 
 namespace pcr {
@@ -172,7 +172,7 @@ Engine::~Engine()
     free_buffers();
     for (auto& e : prof_ev_) cudaEventDestroy(e);
     for (auto& e : ev_snaps_) cudaEventDestroy(e);
-    if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
+    drop_graphs();
     if (pool_) cudaMemPoolDestroy(pool_);
     cudaStreamDestroy(stream_);
 }
@@ -192,6 +192,7 @@ void Engine::alloc_buffers()
     d_give_start_ = dalloc<long long>(kMaxActive, T);
     d_give_ = dalloc<int>(kMaxActive, T);
     d_give_base_ = dalloc<int>(kMaxActive, T);
+    d_path_base_ = dalloc<int>(kMaxActive, T);
     d_active_ = dalloc<int>(kMaxActive, T);
     d_nactive_ = dalloc<int>(1, T);
     d_done_ = dalloc<int>(kMaxActive, T);
@@ -219,6 +220,7 @@ void Engine::alloc_buffers()
     snap_next_ = 0;
     snap_inflight_ = 0;
     CK(cudaMallocHost(&h_params_, sizeof(EngineParams)));
+    CK(cudaMallocHost(&h_cnt_, sizeof(Counters)));
 
     const int fill = tune_.queue_capacity;
     queue_cap_ = fill * 4;   // a dispersive-glass fork turns one path into up to four
@@ -248,6 +250,8 @@ void Engine::free_buffers()
         h = nullptr;
     }
     if (h_params_) cudaFreeHost(h_params_);
+    if (h_cnt_) cudaFreeHost(h_cnt_);
+    h_cnt_ = nullptr;
     h_snap_ = nullptr;
     h_params_ = nullptr;
 }
@@ -280,8 +284,6 @@ void Engine::set_tuning(const EngineTuning& t)
         }
         CK(cudaMemcpy(d_mats_, mats.data(), sizeof(DMaterial) * mat_count_, cudaMemcpyHostToDevice));
     }
-    if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
-    graph_exec_ = nullptr;
     graph_dirty_ = true;
 }
 
@@ -295,6 +297,7 @@ EngineView Engine::view() const
     E.outstanding = d_outstanding_;
     E.give = d_give_;
     E.give_base = d_give_base_;
+    E.path_base = d_path_base_;
     E.active = d_active_;
     E.n_active = d_nactive_;
     E.done_flag = d_done_;
@@ -873,7 +876,7 @@ void Engine::ensure_shadow_capacity(int shadow_samples)
 int64_t Engine::submit(int scene, const pcr_render_desc& desc)
 {
     validate(scene, desc);
-    if ((int64_t)queue_cap_ * desc.shadow_samples > shadow_cap_) {
+    if (!traced_whole(scene) && (int64_t)queue_cap_ * desc.shadow_samples > shadow_cap_) {
         std::lock_guard<std::mutex> g(run_mu_);
         ensure_shadow_capacity(desc.shadow_samples);
     }
@@ -903,41 +906,22 @@ int64_t Engine::submit(int scene, const pcr_render_desc& desc)
     return id;
 }
 
-void Engine::activate(Request& r, int slot)
+// A request's accumulator (cleared) and images, on the engine's stream.
+void Engine::alloc_request(Request& r)
 {
-    const pcr_render_desc& d = r.desc;
-    const int64_t px = (int64_t)d.width * d.height;
+    const int64_t px = (int64_t)r.desc.width * r.desc.height;
     CK(cudaMallocFromPoolAsync(&r.accum, px * 3 * sizeof(double), pool_, stream_));
     CK(cudaMemsetAsync(r.accum, 0, px * 3 * sizeof(double), stream_));
     CK(cudaMallocFromPoolAsync(&r.d_hdr, px * 3 * sizeof(float), pool_, stream_));
     CK(cudaMallocFromPoolAsync(&r.d_rgb, px * 3, pool_, stream_));
-    const SceneEntry& S = scenes_[r.scene];
-    DRequest R{};
-    R.scene = r.scene;
-    R.width = d.width;
-    R.height = d.height;
-    R.depth = d.depth;
-    R.aa = std::max(1, d.aa_samples);
-    R.spp = d.samples;
-    R.sample0 = d.sample_end > 0 ? d.sample_begin : 0;
-    R.local_spp = local_spp(d);
-    R.paths_per_pixel = R.aa * R.local_spp;
-    R.shadow = d.shadow_samples;
-    R.flags = (d.spectral ? kReqSpectral : 0) | (d.mis ? kReqMIS : 0) | (d.russian ? kReqRussian : 0) |
-              (d.stratified ? kReqStratified : 0) | (d.spectral_terminate ? kReqTerminate : 0);
-    R.hero = std::min(4, std::max(1, d.hero_samples <= 0 ? 4 : d.hero_samples));
-    R.strata = d.stratified ? std::max(1, (int)std::lround(std::sqrt((float)d.samples))) : 0;
-    R.cam_x = S.cam[0];
-    R.cam_y = S.cam[1];
-    R.cam_z = S.cam[2];
-    // code/Renderer.cpp:149-150
-    R.aspect = d.width / (float)d.height;
-    R.scale = std::tan((float)3.14159265358979323846 / 180.f * 0.5f * S.fov);
-    const uint64_t seed = d.seed ? d.seed : 1ull;
-    R.seed_lo = (uint32_t)(seed & 0xffffffffu) * 0x9E3779B1u + 0x7F4A7C15u;
-    R.seed_hi = (uint32_t)(seed >> 32) ^ (uint32_t)(seed * 0xD1B54A32D192ED03ull >> 17);
-    R.total = px * R.paths_per_pixel;
-    R.accum = r.accum;
+}
+
+void Engine::activate(Request& r, int slot)
+{
+    const pcr_render_desc& d = r.desc;
+    const int64_t px = (int64_t)d.width * d.height;
+    alloc_request(r);
+    DRequest R = make_request(d, r.scene, r.accum);
     if (adaptive_rounds(d)) {
         R.flags |= kReqAdaptive;
         CK(cudaMallocFromPoolAsync(&r.act[0], px * sizeof(int), pool_, stream_));
@@ -1000,39 +984,59 @@ void Engine::grid_for(const void* kernel, int block, size_t smem, int* grid)
     *grid = std::max(1, per_sm) * sms_;
 }
 
-void Engine::launch_iteration(int cur, bool prof)
+int Engine::active_stages() const
+{
+    int m = 0;
+    for (int slot : active_slots_) {
+        auto it = reqs_.find(slot_owner_[slot]);
+        if (it != reqs_.end()) m |= traced_whole(it->second->scene) ? kStagesPaths : kStagesQueue;
+    }
+    return m ? m : kStagesQueue;
+}
+
+void Engine::launch_iteration(int cur, int stages, bool prof)
 {
     const EngineView E = view();
     const int B = tune_.block_size;
+    // stage index: 0 regen 1 extend 2 shade 3 shadow 4 resolve 5 schedule 6 status (and k_round) 7 other (k_paths)
+    int done = 0;
+    int stage_of[8];
+    auto mark = [&](int stage) {  // the stage just launched ends here
+        stage_launches_[stage]++;
+        if (!prof) return;
+        stage_of[done++] = stage;
+        CK(cudaEventRecord(prof_ev_[done], stream_));
+    };
     if (prof) CK(cudaEventRecord(prof_ev_[0], stream_));
     k_schedule<<<1, kSchedThreads, 0, stream_>>>(E, (const EngineParams*)d_params_, cur);
-    if (prof) CK(cudaEventRecord(prof_ev_[1], stream_));
-    k_regen<<<grid_regen_, B, 0, stream_>>>(E, cur, xyz_scale_);
-    if (prof) CK(cudaEventRecord(prof_ev_[2], stream_));
-    k_extend<<<grid_extend_, B, 0, stream_>>>(E, cur);
-    if (prof) CK(cudaEventRecord(prof_ev_[3], stream_));
-    k_shade<<<grid_shade_, kShadeBlock, shade_smem_, stream_>>>(E, cur, smem_mats_);
-    if (prof) CK(cudaEventRecord(prof_ev_[4], stream_));
-    k_shadow<<<grid_shadow_, B, 0, stream_>>>(E);
-    if (prof) CK(cudaEventRecord(prof_ev_[5], stream_));
+    mark(5);
+    if (stages & kStagesQueue) {
+        k_regen<<<grid_regen_, B, 0, stream_>>>(E, cur, xyz_scale_);
+        mark(0);
+        k_extend<<<grid_extend_, B, 0, stream_>>>(E, cur);
+        mark(1);
+        k_shade<<<grid_shade_, kShadeBlock, shade_smem_, stream_>>>(E, cur, smem_mats_);
+        mark(2);
+        k_shadow<<<grid_shadow_, B, 0, stream_>>>(E);
+        mark(3);
+    }
+    if (stages & kStagesPaths) {
+        k_paths<<<grid_paths_, kPathBlock, kPathSmem, stream_>>>(E, xyz_scale_);
+        mark(7);
+    }
     k_status<<<1, 1024, 0, stream_>>>(E, cur ^ 1);
     k_round<<<grid_round_, 256, 0, stream_>>>(E);
-    if (prof) CK(cudaEventRecord(prof_ev_[6], stream_));
+    mark(6);
+    stage_launches_[6]++;
     CK(cudaGetLastError());
     if (prof) {
-        CK(cudaEventSynchronize(prof_ev_[6]));
-        // stage index: 0 regen 1 extend 2 shade 3 shadow 4 resolve 5 schedule 6 status
-        const int map[6] = {5, 0, 1, 2, 3, 6};
-        for (int k = 0; k < 6; k++) {
+        CK(cudaEventSynchronize(prof_ev_[done]));
+        for (int k = 0; k < done; k++) {
             float ms = 0.f;
             CK(cudaEventElapsedTime(&ms, prof_ev_[k], prof_ev_[k + 1]));
-            stage_ms_[map[k]] += ms;
-            stage_launches_[map[k]]++;
+            stage_ms_[stage_of[k]] += ms;
         }
-    } else {
-        for (int k : {0, 1, 2, 3, 5, 6}) stage_launches_[k]++;
     }
-    stage_launches_[7]++;  // k_round (timed with k_status)
     iterations_++;
 }
 
@@ -1050,7 +1054,7 @@ static void raise_shade_smem(size_t bytes)
         CK(cudaFuncSetAttribute((const void*)k_shade, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
-void Engine::build_graph()
+void Engine::launch_shapes()
 {
     const int B = tune_.block_size;
     // materials staged in shared memory when they fit
@@ -1062,34 +1066,49 @@ void Engine::build_graph()
     grid_for((const void*)k_extend, B, 0, &grid_extend_);
     grid_for((const void*)k_shade, kShadeBlock, shade_smem_, &grid_shade_);
     grid_for((const void*)k_shadow, B, 0, &grid_shadow_);
+    grid_for((const void*)k_paths, kPathBlock, kPathSmem, &grid_paths_);
     grid_round_ = sms_ * 2;  // a round's per-pixel step is light; an idle launch reads one word
-    if (graph_exec_) {
-        cudaGraphExecDestroy(graph_exec_);
-        graph_exec_ = nullptr;
-    }
-    if (use_graph_) {
-        cudaGraph_t g;
-        CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-        for (int it = 0; it < tune_.iters_per_launch; it++) launch_iteration(it & 1, false);
-        CK(cudaStreamEndCapture(stream_, &g));
-        CK(cudaGraphInstantiate(&graph_exec_, g, 0));
-        CK(cudaGraphDestroy(g));
-        // capture counted launches that did not run
-        for (int k : {0, 1, 2, 3, 5, 6, 7}) stage_launches_[k] -= tune_.iters_per_launch;
-        iterations_ -= tune_.iters_per_launch;
-    }
+    drop_graphs();
     graph_dirty_ = false;
 }
 
-void Engine::launch_block()
+void Engine::drop_graphs()
 {
-    if (graph_dirty_) build_graph();
-    if (use_graph_ && !profile_) {
-        CK(cudaGraphLaunch(graph_exec_, stream_));
-        for (int k : {0, 1, 2, 3, 5, 6, 7}) stage_launches_[k] += tune_.iters_per_launch;
+    for (cudaGraphExec_t& g : graphs_)
+        if (g) {
+            cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
+}
+
+void Engine::launch_block(int stages)
+{
+    if (graph_dirty_) launch_shapes();
+    const int64_t iterations = iterations_;
+    int64_t launches[8];
+    std::copy(stage_launches_, stage_launches_ + 8, launches);
+    const bool graph = use_graph_ && !profile_;
+    if (graph && !graphs_[stages]) {
+        cudaGraph_t g;
+        CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+        for (int it = 0; it < tune_.iters_per_launch; it++) launch_iteration(it & 1, stages, false);
+        CK(cudaStreamEndCapture(stream_, &g));
+        CK(cudaGraphInstantiate(&graphs_[stages], g, 0));
+        CK(cudaGraphDestroy(g));
+        // capture counted launches that did not run
+        std::copy(launches, launches + 8, stage_launches_);
+        iterations_ = iterations;
+    }
+    if (graph) {
+        CK(cudaGraphLaunch(graphs_[stages], stream_));
+        stage_launches_[5] += tune_.iters_per_launch;
+        stage_launches_[6] += 2 * tune_.iters_per_launch;
+        if (stages & kStagesQueue)
+            for (int k : {0, 1, 2, 3}) stage_launches_[k] += tune_.iters_per_launch;
+        if (stages & kStagesPaths) stage_launches_[7] += tune_.iters_per_launch;
         iterations_ += tune_.iters_per_launch;
     } else {
-        for (int it = 0; it < tune_.iters_per_launch; it++) launch_iteration(it & 1, profile_);
+        for (int it = 0; it < tune_.iters_per_launch; it++) launch_iteration(it & 1, stages, profile_);
     }
 }
 
@@ -1100,21 +1119,14 @@ void Engine::check_status()
                                                   std::to_string(h_snap_->cnt.status) + ")");
 }
 
-void Engine::finish_request(Request& r, bool after_engine_stream)
+// Resolves a request whose accumulator is final in the order of stream rs.
+void Engine::finish_request(Request& r, cudaStream_t rs)
 {
     const pcr_render_desc& d = r.desc;
     const int64_t px = (int64_t)d.width * d.height;
     // adaptive requests hold each pixel's final mean already
     const double inv = adaptive_rounds(d) ? 1.0 : 1.0 / ((double)d.samples * std::max(1, d.aa_samples));
     int grid = std::min<int64_t>((px + 255) / 256, (int64_t)sms_ * 8);
-    cudaStream_t rs = resolve_stream_;
-    if (after_engine_stream) {
-        // the plain method hands over with work it queued since its last
-        // synchronisation: the resolve follows all of it
-        if (!r.ev_ready) CK(cudaEventCreateWithFlags(&r.ev_ready, cudaEventDisableTiming));
-        CK(cudaEventRecord(r.ev_ready, stream_));
-        CK(cudaStreamWaitEvent(rs, r.ev_ready, 0));
-    }
     k_resolve<<<std::max(1, grid), 256, 0, rs>>>(r.accum, (int)px, inv, d.spectral ? 1 : 0, d.aces ? 1 : 0, r.d_hdr,
                                                  r.d_rgb);
     CK(cudaGetLastError());
@@ -1225,7 +1237,7 @@ void Engine::harvest(bool)
             r.device_ms = (td > tf && tf) ? (double)(td - tf) * 1e-6 : 0.0;
             r.paths = h_snap_->issued[s];  // adaptive requests trace fewer than W*H*spp*aa
             if (r.cancel_running) release_cancelled(r);
-            else finish_request(r);
+            else finish_request(r, resolve_stream_);
             slot_owner_[s] = -1;
             bytes_in_use_ -= r.bytes;
             active_dirty_ = true;
@@ -1256,10 +1268,12 @@ void Engine::harvest(bool)
 bool Engine::engine_step()
 {
     CK(cudaSetDevice(device_));
+    int stages;
     {
         std::lock_guard<std::mutex> g(mu_);
         admit_locked();
         upload_active();
+        stages = active_stages();
         for (int s : active_slots_) {
             Request& r = *reqs_[slot_owner_[s]];
             if (r.cancel_running && !r.cancel_sent) {
@@ -1286,7 +1300,7 @@ bool Engine::engine_step()
             return !pending_.empty();
         }
     }
-    launch_block();
+    launch_block(stages);
     blocks_launched_++;
     const int b = snap_next_;
     snap_block_[b] = blocks_launched_;
@@ -1505,6 +1519,46 @@ double Engine::progress(int64_t id)
 }
 
 // ---------------------------------------------------------------- plain method
+// Traces every path of R, the only request of E, with k_paths: launches of
+// at most kPathsPerLaunch paths, so that other work of the device gets its
+// turn within about a tenth of a second.
+constexpr int64_t kPathsPerLaunch = 1 << 26;
+void Engine::trace_whole(const EngineView& E, const DRequest& R, int grid)
+{
+    for (int64_t at = 0; at < R.total; at += kPathsPerLaunch) {
+        const int n = (int)std::min<int64_t>(kPathsPerLaunch, R.total - at);
+        k_one_request<<<1, 1, 0, stream_>>>(E, R, at, n);
+        if (profile_) CK(cudaEventRecord(prof_ev_[0], stream_));
+        k_paths<<<std::min(grid, (n + kPathBlock - 1) / kPathBlock), kPathBlock, kPathSmem, stream_>>>(E, xyz_scale_);
+        CK(cudaGetLastError());
+        if (profile_) record_other(prof_ev_[0], prof_ev_[1]);
+        else stage_launches_[7]++;
+        iterations_++;
+    }
+}
+
+// Plain render of a scene without a mesh: one k_paths launch, resolve, copy.
+void Engine::render_whole(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats* st)
+{
+    alloc_request(r);
+    const DRequest R = make_request(r.desc, r.scene, r.accum);
+    trace_whole(view(), R, grid_paths_);
+    active_dirty_ = true;  // the active list holds slot 0
+    CK(cudaMemcpyAsync(h_cnt_, d_cnt_, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
+    finish_request(r, stream_);
+    copy_out(r, hdr, rgb);  // waits for the resolve, and so for the counters
+    cudaEventDestroy(r.ev_ready);
+    const Counters& c = *h_cnt_;
+    if (c.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "device reported queue overflow");
+    if (st) {
+        st->device_ms = c.path_end > c.path_begin ? (double)(c.path_end - c.path_begin) * 1e-6 : 0.0;
+        st->queue_ms = 0;
+        st->paths = (uint64_t)R.total;
+        st->rays = 0;
+        st->shadow_rays = 0;
+    }
+}
+
 void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, uint8_t* rgb, pcr_render_stats* st)
 {
     if (adaptive_rounds(desc)) {
@@ -1524,7 +1578,6 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     CK(cudaSetDevice(device_));
     validate(scene, desc);
     if (!active_slots_.empty() || serving_) throw PcrError(PCR_ERR_INVALID, "plain render while batched work is active");
-    ensure_shadow_capacity(desc.shadow_samples);
     auto t0 = std::chrono::steady_clock::now();
     Request r;
     r.id = -1;
@@ -1532,7 +1585,14 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     r.desc = desc;
     r.bytes = request_bytes(desc);
     if (r.bytes > budget_) throw PcrError(PCR_ERR_NO_MEMORY, "request larger than the device memory budget");
-    if (graph_dirty_) build_graph();
+    if (graph_dirty_) launch_shapes();
+    if (traced_whole(scene)) {
+        render_whole(r, hdr, rgb, st);
+        if (st) st->latency_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+        return;
+    }
+    ensure_shadow_capacity(desc.shadow_samples);
+    if (graph_dirty_) launch_shapes();
     // a pass holds one sample per pixel (W*H paths) unless multi_sample asks
     // for passes as large as the queue; no refill until a pass has drained
     const int64_t px = (int64_t)desc.width * desc.height;
@@ -1546,7 +1606,7 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     const int64_t passes = (total + pass - 1) / pass;
     int cur = 0;
     for (int64_t it = 0; it < passes * (int64_t)desc.depth; it++) {
-        launch_iteration(cur, profile_);
+        launch_iteration(cur, kStagesQueue, profile_);
         cur ^= 1;
     }
     int extra = 0;
@@ -1559,18 +1619,18 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
         if (c.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "device reported queue overflow");
         if (done) break;
         if (++extra > 4 * desc.depth + 8) throw PcrError(PCR_ERR_TIMEOUT, "plain render did not finish");
-        launch_iteration(cur, profile_);
+        launch_iteration(cur, kStagesQueue, profile_);
         cur ^= 1;
     }
     // a plain render always ends on queue parity 0 for the next user
     if (cur != 0) {
-        launch_iteration(cur, false);
+        launch_iteration(cur, kStagesQueue, false);
         cur ^= 1;
     }
     unsigned long long tf = 0, td = 0;
     CK(cudaMemcpy(&tf, d_tfirst_, 8, cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(&td, d_tdone_, 8, cudaMemcpyDeviceToHost));
-    finish_request(r, true);
+    finish_request(r, stream_);
     active_slots_.clear();
     active_dirty_ = true;
     bytes_in_use_ -= r.bytes;
@@ -1637,7 +1697,7 @@ static void* noalloc_scratch(int device)
     return g_noalloc_ptr[device];
 }
 
-// The request entry of a render (same fields Engine::activate writes).
+// The request entry of a render (Engine::activate adds the adaptive fields).
 DRequest Engine::make_request(const pcr_render_desc& d, int scene, double* accum) const
 {
     const SceneEntry& S = scenes_[scene];
@@ -1653,12 +1713,14 @@ DRequest Engine::make_request(const pcr_render_desc& d, int scene, double* accum
     R.paths_per_pixel = R.aa * R.local_spp;
     R.shadow = d.shadow_samples;
     R.flags = (d.spectral ? kReqSpectral : 0) | (d.mis ? kReqMIS : 0) | (d.russian ? kReqRussian : 0) |
-              (d.stratified ? kReqStratified : 0) | (d.spectral_terminate ? kReqTerminate : 0);
+              (d.stratified ? kReqStratified : 0) | (d.spectral_terminate ? kReqTerminate : 0) |
+              (traced_whole(scene) ? kReqWhole : 0);
     R.hero = std::min(4, std::max(1, d.hero_samples <= 0 ? 4 : d.hero_samples));
     R.strata = d.stratified ? std::max(1, (int)std::lround(std::sqrt((float)d.samples))) : 0;
     R.cam_x = S.cam[0];
     R.cam_y = S.cam[1];
     R.cam_z = S.cam[2];
+    // code/Renderer.cpp:149-150
     R.aspect = d.width / (float)d.height;
     R.scale = std::tan((float)3.14159265358979323846 / 180.f * 0.5f * S.fov);
     const uint64_t seed = d.seed ? d.seed : 1ull;
@@ -1706,6 +1768,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     long long* give_start = reinterpret_cast<long long*>(take(8));
     int* give = reinterpret_cast<int*>(take(4));
     int* give_base = reinterpret_cast<int*>(take(4));
+    int* path_base = reinterpret_cast<int*>(take(4));
     int* active = reinterpret_cast<int*>(take(4));
     int* n_active = reinterpret_cast<int*>(take(4));
     int* done = reinterpret_cast<int*>(take(4));
@@ -1746,6 +1809,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     E.outstanding = outstanding;
     E.give = give;
     E.give_base = give_base;
+    E.path_base = path_base;
     E.active = active;
     E.n_active = n_active;
     E.done_flag = done;
@@ -1765,51 +1829,57 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     E.queue_cap = kNoAllocQueue;
     E.n_mats = mat_count_;
 
-    DRequest R = make_request(desc, scene, accum);
-    k_admit<<<1, 1, 0, stream_>>>(E, R, 0);
-    ActiveList L;
-    L.n = 1;
-    L.slots[0] = 0;
-    k_set_active<<<1, 32, 0, stream_>>>(E, L);
-    const int pass = (int)std::min<int64_t>(px, kNoAllocFill);
-    k_set_params<<<1, 1, 0, stream_>>>(params, EngineParams{pass, pass, 1, 1});
-    CK(cudaGetLastError());
-
-    // launch shapes from the occupancy calculator (no allocation involved)
-    const int B = tune_.block_size;
-    const size_t mat_bytes = sizeof(DMaterial) * (size_t)std::max(1, mat_count_);
-    const int smem_mats = mat_bytes <= 96 * 1024 ? 1 : 0;
-    const size_t smem = smem_mats ? mat_bytes : 0;
-    raise_shade_smem(smem);
-    int g_regen, g_extend, g_shade, g_shadow;
-    grid_for((const void*)k_regen, B, 0, &g_regen);
-    grid_for((const void*)k_extend, B, 0, &g_extend);
-    grid_for((const void*)k_shade, kShadeBlock, smem, &g_shade);
-    grid_for((const void*)k_shadow, B, 0, &g_shadow);
-    int cur = 0;
-    auto iteration = [&]() {
-        k_schedule<<<1, kSchedThreads, 0, stream_>>>(E, params, cur);
-        k_regen<<<g_regen, B, 0, stream_>>>(E, cur, xyz_scale_);
-        k_extend<<<g_extend, B, 0, stream_>>>(E, cur);
-        k_shade<<<g_shade, kShadeBlock, smem, stream_>>>(E, cur, smem_mats);
-        k_shadow<<<g_shadow, B, 0, stream_>>>(E);
-        k_status<<<1, 1024, 0, stream_>>>(E, cur ^ 1);
+    const DRequest R = make_request(desc, scene, accum);
+    if (traced_whole(scene)) {
+        int g_paths;
+        grid_for((const void*)k_paths, kPathBlock, kPathSmem, &g_paths);
+        trace_whole(E, R, g_paths);
+    } else {
+        k_admit<<<1, 1, 0, stream_>>>(E, R, 0);
+        ActiveList L;
+        L.n = 1;
+        L.slots[0] = 0;
+        k_set_active<<<1, 32, 0, stream_>>>(E, L);
+        const int pass = (int)std::min<int64_t>(px, kNoAllocFill);
+        k_set_params<<<1, 1, 0, stream_>>>(params, EngineParams{pass, pass, 1, 1});
         CK(cudaGetLastError());
-        cur ^= 1;
-    };
-    const int64_t total = px * local_spp(desc) * std::max(1, desc.aa_samples);
-    const int64_t passes = (total + pass - 1) / pass;
-    for (int64_t it = 0; it < passes * (int64_t)desc.depth; it++) iteration();
-    for (int extra = 0;; extra++) {
-        int flag = 0;
-        Counters c;
-        CK(cudaMemcpyAsync(&flag, done, sizeof(int), cudaMemcpyDeviceToHost, stream_));
-        CK(cudaMemcpyAsync(&c, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
-        CK(cudaStreamSynchronize(stream_));
-        if (c.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "pcr_render_noalloc: device reported queue overflow");
-        if (flag) break;
-        if (extra > 4 * desc.depth + 8) throw PcrError(PCR_ERR_TIMEOUT, "pcr_render_noalloc did not finish");
-        iteration();
+
+        // launch shapes from the occupancy calculator (no allocation involved)
+        const int B = tune_.block_size;
+        const size_t mat_bytes = sizeof(DMaterial) * (size_t)std::max(1, mat_count_);
+        const int smem_mats = mat_bytes <= 96 * 1024 ? 1 : 0;
+        const size_t smem = smem_mats ? mat_bytes : 0;
+        raise_shade_smem(smem);
+        int g_regen, g_extend, g_shade, g_shadow;
+        grid_for((const void*)k_regen, B, 0, &g_regen);
+        grid_for((const void*)k_extend, B, 0, &g_extend);
+        grid_for((const void*)k_shade, kShadeBlock, smem, &g_shade);
+        grid_for((const void*)k_shadow, B, 0, &g_shadow);
+        int cur = 0;
+        auto iteration = [&]() {
+            k_schedule<<<1, kSchedThreads, 0, stream_>>>(E, params, cur);
+            k_regen<<<g_regen, B, 0, stream_>>>(E, cur, xyz_scale_);
+            k_extend<<<g_extend, B, 0, stream_>>>(E, cur);
+            k_shade<<<g_shade, kShadeBlock, smem, stream_>>>(E, cur, smem_mats);
+            k_shadow<<<g_shadow, B, 0, stream_>>>(E);
+            k_status<<<1, 1024, 0, stream_>>>(E, cur ^ 1);
+            CK(cudaGetLastError());
+            cur ^= 1;
+        };
+        const int64_t total = px * local_spp(desc) * std::max(1, desc.aa_samples);
+        const int64_t passes = (total + pass - 1) / pass;
+        for (int64_t it = 0; it < passes * (int64_t)desc.depth; it++) iteration();
+        for (int extra = 0;; extra++) {
+            int flag = 0;
+            Counters c;
+            CK(cudaMemcpyAsync(&flag, done, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+            CK(cudaMemcpyAsync(&c, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
+            CK(cudaStreamSynchronize(stream_));
+            if (c.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "pcr_render_noalloc: device reported queue overflow");
+            if (flag) break;
+            if (extra > 4 * desc.depth + 8) throw PcrError(PCR_ERR_TIMEOUT, "pcr_render_noalloc did not finish");
+            iteration();
+        }
     }
     const double inv = 1.0 / ((double)desc.samples * std::max(1, desc.aa_samples));
     const int grid = (int)std::min<int64_t>((px + 255) / 256, (int64_t)sms_ * 8);

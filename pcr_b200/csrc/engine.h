@@ -114,16 +114,25 @@ private:
     void validate(int scene, const pcr_render_desc& d) const;
     int64_t request_bytes(const pcr_render_desc& d) const;
     void admit_locked();
+    void alloc_request(Request& r);
     void activate(Request& r, int slot);
     void upload_active();
-    void launch_iteration(int cur, bool profile);
-    void launch_block();
-    void build_graph();
+    // Which stages an iteration runs: the queue stages for requests on mesh
+    // scenes, k_paths for the others (bits of the active requests).
+    static constexpr int kStagesQueue = 1, kStagesPaths = 2;
+    int active_stages() const;
+    void launch_iteration(int cur, int stages, bool profile);
+    void launch_block(int stages);
+    void launch_shapes();
+    void drop_graphs();
+    void trace_whole(const EngineView& E, const DRequest& R, int grid);
+    void render_whole(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats* st);
     void harvest(bool final_sync);
-    void finish_request(Request& r, bool after_engine_stream = false);
+    void finish_request(Request& r, cudaStream_t rs);
     void release_cancelled(Request& r);
     void copy_out(Request& r, float* hdr, uint8_t* rgb);
     DRequest make_request(const pcr_render_desc& d, int scene, double* accum) const;
+    bool traced_whole(int scene) const { return scenes_[scene].dev.n_nodes == 0; }
     void check_status();
     bool engine_step();
     void serve_loop();
@@ -167,7 +176,7 @@ private:
     unsigned long long *d_issued_ = nullptr, *d_tfirst_ = nullptr, *d_tdone_ = nullptr;
     long long* d_outstanding_ = nullptr;
     long long* d_give_start_ = nullptr;
-    int *d_give_ = nullptr, *d_give_base_ = nullptr, *d_active_ = nullptr, *d_nactive_ = nullptr, *d_done_ = nullptr;
+    int *d_give_ = nullptr, *d_give_base_ = nullptr, *d_path_base_ = nullptr, *d_active_ = nullptr, *d_nactive_ = nullptr, *d_done_ = nullptr;
     int *d_round_state_ = nullptr, *d_round_cnt_ = nullptr, *d_round_list_ = nullptr;
     float4* d_cmf_ = nullptr;  // colour-matching table for raygen
     int* h_active_ = nullptr;     // pinned: [0] = n, then slots
@@ -184,6 +193,7 @@ private:
     // while the host harvests or is briefly descheduled.
     static constexpr int kSnapRing = 4;
     cudaMemPool_t pool_ = nullptr;
+    Counters* h_cnt_ = nullptr;   // pinned: a plain render's counters
     HostSnap* h_snaps_[kSnapRing] = {};
     cudaEvent_t ev_snaps_[kSnapRing] = {};
     HostSnap* h_snap_ = nullptr;  // the snapshot harvest reads (one of h_snaps_)
@@ -203,9 +213,9 @@ private:
     std::vector<void*> qallocs_;
 
     // graph
-    cudaGraphExec_t graph_exec_ = nullptr;
+    cudaGraphExec_t graphs_[4] = {};   // by stages, captured when first launched
     bool graph_dirty_ = true;
-    int grid_regen_ = 0, grid_extend_ = 0, grid_shade_ = 0, grid_shadow_ = 0, grid_round_ = 0;
+    int grid_regen_ = 0, grid_extend_ = 0, grid_shade_ = 0, grid_shadow_ = 0, grid_round_ = 0, grid_paths_ = 0;
     size_t shade_smem_ = 0;
     int smem_mats_ = 0;
 

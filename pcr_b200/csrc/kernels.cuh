@@ -25,14 +25,44 @@ struct EngineParams {
 // ------------------------------------------------------------------ schedule
 // One block.  Decides how many new camera paths each active request gets
 // this iteration: first up to `chunk` each (round-robin fairness), then the
-// remaining free slots oldest-first.
+// remaining free slots oldest-first.  Requests whose paths k_paths traces
+// whole (kReqWhole) share `fill` paths per iteration; the others share the
+// free slots of the path queue.
 constexpr int kSchedThreads = 1024;
+
+struct Share {
+    long long mine, before, all;  // this thread's paths, those of the positions before it, everyone's
+};
+
+// Splits `slots` over the threads' remaining paths `rem`.
+template <typename Scan>
+__device__ __forceinline__ Share share_slots(typename Scan::TempStorage& tmp, long long rem, long long chunk, long long slots)
+{
+    // pass 1: up to chunk each, in active order
+    long long w1 = rem < chunk ? rem : chunk;
+    long long ex1, tot1;
+    Scan(tmp).ExclusiveSum(w1, ex1, tot1);
+    __syncthreads();
+    long long g1 = slots - ex1;
+    g1 = g1 < 0 ? 0 : (g1 > w1 ? w1 : g1);
+    const long long left = slots - (tot1 < slots ? tot1 : slots);
+    const long long rem2 = rem - g1;
+    long long ex2, tot2;
+    Scan(tmp).ExclusiveSum(rem2, ex2, tot2);
+    __syncthreads();
+    long long g2 = left - ex2;
+    g2 = g2 < 0 ? 0 : (g2 > rem2 ? rem2 : g2);
+    Share s;
+    s.mine = g1 + g2;
+    Scan(tmp).ExclusiveSum(s.mine, s.before, s.all);
+    __syncthreads();
+    return s;
+}
 
 __global__ void __launch_bounds__(kSchedThreads) k_schedule(EngineView E, const EngineParams* P, int cur)
 {
-    typedef cub::BlockScan<long long, kSchedThreads> Scan;
+    typedef cub::BlockScan<long long, kSchedThreads, cub::BLOCK_SCAN_WARP_SCANS> Scan;
     __shared__ typename Scan::TempStorage tmp;
-    __shared__ long long s_total;
     Counters* C = E.cnt;
     const int tid = threadIdx.x;
     const int n_act = *E.n_active;
@@ -48,6 +78,7 @@ __global__ void __launch_bounds__(kSchedThreads) k_schedule(EngineView E, const 
     if (p.regen_every > 1 && (C->iter % p.regen_every) != 0 && qn > 0) free_slots = 0;
 
     int slot = -1;
+    bool whole = false;
     long long rem = 0;
     if (tid < n_act) {
         slot = E.active[tid];
@@ -71,27 +102,16 @@ __global__ void __launch_bounds__(kSchedThreads) k_schedule(EngineView E, const 
         }
         rem = E.reqs[slot].total - (long long)E.issued[slot];
         if (rem < 0) rem = 0;
+        whole = (E.reqs[slot].flags & kReqWhole) != 0;
     }
-    // pass 1: up to chunk each, in active order
-    long long w1 = rem < (long long)p.chunk ? rem : (long long)p.chunk;
-    long long ex1, tot1;
-    Scan(tmp).ExclusiveSum(w1, ex1, tot1);
-    __syncthreads();
-    long long g1 = free_slots - ex1;
-    g1 = g1 < 0 ? 0 : (g1 > w1 ? w1 : g1);
-    long long left = free_slots - (tot1 < free_slots ? tot1 : free_slots);
-    long long rem2 = rem - g1;
-    long long ex2, tot2;
-    Scan(tmp).ExclusiveSum(rem2, ex2, tot2);
-    __syncthreads();
-    long long g2 = left - ex2;
-    g2 = g2 < 0 ? 0 : (g2 > rem2 ? rem2 : g2);
-    long long g = g1 + g2;
-    long long exg, totg;
-    Scan(tmp).ExclusiveSum(g, exg, totg);
+    Share q = {0, 0, 0}, w = {0, 0, 0};
+    if (__syncthreads_or(!whole && rem > 0)) q = share_slots<Scan>(tmp, whole ? 0 : rem, p.chunk, free_slots);
+    if (__syncthreads_or(whole && rem > 0)) w = share_slots<Scan>(tmp, whole ? rem : 0, p.chunk, p.fill);
     if (tid < n_act) {
-        E.give[tid] = (int)g;
-        E.give_base[tid] = (int)exg;
+        const long long g = q.mine + w.mine;
+        E.give[tid] = (int)q.mine;
+        E.give_base[tid] = (int)q.before;
+        E.path_base[tid] = (int)w.before;
         E.give_start[tid] = (long long)E.issued[slot];
         if (g > 0) {
             if (E.issued[slot] == 0ull) {
@@ -100,19 +120,19 @@ __global__ void __launch_bounds__(kSchedThreads) k_schedule(EngineView E, const 
                 E.t_first[slot] = t;
             }
             E.issued[slot] += (unsigned long long)g;
-            E.outstanding[slot] += g;
+            E.outstanding[slot] += q.mine;  // a whole path is at its end when k_paths is
         }
     }
-    if (tid == 0) s_total = totg;
-    __syncthreads();
     if (tid == 0) {
         C->n_rounds = 0;  // k_round of the last iteration has read the list
         C->new_base = qn;
-        C->new_n = (int)s_total;
-        C->queue_n[cur] = qn + (int)s_total;
+        C->new_n = (int)q.all;
+        C->queue_n[cur] = qn + (int)q.all;
         C->queue_n[cur ^ 1] = 0;
         C->shadow_n = 0;
-        C->paths += (unsigned long long)s_total;
+        C->path_n = (int)w.all;
+        C->path_next = 0;
+        C->paths += (unsigned long long)(q.all + w.all);
     }
 }
 
@@ -273,6 +293,68 @@ __device__ __noinline__ float4 spec4(const DMaterial& m, int emissive, float4 la
 // ------------------------------------------------------------------ regen
 // Camera rays for the new paths (code/Renderer.cpp:190-239): pixel centre,
 // jitter when aa > 1, hero wavelength and its stratified companions.
+struct CameraPath {
+    uint32_t pixel, sample;
+    float3 d;
+    float lambda0;
+};
+
+// Path number `path` of request R; W receives the XYZ weights of a spectral
+// path's wavelengths (left alone otherwise).
+__device__ __forceinline__ CameraPath camera_path(const EngineView& E, const DRequest& R, long long path, float xyz_scale,
+                                                  XyzWeights& W)
+{
+    CameraPath p;
+    if (R.flags & kReqAdaptive) {
+        // round r: spp paths for each pixel still in the round's list;
+        // sample numbers r*spp.. as in the non-adaptive order
+        const long long q = path - R.round_base;
+        p.pixel = (uint32_t)R.act[R.round & 1][q / R.spp];
+        p.sample = (uint32_t)(R.round * R.spp + (int)(q % R.spp));
+    } else {
+        p.pixel = (uint32_t)(path / R.paths_per_pixel);
+        const int q = (int)(path % R.paths_per_pixel);  // local sample
+        p.sample = (uint32_t)((q / R.local_spp) * R.spp + R.sample0 + q % R.local_spp);
+    }
+    const int px = (int)(p.pixel % (uint32_t)R.width), py = (int)(p.pixel / (uint32_t)R.width);
+    float jx = 0.f, jy = 0.f;
+    if (R.aa > 1) {
+        float4 j = rand4(R, p.pixel, p.sample / (uint32_t)R.spp, 0, 254u, 0);
+        jx = j.x - 0.5f;
+        jy = j.y - 0.5f;
+    }
+    float x = ((2 * (px + 0.5f + jx) / (float)R.width) - 1) * R.scale * R.aspect;
+    float y = -((2 * (py + 0.5f + jy) / (float)R.height) - 1) * R.scale;
+    float inv = rsqrtf(x * x + y * y + 1.f);
+    p.d = make_float3(x * inv, y * inv, -inv);
+    p.lambda0 = 0.f;
+    if (R.flags & kReqSpectral) {
+        float4 u = rand4(R, p.pixel, p.sample, 0, 255u, 0);
+        p.lambda0 = 400.f + u.x * 300.f;
+        const int nch = R.hero;
+        // hero wavelength and its stratified companions (code/Renderer.cpp:227-239)
+        float lam[4];
+        const float span = 300.f, stride_l = span / (float)nch;
+        lam[0] = p.lambda0;
+#pragma unroll
+        for (int k = 1; k < 4; k++) {
+            float l = lam[0] + stride_l * k;
+            if (l > 700.f) l -= span;
+            lam[k] = k < nch ? l : lam[0];
+        }
+        W = xyz_weights(true, lam, nch, 1.f / (float)nch, xyz_scale, E.cmf_table);
+        const DScene& S = E.scenes[R.scene];
+        if (S.emit_mat >= 0) {
+            // emission of the scene's only emissive material, folded in
+            const float4 e = spec4(E.mats[S.mat_base + S.emit_mat], 1, make_float4(lam[0], lam[1], lam[2], lam[3]));
+            W.w[0] = f3mul(W.w[0], e.x);
+            W.w[1] = f3mul(W.w[1], e.y);
+            W.w[2] = f3mul(W.w[2], e.z);
+            W.w[3] = f3mul(W.w[3], e.w);
+        }
+    }
+    return p;
+}
 
 __global__ void k_regen(EngineView E, int cur, float xyz_scale)
 {
@@ -300,63 +382,15 @@ __global__ void k_regen(EngineView E, int cur, float xyz_scale)
         while (lo > 0 && (s_give[lo] == 0 || s_base[lo] > i)) lo--;
         const int slot = s_slot[lo];
         const DRequest& R = E.reqs[slot];
-        const long long path = s_start[lo] + (i - s_base[lo]);
-        uint32_t pixel, sample;
-        if (R.flags & kReqAdaptive) {
-            // round r: spp paths for each pixel still in the round's list;
-            // sample numbers r*spp.. as in the non-adaptive order
-            const long long q = path - R.round_base;
-            pixel = (uint32_t)R.act[R.round & 1][q / R.spp];
-            sample = (uint32_t)(R.round * R.spp + (int)(q % R.spp));
-        } else {
-            pixel = (uint32_t)(path / R.paths_per_pixel);
-            const int q = (int)(path % R.paths_per_pixel);  // local sample
-            sample = (uint32_t)((q / R.local_spp) * R.spp + R.sample0 + q % R.local_spp);
-        }
-        const int px = (int)(pixel % (uint32_t)R.width), py = (int)(pixel / (uint32_t)R.width);
-        float jx = 0.f, jy = 0.f;
-        if (R.aa > 1) {
-            float4 j = rand4(R, pixel, sample / (uint32_t)R.spp, 0, 254u, 0);
-            jx = j.x - 0.5f;
-            jy = j.y - 0.5f;
-        }
-        float x = ((2 * (px + 0.5f + jx) / (float)R.width) - 1) * R.scale * R.aspect;
-        float y = -((2 * (py + 0.5f + jy) / (float)R.height) - 1) * R.scale;
-        float inv = rsqrtf(x * x + y * y + 1.f);
-        float3 d = make_float3(x * inv, y * inv, -inv);
-        float lambda0 = 0.f;
-        int nch = 4;
         const int pos = base + i;
-        if (R.flags & kReqSpectral) {
-            float4 u = rand4(R, pixel, sample, 0, 255u, 0);
-            lambda0 = 400.f + u.x * 300.f;
-            nch = R.hero;
-            // hero wavelength and its stratified companions (code/Renderer.cpp:227-239)
-            float lam[4];
-            const float span = 300.f, stride_l = span / (float)nch;
-            lam[0] = lambda0;
-#pragma unroll
-            for (int k = 1; k < 4; k++) {
-                float l = lam[0] + stride_l * k;
-                if (l > 700.f) l -= span;
-                lam[k] = k < nch ? l : lam[0];
-            }
-            XyzWeights W = xyz_weights(true, lam, nch, 1.f / (float)nch, xyz_scale, E.cmf_table);
-            const DScene& S = E.scenes[R.scene];
-            if (S.emit_mat >= 0) {
-                // emission of the scene's only emissive material, folded in
-                const float4 e = spec4(E.mats[S.mat_base + S.emit_mat], 1, make_float4(lam[0], lam[1], lam[2], lam[3]));
-                W.w[0] = f3mul(W.w[0], e.x);
-                W.w[1] = f3mul(W.w[1], e.y);
-                W.w[2] = f3mul(W.w[2], e.z);
-                W.w[3] = f3mul(W.w[3], e.w);
-            }
-            store_weights(Q, pos, W);
-        }
-        Q.o[pos] = make_float4(R.cam_x, R.cam_y, R.cam_z, lambda0);
-        Q.d[pos] = make_float4(d.x, d.y, d.z, __int_as_float(nch << 12));
+        XyzWeights W;
+        const CameraPath p = camera_path(E, R, s_start[lo] + (i - s_base[lo]), xyz_scale, W);
+        if (R.flags & kReqSpectral) store_weights(Q, pos, W);
+        const int nch = (R.flags & kReqSpectral) ? R.hero : 4;
+        Q.o[pos] = make_float4(R.cam_x, R.cam_y, R.cam_z, p.lambda0);
+        Q.d[pos] = make_float4(p.d.x, p.d.y, p.d.z, __int_as_float(nch << 12));
         Q.tp[pos] = make_float4(1.f, 1.f, 1.f, 1.f);
-        Q.id[pos] = make_int4(slot, (int)pixel, (int)sample, R.scene);
+        Q.id[pos] = make_int4(slot, (int)p.pixel, (int)p.sample, R.scene);
     }
 }
 
@@ -413,6 +447,210 @@ __device__ __forceinline__ void add_xyz(double* acc, float3 c)
     red_add(acc + 0, (double)c.x);
     red_add(acc + 1, (double)c.y);
     red_add(acc + 2, (double)c.z);
+}
+
+// ------------------------------------------------------------------ shading steps
+// The steps of one path vertex (code/Renderer.cpp:656-889 with samples = 1,
+// the GPU's paths-per-pixel estimator), shared by k_shade, which advances a
+// queue of paths by one vertex, and k_paths, which follows a path to its end.
+
+// Wavelengths carried by a path (code/Renderer.cpp:227-239).
+__device__ __forceinline__ float4 path_wavelengths(float l0, int single, int nHero)
+{
+    if (single) return make_float4(l0, l0, l0, l0);
+    const float span = 300.f, stride_l = span / (float)nHero;
+    float l1 = l0 + stride_l * 1, l2 = l0 + stride_l * 2, l3 = l0 + stride_l * 3;
+    if (l1 > 700.f) l1 -= span;
+    if (l2 > 700.f) l2 -= span;
+    if (l3 > 700.f) l3 -= span;
+    return make_float4(l0, 1 < nHero ? l1 : l0, 2 < nHero ? l2 : l0, 3 < nHero ? l3 : l0);
+}
+
+// Hit point, outward normal (not yet turned towards the ray) and material
+// (scene-local) of a hit.  kMesh: the scene may hold triangles.
+struct Surface {
+    float3 hit, N;
+    int mi;
+};
+template <bool kMesh>
+__device__ __forceinline__ Surface surface_at(const DScene& S, uint32_t prim, float t, float hu, float hv, float3 o, float3 d)
+{
+    Surface r;
+    r.hit = make_float3(o.x + d.x * t, o.y + d.y * t, o.z + d.z * t);
+    const uint32_t kind = prim & kPrimKindMask, pidx = prim & kPrimIndexMask;
+    if (kind == kPrimSphere) {
+        const float4 cr = S.spheres[pidx].c_r;
+        float3 v = make_float3(r.hit.x - cr.x, r.hit.y - cr.y, r.hit.z - cr.z);
+        r.N = f3mul(v, rsqrtf(f3dot(v, v)));
+        r.mi = S.spheres[pidx].mat.x;
+    } else if (!kMesh || kind == kPrimPlane) {
+        const float4 na = S.planes[pidx].n_emit;
+        r.N = make_float3(na.x, na.y, na.z);
+        r.mi = __float_as_int(S.planes[pidx].o_mat.w);
+    } else {
+        const DTri& tr = S.tris[pidx];
+        r.mi = __float_as_int(tr.e1_mat.w);
+        if (__float_as_int(tr.e2_flags.w) & 1) {
+            const float4 n0 = S.tri_n[pidx * 3], n1 = S.tri_n[pidx * 3 + 1], n2 = S.tri_n[pidx * 3 + 2];
+            const float w = 1.f - hu - hv;
+            float3 in = make_float3(n0.x * w + n1.x * hu + n2.x * hv, n0.y * w + n1.y * hu + n2.y * hv,
+                                    n0.z * w + n1.z * hu + n2.z * hv);
+            r.N = f3mul(in, rsqrtf(f3dot(in, in)));
+        } else {
+            r.N = xyz(S.tri_flatn[pidx]);
+        }
+    }
+    return r;
+}
+
+// Mirror direction and origin.
+__device__ __forceinline__ void reflect_at(float3 hit, float3 N, float3 d, float cosI, float3& o2, float3& d2)
+{
+    d2 = f3add(d, f3mul(N, 2.f * cosI));
+    o2 = f3add(hit, f3mul(N, 1e-3f));
+}
+
+// Optics::dielectricBounce (code/Includes/Optics.h:59-82) with the coin u;
+// returns whether the path reflects.  Its roundings are written out: left to
+// the compiler, they would depend on the code around the call, and a path's
+// directions with them.
+__device__ __forceinline__ bool dielectric_bounce(float3 hit, float3 N, float3 d, float cosI, bool entering, float ior,
+                                                  float u, float3& bo, float3& bd)
+{
+    const float n1 = entering ? 1.f : ior, n2 = entering ? ior : 1.f;
+    const float eta = n1 / n2;
+    const float e2 = __fmul_rn(eta, eta), s2 = fmaf(-cosI, cosI, 1.f);
+    const float sinT2 = __fmul_rn(e2, s2);
+    bool refl = sinT2 >= 1.f;
+    if (!refl) {
+        float F0 = (n1 - n2) / (n1 + n2);
+        F0 *= F0;
+        const float F = fmaf(1.f - F0, __powf(1.f - cosI, 5.f), F0);
+        refl = u < F;
+    }
+    if (refl) {
+        reflect_at(hit, N, d, cosI, bo, bd);
+    } else {
+        const float cosT = sqrtf(fmaf(-e2, s2, 1.f));
+        const float k = fmaf(eta, cosI, -cosT);
+        bd = make_float3(fmaf(d.x, eta, __fmul_rn(N.x, k)), fmaf(d.y, eta, __fmul_rn(N.y, k)),
+                         fmaf(d.z, eta, __fmul_rn(N.z, k)));
+        bo = f3sub(hit, f3mul(N, 1e-3f));
+    }
+    return refl;
+}
+
+// Optics::cauchyIor, for paths whose wavelengths may bend differently.
+__device__ __forceinline__ float ior_at(const DMaterial& m, bool dispersion, float lambda)
+{
+    float ior = m.ior;
+    if (dispersion) ior = m.ior + m.cauchyB * 1e4f / (lambda * lambda);
+    return ior;
+}
+
+// Light sample s of a diffuse vertex: point, light normal and material.
+struct LightSample {
+    float3 P, Nl;
+    int mat;
+};
+__device__ __forceinline__ LightSample sample_light(const DScene& S, const DRequest& R, uint32_t pixel, uint32_t sample,
+                                                    uint32_t fork, uint32_t bounce, uint32_t s)
+{
+    LightSample r;
+    const float4 rr = rand4(R, pixel, sample, fork, bounce, 1u + s);
+    int pick = 0;
+    if (S.n_lights > 1) {
+        const float target = rr.x * S.total_light_area;
+        float cum = 0.f;
+        for (int l = 0; l < S.n_lights; l++) {
+            cum += S.lights[l].total_area;
+            if (target <= cum) { pick = l; break; }
+        }
+    }
+    const DLight& L = S.lights[pick];
+    if (L.kind == 0) {
+        r.P = make_float3(L.o_mat.x + L.u.x * rr.y + L.v.x * rr.z, L.o_mat.y + L.u.y * rr.y + L.v.y * rr.z,
+                          L.o_mat.z + L.u.z * rr.y + L.v.z * rr.z);
+        r.Nl = xyz(L.n);
+        r.mat = __float_as_int(L.o_mat.w);
+    } else {
+        const float4 r2 = rand4(R, pixel, sample, fork, bounce, 1000u + s);
+        const float rt = rr.y * L.total_area;
+        const float* cum = S.light_cum + L.tri_offset;
+        int lo = 0, hi = L.tri_count;
+        while (lo < hi) { int mid = (lo + hi) >> 1; if (cum[mid] < rt) lo = mid + 1; else hi = mid; }
+        const int ti = lo < L.tri_count - 1 ? lo : L.tri_count - 1;
+        const DTri& lt = S.light_tris[L.tri_offset + ti];
+        float a = rr.z, b = r2.x;
+        if (a + b > 1.f) { a = 1.f - a; b = 1.f - b; }
+        r.P = make_float3(lt.v0_id.x + lt.e1_mat.x * a + lt.e2_flags.x * b,
+                          lt.v0_id.y + lt.e1_mat.y * a + lt.e2_flags.y * b,
+                          lt.v0_id.z + lt.e1_mat.z * a + lt.e2_flags.z * b);
+        r.Nl = xyz(S.light_flatn[L.tri_offset + ti]);
+        r.mat = __float_as_int(lt.e1_mat.w);
+    }
+    return r;
+}
+
+// Shadow segment from the shading point hc (which the lit-facing branch
+// moves, code/Renderer.cpp:857, mutating operator+) to a light sample, and
+// its geometry term G (0 when the sample adds nothing).
+struct ShadowSegment {
+    float3 so, wi;
+    float d2, cosT, cosL, G;
+};
+__device__ __forceinline__ ShadowSegment shadow_segment(const LightSample& L, float3 N, float3& hc)
+{
+    ShadowSegment g;
+    const float3 Li = f3sub(L.P, hc);
+    g.d2 = f3dot(Li, Li);
+    const float inv_d = rsqrtf(g.d2);
+    g.wi = f3mul(Li, inv_d);
+    g.cosT = fmaxf(0.f, f3dot(g.wi, N));
+    if (g.cosT <= 0.f) g.so = f3sub(hc, f3mul(N, 1e-3f));
+    else { hc = f3add(hc, f3mul(N, 1e-3f)); g.so = hc; }
+    g.cosL = fmaxf(0.f, -f3dot(L.Nl, Li));
+    g.G = g.cosT * g.cosL * (inv_d * inv_d);
+    return g;
+}
+// The sample's factor: geometry term times the MIS weight when asked for.
+__device__ __forceinline__ float shadow_factor(const DScene& S, const DRequest& R, const ShadowSegment& g)
+{
+    const float inv_pi = 1.f / 3.14159274f;
+    float w = 1.f;
+    if ((R.flags & kReqMIS) && g.cosL > 1e-6f) {
+        const float pL = g.d2 / (g.cosL * S.total_light_area), pB = g.cosT * inv_pi;
+        w = (pL * pL) / (pL * pL + pB * pB);
+    }
+    return g.G * w;
+}
+
+// Continuation of a diffuse vertex: Russian roulette and the cosine
+// hemisphere.  Returns whether the path goes on; nd its direction and
+// rr_scale its throughput factor.
+__device__ __forceinline__ bool diffuse_bounce(const DRequest& R, uint32_t pixel, uint32_t sample, uint32_t fork, int bounce,
+                                               bool last, bool spectral, float4 al, float3 N, float3& nd, float& rr_scale)
+{
+    const float4 r0 = rand4(R, pixel, sample, fork, (uint32_t)bounce, 0u);
+    bool survive = !last;
+    rr_scale = 1.f;
+    if (survive && (R.flags & kReqRussian) && bounce >= 1) {
+        float pr = spectral ? al.x : fmaxf(fmaxf(al.x, al.y), al.z);
+        pr = fminf(0.95f, fmaxf(0.05f, pr));
+        if (r0.w > pr) survive = false;
+        else rr_scale = 1.f / pr;
+    }
+    if (survive) {
+        float r1 = r0.x, r2 = r0.y;
+        if ((R.flags & kReqStratified) && bounce == 0 && R.strata > 0) {
+            const int sin_ = (int)sample % R.spp;
+            const int sx = sin_ % R.strata, sy = (sin_ / R.strata) % R.strata;
+            r1 = ((float)sx + r0.x) / (float)R.strata;
+            r2 = ((float)sy + r0.y) / (float)R.strata;
+        }
+        nd = hemisphere(N, r1, r2);
+    }
+    return survive;
 }
 
 // ------------------------------------------------------------------ shade
@@ -565,50 +803,13 @@ __global__ void __launch_bounds__(kShadeBlock, PCR_SHADE_MIN_BLOCKS) k_shade(Eng
             const DScene& S = E.scenes[id.w];
             const bool spectral = (R.flags & kReqSpectral) != 0;
             spec_path = spectral;
-            // wavelengths carried by this path (code/Renderer.cpp:227-239)
-            float4 lam4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (spectral) {
-                const float l0 = o4.w;
-                if (single) {
-                    lam4 = make_float4(l0, l0, l0, l0);
-                } else {
-                    const float span = 300.f, stride_l = span / (float)nHero;
-                    float l1 = l0 + stride_l * 1, l2 = l0 + stride_l * 2, l3 = l0 + stride_l * 3;
-                    if (l1 > 700.f) l1 -= span;
-                    if (l2 > 700.f) l2 -= span;
-                    if (l3 > 700.f) l3 -= span;
-                    lam4 = make_float4(l0, 1 < nHero ? l1 : l0, 2 < nHero ? l2 : l0, 3 < nHero ? l3 : l0);
-                }
-            }
+            const float4 lam4 = spectral ? path_wavelengths(o4.w, single, nHero) : make_float4(0.f, 0.f, 0.f, 0.f);
             acc = R.accum + (size_t)id.y * 3;
             const float3 o = xyz(o4), d = xyz(d4);
-            const float t = h.x;
-            const float3 hit = make_float3(o.x + d.x * t, o.y + d.y * t, o.z + d.z * t);
-            float3 N;
-            int mi;
-            const uint32_t kind = prim & kPrimKindMask, pidx = prim & kPrimIndexMask;
-            if (kind == kPrimSphere) {
-                const float4 cr = S.spheres[pidx].c_r;
-                float3 v = make_float3(hit.x - cr.x, hit.y - cr.y, hit.z - cr.z);
-                N = f3mul(v, rsqrtf(f3dot(v, v)));
-                mi = S.spheres[pidx].mat.x;
-            } else if (kind == kPrimPlane) {
-                const float4 na = S.planes[pidx].n_emit;
-                N = make_float3(na.x, na.y, na.z);
-                mi = __float_as_int(S.planes[pidx].o_mat.w);
-            } else {
-                const DTri& tr = S.tris[pidx];
-                mi = __float_as_int(tr.e1_mat.w);
-                if (__float_as_int(tr.e2_flags.w) & 1) {
-                    const float4 n0 = S.tri_n[pidx * 3], n1 = S.tri_n[pidx * 3 + 1], n2 = S.tri_n[pidx * 3 + 2];
-                    const float w = 1.f - h.z - h.w;
-                    float3 in = make_float3(n0.x * w + n1.x * h.z + n2.x * h.w, n0.y * w + n1.y * h.z + n2.y * h.w,
-                                            n0.z * w + n1.z * h.z + n2.z * h.w);
-                    N = f3mul(in, rsqrtf(f3dot(in, in)));
-                } else {
-                    N = xyz(S.tri_flatn[pidx]);
-                }
-            }
+            const Surface sf = surface_at<true>(S, prim, h.x, h.z, h.w, o, d);
+            const float3 hit = sf.hit;
+            float3 N = sf.N;
+            const int mi = sf.mi;
             const bool entering = f3dot(d, N) < 0.f;
             if (!entering) N = f3neg(N);
             const DMaterial& m = M[S.mat_base + mi];
@@ -623,8 +824,7 @@ __global__ void __launch_bounds__(kShadeBlock, PCR_SHADE_MIN_BLOCKS) k_shade(Eng
             } else if (m.flags & kMatMetallic) {
                 if (!last) {
                     const float cosI = -f3dot(d, N);
-                    nd = f3add(d, f3mul(N, 2.f * cosI));
-                    no = f3add(hit, f3mul(N, 1e-3f));
+                    reflect_at(hit, N, d, cosI, no, nd);
                     ntp = mul4(tp4, spectral ? spec4(m, 0, lam4) : rgb4(m.albedo));
                     cont = true;
                 }
@@ -647,30 +847,9 @@ __global__ void __launch_bounds__(kShadeBlock, PCR_SHADE_MIN_BLOCKS) k_shade(Eng
                     }
                     for (int k = 0; k < ways; k++) {
                         const float lk = comp4(lam4, k);
-                        float ior = m.ior;
-                        if (spectral && m.cauchyB != 0.f && (dispersive || single))
-                            ior = m.ior + m.cauchyB * 1e4f / (lk * lk);  // Optics::cauchyIor
-                        // Optics::dielectricBounce (code/Includes/Optics.h:59-82)
-                        const float n1 = entering ? 1.f : ior, n2 = entering ? ior : 1.f;
-                        const float eta = n1 / n2;
-                        const float sinT2 = eta * eta * (1.f - cosI * cosI);
-                        const float u = comp4(coins, k);
+                        const float ior = ior_at(m, spectral && m.cauchyB != 0.f && (dispersive || single), lk);
                         float3 bd, bo;
-                        bool refl = sinT2 >= 1.f;
-                        if (!refl) {
-                            float F0 = (n1 - n2) / (n1 + n2);
-                            F0 *= F0;
-                            const float F = F0 + (1.f - F0) * __powf(1.f - cosI, 5.f);
-                            refl = u < F;
-                        }
-                        if (refl) {
-                            bd = f3add(d, f3mul(N, 2.f * cosI));
-                            bo = f3add(hit, f3mul(N, 1e-3f));
-                        } else {
-                            const float cosT = sqrtf(1.f - sinT2);
-                            bd = f3add(f3mul(d, eta), f3mul(N, eta * cosI - cosT));
-                            bo = f3sub(hit, f3mul(N, 1e-3f));
-                        }
+                        const bool refl = dielectric_bounce(hit, N, d, cosI, entering, ior, comp4(coins, k), bo, bd);
                         if (disperse) {
                             // sub-path k carries wavelength k alone (code/Renderer.cpp:736-753)
                             const int pos = fpos + k;
@@ -735,95 +914,30 @@ __global__ void __launch_bounds__(kShadeBlock, PCR_SHADE_MIN_BLOCKS) k_shade(Eng
                     const int nsh = spos + (R.shadow - 1) * sstride < E.shadow_cap ? R.shadow : 0;
                     if (nsh == 0) atomicOr(&C->status, 1);
                     for (int s = 0; s < nsh; s++) {
-                        const float4 rr = rand4(R, (uint32_t)id.y, (uint32_t)id.z, (uint32_t)fork, (uint32_t)bounce,
-                                                1u + (uint32_t)s);
-                        int pick = 0;
-                        if (S.n_lights > 1) {
-                            const float target = rr.x * S.total_light_area;
-                            float cum = 0.f;
-                            for (int l = 0; l < S.n_lights; l++) {
-                                cum += S.lights[l].total_area;
-                                if (target <= cum) { pick = l; break; }
-                            }
-                        }
-                        const DLight& L = S.lights[pick];
-                        float3 P, Nl;
-                        int lm;
-                        if (L.kind == 0) {
-                            P = make_float3(L.o_mat.x + L.u.x * rr.y + L.v.x * rr.z, L.o_mat.y + L.u.y * rr.y + L.v.y * rr.z,
-                                            L.o_mat.z + L.u.z * rr.y + L.v.z * rr.z);
-                            Nl = xyz(L.n);
-                            lm = __float_as_int(L.o_mat.w);
-                        } else {
-                            const float4 r2 = rand4(R, (uint32_t)id.y, (uint32_t)id.z, (uint32_t)fork, (uint32_t)bounce,
-                                                    1000u + (uint32_t)s);
-                            const float rt = rr.y * L.total_area;
-                            const float* cum = S.light_cum + L.tri_offset;
-                            int lo = 0, hi = L.tri_count;
-                            while (lo < hi) { int mid = (lo + hi) >> 1; if (cum[mid] < rt) lo = mid + 1; else hi = mid; }
-                            const int ti = lo < L.tri_count - 1 ? lo : L.tri_count - 1;
-                            const DTri& lt = S.light_tris[L.tri_offset + ti];
-                            float a = rr.z, b = r2.x;
-                            if (a + b > 1.f) { a = 1.f - a; b = 1.f - b; }
-                            P = make_float3(lt.v0_id.x + lt.e1_mat.x * a + lt.e2_flags.x * b,
-                                            lt.v0_id.y + lt.e1_mat.y * a + lt.e2_flags.y * b,
-                                            lt.v0_id.z + lt.e1_mat.z * a + lt.e2_flags.z * b);
-                            Nl = xyz(S.light_flatn[L.tri_offset + ti]);
-                            lm = __float_as_int(lt.e1_mat.w);
-                        }
-                        const float3 Li = f3sub(P, hc);
-                        const float d2 = f3dot(Li, Li);
-                        const float inv_d = rsqrtf(d2);
-                        const float3 wi = f3mul(Li, inv_d);
-                        const float cosT = fmaxf(0.f, f3dot(wi, N));
-                        float3 so;
-                        // the lit-facing branch moves the shading point again
-                        // (code/Renderer.cpp:857, mutating operator+)
-                        if (cosT <= 0.f) so = f3sub(hc, f3mul(N, 1e-3f));
-                        else { hc = f3add(hc, f3mul(N, 1e-3f)); so = hc; }
-                        const float cosL = fmaxf(0.f, -f3dot(Nl, Li));
-                        const float G = cosT * cosL * (inv_d * inv_d);
+                        const LightSample L = sample_light(S, R, (uint32_t)id.y, (uint32_t)id.z, (uint32_t)fork,
+                                                           (uint32_t)bounce, (uint32_t)s);
+                        const ShadowSegment g = shadow_segment(L, N, hc);
                         const int pos = spos + s * sstride;
-                        if (!(G > 0.f)) {
+                        if (!(g.G > 0.f)) {
                             SQ.o[pos] = make_float4(0.f, 0.f, 0.f, -1.f);  // skip record
                             continue;
                         }
-                        if (lm != cached) {
+                        if (L.mat != cached) {
                             // product of this light material, once per vertex
-                            const DMaterial& lmat = M[S.mat_base + lm];
+                            const DMaterial& lmat = M[S.mat_base + L.mat];
                             const float4 c = spectral ? mul4(tpal, spec4(lmat, 1, lam4)) : mul4(tpal, rgb4(lmat.emissive));
                             V = f3mul(apply_xyz(spectral ? load_weights(Q, i) : rgb_weights(), c), scaleS);
-                            cached = lm;
+                            cached = L.mat;
                         }
-                        float w = 1.f;
-                        if ((R.flags & kReqMIS) && cosL > 1e-6f) {
-                            const float pL = d2 / (cosL * S.total_light_area), pB = cosT * inv_pi;
-                            w = (pL * pL) / (pL * pL + pB * pB);
-                        }
-                        const float f = G * w;
-                        SQ.o[pos] = make_float4(so.x, so.y, so.z, d2);
-                        SQ.d[pos] = make_float4(wi.x, wi.y, wi.z, __int_as_float(id.y));
+                        const float f = shadow_factor(S, R, g);
+                        SQ.o[pos] = make_float4(g.so.x, g.so.y, g.so.z, g.d2);
+                        SQ.d[pos] = make_float4(g.wi.x, g.wi.y, g.wi.z, __int_as_float(id.y));
                         SQ.c[pos] = make_float4(V.x * f, V.y * f, V.z * f, __int_as_float(slot | (id.w << 16)));
                     }
                 }
-                const float4 r0 = rand4(R, (uint32_t)id.y, (uint32_t)id.z, (uint32_t)fork, (uint32_t)bounce, 0u);
-                bool survive = !last;
-                float rr_scale = 1.f;
-                if (survive && (R.flags & kReqRussian) && bounce >= 1) {
-                    float pr = spectral ? al.x : fmaxf(fmaxf(al.x, al.y), al.z);
-                    pr = fminf(0.95f, fmaxf(0.05f, pr));
-                    if (r0.w > pr) survive = false;
-                    else rr_scale = 1.f / pr;
-                }
-                if (survive) {
-                    float r1 = r0.x, r2 = r0.y;
-                    if ((R.flags & kReqStratified) && bounce == 0 && R.strata > 0) {
-                        const int sin_ = id.z % R.spp;
-                        const int sx = sin_ % R.strata, sy = (sin_ / R.strata) % R.strata;
-                        r1 = ((float)sx + r0.x) / (float)R.strata;
-                        r2 = ((float)sy + r0.y) / (float)R.strata;
-                    }
-                    nd = hemisphere(N, r1, r2);
+                float rr_scale;
+                if (diffuse_bounce(R, (uint32_t)id.y, (uint32_t)id.z, (uint32_t)fork, bounce, last, spectral, al, N, nd,
+                                   rr_scale)) {
                     no = h1;
                     ntp = make_float4(tp4.x * al.x * rr_scale, tp4.y * al.y * rr_scale, tp4.z * al.z * rr_scale,
                                       tp4.w * al.w * rr_scale);

@@ -132,7 +132,8 @@ struct DScene {
 
 // Request flags
 constexpr int kReqSpectral = 1, kReqMIS = 2, kReqRussian = 4, kReqStratified = 8, kReqAdaptive = 16,
-              kReqTerminate = 32, kReqCancelled = 64;
+              kReqTerminate = 32, kReqCancelled = 64,
+              kReqWhole = 128;      // traced by k_paths (scene without a mesh), not through the queues
 
 struct DRequest {
     int scene, width, height, depth;
@@ -186,6 +187,8 @@ struct Counters {
     int idle;             // 1 when no request has work left
     int n_rounds;         // adaptive requests whose round ended this iteration (k_status -> k_round)
     unsigned long long rays, shadow_rays, paths;
+    int path_n, path_next;        // k_paths: paths of this launch, next one to take
+    unsigned long long path_begin, path_end;  // plain k_paths: globaltimer at its setup and its last block's end
 };
 
 // Device view of the engine, passed by value to every kernel.
@@ -197,6 +200,7 @@ struct EngineView {
     long long* outstanding;          // per slot
     int* give;                       // per active position: paths this iteration
     int* give_base;                  // per active position: exclusive prefix
+    int* path_base;                  // the same for the paths k_paths traces whole
     int* active;                     // active slot list (admission order)
     int* n_active;
     int* done_flag;                  // per slot: 1 once finished

@@ -1,0 +1,358 @@
+// Whole-path kernel for scenes without a triangle mesh.
+#pragma once
+
+#include "kernels.cuh"
+
+namespace pcr {
+
+// k_paths follows each path from its camera ray to its end in one thread:
+// closest hit, shading, shadow rays and the next direction, vertex after
+// vertex, with the path's state in registers.
+//
+// Why not the queue stages (k_extend / k_shade / k_shadow) here: a ray meets
+// at most a few dozen quads and spheres, so its trace is short, and what the
+// stages pass through memory outweighs it: 400 B of path and hit records per
+// vertex and 96 B per shadow ray, besides three FP64 reductions per lit
+// sample, and five launches per vertex of a path.  Mesh scenes keep the
+// queues, where the lanes of a warp at least start their long BVH walks
+// together.
+//
+// A warp keeps its lanes filled: a lane whose path has ended takes a pending
+// sub-path of a dispersive fork from the warp's stack, and when the stack is
+// empty and kPathRefill lanes wait (raygen costs about one vertex, so it is
+// not run for a lane or two at a time), they take the next camera paths from
+// a counter shared by the grid.
+//
+// The samples of a path are added up in double and go to the pixel's FP64
+// accumulator once, when the path ends.
+//
+// What bounds it: instruction issue (50 % of the slots; 16 warps per SM at
+// 128 registers, instruction fetches the most frequent stall).  4 blocks per
+// SM without spills beat 5 (96 registers, 180 B of spills) and 6: Cornell
+// 256x256, 16 paths a pixel, 4 vertices, 4 shadow rays: queue stages 4.39 ms,
+// 1.08 ms at 5 blocks, 1.02 ms at 4.  64x64, one path a pixel: 240 -> 98 us.
+constexpr int kPathBlock = 128;
+#ifndef PCR_PATH_MIN_BLOCKS
+#define PCR_PATH_MIN_BLOCKS 4
+#endif
+#ifndef PCR_PATH_REFILL
+#define PCR_PATH_REFILL 12
+#endif
+constexpr int kPathRefill = PCR_PATH_REFILL;
+// A path forks at most once, into at most four sub-paths of which one stays
+// in its lane; new camera paths are taken only when the stack is empty.  So
+// pending entries + 3 x (lanes that may still fork) never exceed 3 x 32.
+constexpr int kForkStack = 96;
+constexpr int kForkWords = 14;
+
+struct PathWarp {
+    float w[12][32];                     // XYZ weights of each lane's path
+    uint32_t fork[kForkWords][kForkStack];  // pending sub-paths
+    int pending;
+};
+
+constexpr size_t kPathSmem = (kPathBlock / 32) * sizeof(PathWarp);
+
+// The work of one k_paths launch for a single request (the plain method):
+// `n` paths from number `first` on, in slot 0.
+__global__ void k_one_request(EngineView E, DRequest r, long long first, int n)
+{
+    Counters* C = E.cnt;
+    const_cast<DRequest*>(E.reqs)[0] = r;
+    E.active[0] = 0;
+    *E.n_active = 1;
+    E.path_base[0] = 0;
+    E.give_start[0] = first;
+    C->path_n = n;
+    C->path_next = 0;
+    C->paths += (unsigned long long)n;
+    if (first == 0) {
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        C->path_begin = t;
+        C->path_end = 0;
+    }
+}
+
+__device__ __forceinline__ XyzWeights lane_weights(const PathWarp& P, int lane)
+{
+    XyzWeights W;
+    W.w[0] = make_float3(P.w[0][lane], P.w[1][lane], P.w[2][lane]);
+    W.w[1] = make_float3(P.w[3][lane], P.w[4][lane], P.w[5][lane]);
+    W.w[2] = make_float3(P.w[6][lane], P.w[7][lane], P.w[8][lane]);
+    W.w[3] = make_float3(P.w[9][lane], P.w[10][lane], P.w[11][lane]);
+    return W;
+}
+__device__ __forceinline__ void set_lane_weights(PathWarp& P, int lane, const XyzWeights& W)
+{
+    P.w[0][lane] = W.w[0].x; P.w[1][lane] = W.w[0].y; P.w[2][lane] = W.w[0].z;
+    P.w[3][lane] = W.w[1].x; P.w[4][lane] = W.w[1].y; P.w[5][lane] = W.w[1].z;
+    P.w[6][lane] = W.w[2].x; P.w[7][lane] = W.w[2].y; P.w[8][lane] = W.w[2].z;
+    P.w[9][lane] = W.w[3].x; P.w[10][lane] = W.w[3].y; P.w[11][lane] = W.w[3].z;
+}
+// Only the hero wavelength is left.
+__device__ __forceinline__ void single_lane_weights(PathWarp& P, int lane, float3 w)
+{
+    P.w[0][lane] = w.x; P.w[1][lane] = w.y; P.w[2][lane] = w.z;
+#pragma unroll
+    for (int k = 3; k < 12; k++) P.w[k][lane] = 0.f;
+}
+
+// Work of one launch: Counters::path_n paths, numbered over the active list;
+// position r's paths start at path_base[r] and are the request's paths
+// give_start[r], give_start[r] + 1, ...
+__global__ void __launch_bounds__(kPathBlock, PCR_PATH_MIN_BLOCKS) k_paths(const __grid_constant__ EngineView E, float xyz_scale)
+{
+    extern __shared__ __align__(16) unsigned char s_paths[];
+    PathWarp& P = reinterpret_cast<PathWarp*>(s_paths)[threadIdx.x >> 5];
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    Counters* C = E.cnt;
+    const int n = C->path_n, n_act = *E.n_active;
+    if (lane == 0) P.pending = 0;
+    __syncwarp();
+
+    bool alive = false, more = n > 0;
+    float3 o = make_float3(0.f, 0.f, 0.f), d = o;
+    float4 tp = make_float4(0.f, 0.f, 0.f, 0.f);
+    float lambda0 = 0.f;
+    int meta = 0, slot = 0;
+    uint32_t pixel = 0, sample = 0;
+    double ax = 0.0, ay = 0.0, az = 0.0;
+    unsigned rays = 0, shadows = 0;
+
+    while (true) {
+        // ---- refill
+        unsigned dead = __ballot_sync(kAll, !alive);
+        if (dead) {
+            const int pending = P.pending;
+            if (pending) {
+                const int k = pending - 1 - __popc(dead & below);
+                if (!alive && k >= 0) {
+                    o = make_float3(__uint_as_float(P.fork[0][k]), __uint_as_float(P.fork[1][k]), __uint_as_float(P.fork[2][k]));
+                    d = make_float3(__uint_as_float(P.fork[3][k]), __uint_as_float(P.fork[4][k]), __uint_as_float(P.fork[5][k]));
+                    lambda0 = __uint_as_float(P.fork[6][k]);
+                    const float f = __uint_as_float(P.fork[7][k]);
+                    tp = make_float4(f, f, f, f);
+                    single_lane_weights(P, lane, make_float3(__uint_as_float(P.fork[8][k]), __uint_as_float(P.fork[9][k]),
+                                                             __uint_as_float(P.fork[10][k])));
+                    pixel = P.fork[11][k];
+                    sample = P.fork[12][k];
+                    meta = (int)(P.fork[13][k] & 0xffffu);
+                    slot = (int)(P.fork[13][k] >> 16);
+                    alive = true;
+                }
+                __syncwarp();
+                if (lane == 0) P.pending = max(0, pending - __popc(dead));
+                __syncwarp();
+                dead = __ballot_sync(kAll, !alive);
+            }
+            if (more && __popc(dead) >= kPathRefill) {
+                int first = 0;
+                if (lane == 0) first = atomicAdd(&C->path_next, __popc(dead));
+                first = __shfl_sync(kAll, first, 0);
+                more = first + __popc(dead) < n;
+                const int i = first + __popc(dead & below);
+                if (!alive && i < n) {
+                    int lo = 0, hi = n_act - 1;
+                    while (lo < hi) {  // last r with path_base[r] <= i: it has paths in this launch
+                        const int mid = (lo + hi + 1) >> 1;
+                        if (E.path_base[mid] <= i) lo = mid; else hi = mid - 1;
+                    }
+                    slot = E.active[lo];
+                    const DRequest& R = E.reqs[slot];
+                    XyzWeights W = rgb_weights();
+                    const CameraPath p = camera_path(E, R, E.give_start[lo] + (i - E.path_base[lo]), xyz_scale, W);
+                    set_lane_weights(P, lane, W);
+                    pixel = p.pixel;
+                    sample = p.sample;
+                    o = make_float3(R.cam_x, R.cam_y, R.cam_z);
+                    d = p.d;
+                    lambda0 = p.lambda0;
+                    tp = make_float4(1.f, 1.f, 1.f, 1.f);
+                    meta = ((R.flags & kReqSpectral) ? R.hero : 4) << 12;
+                    alive = true;
+                }
+            }
+            if (!__any_sync(kAll, alive)) {
+                if (more) continue;
+                break;
+            }
+        }
+
+        // ---- one vertex of each live path
+        if (alive) {
+            const DRequest& R = E.reqs[slot];
+            const DScene& S = E.scenes[R.scene];
+            alive = false;
+            rays++;
+            float t = FLT_MAX;
+            const uint32_t prim = scene_analytic(S, o, d, t);
+            if (prim != kPrimNone) {
+                const int bounce = meta & 0xFF, fork = (meta >> 8) & 7, single = (meta >> 11) & 1, nHero = (meta >> 12) & 7;
+                const bool spectral = (R.flags & kReqSpectral) != 0;
+                const float4 lam4 = spectral ? path_wavelengths(lambda0, single, nHero) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const Surface sf = surface_at<false>(S, prim, t, 0.f, 0.f, o, d);
+                const float3 hit = sf.hit;
+                float3 N = sf.N;
+                const bool entering = f3dot(d, N) < 0.f;
+                if (!entering) N = f3neg(N);
+                const DMaterial& m = E.mats[S.mat_base + sf.mi];
+                const bool last = bounce + 1 >= R.depth;
+                if (m.flags & kMatEmissive) {
+                    const float4 c = !spectral ? mul4(tp, rgb4(m.emissive))
+                                   : S.emit_mat >= 0 ? tp : mul4(tp, spec4(m, 1, lam4));
+                    const float3 e = apply_xyz(lane_weights(P, lane), c);
+                    ax += (double)e.x;
+                    ay += (double)e.y;
+                    az += (double)e.z;
+                } else if (m.flags & kMatMetallic) {
+                    if (!last) {
+                        const float cosI = -f3dot(d, N);
+                        reflect_at(hit, N, d, cosI, o, d);
+                        tp = mul4(tp, spectral ? spec4(m, 0, lam4) : rgb4(m.albedo));
+                        meta++;
+                        alive = true;
+                    }
+                } else if (m.flags & kMatTransparent) {
+                    if (!last) {
+                        const float cosI = -f3dot(d, N);
+                        const bool dispersive = spectral && m.cauchyB != 0.f && !single && nHero > 1;
+                        // fork: one sub-path per wavelength (code/Renderer.cpp:736-753);
+                        // terminate: the hero wavelength's bounce alone
+                        // (code/Gpu/Metal/MetalRenderer.mm:2143-2252)
+                        const bool terminate = dispersive && (R.flags & kReqTerminate);
+                        const bool disperse = dispersive && !terminate;
+                        const int ways = disperse ? nHero : 1;
+                        const float4 coins = rand4(R, pixel, sample, (uint32_t)fork, (uint32_t)bounce, 63u);
+                        const float4 alg = spectral ? spec4(m, 0, lam4) : rgb4(m.albedo);
+                        int at = 0;
+                        if (disperse) at = atomicAdd(&P.pending, ways - 1);
+                        float3 no = o, nd = d;
+                        bool refl = false;
+                        // the lane keeps sub-path 0, the last one computed
+                        for (int k = ways - 1; k >= 0; k--) {
+                            const float lk = comp4(lam4, k);
+                            const float ior = ior_at(m, spectral && m.cauchyB != 0.f && (dispersive || single), lk);
+                            refl = dielectric_bounce(hit, N, d, cosI, entering, ior, comp4(coins, k), no, nd);
+                            if (k > 0 && at >= kForkStack) {
+                                atomicOr(&C->status, 2);  // never expected, see kForkStack
+                            } else if (k > 0) {
+                                // sub-path k carries wavelength k alone
+                                P.fork[0][at] = __float_as_uint(no.x);
+                                P.fork[1][at] = __float_as_uint(no.y);
+                                P.fork[2][at] = __float_as_uint(no.z);
+                                P.fork[3][at] = __float_as_uint(nd.x);
+                                P.fork[4][at] = __float_as_uint(nd.y);
+                                P.fork[5][at] = __float_as_uint(nd.z);
+                                P.fork[6][at] = __float_as_uint(lk);
+                                P.fork[7][at] = __float_as_uint(comp4(tp, k) * comp4(alg, k));
+                                P.fork[8][at] = __float_as_uint(P.w[3 * k][lane]);
+                                P.fork[9][at] = __float_as_uint(P.w[3 * k + 1][lane]);
+                                P.fork[10][at] = __float_as_uint(P.w[3 * k + 2][lane]);
+                                P.fork[11][at] = pixel;
+                                P.fork[12][at] = sample;
+                                P.fork[13][at] = (uint32_t)((bounce + 1) | ((k + 1) << 8) | (1 << 11) | (nHero << 12)) |
+                                                 ((uint32_t)slot << 16);
+                                at++;
+                            }
+                        }
+                        o = no;
+                        d = nd;
+                        if (disperse) {
+                            const float f = tp.x * alg.x;
+                            tp = make_float4(f, f, f, f);
+                            meta = (bounce + 1) | (1 << 8) | (1 << 11) | (nHero << 12);
+                            single_lane_weights(P, lane, make_float3(P.w[0][lane], P.w[1][lane], P.w[2][lane]));
+                        } else {
+                            tp = mul4(tp, alg);
+                            meta++;
+                            // a refraction ends the other wavelengths; the
+                            // hero's share is scaled by their number so the
+                            // estimate stays unbiased (a reflection does not
+                            // depend on the wavelength and keeps them all)
+                            if (terminate && !refl) {
+                                const float h0 = tp.x * (float)nHero;
+                                tp = make_float4(h0, h0, h0, h0);
+                                meta |= 1 << 11;
+                                single_lane_weights(P, lane, make_float3(P.w[0][lane], P.w[1][lane], P.w[2][lane]));
+                            }
+                        }
+                        alive = true;
+                    }
+                } else {
+                    // diffuse; the continuation starts at the hit moved once
+                    // by 1e-3*N (the reference's mutating `hit + N * 1e-3`,
+                    // code/Renderer.cpp:782 with samples = 1)
+                    const float4 al = spectral ? spec4(m, 0, lam4) : rgb4(m.albedo);
+                    float3 hc = f3add(hit, f3mul(N, 1e-3f));
+                    o = hc;
+                    if (S.total_light_area > 0.f) {
+                        const float inv_pi = 1.f / 3.14159274f;
+                        const float scaleS = S.total_light_area * inv_pi / (float)R.shadow;
+                        const float4 tpal = mul4(tp, al);
+                        int cached = -1;
+                        float3 V = make_float3(0.f, 0.f, 0.f);
+                        if (spectral && S.emit_mat >= 0) {
+                            // every light has the one emissive material, whose
+                            // emission the weights already hold
+                            V = f3mul(apply_xyz(lane_weights(P, lane), tpal), scaleS);
+                            cached = S.emit_mat;
+                        }
+                        for (int s = 0; s < R.shadow; s++) {
+                            const LightSample L = sample_light(S, R, pixel, sample, (uint32_t)fork, (uint32_t)bounce, (uint32_t)s);
+                            const ShadowSegment g = shadow_segment(L, N, hc);
+                            if (!(g.G > 0.f)) continue;
+                            shadows++;
+                            float bound;
+                            if (scene_blocked_analytic<false>(S, E.mats, g.so, g.wi, g.d2, bound) == kShadowBlocked) continue;
+                            if (L.mat != cached) {
+                                // product of this light material, once per vertex
+                                const DMaterial& lmat = E.mats[S.mat_base + L.mat];
+                                const float4 c = spectral ? mul4(tpal, spec4(lmat, 1, lam4)) : mul4(tpal, rgb4(lmat.emissive));
+                                V = f3mul(apply_xyz(lane_weights(P, lane), c), scaleS);
+                                cached = L.mat;
+                            }
+                            const float f = shadow_factor(S, R, g);
+                            ax += (double)(V.x * f);
+                            ay += (double)(V.y * f);
+                            az += (double)(V.z * f);
+                        }
+                    }
+                    float3 nd;
+                    float rr_scale;
+                    if (diffuse_bounce(R, pixel, sample, (uint32_t)fork, bounce, last, spectral, al, N, nd, rr_scale)) {
+                        d = nd;
+                        tp = make_float4(tp.x * al.x * rr_scale, tp.y * al.y * rr_scale, tp.z * al.z * rr_scale,
+                                         tp.w * al.w * rr_scale);
+                        meta++;
+                        alive = true;
+                    }
+                }
+            }
+            if (!alive && (ax != 0.0 || ay != 0.0 || az != 0.0)) {
+                double* acc = R.accum + (size_t)pixel * 3;
+                red_add(acc + 0, ax);
+                red_add(acc + 1, ay);
+                red_add(acc + 2, az);
+                ax = ay = az = 0.0;
+            }
+        }
+        __syncwarp();
+    }
+    rays = __reduce_add_sync(kAll, rays);
+    shadows = __reduce_add_sync(kAll, shadows);
+    if (lane == 0 && rays) {
+        atomicAdd(&C->rays, (unsigned long long)rays);
+        atomicAdd(&C->shadow_rays, (unsigned long long)shadows);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        atomicMax(&C->path_end, now);
+    }
+}
+
+}  // namespace pcr

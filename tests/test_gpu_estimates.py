@@ -160,3 +160,40 @@ def test_estimates_agree_with_exact_tests(ctx, tmp_path, kind):
     assert 0.02 < b0.mean() < 0.98
     for sid in (fast, exact):
         ctx.release_scene(sid)
+
+
+@pytest.mark.parametrize("scene,kw", [
+    ("cornell", dict(depth=1, samples=1, shadow=1, spectral=False)),
+    ("cornell", dict(depth=6, samples=5, shadow=3, spectral=True, hero=1)),
+    ("cornell-spheres", dict(depth=4, samples=4, shadow=2, spectral=False, mis=True, russian=True, stratified=True, aa=2)),
+    ("cornell-glass", dict(depth=8, samples=3, shadow=2, spectral=True, hero=3)),
+    ("cornell-glass", dict(depth=8, samples=3, shadow=2, spectral=True, terminate=True)),
+    ("closed-cornell-glass", dict(depth=8, samples=2, shadow=8, spectral=True)),
+])
+@pytest.mark.parametrize("size", [(1, 1), (33, 7), (128, 96)])
+def test_whole_paths_equal_queue_stages(ctx, tmp_path, scene, kw, size):
+    """The whole-path kernel (scenes without a mesh) against the queue stages:
+    the same scene with a triangle far behind the camera goes through the
+    queues and must give the same image (each sample's value is the same;
+    only the FP64 summation order differs)."""
+    from conftest import GOLDEN, scene_path
+    from pcr_b200 import capi, workloads
+    sc = workloads.read_scene_json(scene_path(scene))
+    (tmp_path / "tri.obj").write_text("v 0 0 0\nv 0.001 0 0\nv 0 0.001 0\nf 1 2 3\n")
+    sc["primitives"].insert(0, {"type": "mesh", "file": "tri.obj", "position": [0, 0, 5000.0],
+                                "material": next(k for k, m in sc["materials"].items() if "emissive" not in m)})
+    p = tmp_path / "queue.json"
+    p.write_text(json.dumps(sc))
+    import shutil, os
+    if os.path.isdir(os.path.join(GOLDEN, "spd")):
+        shutil.copytree(os.path.join(GOLDEN, "spd"), tmp_path / "spd")
+    a, b = ctx.load_scene_json(scene_path(scene), GOLDEN), ctx.load_scene_json(str(p), str(tmp_path))
+    d = capi.render_desc(size[0], size[1], seed=11, **kw)
+    whole, queue = ctx.render(a, d), ctx.render(b, d)
+    assert np.allclose(whole[0], queue[0], rtol=1e-6, atol=1e-7)
+    ids = [ctx.submit(s, d) for s in (a, b)]
+    ctx.run_until_idle()
+    for rid in ids:
+        assert np.allclose(ctx.fetch(rid)[0], whole[0], rtol=1e-6, atol=1e-7)
+    for sid in (a, b):
+        ctx.release_scene(sid)
