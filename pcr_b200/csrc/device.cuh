@@ -677,39 +677,53 @@ __device__ __noinline__ int scene_blocked_exact(const DScene& S, const DMaterial
 // The analytic shadow query where the estimates decide it, else -1.  `light`
 // receives the plane index of the emissive rectangle that bounds the query
 // (-1: none, the query's end does).
-__device__ __forceinline__ int flat_blocked(const DScene& S, float3 o, float3 d, float tmax, float d2, int& light)
+//
+// Most shadow rays run between two points of the cell, the box that the
+// room's walls enclose with everything else in it (flat_scene), where no wall
+// can be met.  So the walls are tested only for a ray that starts outside the
+// cell or that no light inside it bounds: the Cornell box's query then tests
+// one rectangle and two boxes instead of six and two.
+__device__ __forceinline__ int flat_blocked(const DScene& S, float3 o, float3 d, float d2, int& light)
 {
     const float inf = __int_as_float(0x7f800000);
     FlatRay r = flat_ray(S, o, d);
     const float pad = S.flat_pad;
-    float bound = tmax;     // closest emissive hit, or the query's end
+    float bound = sqrt_approx(d2) * 1.0001f + 1e-4f;  // closest emissive hit, or the query's end
     float may_t = inf;      // no other hit lies in front of this
     float hit_t = inf;      // one surely lies in front of this
     light = -1;
     bool clear = true;      // the bound is beyond doubt
-    const DRect* q = S.rects;
-    AxisRay ar(r);
+    bool walls = !(o.x > S.cell_lo[0] && o.y > S.cell_lo[1] && o.z > S.cell_lo[2] && o.x < S.cell_hi[0] &&
+                   o.y < S.cell_hi[1] && o.z < S.cell_hi[2]);
+    bool cell_light = false;
+    const DRect* q = S.srects;
+    const DRect* const all = q + S.n_srects;
+    const DRect* end = q + S.n_inner;
+    while (true) {
 #pragma unroll 1
-    for (int axis = 0; axis < 3; axis++) {
-        bool met = false;   // an emissive rectangle of the same plane has the point: the others tie with the bound
-#pragma unroll 1
-        for (const DRect* end = q + S.n_rects[axis]; q < end; q++) {
-            float t;
-            int pid, flags;
-            const float e = rect_excess(*q, ar, t, pid, flags);
-            met = met && (flags & kRectSamePlane);
-            const bool may = e < pad && t > 5e-7f && !met, sure = e < -pad && t > 2e-6f;
-            const bool emissive = flags & kRectEmissive;
-            if (emissive) {
+        for (; q < end; q++) {
+            const float4 a = __ldg(&q->a), b = __ldg(&q->b);
+            const int flags = __float_as_int(b.z), axis = flags >> kRectAxisShift;
+            const bool ax = axis == 0, az = axis == 2;
+            const float ok = ax ? o.x : (az ? o.z : o.y), rk = ax ? r.rd.x : (az ? r.rd.z : r.rd.y);
+            const float oi = ax ? o.y : o.x, di = ax ? d.y : d.x, oj = az ? o.y : o.z, dj = az ? d.y : d.z;
+            const float t = (a.x - ok) * rk;
+            const float e = fmaxf(fabsf(fmaf(t, di, oi) - a.y) - b.x, fabsf(fmaf(t, dj, oj) - a.z) - b.y);
+            const bool may = e < pad && t > 5e-7f, sure = e < -pad && t > 2e-6f;
+            if (flags & kRectEmissive) {
                 clear = clear && (sure || !may);
-                if (may && t < bound) { bound = t; light = pid; }
-                met = may;
+                if (may && t < bound) {
+                    bound = t;
+                    light = __float_as_int(a.w);
+                    cell_light = flags & kRectCellLight;
+                }
             } else {
                 may_t = fminf(may_t, may ? t : inf);
                 hit_t = fminf(hit_t, may && sure ? t : inf);
             }
         }
-        ar.next();
+        if (end == all || (!walls && cell_light)) break;
+        end = all;
     }
 #pragma unroll 1
     for (int i = 0; i < S.n_boxes; i++) {
@@ -736,21 +750,22 @@ __device__ __forceinline__ int flat_blocked(const DScene& S, float3 o, float3 d,
     return -1;
 }
 
+// A hit beyond the light cannot block: the query ends just past it.
+__device__ __forceinline__ float shadow_end(float d2) { return sqrtf(d2) * 1.0001f + 1e-4f; }
+
 // The part of the shadow query before the triangle BVH (see
 // scene_blocked_exact).
 template <bool kMesh>
 __device__ __forceinline__ int scene_blocked_analytic(const DScene& S, const DMaterial* mats, float3 o, float3 d,
                                                       float d2, float& bound)
 {
-    // a hit beyond the light cannot block: bound the query just past it
-    const float tmax = sqrtf(d2) * 1.0001f + 1e-4f;
     if (S.flat_ok && !(kMesh && S.emissive_tris)) {
         int light;
-        const int r = flat_blocked(S, o, d, tmax, d2, light);
+        const int r = flat_blocked(S, o, d, d2, light);
         if (r == kShadowBlocked) return r;
         if (r == kShadowLit) {
             if (!kMesh || S.n_nodes <= 0) return r;
-            bound = tmax;
+            bound = shadow_end(d2);
             if (light >= 0) {
                 const float3 N = xyz(S.planes[light].n_emit), po = xyz(S.planes[light].o_mat);
                 bound = ex::div(ex::dot(ex::sub3(po, o), N), ex::dot(d, N));
@@ -758,7 +773,7 @@ __device__ __forceinline__ int scene_blocked_analytic(const DScene& S, const DMa
             return kShadowWalk;
         }
     }
-    return scene_blocked_exact<kMesh>(S, mats, o, d, tmax, (double)d2 - 1e-3, bound);
+    return scene_blocked_exact<kMesh>(S, mats, o, d, shadow_end(d2), (double)d2 - 1e-3, bound);
 }
 
 __device__ __forceinline__ bool scene_blocked(const DScene& S, const DMaterial* mats, float3 o, float3 d, float d2)

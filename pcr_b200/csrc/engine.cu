@@ -398,9 +398,10 @@ static std::vector<float4> plane_groups(const pcr_plane* p, int n)
 // the exact tests' grouped culling skips more than it costs.
 constexpr int kMaxFlatPrims = 64;
 struct FlatScene {
-    std::vector<DRect> rects;
+    std::vector<DRect> rects, srects;
     std::vector<DBox> boxes;
-    int n_rects[3] = {0, 0, 0};
+    int n_rects[3] = {0, 0, 0}, n_inner = 0;
+    float cell_lo[3] = {0, 0, 0}, cell_hi[3] = {0, 0, 0};
     bool ok = false;
     float pad = 0.f, reach = 0.f;
 };
@@ -512,13 +513,64 @@ static FlatScene flat_scene(const pcr_scene_desc& d, const std::vector<DPlane>& 
         const pcr_plane& p = d.planes[i];
         const int a = axis == 0 ? 1 : 0, b = axis == 2 ? 1 : 2;  // the two other axes, in order
         auto span = [&](int x) { return (double)p.u[x] + (double)p.v[x]; };  // one of them is zero
-        int flags = planes[i].n_emit.w != 0.f ? kRectEmissive : 0;
+        int flags = (planes[i].n_emit.w != 0.f ? kRectEmissive : 0) | axis << kRectAxisShift;
         if (k > 0 && std::get<0>(flat[k - 1]) == axis && std::get<1>(flat[k - 1]) == at) flags |= kRectSamePlane;
         DRect q;
         q.a = make_float4(at, (float)(p.origin[a] + 0.5 * span(a)), (float)(p.origin[b] + 0.5 * span(b)), __int_as_float_host(i));
         q.b = make_float4((float)(0.5 * std::fabs(span(a))), (float)(0.5 * std::fabs(span(b))), __int_as_float_host(flags), 0.f);
         F.rects.push_back(q);
         F.n_rects[axis]++;
+    }
+
+    // The cell: everything that is no wall, the camera included, lies in it;
+    // a wall is a rectangle whose plane has all of that on one side.
+    double in_lo[3], in_hi[3];
+    for (int x = 0; x < 3; x++) in_lo[x] = in_hi[x] = d.cam_pos[x];
+    auto hold = [&](const V& c, double r) {
+        for (int x = 0; x < 3; x++) {
+            in_lo[x] = std::min(in_lo[x], c[x] - r);
+            in_hi[x] = std::max(in_hi[x], c[x] + r);
+        }
+    };
+    for (const DBox& B : F.boxes)
+        for (int i : {B.lo.x, B.hi.x}) {
+            const V o = vec(d.planes[i].origin), u = vec(d.planes[i].u), v = vec(d.planes[i].v);
+            for (const V& c : {o, add(o, u), add(o, v), add(add(o, u), v)}) hold(c, 0.0);
+        }
+    for (int i = 0; i < d.n_spheres; i++) hold(vec(d.spheres[i].center), d.spheres[i].radius);
+    for (const DRect& q : F.rects)
+        if (__float_as_int_host(q.b.z) & kRectEmissive) {
+            const pcr_plane& p = d.planes[__float_as_int_host(q.a.w)];
+            hold(vec(p.origin), 0.0);
+            hold(add(vec(p.origin), add(vec(p.u), vec(p.v))), 0.0);
+        }
+    double lo[3], hi[3];
+    for (int x = 0; x < 3; x++) { lo[x] = -HUGE_VAL; hi[x] = HUGE_VAL; }
+    std::vector<DRect> walls;
+    for (DRect q : F.rects) {
+        const int flags = __float_as_int_host(q.b.z), x = flags >> kRectAxisShift;
+        const bool above = q.a.x >= in_hi[x] - F.pad, below = q.a.x <= in_lo[x] + F.pad;
+        if ((flags & kRectEmissive) || above == below) { F.srects.push_back(q); continue; }
+        if (above) hi[x] = std::min(hi[x], (double)q.a.x);
+        else lo[x] = std::max(lo[x], (double)q.a.x);
+        walls.push_back(q);
+    }
+    F.n_inner = (int)F.srects.size();
+    for (DRect& q : F.srects) {
+        // the light's points lie in the cell, away from the walls except
+        // one in its own plane, which any ray meets at the light's t
+        int flags = __float_as_int_host(q.b.z);
+        const int x = flags >> kRectAxisShift, y = x == 0 ? 1 : 0, z = x == 2 ? 1 : 2;
+        auto clear = [&](int k, double c, double h) { return c - h > lo[k] + 4.0 * F.pad && c + h < hi[k] - 4.0 * F.pad; };
+        if ((flags & kRectEmissive) && clear(y, q.a.y, q.b.x) && clear(z, q.a.z, q.b.y) &&
+            (q.a.x == lo[x] || q.a.x == hi[x] || clear(x, q.a.x, 0.0)))
+            flags |= kRectCellLight;
+        q.b.z = __int_as_float_host(flags);
+    }
+    F.srects.insert(F.srects.end(), walls.begin(), walls.end());
+    for (int x = 0; x < 3; x++) {
+        F.cell_lo[x] = (float)(lo[x] + F.pad);
+        F.cell_hi[x] = (float)(hi[x] - F.pad);
     }
     F.ok = true;
     return F;
@@ -735,6 +787,13 @@ int Engine::upload_scene(const pcr_scene_desc& d)
     S.boxes = dupload(flat.boxes, e.allocs, bytes);
     for (int k = 0; k < 3; k++) S.n_rects[k] = flat.n_rects[k];
     S.n_boxes = (int)flat.boxes.size();
+    S.srects = dupload(flat.srects, e.allocs, bytes);
+    S.n_srects = (int)flat.srects.size();
+    S.n_inner = flat.n_inner;
+    for (int k = 0; k < 3; k++) {
+        S.cell_lo[k] = flat.cell_lo[k];
+        S.cell_hi[k] = flat.cell_hi[k];
+    }
     S.flat_ok = flat.ok ? 1 : 0;
     S.flat_pad = flat.pad;
     S.flat_reach = flat.reach;

@@ -79,6 +79,8 @@ struct alignas(16) DLight {
 // a = (plane coordinate p, centre on the two other axes in x y z order, plane
 // index (bits)), b = (half extents on those axes, kRect* flags (bits), 0).
 constexpr int kRectEmissive = 1, kRectSamePlane = 2;  // SamePlane: as the rectangle before it in the list
+constexpr int kRectCellLight = 4;  // emissive, and no wall can lie between it and a point of the cell
+constexpr int kRectAxisShift = 4;  // normal axis
 struct alignas(16) DRect {
     float4 a, b;
 };
@@ -127,6 +129,11 @@ struct DScene {
     const DRect* rects;
     const DBox* boxes;
     int n_rects[3], n_boxes, flat_ok;
+    // The rectangles again for shadow rays, the n_inner that are not walls of
+    // the cell first: between two points of the cell no wall can lie.
+    const DRect* srects;
+    int n_srects, n_inner;
+    float cell_lo[3], cell_hi[3];  // flat_pad inside the walls
     float flat_pad, flat_reach;  // distance margin; largest |origin coordinate| it holds for
 };
 

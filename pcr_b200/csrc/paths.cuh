@@ -26,17 +26,23 @@ namespace pcr {
 // The samples of a path are added up in double and go to the pixel's FP64
 // accumulator once, when the path ends.
 //
-// What bounds it: instruction issue (50 % of the slots; 16 warps per SM at
-// 128 registers, instruction fetches the most frequent stall).  4 blocks per
-// SM without spills beat 5 (96 registers, 180 B of spills) and 6: Cornell
-// 256x256, 16 paths a pixel, 4 vertices, 4 shadow rays: queue stages 4.39 ms,
-// 1.08 ms at 5 blocks, 1.02 ms at 4.  64x64, one path a pixel: 240 -> 98 us.
+// What bounds it: instruction fetch and issue (46 % of the issue slots used, 23
+// of 32 lanes active; 16 warps per SM at 128 registers; waits for instructions
+// are the most frequent stall, as warps are spread over 40 KB of hot code).
+// 4 blocks per SM without spills beat 5 (96 registers, 180 B of spills) and 6.
+// Cornell 256x256, 16 paths a pixel, 4 vertices, 4 shadow rays: queue stages
+// 4.39 ms, first form of this kernel 1.02 ms.  64x64, one path a pixel:
+// 240 -> 98 us.  Refilling at 4 / 12 / 24 / 32 dead lanes: 1015 / 947 / 909 /
+// 900 us, 24 uneven renders 103.6 / 102.7 / 98.3 / 98.3 ms, adaptive rounds
+// 1569 / 1535 / 1537 / 1545 us.  Barriers that keep the warps of 256 or 512
+// threads at the same vertex: glass 4.84 -> 4.44 ms, everything else 2 to 15 %
+// slower.
 constexpr int kPathBlock = 128;
 #ifndef PCR_PATH_MIN_BLOCKS
 #define PCR_PATH_MIN_BLOCKS 4
 #endif
 #ifndef PCR_PATH_REFILL
-#define PCR_PATH_REFILL 12
+#define PCR_PATH_REFILL 24
 #endif
 constexpr int kPathRefill = PCR_PATH_REFILL;
 // A path forks at most once, into at most four sub-paths of which one stays

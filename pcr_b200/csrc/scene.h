@@ -22,6 +22,13 @@ inline float __int_as_float_host(int x)
     return f;
 }
 
+inline int __float_as_int_host(float f)
+{
+    int x;
+    std::memcpy(&x, &f, 4);
+    return x;
+}
+
 struct HostScene {
     std::string name, version;
     float cam[3] = {0, 0, 0};
