@@ -788,38 +788,41 @@ __device__ __forceinline__ bool scene_blocked(const DScene& S, const DMaterial* 
 // The stage functions below use the exact (never-contracted) ops: the
 // sigmoid 0.5 + p / (2 sqrt(1 + p^2)) cancels for strongly negative p, where
 // a fused multiply-add would move the result by more than 1e-5 relative.
+//
+// kVisible: lambda lies in 400..700 nm, as every wavelength a path carries
+// does.  The divisions by 150 and 5 are then Markstein's: with y the rounded
+// reciprocal of c, q = x y, r = x - q c (exact by one fused multiply-add),
+// q + r y is x / c correctly rounded (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990; equal to the
+// division for every float in 400..700).
+template <bool kVisible>
+__device__ __forceinline__ float div_const(float x, float c)
+{
+    if (!kVisible) return ex::div(x, c);
+    const float y = 1.f / c, q = ex::mul(x, y);
+    return fmaf(fmaf(-q, c, x), y, q);
+}
+template <bool kVisible>
 __device__ __forceinline__ float sigmoid_fit(float4 f, float lambda)
 {
     // RGBToSpectrum::evalSigmoidFit (code/Includes/RGBToSpectrum.h:118-125)
     using namespace ex;
-    float L = div(sub(lambda, 550.f), 150.f);
+    float L = div_const<kVisible>(sub(lambda, 550.f), 150.f);
     float p = add(f.x, mul(L, add(f.y, mul(L, f.z))));
     return mul(add(0.5f, div(p, mul(2.f, __fsqrt_rn(add(1.f, mul(p, p)))))), f.w);
 }
 
+template <bool kVisible>
 __device__ __forceinline__ float spectrum_lerp(const float* s, float lambda)
 {
     // Spectrum::operator() (code/Includes/Spectrum.h:82-90)
     using namespace ex;
-    if (lambda < 400.f || lambda > 700.f) return 0.f;
-    float t = div(sub(lambda, 400.f), 5.0f);
+    if (!kVisible && (lambda < 400.f || lambda > 700.f)) return 0.f;
+    float t = div_const<kVisible>(sub(lambda, 400.f), 5.0f);
     int i = (int)t;
     if (i >= kSpecN - 1) return s[kSpecN - 1];
     float f = sub(t, (float)i);
     return add(mul(s[i], sub(1.f, f)), mul(s[i + 1], f));
-}
-
-// Material::albedoAt / emissiveAt (code/Includes/Material.h:92-101)
-__device__ __forceinline__ float albedo_at(const DMaterial& m, float lambda)
-{
-    if (m.flags & kMatTabA) return spectrum_lerp(m.tabA, lambda);
-    float v = sigmoid_fit(m.afit, lambda);
-    return v > 1.f ? 1.f : v;
-}
-__device__ __forceinline__ float emissive_at(const DMaterial& m, float lambda)
-{
-    if (m.flags & kMatTabE) return spectrum_lerp(m.tabE, lambda);
-    return sigmoid_fit(m.efit, lambda);
 }
 
 // Wyman-Sloan-Shirley piecewise Gaussians (code/Includes/CIE.h:27-53)

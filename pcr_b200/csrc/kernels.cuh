@@ -275,20 +275,16 @@ __device__ __forceinline__ float4 rgb4(float4 c) { return make_float4(c.x, c.y, 
 // instruction footprint small.
 __device__ __noinline__ float4 spec4(const DMaterial& m, int emissive, float4 lam)
 {
-    const bool tab = (m.flags & (emissive ? kMatTabE : kMatTabA)) != 0;
-    const float* table = emissive ? m.tabE : m.tabA;
-    const float4 fit = emissive ? m.efit : m.afit;
-    float v[4];
-    const float l[4] = {lam.x, lam.y, lam.z, lam.w};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        float x = tab ? spectrum_lerp(table, l[k]) : sigmoid_fit(fit, l[k]);
-        if (!emissive && !tab && x > 1.f) x = 1.f;
-        v[k] = x;
+    if (m.flags & (emissive ? kMatTabE : kMatTabA)) {
+        const float* table = emissive ? m.tabE : m.tabA;
+        return make_float4(spectrum_lerp<true>(table, lam.x), spectrum_lerp<true>(table, lam.y),
+                           spectrum_lerp<true>(table, lam.z), spectrum_lerp<true>(table, lam.w));
     }
-    return make_float4(v[0], v[1], v[2], v[3]);
+    const float4 fit = emissive ? m.efit : m.afit;
+    const float4 v = make_float4(sigmoid_fit<true>(fit, lam.x), sigmoid_fit<true>(fit, lam.y), sigmoid_fit<true>(fit, lam.z),
+                                 sigmoid_fit<true>(fit, lam.w));
+    return emissive ? v : make_float4(v.x > 1.f ? 1.f : v.x, v.y > 1.f ? 1.f : v.y, v.z > 1.f ? 1.f : v.z, v.w > 1.f ? 1.f : v.w);
 }
-
 
 // ------------------------------------------------------------------ regen
 // Camera rays for the new paths (code/Renderer.cpp:190-239): pixel centre,
@@ -299,24 +295,48 @@ struct CameraPath {
     float lambda0;
 };
 
+// 300 nm / n for n = 1..4 wavelengths (all exact)
+__device__ __forceinline__ float wavelength_stride(int n)
+{
+    return n == 4 ? 75.f : (n == 3 ? 100.f : (n == 2 ? 150.f : 300.f));
+}
+
+// Pixel (returned) and local sample of a path number past 2^32.
+__device__ __noinline__ uint32_t split_path(long long path, uint32_t per_pixel, uint32_t& q)
+{
+    const long long px = path / (long long)per_pixel;
+    q = (uint32_t)(path - px * (long long)per_pixel);
+    return (uint32_t)px;
+}
+
 // Path number `path` of request R; W receives the XYZ weights of a spectral
 // path's wavelengths (left alone otherwise).
 __device__ __forceinline__ CameraPath camera_path(const EngineView& E, const DRequest& R, long long path, float xyz_scale,
                                                   XyzWeights& W)
 {
     CameraPath p;
-    if (R.flags & kReqAdaptive) {
-        // round r: spp paths for each pixel still in the round's list;
-        // sample numbers r*spp.. as in the non-adaptive order
-        const long long q = path - R.round_base;
-        p.pixel = (uint32_t)R.act[R.round & 1][q / R.spp];
-        p.sample = (uint32_t)(R.round * R.spp + (int)(q % R.spp));
+    const bool adaptive = R.flags & kReqAdaptive;
+    // adaptive round r: spp paths for each pixel still in the round's list
+    const long long at = adaptive ? path - R.round_base : path;
+    const uint32_t per = (uint32_t)(adaptive ? R.spp : R.paths_per_pixel);
+    uint32_t q;
+    if ((at >> 32) == 0) {
+        p.pixel = (uint32_t)at / per;
+        q = (uint32_t)at - p.pixel * per;
     } else {
-        p.pixel = (uint32_t)(path / R.paths_per_pixel);
-        const int q = (int)(path % R.paths_per_pixel);  // local sample
-        p.sample = (uint32_t)((q / R.local_spp) * R.spp + R.sample0 + q % R.local_spp);
+        p.pixel = split_path(at, per, q);
     }
-    const int px = (int)(p.pixel % (uint32_t)R.width), py = (int)(p.pixel / (uint32_t)R.width);
+    if (adaptive) {
+        // sample numbers r*spp.. as in the non-adaptive order
+        p.pixel = (uint32_t)R.act[R.round & 1][p.pixel];
+        p.sample = (uint32_t)R.round * (uint32_t)R.spp + q;
+    } else if (R.local_spp == R.spp) {
+        p.sample = q;
+    } else {  // local sample q of a sample range
+        const uint32_t round = q / (uint32_t)R.local_spp;
+        p.sample = round * (uint32_t)(R.spp - R.local_spp) + (uint32_t)R.sample0 + q;
+    }
+    const int py = (int)(p.pixel / (uint32_t)R.width), px = (int)p.pixel - py * R.width;
     float jx = 0.f, jy = 0.f;
     if (R.aa > 1) {
         float4 j = rand4(R, p.pixel, p.sample / (uint32_t)R.spp, 0, 254u, 0);
@@ -334,7 +354,7 @@ __device__ __forceinline__ CameraPath camera_path(const EngineView& E, const DRe
         const int nch = R.hero;
         // hero wavelength and its stratified companions (code/Renderer.cpp:227-239)
         float lam[4];
-        const float span = 300.f, stride_l = span / (float)nch;
+        const float span = 300.f, stride_l = wavelength_stride(nch);
         lam[0] = p.lambda0;
 #pragma unroll
         for (int k = 1; k < 4; k++) {
@@ -458,7 +478,7 @@ __device__ __forceinline__ void add_xyz(double* acc, float3 c)
 __device__ __forceinline__ float4 path_wavelengths(float l0, int single, int nHero)
 {
     if (single) return make_float4(l0, l0, l0, l0);
-    const float span = 300.f, stride_l = span / (float)nHero;
+    const float span = 300.f, stride_l = wavelength_stride(nHero);
     float l1 = l0 + stride_l * 1, l2 = l0 + stride_l * 2, l3 = l0 + stride_l * 3;
     if (l1 > 700.f) l1 -= span;
     if (l2 > 700.f) l2 -= span;
@@ -1247,8 +1267,8 @@ __global__ void k_eval_stage(int what, const float* __restrict__ params, const f
 {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         switch (what) {
-        case 0: out[i] = sigmoid_fit(make_float4(params[0], params[1], params[2], params[3]), in[i]); break;
-        case 1: out[i] = spectrum_lerp(params, in[i]); break;
+        case 0: out[i] = sigmoid_fit<false>(make_float4(params[0], params[1], params[2], params[3]), in[i]); break;
+        case 1: out[i] = spectrum_lerp<false>(params, in[i]); break;
         case 2: { float3 c = cmf(in[i]); out[i * 3] = c.x; out[i * 3 + 1] = c.y; out[i * 3 + 2] = c.z; } break;
         case 3: {
             float3 c = cmf(in[i * 2]);
