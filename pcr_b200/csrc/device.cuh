@@ -595,6 +595,15 @@ __device__ __forceinline__ uint32_t scene_analytic(const DScene& S, float3 o, fl
     return scene_analytic_exact(S, o, d, closest);
 }
 
+// Whether the mesh can hold a hit closer than `closest`: the padded box test
+// of the plane groups, on the mesh's box.
+__device__ __forceinline__ bool mesh_may_hit(const DScene& S, float3 o, float3 d, float closest)
+{
+    if (S.n_nodes <= 0) return false;
+    const float3 rd = make_float3(rcp_approx(d.x), rcp_approx(d.y), rcp_approx(d.z));
+    return group_may_hit(S.mesh_lo, S.mesh_hi, o, d, rd, closest);
+}
+
 // Renderer::sceneIntersect: the analytic primitives, then the triangle BVH.
 // Returns the primitive code; t and barycentrics through refs.
 __device__ __forceinline__ uint32_t scene_closest(const DScene& S, float3 o, float3 d, float tmax, float& t, float& hu,

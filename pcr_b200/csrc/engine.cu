@@ -768,6 +768,21 @@ int Engine::upload_scene(const pcr_scene_desc& d)
     S.light_tris = dupload(ltris, e.allocs, bytes);
     S.light_flatn = dupload(lflat, e.allocs, bytes);
     S.light_cum = dupload(lcum, e.allocs, bytes);
+    // The mesh's box, padded as the plane groups' are; a scene without a mesh
+    // has an empty one.
+    {
+        float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX}, big = 1.f;
+        for (int i = 0; i < d.n_triangles; i++)
+            for (const float* v : {tris[i].v0, tris[i].v1, tris[i].v2})
+                for (int k = 0; k < 3; k++) {
+                    lo[k] = std::min(lo[k], v[k]);
+                    hi[k] = std::max(hi[k], v[k]);
+                    big = std::max(big, std::fabs(v[k]));
+                }
+        const float pad = 1e-4f * big;
+        S.mesh_lo = make_float4(lo[0] - pad, lo[1] - pad, lo[2] - pad, 0.f);
+        S.mesh_hi = make_float4(hi[0] + pad, hi[1] + pad, hi[2] + pad, 0.f);
+    }
     const std::vector<float4> pgroups = plane_groups(d.planes, d.n_planes);
     S.pgroups = dupload(pgroups, e.allocs, bytes);
     S.n_pgroups = (int)pgroups.size() / 2;
@@ -1056,7 +1071,7 @@ int Engine::active_stages() const
 void Engine::launch_iteration(int cur, int stages, bool prof)
 {
     const EngineView E = view();
-    const int B = tune_.block_size;
+    const int B = trace_block();
     // stage index: 0 regen 1 extend 2 shade 3 shadow 4 resolve 5 schedule 6 status (and k_round) 7 other (k_paths)
     int done = 0;
     int stage_of[8];
@@ -1115,7 +1130,7 @@ static void raise_shade_smem(size_t bytes)
 
 void Engine::launch_shapes()
 {
-    const int B = tune_.block_size;
+    const int B = trace_block();
     // materials staged in shared memory when they fit
     const size_t mat_bytes = sizeof(DMaterial) * (size_t)std::max(1, mat_count_);
     smem_mats_ = mat_bytes <= 96 * 1024 ? 1 : 0;
@@ -1904,7 +1919,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
         CK(cudaGetLastError());
 
         // launch shapes from the occupancy calculator (no allocation involved)
-        const int B = tune_.block_size;
+        const int B = trace_block();
         const size_t mat_bytes = sizeof(DMaterial) * (size_t)std::max(1, mat_count_);
         const int smem_mats = mat_bytes <= 96 * 1024 ? 1 : 0;
         const size_t smem = smem_mats ? mat_bytes : 0;

@@ -124,6 +124,7 @@ private:
     void launch_iteration(int cur, int stages, bool profile);
     void launch_block(int stages);
     void launch_shapes();
+    int trace_block() const { return (tune_.block_size + 31) / 32 * 32; }  // whole warps
     void drop_graphs();
     void trace_whole(const EngineView& E, const DRequest& R, int grid);
     void render_whole(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats* st);

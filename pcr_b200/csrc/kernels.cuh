@@ -433,25 +433,73 @@ __device__ __forceinline__ void prefetch_l2(const void* p)
 #endif
 constexpr int kTraceMaxBlock = 256, kTraceMinBlocks = PCR_TRACE_MIN_BLOCKS, kShadowMinBlocks = PCR_SHADOW_MIN_BLOCKS;
 
+// Rays of a warp that have a mesh to walk.  Many rays miss the mesh's box;
+// walked where they stand, the others left 9 of 32 lanes active.  So each warp
+// first runs the analytic tests and the box test for its rays, keeps those
+// that go on in shared memory, and walks the BVH whenever 32 of them have come
+// together (14 to 16 lanes active over the whole kernel).  Six mesh renders
+// batched: k_extend 11.0 -> 8.5 ms, k_shadow 9.3 -> 6.1 ms; 24 uneven renders
+// 14.0 -> 7.7 and 24.9 -> 18.3 ms.
+struct WalkQueue {
+    int ray[64];
+    float t[64];
+    uint32_t prim[64];
+};
+
 // Closest hit for every queued path (trace_closest).
 __global__ void __launch_bounds__(kTraceMaxBlock, kTraceMinBlocks) k_extend(EngineView E, int cur)
 {
+    __shared__ WalkQueue s_walk[kTraceMaxBlock / 32];
+    WalkQueue& W = s_walk[threadIdx.x >> 5];
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
     const Counters* C = E.cnt;
     const int n = min(C->queue_n[cur], E.queue_cap);
     const PathQueue Q = E.q[cur];
-    unsigned long long mine = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int nx = i + gridDim.x * blockDim.x;
+    const int stride = gridDim.x * blockDim.x;
+    unsigned mine = 0;
+    int pending = 0;
+    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
+        const int i = base + lane, nx = i + stride;
         if (nx < n) { prefetch_l2(Q.o + nx); prefetch_l2(Q.d + nx); prefetch_l2(Q.id + nx); }
-        const DScene& S = E.scenes[Q.id[i].w];
-        float4 o = Q.o[i], d = Q.d[i];
-        float t = FLT_MAX, u = 0.f, v = 0.f;
-        uint32_t prim = scene_closest(S, xyz(o), xyz(d), FLT_MAX, t, u, v);
-        E.hit[i] = make_float4(t, __uint_as_float(prim), u, v);
-        mine++;
+        bool walk = false;
+        float t = FLT_MAX;
+        uint32_t prim = kPrimNone;
+        if (i < n) {
+            const DScene& S = E.scenes[Q.id[i].w];
+            const float3 o = xyz(Q.o[i]), d = xyz(Q.d[i]);
+            prim = scene_analytic(S, o, d, t);
+            walk = mesh_may_hit(S, o, d, t);
+            if (!walk) E.hit[i] = make_float4(t, __uint_as_float(prim), 0.f, 0.f);
+            mine++;
+        }
+        const unsigned m = __ballot_sync(kAll, walk);
+        if (walk) {
+            const int k = pending + __popc(m & ((1u << lane) - 1u));
+            W.ray[k] = i;
+            W.t[k] = t;
+            W.prim[k] = prim;
+        }
+        pending += __popc(m);
+        __syncwarp();
+        const bool last = base >= n - stride;
+        while (pending >= 32 || (last && pending > 0)) {
+            const int first = max(0, pending - 32), k = first + lane;
+            if (k < pending) {
+                const int r = W.ray[k];
+                const DScene& S = E.scenes[Q.id[r].w];
+                float u = 0.f, v = 0.f, c = W.t[k];
+                const int tri = bvh4_closest<false>(S, xyz(Q.o[r]), xyz(Q.d[r]), c, u, v, nullptr);
+                const uint32_t p = tri >= 0 ? kPrimTri | (uint32_t)tri : W.prim[k];
+                E.hit[r] = make_float4(c, __uint_as_float(p), u, v);
+            }
+            pending = first;
+            __syncwarp();
+        }
+        if (last) break;
     }
-    for (int off = 16; off > 0; off >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, off);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&E.cnt->rays, mine);
+    mine = __reduce_add_sync(kAll, mine);
+    if (lane == 0 && mine) atomicAdd(&E.cnt->rays, (unsigned long long)mine);
 }
 
 // ------------------------------------------------------------------ helpers
@@ -1016,32 +1064,66 @@ __global__ void __launch_bounds__(kShadeBlock, PCR_SHADE_MIN_BLOCKS) k_shade(Eng
 // 1e-3 (compared in double, as the reference's double literal promotes it);
 // scene_blocked answers it with an early exit.  Lit samples add their XYZ
 // contribution to the pixel's FP64 accumulator.
+__device__ __forceinline__ void add_lit(const EngineView& E, int i)
+{
+    const float4 c = E.sq.c[i];
+    const int pixel = __float_as_int(E.sq.d[i].w);
+    add_xyz(E.reqs[__float_as_int(c.w) & 0xFFFF].accum + (size_t)pixel * 3, make_float3(c.x, c.y, c.z));
+}
 __global__ void __launch_bounds__(kTraceMaxBlock, kShadowMinBlocks) k_shadow(EngineView E)
 {
+    __shared__ WalkQueue s_walk[kTraceMaxBlock / 32];  // t: the query's bound
+    WalkQueue& W = s_walk[threadIdx.x >> 5];
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
     Counters* C = E.cnt;
     const int n = min(C->shadow_n, E.shadow_cap);
     const ShadowQueue SQ = E.sq;
+    const int stride = gridDim.x * blockDim.x;
     unsigned mine = 0;  // shadow rays of this thread (one launch: < 2^32)
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int nx = i + gridDim.x * blockDim.x;
+    int pending = 0;
+    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
+        const int i = base + lane, nx = i + stride;
         if (nx < n) { prefetch_l2(SQ.o + nx); prefetch_l2(SQ.d + nx); prefetch_l2(SQ.c + nx); }
-        const float4 o = SQ.o[i];
-        if (!(o.w >= 0.f)) continue;  // skip record (zero geometry term)
-        const float4 d = SQ.d[i];
-        // only the scene is needed for the query; the contribution is read
-        // afterwards, for lit samples, so it holds no registers across it
-        const DScene& S = E.scenes[__float_as_int(SQ.c[i].w) >> 16];
-        const float d2 = o.w;
-        mine++;
-        if (!scene_blocked(S, E.mats, xyz(o), xyz(d), d2)) {
-            const float4 c = SQ.c[i];
-            const int pixel = __float_as_int(SQ.d[i].w);
-            add_xyz(E.reqs[__float_as_int(c.w) & 0xFFFF].accum + (size_t)pixel * 3, make_float3(c.x, c.y, c.z));
+        bool walk = false;
+        float bound = 0.f;
+        if (i < n) {
+            const float4 o = SQ.o[i];
+            if (o.w >= 0.f) {  // else a skip record (zero geometry term)
+                const float4 d = SQ.d[i];
+                const DScene& S = E.scenes[__float_as_int(SQ.c[i].w) >> 16];
+                mine++;
+                const int r = scene_blocked_analytic<true>(S, E.mats, xyz(o), xyz(d), o.w, bound);
+                walk = r == kShadowWalk && mesh_may_hit(S, xyz(o), xyz(d), bound);
+                if (r != kShadowBlocked && !walk) add_lit(E, i);
+            }
         }
+        const unsigned m = __ballot_sync(kAll, walk);
+        if (walk) {
+            const int k = pending + __popc(m & ((1u << lane) - 1u));
+            W.ray[k] = i;
+            W.t[k] = bound;
+        }
+        pending += __popc(m);
+        __syncwarp();
+        const bool last = base >= n - stride;
+        while (pending >= 32 || (last && pending > 0)) {
+            const int first = max(0, pending - 32), k = first + lane;
+            if (k < pending) {
+                const int r = W.ray[k];
+                const float4 o = SQ.o[r];
+                const DScene& S = E.scenes[__float_as_int(SQ.c[r].w) >> 16];
+                float c = W.t[k], u, v;
+                if (bvh4_closest<false, true>(S, xyz(o), xyz(SQ.d[r]), c, u, v, nullptr, (double)o.w - 1e-3) != -2)
+                    add_lit(E, r);
+            }
+            pending = first;
+            __syncwarp();
+        }
+        if (last) break;
     }
-    unsigned long long warp_rays = mine;
-    for (int off = 16; off > 0; off >>= 1) warp_rays += __shfl_down_sync(0xffffffffu, warp_rays, off);
-    if ((threadIdx.x & 31) == 0 && warp_rays) atomicAdd(&C->shadow_rays, warp_rays);
+    mine = __reduce_add_sync(kAll, mine);
+    if (lane == 0 && mine) atomicAdd(&C->shadow_rays, (unsigned long long)mine);
 }
 
 // ------------------------------------------------------------------ status

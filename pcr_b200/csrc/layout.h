@@ -111,6 +111,7 @@ struct DScene {
     // query (which tests emissive planes separately and needs no tie order).
     const DPlane* splanes;
     const float4* sgroups;
+    float4 mesh_lo, mesh_hi;  // padded box of the triangle mesh
     int n_planes, n_spheres, n_nodes, n_tris, n_lights, mat_base, n_mats, n_pgroups;
     int n_sgroups;
     int emissive_tris;        // 1 when any triangle's material is emissive
