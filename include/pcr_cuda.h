@@ -95,11 +95,10 @@ typedef struct {
     uint64_t seed;           /* 0 -> 1 */
     int32_t priority;        /* batched / served: pending requests are admitted lowest value
                               * first, in submit order among equals (0 default) */
-    /* plain method on scenes with a triangle mesh: 0 = one sample per pixel per
-     * pass, the reference wavefront's default
-     * (code/Includes/GpuDefaults.h:44-50); 1 = passes as large as the queue
-     * (wavefrontMultiSample).  Other scenes are traced path by path, without
-     * passes.  The image is the same either way. */
+    /* The reference wavefront's choice between passes of one sample per pixel
+     * (0, code/Includes/GpuDefaults.h:44-50) and larger ones
+     * (wavefrontMultiSample).  Paths are taken from a common counter here, so
+     * neither changes the image nor the work; kept for callers that set it. */
     int32_t multi_sample;
     /* Sample range [sample_begin, sample_end) of `samples` (0, 0 = all).  A
      * render split across GPUs gives each one a range; the HDR images are

@@ -190,7 +190,6 @@ void Engine::alloc_buffers()
     d_tdone_ = dalloc<unsigned long long>(kMaxActive, T);
     d_outstanding_ = dalloc<long long>(kMaxActive, T);
     d_give_start_ = dalloc<long long>(kMaxActive, T);
-    d_give_ = dalloc<int>(kMaxActive, T);
     d_give_base_ = dalloc<int>(kMaxActive, T);
     d_path_base_ = dalloc<int>(kMaxActive, T);
     d_active_ = dalloc<int>(kMaxActive, T);
@@ -231,12 +230,13 @@ void Engine::alloc_buffers()
         q_[b].tp = dalloc<float4>(queue_cap_, T);
         q_[b].id = dalloc<int4>(queue_cap_, T);
         for (int k = 0; k < 3; k++) q_[b].w[k] = dalloc<float4>(queue_cap_, T);
+        q_[b].hit = dalloc<float4>(queue_cap_, T);
     }
-    d_hit_ = dalloc<float4>(queue_cap_, T);
     sq_.o = dalloc<float4>(shadow_cap_, T);
     sq_.d = dalloc<float4>(shadow_cap_, T);
     sq_.c = dalloc<float4>(shadow_cap_, T);
-    EngineParams p{fill, tune_.chunk_paths, tune_.regen_every, 0};
+    sq_.bound = dalloc<float>(shadow_cap_, T);
+    EngineParams p{fill, tune_.chunk_paths, tune_.regen_every};
     CK(cudaMemcpy(d_params_, &p, sizeof(p), cudaMemcpyHostToDevice));
     graph_dirty_ = true;
 }
@@ -295,7 +295,6 @@ EngineView Engine::view() const
     E.reqs = d_reqs_;
     E.issued = d_issued_;
     E.outstanding = d_outstanding_;
-    E.give = d_give_;
     E.give_base = d_give_base_;
     E.path_base = d_path_base_;
     E.active = d_active_;
@@ -306,12 +305,10 @@ EngineView Engine::view() const
     E.cnt = d_cnt_;
     E.q[0] = q_[0];
     E.q[1] = q_[1];
-    E.hit = d_hit_;
     E.sq = sq_;
     E.give_start = d_give_start_;
-    E.shadow_cap = shadow_cap_;
+    E.shadow_cap = std::min(shadow_cap_, INT32_MAX - (1 << 22));  // shadow_slots may count past it
     E.queue_cap = queue_cap_;
-    E.n_mats = mat_count_;
     E.round_state = d_round_state_;
     E.round_cnt = d_round_cnt_;
     E.round_list = d_round_list_;
@@ -935,8 +932,8 @@ void Engine::ensure_shadow_capacity(int shadow_samples)
                                             " paths in flight exceed the 2^31-record shadow queue; use a smaller "
                                             "queue capacity");
     CK(cudaStreamSynchronize(stream_));
-    for (float4* p : {sq_.o, sq_.d, sq_.c}) {
-        auto it = std::find(qallocs_.begin(), qallocs_.end(), (void*)p);
+    for (void* p : {(void*)sq_.o, (void*)sq_.d, (void*)sq_.c, (void*)sq_.bound}) {
+        auto it = std::find(qallocs_.begin(), qallocs_.end(), p);
         if (it != qallocs_.end()) qallocs_.erase(it);
         CK(cudaFree(p));
     }
@@ -944,13 +941,14 @@ void Engine::ensure_shadow_capacity(int shadow_samples)
     sq_.o = dalloc<float4>(shadow_cap_, qallocs_);
     sq_.d = dalloc<float4>(shadow_cap_, qallocs_);
     sq_.c = dalloc<float4>(shadow_cap_, qallocs_);
+    sq_.bound = dalloc<float>(shadow_cap_, qallocs_);
     graph_dirty_ = true;
 }
 
 int64_t Engine::submit(int scene, const pcr_render_desc& desc)
 {
     validate(scene, desc);
-    if (!traced_whole(scene) && (int64_t)queue_cap_ * desc.shadow_samples > shadow_cap_) {
+    if (!flat(scene) && (int64_t)queue_cap_ * desc.shadow_samples > shadow_cap_) {
         std::lock_guard<std::mutex> g(run_mu_);
         ensure_shadow_capacity(desc.shadow_samples);
     }
@@ -1063,16 +1061,17 @@ int Engine::active_stages() const
     int m = 0;
     for (int slot : active_slots_) {
         auto it = reqs_.find(slot_owner_[slot]);
-        if (it != reqs_.end()) m |= traced_whole(it->second->scene) ? kStagesPaths : kStagesQueue;
+        if (it != reqs_.end()) m |= flat(it->second->scene) ? kStagesFlat : kStagesMesh;
     }
-    return m ? m : kStagesQueue;
+    return m ? m : kStagesMesh;
 }
 
 void Engine::launch_iteration(int cur, int stages, bool prof)
 {
     const EngineView E = view();
     const int B = trace_block();
-    // stage index: 0 regen 1 extend 2 shade 3 shadow 4 resolve 5 schedule 6 status (and k_round) 7 other (k_paths)
+    // stage index: 1 extend 2 shade (k_paths on mesh scenes) 3 shadow 5 schedule 6 status (and k_round)
+    // 7 other (k_paths on scenes without a mesh)
     int done = 0;
     int stage_of[8];
     auto mark = [&](int stage) {  // the stage just launched ends here
@@ -1084,18 +1083,16 @@ void Engine::launch_iteration(int cur, int stages, bool prof)
     if (prof) CK(cudaEventRecord(prof_ev_[0], stream_));
     k_schedule<<<1, kSchedThreads, 0, stream_>>>(E, (const EngineParams*)d_params_, cur);
     mark(5);
-    if (stages & kStagesQueue) {
-        k_regen<<<grid_regen_, B, 0, stream_>>>(E, cur, xyz_scale_);
-        mark(0);
-        k_extend<<<grid_extend_, B, 0, stream_>>>(E, cur);
-        mark(1);
-        k_shade<<<grid_shade_, kShadeBlock, shade_smem_, stream_>>>(E, cur, smem_mats_);
+    if (stages & kStagesMesh) {
+        k_paths<true><<<grid_mesh_, kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
         mark(2);
+        k_extend<<<grid_extend_, B, 0, stream_>>>(E, cur ^ 1);
+        mark(1);
         k_shadow<<<grid_shadow_, B, 0, stream_>>>(E);
         mark(3);
     }
-    if (stages & kStagesPaths) {
-        k_paths<<<grid_paths_, kPathBlock, kPathSmem, stream_>>>(E, xyz_scale_);
+    if (stages & kStagesFlat) {
+        k_paths<false><<<grid_flat_, kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
         mark(7);
     }
     k_status<<<1, 1024, 0, stream_>>>(E, cur ^ 1);
@@ -1114,33 +1111,13 @@ void Engine::launch_iteration(int cur, int stages, bool prof)
     iterations_++;
 }
 
-// k_shade's limit on dynamic shared memory is one attribute of the function
-// on the current device, shared by every context of the process.  It is only
-// ever raised: a context with a smaller material table must not lower it
-// below the size another context's launches (or captured graph) use.
-static void raise_shade_smem(size_t bytes)
-{
-    static std::mutex mu;
-    std::lock_guard<std::mutex> g(mu);
-    cudaFuncAttributes a{};
-    CK(cudaFuncGetAttributes(&a, (const void*)k_shade));
-    if ((int)bytes > a.maxDynamicSharedSizeBytes)
-        CK(cudaFuncSetAttribute((const void*)k_shade, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-}
-
 void Engine::launch_shapes()
 {
     const int B = trace_block();
-    // materials staged in shared memory when they fit
-    const size_t mat_bytes = sizeof(DMaterial) * (size_t)std::max(1, mat_count_);
-    smem_mats_ = mat_bytes <= 96 * 1024 ? 1 : 0;
-    shade_smem_ = smem_mats_ ? mat_bytes : 0;
-    raise_shade_smem(shade_smem_);
-    grid_for((const void*)k_regen, B, 0, &grid_regen_);
     grid_for((const void*)k_extend, B, 0, &grid_extend_);
-    grid_for((const void*)k_shade, kShadeBlock, shade_smem_, &grid_shade_);
     grid_for((const void*)k_shadow, B, 0, &grid_shadow_);
-    grid_for((const void*)k_paths, kPathBlock, kPathSmem, &grid_paths_);
+    grid_for((const void*)k_paths<false>, kPathBlock, kPathSmem, &grid_flat_);
+    grid_for((const void*)k_paths<true>, kPathBlock, kPathSmem, &grid_mesh_);
     grid_round_ = sms_ * 2;  // a round's per-pixel step is light; an idle launch reads one word
     drop_graphs();
     graph_dirty_ = false;
@@ -1177,9 +1154,9 @@ void Engine::launch_block(int stages)
         CK(cudaGraphLaunch(graphs_[stages], stream_));
         stage_launches_[5] += tune_.iters_per_launch;
         stage_launches_[6] += 2 * tune_.iters_per_launch;
-        if (stages & kStagesQueue)
-            for (int k : {0, 1, 2, 3}) stage_launches_[k] += tune_.iters_per_launch;
-        if (stages & kStagesPaths) stage_launches_[7] += tune_.iters_per_launch;
+        if (stages & kStagesMesh)
+            for (int k : {1, 2, 3}) stage_launches_[k] += tune_.iters_per_launch;
+        if (stages & kStagesFlat) stage_launches_[7] += tune_.iters_per_launch;
         iterations_ += tune_.iters_per_launch;
     } else {
         for (int it = 0; it < tune_.iters_per_launch; it++) launch_iteration(it & 1, stages, profile_);
@@ -1597,13 +1574,13 @@ double Engine::progress(int64_t id)
 // at most kPathsPerLaunch paths, so that other work of the device gets its
 // turn within about a tenth of a second.
 constexpr int64_t kPathsPerLaunch = 1 << 26;
-void Engine::trace_whole(const EngineView& E, const DRequest& R, int grid)
+void Engine::trace_flat(const EngineView& E, const DRequest& R, int grid)
 {
     for (int64_t at = 0; at < R.total; at += kPathsPerLaunch) {
         const int n = (int)std::min<int64_t>(kPathsPerLaunch, R.total - at);
         k_one_request<<<1, 1, 0, stream_>>>(E, R, at, n);
         if (profile_) CK(cudaEventRecord(prof_ev_[0], stream_));
-        k_paths<<<std::min(grid, (n + kPathBlock - 1) / kPathBlock), kPathBlock, kPathSmem, stream_>>>(E, xyz_scale_);
+        k_paths<false><<<std::min(grid, (n + kPathBlock - 1) / kPathBlock), kPathBlock, kPathSmem, stream_>>>(E, 0, xyz_scale_);
         CK(cudaGetLastError());
         if (profile_) record_other(prof_ev_[0], prof_ev_[1]);
         else stage_launches_[7]++;
@@ -1612,11 +1589,11 @@ void Engine::trace_whole(const EngineView& E, const DRequest& R, int grid)
 }
 
 // Plain render of a scene without a mesh: one k_paths launch, resolve, copy.
-void Engine::render_whole(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats* st)
+void Engine::render_flat(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats* st)
 {
     alloc_request(r);
     const DRequest R = make_request(r.desc, r.scene, r.accum);
-    trace_whole(view(), R, grid_paths_);
+    trace_flat(view(), R, grid_flat_);
     active_dirty_ = true;  // the active list holds slot 0
     CK(cudaMemcpyAsync(h_cnt_, d_cnt_, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
     finish_request(r, stream_);
@@ -1660,30 +1637,28 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     r.bytes = request_bytes(desc);
     if (r.bytes > budget_) throw PcrError(PCR_ERR_NO_MEMORY, "request larger than the device memory budget");
     if (graph_dirty_) launch_shapes();
-    if (traced_whole(scene)) {
-        render_whole(r, hdr, rgb, st);
+    if (flat(scene)) {
+        render_flat(r, hdr, rgb, st);
         if (st) st->latency_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         return;
     }
     ensure_shadow_capacity(desc.shadow_samples);
     if (graph_dirty_) launch_shapes();
-    // a pass holds one sample per pixel (W*H paths) unless multi_sample asks
-    // for passes as large as the queue; no refill until a pass has drained
     const int64_t px = (int64_t)desc.width * desc.height;
-    const int pass = desc.multi_sample ? tune_.queue_capacity : (int)std::min<int64_t>(px, tune_.queue_capacity);
-    EngineParams p{pass, pass, 1, 1};
+    EngineParams p{tune_.queue_capacity, tune_.queue_capacity, 1};
     k_set_params<<<1, 1, 0, stream_>>>((EngineParams*)d_params_, p);
     activate(r, 0);
     slot_owner_[0] = -1;  // the plain request is not in the request map
     upload_active();
     const int64_t total = px * local_spp(desc) * std::max(1, desc.aa_samples);
-    const int64_t passes = (total + pass - 1) / pass;
+    const int64_t fills = (total + tune_.queue_capacity - 1) / tune_.queue_capacity;
     int cur = 0;
-    for (int64_t it = 0; it < passes * (int64_t)desc.depth; it++) {
-        launch_iteration(cur, kStagesQueue, profile_);
+    // a path waits for the mesh at most `depth` times
+    for (int64_t it = 0; it < fills + desc.depth; it++) {
+        launch_iteration(cur, kStagesMesh, profile_);
         cur ^= 1;
     }
-    int extra = 0;
+    int64_t extra = 0;
     while (true) {
         int done = 0;
         CK(cudaMemcpyAsync(&done, d_done_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
@@ -1692,13 +1667,13 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
         CK(cudaMemcpy(&c, d_cnt_, sizeof(c), cudaMemcpyDeviceToHost));
         if (c.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "device reported queue overflow");
         if (done) break;
-        if (++extra > 4 * desc.depth + 8) throw PcrError(PCR_ERR_TIMEOUT, "plain render did not finish");
-        launch_iteration(cur, kStagesQueue, profile_);
+        if (++extra > fills * (4 * (int64_t)desc.depth + 8)) throw PcrError(PCR_ERR_TIMEOUT, "plain render did not finish");
+        launch_iteration(cur, kStagesMesh, profile_);
         cur ^= 1;
     }
     // a plain render always ends on queue parity 0 for the next user
     if (cur != 0) {
-        launch_iteration(cur, kStagesQueue, false);
+        launch_iteration(cur, kStagesMesh, false);
         cur ^= 1;
     }
     unsigned long long tf = 0, td = 0;
@@ -1709,7 +1684,7 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     active_dirty_ = true;
     bytes_in_use_ -= r.bytes;
     upload_active();
-    EngineParams q{tune_.queue_capacity, tune_.chunk_paths, tune_.regen_every, 0};
+    EngineParams q{tune_.queue_capacity, tune_.chunk_paths, tune_.regen_every};
     k_set_params<<<1, 1, 0, stream_>>>((EngineParams*)d_params_, q);
     copy_out(r, hdr, rgb);
     cudaEventDestroy(r.ev_ready);
@@ -1738,12 +1713,11 @@ constexpr int64_t kNoAllocMaxPixels = 256 * 256;
 constexpr size_t kNoAllocAlign = 256;
 constexpr size_t align_up(size_t x) { return (x + kNoAllocAlign - 1) / kNoAllocAlign * kNoAllocAlign; }
 constexpr size_t kNoAllocHeader = 64 * 1024;             // counters, request table, per-slot words
-constexpr size_t kNoAllocQueueBytes = align_up((size_t)kNoAllocQueue * 112);  // 7 x 16 B per path
-constexpr size_t kNoAllocHitBytes = align_up((size_t)kNoAllocQueue * 16);
-constexpr size_t kNoAllocShadowBytes = align_up((size_t)kNoAllocShadow * 48);
+constexpr size_t kNoAllocQueueBytes = align_up((size_t)kNoAllocQueue * 128);  // 8 x 16 B per path
+constexpr size_t kNoAllocShadowBytes = align_up((size_t)kNoAllocShadow * 52);
 constexpr size_t kNoAllocAccumBytes = align_up((size_t)kNoAllocMaxPixels * 3 * sizeof(double));
 constexpr size_t kNoAllocBytes =
-    kNoAllocHeader + 2 * kNoAllocQueueBytes + kNoAllocHitBytes + kNoAllocShadowBytes + kNoAllocAccumBytes;
+    kNoAllocHeader + 2 * kNoAllocQueueBytes + kNoAllocShadowBytes + kNoAllocAccumBytes;
 
 // The scratch array.  In host code `g_noalloc_scratch` is only a host-side
 // stand-in for the symbol; its device address comes from
@@ -1788,7 +1762,7 @@ DRequest Engine::make_request(const pcr_render_desc& d, int scene, double* accum
     R.shadow = d.shadow_samples;
     R.flags = (d.spectral ? kReqSpectral : 0) | (d.mis ? kReqMIS : 0) | (d.russian ? kReqRussian : 0) |
               (d.stratified ? kReqStratified : 0) | (d.spectral_terminate ? kReqTerminate : 0) |
-              (traced_whole(scene) ? kReqWhole : 0);
+              (flat(scene) ? kReqFlat : 0);
     R.hero = std::min(4, std::max(1, d.hero_samples <= 0 ? 4 : d.hero_samples));
     R.strata = d.stratified ? std::max(1, (int)std::lround(std::sqrt((float)d.samples))) : 0;
     R.cam_x = S.cam[0];
@@ -1840,7 +1814,6 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     unsigned long long* tfirst = reinterpret_cast<unsigned long long*>(take(8));
     unsigned long long* tdone = reinterpret_cast<unsigned long long*>(take(8));
     long long* give_start = reinterpret_cast<long long*>(take(8));
-    int* give = reinterpret_cast<int*>(take(4));
     int* give_base = reinterpret_cast<int*>(take(4));
     int* path_base = reinterpret_cast<int*>(take(4));
     int* active = reinterpret_cast<int*>(take(4));
@@ -1861,12 +1834,13 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
         q[b].w[0] = reinterpret_cast<float4*>(q[b].id + kNoAllocQueue);
         q[b].w[1] = q[b].w[0] + kNoAllocQueue;
         q[b].w[2] = q[b].w[1] + kNoAllocQueue;
+        q[b].hit = q[b].w[2] + kNoAllocQueue;
     }
-    float4* hit = reinterpret_cast<float4*>(take(kNoAllocHitBytes));
     ShadowQueue sq;
     sq.o = reinterpret_cast<float4*>(take(kNoAllocShadowBytes));
     sq.d = sq.o + kNoAllocShadow;
     sq.c = sq.d + kNoAllocShadow;
+    sq.bound = reinterpret_cast<float*>(sq.c + kNoAllocShadow);
     double* accum = reinterpret_cast<double*>(take(kNoAllocAccumBytes));
     if (off > kNoAllocBytes || header_used > kNoAllocHeader)
         throw PcrError(PCR_ERR_INVALID, "pcr_render_noalloc: scratch layout overflow");
@@ -1881,7 +1855,6 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     E.reqs = reqs;
     E.issued = issued;
     E.outstanding = outstanding;
-    E.give = give;
     E.give_base = give_base;
     E.path_base = path_base;
     E.active = active;
@@ -1892,7 +1865,6 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     E.cnt = cnt;
     E.q[0] = q[0];
     E.q[1] = q[1];
-    E.hit = hit;
     E.sq = sq;
     E.give_start = give_start;
     E.shadow_cap = kNoAllocShadow;
@@ -1901,13 +1873,12 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     E.round_list = round_list;
     E.cmf_table = d_cmf_;
     E.queue_cap = kNoAllocQueue;
-    E.n_mats = mat_count_;
 
     const DRequest R = make_request(desc, scene, accum);
-    if (traced_whole(scene)) {
+    if (flat(scene)) {
         int g_paths;
-        grid_for((const void*)k_paths, kPathBlock, kPathSmem, &g_paths);
-        trace_whole(E, R, g_paths);
+        grid_for((const void*)k_paths<false>, kPathBlock, kPathSmem, &g_paths);
+        trace_flat(E, R, g_paths);
     } else {
         k_admit<<<1, 1, 0, stream_>>>(E, R, 0);
         ActiveList L;
@@ -1915,35 +1886,29 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
         L.slots[0] = 0;
         k_set_active<<<1, 32, 0, stream_>>>(E, L);
         const int pass = (int)std::min<int64_t>(px, kNoAllocFill);
-        k_set_params<<<1, 1, 0, stream_>>>(params, EngineParams{pass, pass, 1, 1});
+        k_set_params<<<1, 1, 0, stream_>>>(params, EngineParams{pass, pass, 1});
         CK(cudaGetLastError());
 
         // launch shapes from the occupancy calculator (no allocation involved)
         const int B = trace_block();
-        const size_t mat_bytes = sizeof(DMaterial) * (size_t)std::max(1, mat_count_);
-        const int smem_mats = mat_bytes <= 96 * 1024 ? 1 : 0;
-        const size_t smem = smem_mats ? mat_bytes : 0;
-        raise_shade_smem(smem);
-        int g_regen, g_extend, g_shade, g_shadow;
-        grid_for((const void*)k_regen, B, 0, &g_regen);
+        int g_paths, g_extend, g_shadow;
+        grid_for((const void*)k_paths<true>, kPathBlock, kPathSmem, &g_paths);
         grid_for((const void*)k_extend, B, 0, &g_extend);
-        grid_for((const void*)k_shade, kShadeBlock, smem, &g_shade);
         grid_for((const void*)k_shadow, B, 0, &g_shadow);
         int cur = 0;
         auto iteration = [&]() {
             k_schedule<<<1, kSchedThreads, 0, stream_>>>(E, params, cur);
-            k_regen<<<g_regen, B, 0, stream_>>>(E, cur, xyz_scale_);
-            k_extend<<<g_extend, B, 0, stream_>>>(E, cur);
-            k_shade<<<g_shade, kShadeBlock, smem, stream_>>>(E, cur, smem_mats);
+            k_paths<true><<<g_paths, kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
+            k_extend<<<g_extend, B, 0, stream_>>>(E, cur ^ 1);
             k_shadow<<<g_shadow, B, 0, stream_>>>(E);
             k_status<<<1, 1024, 0, stream_>>>(E, cur ^ 1);
             CK(cudaGetLastError());
             cur ^= 1;
         };
         const int64_t total = px * local_spp(desc) * std::max(1, desc.aa_samples);
-        const int64_t passes = (total + pass - 1) / pass;
-        for (int64_t it = 0; it < passes * (int64_t)desc.depth; it++) iteration();
-        for (int extra = 0;; extra++) {
+        const int64_t fills = (total + pass - 1) / pass;
+        for (int64_t it = 0; it < fills + desc.depth; it++) iteration();
+        for (int64_t extra = 0;; extra++) {
             int flag = 0;
             Counters c;
             CK(cudaMemcpyAsync(&flag, done, sizeof(int), cudaMemcpyDeviceToHost, stream_));
@@ -1951,7 +1916,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
             CK(cudaStreamSynchronize(stream_));
             if (c.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "pcr_render_noalloc: device reported queue overflow");
             if (flag) break;
-            if (extra > 4 * desc.depth + 8) throw PcrError(PCR_ERR_TIMEOUT, "pcr_render_noalloc did not finish");
+            if (extra > fills * (4 * (int64_t)desc.depth + 8)) throw PcrError(PCR_ERR_TIMEOUT, "pcr_render_noalloc did not finish");
             iteration();
         }
     }

@@ -117,23 +117,24 @@ private:
     void alloc_request(Request& r);
     void activate(Request& r, int slot);
     void upload_active();
-    // Which stages an iteration runs: the queue stages for requests on mesh
-    // scenes, k_paths for the others (bits of the active requests).
-    static constexpr int kStagesQueue = 1, kStagesPaths = 2;
+    // Which kernels an iteration runs: k_paths and the BVH walks for requests
+    // on mesh scenes, the mesh-free k_paths for the others (bits of the active
+    // requests).
+    static constexpr int kStagesMesh = 1, kStagesFlat = 2;
     int active_stages() const;
     void launch_iteration(int cur, int stages, bool profile);
     void launch_block(int stages);
     void launch_shapes();
     int trace_block() const { return (tune_.block_size + 31) / 32 * 32; }  // whole warps
     void drop_graphs();
-    void trace_whole(const EngineView& E, const DRequest& R, int grid);
-    void render_whole(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats* st);
+    void trace_flat(const EngineView& E, const DRequest& R, int grid);
+    void render_flat(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats* st);
     void harvest(bool final_sync);
     void finish_request(Request& r, cudaStream_t rs);
     void release_cancelled(Request& r);
     void copy_out(Request& r, float* hdr, uint8_t* rgb);
     DRequest make_request(const pcr_render_desc& d, int scene, double* accum) const;
-    bool traced_whole(int scene) const { return scenes_[scene].dev.n_nodes == 0; }
+    bool flat(int scene) const { return scenes_[scene].dev.n_nodes == 0; }
     void check_status();
     bool engine_step();
     void serve_loop();
@@ -177,7 +178,7 @@ private:
     unsigned long long *d_issued_ = nullptr, *d_tfirst_ = nullptr, *d_tdone_ = nullptr;
     long long* d_outstanding_ = nullptr;
     long long* d_give_start_ = nullptr;
-    int *d_give_ = nullptr, *d_give_base_ = nullptr, *d_path_base_ = nullptr, *d_active_ = nullptr, *d_nactive_ = nullptr, *d_done_ = nullptr;
+    int *d_give_base_ = nullptr, *d_path_base_ = nullptr, *d_active_ = nullptr, *d_nactive_ = nullptr, *d_done_ = nullptr;
     int *d_round_state_ = nullptr, *d_round_cnt_ = nullptr, *d_round_list_ = nullptr;
     float4* d_cmf_ = nullptr;  // colour-matching table for raygen
     int* h_active_ = nullptr;     // pinned: [0] = n, then slots
@@ -208,7 +209,6 @@ private:
 
     // queues
     PathQueue q_[2]{};
-    float4* d_hit_ = nullptr;
     ShadowQueue sq_{};
     int queue_cap_ = 0, shadow_cap_ = 0;
     std::vector<void*> qallocs_;
@@ -216,9 +216,7 @@ private:
     // graph
     cudaGraphExec_t graphs_[4] = {};   // by stages, captured when first launched
     bool graph_dirty_ = true;
-    int grid_regen_ = 0, grid_extend_ = 0, grid_shade_ = 0, grid_shadow_ = 0, grid_round_ = 0, grid_paths_ = 0;
-    size_t shade_smem_ = 0;
-    int smem_mats_ = 0;
+    int grid_extend_ = 0, grid_shadow_ = 0, grid_round_ = 0, grid_flat_ = 0, grid_mesh_ = 0;
 
     // requests
     std::mutex mu_;

@@ -1,14 +1,15 @@
 // Wavefront stage kernels.  One iteration of the persistent wavefront is
-//   schedule -> regen -> extend -> shade -> shadow -> status
-// over the current path queue; shade writes surviving paths into the other
-// queue.  Every kernel is a grid-stride loop over a device-side count, so
-// a whole iteration (and several in a row) can be captured in one CUDA
-// graph with no host round trip.  No kernel waits on another block or on
+//   schedule -> paths -> extend -> shadow -> status
+// k_paths (paths.cuh) takes the queued paths, whose ray has been traced, and
+// new camera paths, and follows each until it ends or its next ray has a
+// triangle mesh to walk: then the path waits in the other queue, where
+// k_extend walks it, as k_shadow does the shadow rays that meet the mesh.
+// Paths on scenes without a mesh never wait.  Every kernel loops over a
+// device-side count, so a whole iteration (and several in a row) can be
+// captured in one CUDA graph with no host round trip.  No kernel waits on another block or on
 // the host: there is no spin anywhere.
 #pragma once
 
-#include <cooperative_groups.h>
-#include <cooperative_groups/scan.h>
 #include <cub/block/block_scan.cuh>
 
 #include "device.cuh"
@@ -19,15 +20,14 @@ struct EngineParams {
     int fill;          // refill target (paths in flight)
     int chunk;         // per-request issue chunk per refill
     int regen_every;   // refill cadence in iterations
-    int plain;         // 1: refill only when the queue is empty (pass-wise)
 };
 
 // ------------------------------------------------------------------ schedule
 // One block.  Decides how many new camera paths each active request gets
 // this iteration: first up to `chunk` each (round-robin fairness), then the
-// remaining free slots oldest-first.  Requests whose paths k_paths traces
-// whole (kReqWhole) share `fill` paths per iteration; the others share the
-// free slots of the path queue.
+// remaining free slots oldest-first.  Requests on scenes without a mesh
+// (kReqFlat) share `fill` paths per iteration; the others share what the
+// waiting paths leave of `fill`.
 constexpr int kSchedThreads = 1024;
 
 struct Share {
@@ -67,18 +67,17 @@ __global__ void __launch_bounds__(kSchedThreads) k_schedule(EngineView E, const 
     const int tid = threadIdx.x;
     const int n_act = *E.n_active;
     int qn = C->queue_n[cur];
-    if (qn > E.queue_cap) {  // never expected: shade guards every append
+    if (qn > E.queue_cap) {  // never expected: k_paths guards every append
         qn = E.queue_cap;
         if (tid == 0) atomicOr(&C->status, 4);
     }
     const EngineParams p = *P;
     long long free_slots = (long long)p.fill - qn;
     if (free_slots < 0) free_slots = 0;
-    if (p.plain && qn > 0) free_slots = 0;
     if (p.regen_every > 1 && (C->iter % p.regen_every) != 0 && qn > 0) free_slots = 0;
 
     int slot = -1;
-    bool whole = false;
+    bool flat = false;
     long long rem = 0;
     if (tid < n_act) {
         slot = E.active[tid];
@@ -102,14 +101,13 @@ __global__ void __launch_bounds__(kSchedThreads) k_schedule(EngineView E, const 
         }
         rem = E.reqs[slot].total - (long long)E.issued[slot];
         if (rem < 0) rem = 0;
-        whole = (E.reqs[slot].flags & kReqWhole) != 0;
+        flat = (E.reqs[slot].flags & kReqFlat) != 0;
     }
     Share q = {0, 0, 0}, w = {0, 0, 0};
-    if (__syncthreads_or(!whole && rem > 0)) q = share_slots<Scan>(tmp, whole ? 0 : rem, p.chunk, free_slots);
-    if (__syncthreads_or(whole && rem > 0)) w = share_slots<Scan>(tmp, whole ? rem : 0, p.chunk, p.fill);
+    if (__syncthreads_or(!flat && rem > 0)) q = share_slots<Scan>(tmp, flat ? 0 : rem, p.chunk, free_slots);
+    if (__syncthreads_or(flat && rem > 0)) w = share_slots<Scan>(tmp, flat ? rem : 0, p.chunk, p.fill);
     if (tid < n_act) {
         const long long g = q.mine + w.mine;
-        E.give[tid] = (int)q.mine;
         E.give_base[tid] = (int)q.before;
         E.path_base[tid] = (int)w.before;
         E.give_start[tid] = (long long)E.issued[slot];
@@ -120,18 +118,17 @@ __global__ void __launch_bounds__(kSchedThreads) k_schedule(EngineView E, const 
                 E.t_first[slot] = t;
             }
             E.issued[slot] += (unsigned long long)g;
-            E.outstanding[slot] += q.mine;  // a whole path is at its end when k_paths is
         }
+        E.outstanding[slot] = 0;  // k_extend counts the paths that wait
     }
     if (tid == 0) {
         C->n_rounds = 0;  // k_round of the last iteration has read the list
-        C->new_base = qn;
         C->new_n = (int)q.all;
-        C->queue_n[cur] = qn + (int)q.all;
+        C->queue_n[cur] = qn;
         C->queue_n[cur ^ 1] = 0;
         C->shadow_n = 0;
         C->path_n = (int)w.all;
-        C->path_next = 0;
+        C->next[0] = C->next[1] = C->next[2] = 0;
         C->paths += (unsigned long long)(q.all + w.all);
     }
 }
@@ -271,7 +268,7 @@ __device__ __forceinline__ float4 rgb4(float4 c) { return make_float4(c.x, c.y, 
 
 // A material spectrum at the four carried wavelengths (Material::albedoAt /
 // emissiveAt, code/Includes/Material.h:92-101).  Kept out of line: one copy
-// of the sigmoid / table code instead of one per call site keeps k_shade's
+// of the sigmoid / table code instead of one per call site keeps k_paths'
 // instruction footprint small.
 __device__ __noinline__ float4 spec4(const DMaterial& m, int emissive, float4 lam)
 {
@@ -286,7 +283,7 @@ __device__ __noinline__ float4 spec4(const DMaterial& m, int emissive, float4 la
     return emissive ? v : make_float4(v.x > 1.f ? 1.f : v.x, v.y > 1.f ? 1.f : v.y, v.z > 1.f ? 1.f : v.z, v.w > 1.f ? 1.f : v.w);
 }
 
-// ------------------------------------------------------------------ regen
+// ------------------------------------------------------------------ raygen
 // Camera rays for the new paths (code/Renderer.cpp:190-239): pixel centre,
 // jitter when aa > 1, hero wavelength and its stratified companions.
 struct CameraPath {
@@ -376,44 +373,6 @@ __device__ __forceinline__ CameraPath camera_path(const EngineView& E, const DRe
     return p;
 }
 
-__global__ void k_regen(EngineView E, int cur, float xyz_scale)
-{
-    __shared__ int s_base[kMaxActive];
-    __shared__ int s_give[kMaxActive];
-    __shared__ int s_slot[kMaxActive];
-    __shared__ long long s_start[kMaxActive];
-    const Counters* C = E.cnt;
-    const int n_act = *E.n_active;
-    for (int i = threadIdx.x; i < n_act; i += blockDim.x) {
-        s_base[i] = E.give_base[i];
-        s_give[i] = E.give[i];
-        s_slot[i] = E.active[i];
-        s_start[i] = E.give_start[i];
-    }
-    __syncthreads();
-    const int n_new = C->new_n, base = C->new_base;
-    const PathQueue Q = E.q[cur];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_new; i += gridDim.x * blockDim.x) {
-        int lo = 0, hi = n_act - 1;
-        while (lo < hi) {  // last r with base[r] <= i and give[r] > 0
-            int mid = (lo + hi + 1) >> 1;
-            if (s_base[mid] <= i) lo = mid; else hi = mid - 1;
-        }
-        while (lo > 0 && (s_give[lo] == 0 || s_base[lo] > i)) lo--;
-        const int slot = s_slot[lo];
-        const DRequest& R = E.reqs[slot];
-        const int pos = base + i;
-        XyzWeights W;
-        const CameraPath p = camera_path(E, R, s_start[lo] + (i - s_base[lo]), xyz_scale, W);
-        if (R.flags & kReqSpectral) store_weights(Q, pos, W);
-        const int nch = (R.flags & kReqSpectral) ? R.hero : 4;
-        Q.o[pos] = make_float4(R.cam_x, R.cam_y, R.cam_z, p.lambda0);
-        Q.d[pos] = make_float4(p.d.x, p.d.y, p.d.z, __int_as_float(nch << 12));
-        Q.tp[pos] = make_float4(1.f, 1.f, 1.f, 1.f);
-        Q.id[pos] = make_int4(slot, (int)p.pixel, (int)p.sample, R.scene);
-    }
-}
-
 // Brings the next grid-stride record's line into L2 while this one is
 // processed (no register cost; the record is read again when its turn comes).
 __device__ __forceinline__ void prefetch_l2(const void* p)
@@ -433,73 +392,33 @@ __device__ __forceinline__ void prefetch_l2(const void* p)
 #endif
 constexpr int kTraceMaxBlock = 256, kTraceMinBlocks = PCR_TRACE_MIN_BLOCKS, kShadowMinBlocks = PCR_SHADOW_MIN_BLOCKS;
 
-// Rays of a warp that have a mesh to walk.  Many rays miss the mesh's box;
-// walked where they stand, the others left 9 of 32 lanes active.  So each warp
-// first runs the analytic tests and the box test for its rays, keeps those
-// that go on in shared memory, and walks the BVH whenever 32 of them have come
-// together (14 to 16 lanes active over the whole kernel).  Six mesh renders
-// batched: k_extend 11.0 -> 8.5 ms, k_shadow 9.3 -> 6.1 ms; 24 uneven renders
-// 14.0 -> 7.7 and 24.9 -> 18.3 ms.
-struct WalkQueue {
-    int ray[64];
-    float t[64];
-    uint32_t prim[64];
-};
-
-// Closest hit for every queued path (trace_closest).
-__global__ void __launch_bounds__(kTraceMaxBlock, kTraceMinBlocks) k_extend(EngineView E, int cur)
+// Closest hit of the paths that wait in queue q: the BVH walk, bounded by the
+// analytic hit.  Every ray here meets the mesh's box (others never wait), so
+// warps walk with all lanes from the start.  Also counts each request's
+// waiting paths.
+__global__ void __launch_bounds__(kTraceMaxBlock, kTraceMinBlocks) k_extend(EngineView E, int q)
 {
-    __shared__ WalkQueue s_walk[kTraceMaxBlock / 32];
-    WalkQueue& W = s_walk[threadIdx.x >> 5];
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const Counters* C = E.cnt;
-    const int n = min(C->queue_n[cur], E.queue_cap);
-    const PathQueue Q = E.q[cur];
+    const int n = min(E.cnt->queue_n[q], E.queue_cap);
+    const PathQueue Q = E.q[q];
     const int stride = gridDim.x * blockDim.x;
-    unsigned mine = 0;
-    int pending = 0;
     for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
         const int i = base + lane, nx = i + stride;
-        if (nx < n) { prefetch_l2(Q.o + nx); prefetch_l2(Q.d + nx); prefetch_l2(Q.id + nx); }
-        bool walk = false;
-        float t = FLT_MAX;
-        uint32_t prim = kPrimNone;
+        if (nx < n) { prefetch_l2(Q.o + nx); prefetch_l2(Q.d + nx); prefetch_l2(Q.id + nx); prefetch_l2(Q.hit + nx); }
+        int slot = -1;
         if (i < n) {
-            const DScene& S = E.scenes[Q.id[i].w];
-            const float3 o = xyz(Q.o[i]), d = xyz(Q.d[i]);
-            prim = scene_analytic(S, o, d, t);
-            walk = mesh_may_hit(S, o, d, t);
-            if (!walk) E.hit[i] = make_float4(t, __uint_as_float(prim), 0.f, 0.f);
-            mine++;
+            const int4 id = Q.id[i];
+            slot = id.x;
+            float t = Q.hit[i].x, u = 0.f, v = 0.f;
+            const int tri = bvh4_closest<false>(E.scenes[id.w], xyz(Q.o[i]), xyz(Q.d[i]), t, u, v, nullptr);
+            if (tri >= 0) Q.hit[i] = make_float4(t, __uint_as_float(kPrimTri | (uint32_t)tri), u, v);
         }
-        const unsigned m = __ballot_sync(kAll, walk);
-        if (walk) {
-            const int k = pending + __popc(m & ((1u << lane) - 1u));
-            W.ray[k] = i;
-            W.t[k] = t;
-            W.prim[k] = prim;
-        }
-        pending += __popc(m);
-        __syncwarp();
-        const bool last = base >= n - stride;
-        while (pending >= 32 || (last && pending > 0)) {
-            const int first = max(0, pending - 32), k = first + lane;
-            if (k < pending) {
-                const int r = W.ray[k];
-                const DScene& S = E.scenes[Q.id[r].w];
-                float u = 0.f, v = 0.f, c = W.t[k];
-                const int tri = bvh4_closest<false>(S, xyz(Q.o[r]), xyz(Q.d[r]), c, u, v, nullptr);
-                const uint32_t p = tri >= 0 ? kPrimTri | (uint32_t)tri : W.prim[k];
-                E.hit[r] = make_float4(c, __uint_as_float(p), u, v);
-            }
-            pending = first;
-            __syncwarp();
-        }
-        if (last) break;
+        const unsigned same = __match_any_sync(kAll, slot);
+        if (slot >= 0 && lane == __ffs(same) - 1)
+            atomicAdd((unsigned long long*)&E.outstanding[slot], (unsigned long long)__popc(same));
+        if (base >= n - stride) break;
     }
-    mine = __reduce_add_sync(kAll, mine);
-    if (lane == 0 && mine) atomicAdd(&E.cnt->rays, (unsigned long long)mine);
 }
 
 // ------------------------------------------------------------------ helpers
@@ -519,8 +438,7 @@ __device__ __forceinline__ void add_xyz(double* acc, float3 c)
 
 // ------------------------------------------------------------------ shading steps
 // The steps of one path vertex (code/Renderer.cpp:656-889 with samples = 1,
-// the GPU's paths-per-pixel estimator), shared by k_shade, which advances a
-// queue of paths by one vertex, and k_paths, which follows a path to its end.
+// the GPU's paths-per-pixel estimator).
 
 // Wavelengths carried by a path (code/Renderer.cpp:227-239).
 __device__ __forceinline__ float4 path_wavelengths(float l0, int single, int nHero)
@@ -693,6 +611,13 @@ __device__ __forceinline__ float shadow_factor(const DScene& S, const DRequest& 
     return g.G * w;
 }
 
+// What every sample of a vertex is scaled by: light area / (pi S).
+__device__ __forceinline__ float light_scale(const DScene& S, const DRequest& R)
+{
+    const float inv_pi = 1.f / 3.14159274f;
+    return S.total_light_area * inv_pi / (float)R.shadow;
+}
+
 // Continuation of a diffuse vertex: Russian roulette and the cosine
 // hemisphere.  Returns whether the path goes on; nd its direction and
 // rr_scale its throughput factor.
@@ -721,409 +646,33 @@ __device__ __forceinline__ bool diffuse_bounce(const DRequest& R, uint32_t pixel
     return survive;
 }
 
-// ------------------------------------------------------------------ shade
-// Appends `count` records for the calling lane among the lanes that reach the
-// call together (divergent code): one atomic per coalesced group.
-__device__ __forceinline__ int group_append(int* counter, int count)
-{
-    namespace cg = cooperative_groups;
-    cg::coalesced_group g = cg::coalesced_threads();
-    const int ex = cg::exclusive_scan(g, count);
-    const int tot = g.shfl(ex + count, g.size() - 1);
-    int base = 0;
-    if (g.thread_rank() == 0 && tot) base = atomicAdd(counter, tot);
-    return g.shfl(base, 0) + ex;
-}
-
-// k_shade's block shape is fixed: its register budget (launch bounds) is
-// set for 128-thread blocks, PCR_SHADE_MIN_BLOCKS per SM.
-#ifndef PCR_SHADE_MIN_BLOCKS
-#define PCR_SHADE_MIN_BLOCKS 5
-#endif
-constexpr int kShadeBlock = 128;
-
-// Per-path shading of the hit found by k_extend (code/Renderer.cpp:656-889
-// with samples = 1, the GPU's paths-per-pixel estimator): emission,
-// mirror, dielectric (with the 4-way hero fork at dispersive glass),
-// diffuse direct lighting via explicit shadow rays, Russian roulette and the
-// cosine-hemisphere continuation.  Materials are staged in shared memory.
-//
-// A diffuse vertex reserves R.shadow shadow records with one append; samples
-// whose geometry term is zero are written as skip records (lightDist2 < 0).
-// The spectral product albedo * emission * XYZ weight is formed once per
-// vertex and light material, so each shadow sample only scales it by its
-// geometry term.
-//
-// Per-channel values live in float4 registers (no per-thread arrays, so no
-// local memory); channels a path does not carry have zero XYZ weight, so
-// they are evaluated but contribute nothing.
-__global__ void __launch_bounds__(kShadeBlock, PCR_SHADE_MIN_BLOCKS) k_shade(EngineView E, int cur, int smem_mats)
-{
-    extern __shared__ DMaterial s_mat[];
-    const DMaterial* M = E.mats;
-    if (smem_mats) {
-        const int words = E.n_mats * (int)(sizeof(DMaterial) / 16);
-        const float4* src = reinterpret_cast<const float4*>(E.mats);
-        float4* dst = reinterpret_cast<float4*>(s_mat);
-        for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
-        __syncthreads();
-        M = s_mat;
-    }
-    Counters* C = E.cnt;
-    const int n = min(C->queue_n[cur], E.queue_cap);
-    const PathQueue Q = E.q[cur];
-    const PathQueue NQ = E.q[cur ^ 1];
-    const ShadowQueue SQ = E.sq;
-    const float inv_pi = 1.f / 3.14159274f;
-    const int lane = threadIdx.x & 31;
-    // block-uniform trip count: every thread of a block runs the same
-    // iterations, so the block-wide append at the bottom sees all of them
-    __shared__ int s_app[2][kShadeBlock / 32 + 1];
-    __shared__ int s_shd[2][kShadeBlock / 32 + 1];
-    int parity = 0;
-    const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
-        const int i = base + threadIdx.x;
-        const bool live = i < n;
-        int4 id = make_int4(0, 0, 0, 0);
-        float4 o4 = make_float4(0, 0, 0, 0), d4 = o4, tp4 = o4, h = o4;
-        if (i + stride < n) {
-            const int nx = i + stride;
-            prefetch_l2(Q.id + nx); prefetch_l2(Q.o + nx); prefetch_l2(Q.d + nx); prefetch_l2(Q.tp + nx);
-            prefetch_l2(E.hit + nx);
-            prefetch_l2(Q.w[0] + nx); prefetch_l2(Q.w[1] + nx); prefetch_l2(Q.w[2] + nx);
-        }
-        if (live) { id = Q.id[i]; o4 = Q.o[i]; d4 = Q.d[i]; tp4 = Q.tp[i]; h = E.hit[i]; }
-        const int slot = id.x;
-        const uint32_t prim = __float_as_uint(h.y);
-        const int meta = __float_as_int(d4.w);
-        const int bounce = meta & 0xFF, fork = (meta >> 8) & 7, single = (meta >> 11) & 1, nHero = (meta >> 12) & 7;
-        bool cont = false;    // continue into the next queue
-        int forked = 0;       // sub-paths written by a dispersive fork
-        float3 no = make_float3(0, 0, 0), nd = no;
-        float4 ntp = make_float4(0, 0, 0, 0);
-        bool term = false;    // continues with its hero wavelength alone
-        double* acc = nullptr;
-        float3 emit_xyz = make_float3(0, 0, 0);
-        bool emit = false;
-        bool spec_path = false;
-
-        // Shadow records: a diffuse vertex with a light in its scene writes
-        // R.shadow of them.  They are reserved for the whole block at once
-        // (one contiguous range, its warps in order), so k_shadow's warps
-        // rarely straddle two blocks' records, which may belong to
-        // different scenes.
-        int nee = 0;
-        bool mesh = false;  // casts over a BVH
-        if (live && (prim & kPrimKindMask) != kPrimNone) {
-            const DScene& S0 = E.scenes[id.w];
-            if (S0.total_light_area > 0.f) {
-                const uint32_t k0 = prim & kPrimKindMask, p0 = prim & kPrimIndexMask;
-                const int mi0 = k0 == kPrimSphere ? S0.spheres[p0].mat.x
-                              : k0 == kPrimPlane  ? __float_as_int(S0.planes[p0].o_mat.w)
-                                                  : __float_as_int(S0.tris[p0].e1_mat.w);
-                if (!(M[S0.mat_base + mi0].flags & (kMatEmissive | kMatMetallic | kMatTransparent))) {
-                    nee = E.reqs[slot].shadow;
-                    mesh = S0.n_nodes > 0;
-                }
-            }
-        }
-        int spos_block, sstride;
-        {
-            int ex = nee;  // inclusive scan across the warp
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, ex, off);
-                if (lane >= off) ex += v;
-            }
-            int* sw = s_shd[parity];
-            const int wid = threadIdx.x >> 5;
-            if (lane == 31) sw[wid] = ex;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int tot = 0;
-                for (int k = 0; k < kShadeBlock / 32; k++) { const int c = sw[k]; sw[k] = tot; tot += c; }
-                sw[kShadeBlock / 32] = tot ? atomicAdd(&C->shadow_n, tot) : 0;
-            }
-            __syncthreads();
-            const int wbase = sw[kShadeBlock / 32] + sw[wid];
-            // Sample-major order inside the warp when its vertices all cast
-            // the same number of shadow rays (one request, the usual case)
-            // into scenes without a mesh: record s of the warp's k-th
-            // casting lane sits at wbase + s * casters + k, so each sample's
-            // stores are one contiguous run.  Otherwise each lane's records
-            // are adjacent: over a BVH, the rays of one vertex then share a
-            // k_shadow warp and walk mostly the same nodes.
-            const unsigned cm = __ballot_sync(0xffffffffu, nee > 0);
-            const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)nee);
-            const unsigned lo = __reduce_min_sync(0xffffffffu, nee > 0 ? (unsigned)nee : 0xffffffffu);
-            if (hi == lo && !__any_sync(0xffffffffu, mesh)) {
-                spos_block = wbase + __popc(cm & ((1u << lane) - 1u));
-                sstride = __popc(cm);
-            } else {
-                spos_block = wbase + ex - nee;
-                sstride = 1;
-            }
-        }
-
-        if (live && (prim & kPrimKindMask) != kPrimNone) {
-            const DRequest& R = E.reqs[slot];
-            const DScene& S = E.scenes[id.w];
-            const bool spectral = (R.flags & kReqSpectral) != 0;
-            spec_path = spectral;
-            const float4 lam4 = spectral ? path_wavelengths(o4.w, single, nHero) : make_float4(0.f, 0.f, 0.f, 0.f);
-            acc = R.accum + (size_t)id.y * 3;
-            const float3 o = xyz(o4), d = xyz(d4);
-            const Surface sf = surface_at<true>(S, prim, h.x, h.z, h.w, o, d);
-            const float3 hit = sf.hit;
-            float3 N = sf.N;
-            const int mi = sf.mi;
-            const bool entering = f3dot(d, N) < 0.f;
-            if (!entering) N = f3neg(N);
-            const DMaterial& m = M[S.mat_base + mi];
-            const bool last = bounce + 1 >= R.depth;
-            if (m.flags & kMatEmissive) {
-                // with emit_mat the carried weights already hold the emission
-                const float4 c = !spectral ? mul4(tp4, rgb4(m.emissive))
-                               : S.emit_mat >= 0 ? tp4 : mul4(tp4, spec4(m, 1, lam4));
-                const XyzWeights W = spectral ? load_weights(Q, i) : rgb_weights();
-                emit_xyz = apply_xyz(W, c);
-                emit = true;
-            } else if (m.flags & kMatMetallic) {
-                if (!last) {
-                    const float cosI = -f3dot(d, N);
-                    reflect_at(hit, N, d, cosI, no, nd);
-                    ntp = mul4(tp4, spectral ? spec4(m, 0, lam4) : rgb4(m.albedo));
-                    cont = true;
-                }
-            } else if (m.flags & kMatTransparent) {
-                if (!last) {
-                    const float cosI = -f3dot(d, N);
-                    const bool dispersive = spectral && m.cauchyB != 0.f && !single && nHero > 1;
-                    // fork: one sub-path per wavelength (code/Renderer.cpp:736-753);
-                    // terminate: the hero wavelength's bounce alone
-                    // (code/Gpu/Metal/MetalRenderer.mm:2143-2252)
-                    const bool terminate = dispersive && (R.flags & kReqTerminate);
-                    const bool disperse = dispersive && !terminate;
-                    const int ways = disperse ? nHero : 1;
-                    const float4 coins = rand4(R, (uint32_t)id.y, (uint32_t)id.z, (uint32_t)fork, (uint32_t)bounce, 63u);
-                    const float4 alg = spectral ? spec4(m, 0, lam4) : rgb4(m.albedo);
-                    int fpos = 0;
-                    if (disperse) {
-                        fpos = group_append(&C->queue_n[cur ^ 1], ways);
-                        forked = ways;
-                    }
-                    for (int k = 0; k < ways; k++) {
-                        const float lk = comp4(lam4, k);
-                        const float ior = ior_at(m, spectral && m.cauchyB != 0.f && (dispersive || single), lk);
-                        float3 bd, bo;
-                        const bool refl = dielectric_bounce(hit, N, d, cosI, entering, ior, comp4(coins, k), bo, bd);
-                        if (disperse) {
-                            // sub-path k carries wavelength k alone (code/Renderer.cpp:736-753)
-                            const int pos = fpos + k;
-                            if (pos < E.queue_cap) {
-                                const float ftp = comp4(tp4, k) * comp4(alg, k);
-                                const int fm = (bounce + 1) | ((k + 1) << 8) | (1 << 11) | (nHero << 12);
-                                NQ.o[pos] = make_float4(bo.x, bo.y, bo.z, lk);
-                                NQ.d[pos] = make_float4(bd.x, bd.y, bd.z, __int_as_float(fm));
-                                NQ.tp[pos] = make_float4(ftp, ftp, ftp, ftp);
-                                NQ.id[pos] = id;
-                                // the sub-path keeps wavelength k's weight alone
-                                const float4 w0 = Q.w[0][i], w1 = Q.w[1][i], w2 = Q.w[2][i];
-                                const float3 wk = k == 0 ? make_float3(w0.x, w0.y, w0.z)
-                                                : k == 1 ? make_float3(w0.w, w1.x, w1.y)
-                                                : k == 2 ? make_float3(w1.z, w1.w, w2.x)
-                                                         : make_float3(w2.y, w2.z, w2.w);
-                                NQ.w[0][pos] = make_float4(wk.x, wk.y, wk.z, 0.f);
-                                NQ.w[1][pos] = make_float4(0.f, 0.f, 0.f, 0.f);
-                                NQ.w[2][pos] = make_float4(0.f, 0.f, 0.f, 0.f);
-                            } else {
-                                atomicOr(&C->status, 2);
-                            }
-                        } else {
-                            no = bo;
-                            nd = bd;
-                            // a refraction ends the other wavelengths; the
-                            // hero's share is scaled by their number so the
-                            // estimate stays unbiased (a reflection does not
-                            // depend on the wavelength and keeps them all)
-                            term = terminate && !refl;
-                        }
-                    }
-                    if (!disperse) {
-                        ntp = mul4(tp4, alg);
-                        if (term) {
-                            const float h0 = ntp.x * (float)nHero;
-                            ntp = make_float4(h0, h0, h0, h0);
-                        }
-                        cont = true;
-                    }
-                }
-            } else {
-                // diffuse
-                const float4 al = spectral ? spec4(m, 0, lam4) : rgb4(m.albedo);
-                // indirect origin: hit moved once by 1e-3*N (the reference's
-                // mutating `hit + N * 1e-3`, code/Renderer.cpp:782 with samples = 1)
-                float3 hc = f3add(hit, f3mul(N, 1e-3f));
-                const float3 h1 = hc;
-                if (S.total_light_area > 0.f) {
-                    const float scaleS = S.total_light_area * inv_pi / (float)R.shadow;
-                    const float4 tpal = mul4(tp4, al);
-                    int cached = -1;
-                    float3 V = make_float3(0.f, 0.f, 0.f);
-                    if (spectral && S.emit_mat >= 0) {
-                        // every light has the one emissive material, whose
-                        // emission the carried weights already hold: the
-                        // vertex's product is known before any sample
-                        V = f3mul(apply_xyz(load_weights(Q, i), tpal), scaleS);
-                        cached = S.emit_mat;
-                    }
-                    const int spos = spos_block;
-                    const int nsh = spos + (R.shadow - 1) * sstride < E.shadow_cap ? R.shadow : 0;
-                    if (nsh == 0) atomicOr(&C->status, 1);
-                    for (int s = 0; s < nsh; s++) {
-                        const LightSample L = sample_light(S, R, (uint32_t)id.y, (uint32_t)id.z, (uint32_t)fork,
-                                                           (uint32_t)bounce, (uint32_t)s);
-                        const ShadowSegment g = shadow_segment(L, N, hc);
-                        const int pos = spos + s * sstride;
-                        if (!(g.G > 0.f)) {
-                            SQ.o[pos] = make_float4(0.f, 0.f, 0.f, -1.f);  // skip record
-                            continue;
-                        }
-                        if (L.mat != cached) {
-                            // product of this light material, once per vertex
-                            const DMaterial& lmat = M[S.mat_base + L.mat];
-                            const float4 c = spectral ? mul4(tpal, spec4(lmat, 1, lam4)) : mul4(tpal, rgb4(lmat.emissive));
-                            V = f3mul(apply_xyz(spectral ? load_weights(Q, i) : rgb_weights(), c), scaleS);
-                            cached = L.mat;
-                        }
-                        const float f = shadow_factor(S, R, g);
-                        SQ.o[pos] = make_float4(g.so.x, g.so.y, g.so.z, g.d2);
-                        SQ.d[pos] = make_float4(g.wi.x, g.wi.y, g.wi.z, __int_as_float(id.y));
-                        SQ.c[pos] = make_float4(V.x * f, V.y * f, V.z * f, __int_as_float(slot | (id.w << 16)));
-                    }
-                }
-                float rr_scale;
-                if (diffuse_bounce(R, (uint32_t)id.y, (uint32_t)id.z, (uint32_t)fork, bounce, last, spectral, al, N, nd,
-                                   rr_scale)) {
-                    no = h1;
-                    ntp = make_float4(tp4.x * al.x * rr_scale, tp4.y * al.y * rr_scale, tp4.z * al.z * rr_scale,
-                                      tp4.w * al.w * rr_scale);
-                    cont = true;
-                }
-            }
-        }
-
-        // ---- emit work (block-uniform control flow from here)
-        if (emit) add_xyz(acc, emit_xyz);
-        {
-            const int newMeta = (bounce + 1) | (fork << 8) | ((single | (term ? 1 : 0)) << 11) | (nHero << 12);
-            // one contiguous range per block (its warps in order), so the
-            // next launch's warps rarely straddle two blocks' outputs, which
-            // may belong to different scenes
-            int* sw = s_app[parity];
-            parity ^= 1;
-            const unsigned am = __ballot_sync(0xffffffffu, cont);
-            const int wid = threadIdx.x >> 5;
-            if (lane == 0) sw[wid] = __popc(am);
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int tot = 0;
-                for (int k = 0; k < kShadeBlock / 32; k++) { const int c = sw[k]; sw[k] = tot; tot += c; }
-                sw[kShadeBlock / 32] = tot ? atomicAdd(&C->queue_n[cur ^ 1], tot) : 0;
-            }
-            __syncthreads();
-            int pos = cont ? sw[kShadeBlock / 32] + sw[wid] + __popc(am & ((1u << lane) - 1u)) : -1;
-            if (pos >= E.queue_cap) { atomicOr(&C->status, 2); pos = -1; }
-            if (pos >= 0) {
-                NQ.o[pos] = make_float4(no.x, no.y, no.z, o4.w);
-                NQ.d[pos] = make_float4(nd.x, nd.y, nd.z, __int_as_float(newMeta));
-                NQ.tp[pos] = ntp;
-                NQ.id[pos] = id;
-                if (spec_path) {
-                    const float4 w0 = Q.w[0][i];
-                    NQ.w[0][pos] = term ? make_float4(w0.x, w0.y, w0.z, 0.f) : w0;
-                    NQ.w[1][pos] = term ? make_float4(0.f, 0.f, 0.f, 0.f) : Q.w[1][i];
-                    NQ.w[2][pos] = term ? make_float4(0.f, 0.f, 0.f, 0.f) : Q.w[2][i];
-                }
-            }
-        }
-        // path bookkeeping per request, one atomic per request per warp:
-        // -1 for a retired path, ways-1 for a fork
-        const long long delta = live ? (long long)((cont ? 0 : -1) + forked) : 0;
-        const unsigned same = __match_any_sync(0xffffffffu, live ? slot : -1);
-        const int sum = __reduce_add_sync(same, (int)delta);
-        if (live && sum != 0 && lane == __ffs(same) - 1)
-            atomicAdd((unsigned long long*)&E.outstanding[slot], (unsigned long long)(long long)sum);
-    }
-}
-
 // ------------------------------------------------------------------ shadow
-// Shadow-ray test (code/Renderer.cpp:852-860): blocked when the closest hit
-// within the light distance is non-emissive and closer than lightDist2 -
-// 1e-3 (compared in double, as the reference's double literal promotes it);
-// scene_blocked answers it with an early exit.  Lit samples add their XYZ
-// contribution to the pixel's FP64 accumulator.
-__device__ __forceinline__ void add_lit(const EngineView& E, int i)
-{
-    const float4 c = E.sq.c[i];
-    const int pixel = __float_as_int(E.sq.d[i].w);
-    add_xyz(E.reqs[__float_as_int(c.w) & 0xFFFF].accum + (size_t)pixel * 3, make_float3(c.x, c.y, c.z));
-}
+// The BVH part of the shadow test (code/Renderer.cpp:852-860) for the shadow
+// rays that meet the mesh's box and that k_paths found lit otherwise: blocked
+// by a hit in front of the bound and closer than lightDist2 - 1e-3 (compared
+// in double, as the reference's double literal promotes it).  Lit samples add
+// their XYZ contribution to the pixel's FP64 accumulator.
 __global__ void __launch_bounds__(kTraceMaxBlock, kShadowMinBlocks) k_shadow(EngineView E)
 {
-    __shared__ WalkQueue s_walk[kTraceMaxBlock / 32];  // t: the query's bound
-    WalkQueue& W = s_walk[threadIdx.x >> 5];
-    constexpr unsigned kAll = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    Counters* C = E.cnt;
-    const int n = min(C->shadow_n, E.shadow_cap);
+    const int n = min(E.cnt->shadow_n, E.shadow_cap);
     const ShadowQueue SQ = E.sq;
     const int stride = gridDim.x * blockDim.x;
-    unsigned mine = 0;  // shadow rays of this thread (one launch: < 2^32)
-    int pending = 0;
-    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
-        const int i = base + lane, nx = i + stride;
-        if (nx < n) { prefetch_l2(SQ.o + nx); prefetch_l2(SQ.d + nx); prefetch_l2(SQ.c + nx); }
-        bool walk = false;
-        float bound = 0.f;
-        if (i < n) {
-            const float4 o = SQ.o[i];
-            if (o.w >= 0.f) {  // else a skip record (zero geometry term)
-                const float4 d = SQ.d[i];
-                const DScene& S = E.scenes[__float_as_int(SQ.c[i].w) >> 16];
-                mine++;
-                const int r = scene_blocked_analytic<true>(S, E.mats, xyz(o), xyz(d), o.w, bound);
-                walk = r == kShadowWalk && mesh_may_hit(S, xyz(o), xyz(d), bound);
-                if (r != kShadowBlocked && !walk) add_lit(E, i);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const int nx = i + stride;
+        if (nx < n) { prefetch_l2(SQ.o + nx); prefetch_l2(SQ.d + nx); prefetch_l2(SQ.c + nx); prefetch_l2(SQ.bound + nx); }
+        const float4 o = SQ.o[i];
+        if (o.w >= 0.f) {
+            const DScene& S = E.scenes[__float_as_int(SQ.c[i].w) >> 16];
+            float t = SQ.bound[i], u, v;
+            if (bvh4_closest<false, true>(S, xyz(o), xyz(SQ.d[i]), t, u, v, nullptr, (double)o.w - 1e-3) != -2) {
+                // read after the walk, so that it holds no registers across it
+                const float4 c = SQ.c[i];
+                const int pixel = __float_as_int(SQ.d[i].w);
+                add_xyz(E.reqs[__float_as_int(c.w) & 0xFFFF].accum + (size_t)pixel * 3, make_float3(c.x, c.y, c.z));
             }
         }
-        const unsigned m = __ballot_sync(kAll, walk);
-        if (walk) {
-            const int k = pending + __popc(m & ((1u << lane) - 1u));
-            W.ray[k] = i;
-            W.t[k] = bound;
-        }
-        pending += __popc(m);
-        __syncwarp();
-        const bool last = base >= n - stride;
-        while (pending >= 32 || (last && pending > 0)) {
-            const int first = max(0, pending - 32), k = first + lane;
-            if (k < pending) {
-                const int r = W.ray[k];
-                const float4 o = SQ.o[r];
-                const DScene& S = E.scenes[__float_as_int(SQ.c[r].w) >> 16];
-                float c = W.t[k], u, v;
-                if (bvh4_closest<false, true>(S, xyz(o), xyz(SQ.d[r]), c, u, v, nullptr, (double)o.w - 1e-3) != -2)
-                    add_lit(E, r);
-            }
-            pending = first;
-            __syncwarp();
-        }
-        if (last) break;
+        if (i >= n - stride) break;
     }
-    mine = __reduce_add_sync(kAll, mine);
-    if (lane == 0 && mine) atomicAdd(&C->shadow_rays, (unsigned long long)mine);
 }
 
 // ------------------------------------------------------------------ status

@@ -141,7 +141,7 @@ struct DScene {
 // Request flags
 constexpr int kReqSpectral = 1, kReqMIS = 2, kReqRussian = 4, kReqStratified = 8, kReqAdaptive = 16,
               kReqTerminate = 32, kReqCancelled = 64,
-              kReqWhole = 128;      // traced by k_paths (scene without a mesh), not through the queues
+              kReqFlat = 128;       // on a scene without a mesh: its paths never wait in the queues
 
 struct DRequest {
     int scene, width, height, depth;
@@ -165,37 +165,43 @@ struct DRequest {
     int sample0, local_spp;
 };
 
-// Path state, structure of arrays, one entry per queued path.
+// Paths whose next ray has a mesh to walk, structure of arrays, one entry per
+// path.
 struct PathQueue {
     float4* o;     // origin, hero lambda
     float4* d;     // direction, meta (bits): bounce | fork<<8 | single<<11 | n<<12
     float4* tp;    // throughput per channel
-    int4* id;      // request slot, pixel, sample, scene (copied by continuations and forks)
+    int4* id;      // request slot, pixel, sample, scene
     // XYZ weight of each carried wavelength, cmf(lambda_k) * 300/yBarIntegral / N
     // (spectral paths only): w[0] = x0 y0 z0 x1, w[1] = y1 z1 x2 y2, w[2] = z2 x3 y3 z3.
     // Computed once at raygen; a path's wavelengths never change.  In a scene
     // with one emissive material (DScene::emit_mat >= 0) each weight is
     // multiplied by that material's emission at the wavelength.
     float4* w[3];
+    // The ray's analytic hit (t, primitive), which k_extend replaces by a
+    // triangle's (t, primitive, u, v) where the mesh is hit first.
+    float4* hit;
 };
 
+// Shadow rays that have a mesh to walk.
 struct ShadowQueue {
-    float4* o;     // origin, lightDist2
+    float4* o;     // origin, lightDist2 (below zero: an unused record)
     float4* d;     // direction, pixel (bits)
     float4* c;     // contribution (XYZ or RGB), request slot | scene << 16 (bits)
+    float* bound;  // no hit at or past it matters
 };
 
 struct Counters {
     int queue_n[2];
     int shadow_n;
-    int new_n;
-    int new_base;
+    int new_n;            // mesh scenes: new paths of this iteration
     int iter;
     int status;           // non-zero: a kernel reported an error
     int idle;             // 1 when no request has work left
     int n_rounds;         // adaptive requests whose round ended this iteration (k_status -> k_round)
     unsigned long long rays, shadow_rays, paths;
-    int path_n, path_next;        // k_paths: paths of this launch, next one to take
+    int path_n;                   // scenes without a mesh: paths of this iteration
+    int next[3];                  // k_paths: paths taken without / with a mesh, queued paths taken up
     unsigned long long path_begin, path_end;  // plain k_paths: globaltimer at its setup and its last block's end
 };
 
@@ -205,10 +211,9 @@ struct EngineView {
     const DMaterial* mats;
     const DRequest* reqs;
     unsigned long long* issued;      // per slot
-    long long* outstanding;          // per slot
-    int* give;                       // per active position: paths this iteration
-    int* give_base;                  // per active position: exclusive prefix
-    int* path_base;                  // the same for the paths k_paths traces whole
+    long long* outstanding;          // per slot: paths waiting in the queue
+    int* give_base;                  // per active position: new paths of this iteration before it (mesh scenes)
+    int* path_base;                  // the same for requests on scenes without a mesh
     int* active;                     // active slot list (admission order)
     int* n_active;
     int* done_flag;                  // per slot: 1 once finished
@@ -216,12 +221,10 @@ struct EngineView {
     unsigned long long* t_done;      // per slot: globaltimer at completion
     Counters* cnt;
     PathQueue q[2];
-    float4* hit;
     ShadowQueue sq;
     long long* give_start;           // per active position: first path index issued
     int shadow_cap;                  // shadow-queue entries
     int queue_cap;                   // entries per path queue
-    int n_mats;
     int* round_state;                // per slot: 1 while an adaptive round's per-pixel step is pending
     int* round_cnt;                  // per slot: pixels kept for the next adaptive round
     int* round_list;                 // slots of Counters::n_rounds

@@ -1,42 +1,48 @@
-// Whole-path kernel for scenes without a triangle mesh.
+// The path kernel: raygen, analytic trace, shading and shadow rays.
 #pragma once
 
 #include "kernels.cuh"
 
 namespace pcr {
 
-// k_paths follows each path from its camera ray to its end in one thread:
-// closest hit, shading, shadow rays and the next direction, vertex after
-// vertex, with the path's state in registers.
+// k_paths follows each path in one thread, vertex after vertex, with its state
+// in registers: closest hit, shading, shadow rays, next direction.  On a scene
+// without a mesh (kMesh = false) it goes on to the path's end.  Where a ray
+// meets the mesh's box, the path waits in the queue for k_extend's walk and is
+// taken up again in the next iteration; a shadow ray that would be lit but
+// meets the box becomes a record for k_shadow.
 //
-// Why not the queue stages (k_extend / k_shade / k_shadow) here: a ray meets
-// at most a few dozen quads and spheres, so its trace is short, and what the
+// Why one kernel and not one per stage: a ray meets at most a few dozen quads
+// and spheres outside the mesh, so that part of its trace is short, and what
 // stages pass through memory outweighs it: 400 B of path and hit records per
 // vertex and 96 B per shadow ray, besides three FP64 reductions per lit
-// sample, and five launches per vertex of a path.  Mesh scenes keep the
-// queues, where the lanes of a warp at least start their long BVH walks
-// together.
+// sample, and five launches per vertex of a path.  The BVH walk is left out
+// because it needs its own registers and full warps: inlined here, six mesh
+// renders took 48 ms instead of 28.
 //
 // A warp keeps its lanes filled: a lane whose path has ended takes a pending
-// sub-path of a dispersive fork from the warp's stack, and when the stack is
-// empty and kPathRefill lanes wait (raygen costs about one vertex, so it is
-// not run for a lane or two at a time), they take the next camera paths from
-// a counter shared by the grid.
+// sub-path of a dispersive fork from the warp's stack, then a queued path, and
+// when kPathRefill lanes wait (raygen costs about one vertex, so it is not run
+// for a lane or two at a time), they take the next camera paths; queue and
+// camera paths are numbered by one counter shared by the grid.
 //
 // The samples of a path are added up in double and go to the pixel's FP64
-// accumulator once, when the path ends.
+// accumulator when the path ends or waits.
 //
-// What bounds it: instruction fetch and issue (46 % of the issue slots used, 23
+// What bounds it: instruction fetch and issue (50 % of the issue slots used, 24
 // of 32 lanes active; 16 warps per SM at 128 registers; waits for instructions
-// are the most frequent stall, as warps are spread over 40 KB of hot code).
-// 4 blocks per SM without spills beat 5 (96 registers, 180 B of spills) and 6.
-// Cornell 256x256, 16 paths a pixel, 4 vertices, 4 shadow rays: queue stages
-// 4.39 ms, first form of this kernel 1.02 ms.  64x64, one path a pixel:
-// 240 -> 98 us.  Refilling at 4 / 12 / 24 / 32 dead lanes: 1015 / 947 / 909 /
-// 900 us, 24 uneven renders 103.6 / 102.7 / 98.3 / 98.3 ms, adaptive rounds
-// 1569 / 1535 / 1537 / 1545 us.  Barriers that keep the warps of 256 or 512
-// threads at the same vertex: glass 4.84 -> 4.44 ms, everything else 2 to 15 %
-// slower.
+// are the most frequent stall, as warps are spread over 40 KB of hot code:
+// 1, 2, 3, 4 blocks per SM take 1923, 1173, 950, 842 us, but 5 and 6 blocks at
+// 96 and 80 registers 943 and 1034 us).  Cornell 256x256, 16 paths a pixel, 4
+// vertices, 4 shadow rays: stages of a queue 4.39 ms, this kernel 0.84 ms.
+// 64x64, one path a pixel: 240 -> 98 us.  Refilling at 4 / 12 / 24 / 32 dead
+// lanes: 1015 / 947 / 909 / 900 us, 24 uneven renders 103.6 / 102.7 / 98.3 /
+// 98.3 ms.  Barriers that keep the warps of a scheduler at the same vertex end
+// the instruction waits but cost as much in barrier waits.
+//
+// With a mesh, against queue stages of one vertex each: bunny 320x320, 8 paths
+// a pixel 4.97 -> 2.01 ms, 24 uneven renders 80.8 -> 75.6 ms; six renders half
+// of them through a glass mesh, where most vertices wait, 22.4 -> 26.0 ms.
 constexpr int kPathBlock = 128;
 #ifndef PCR_PATH_MIN_BLOCKS
 #define PCR_PATH_MIN_BLOCKS 4
@@ -50,11 +56,18 @@ constexpr int kPathRefill = PCR_PATH_REFILL;
 // pending entries + 3 x (lanes that may still fork) never exceed 3 x 32.
 constexpr int kForkStack = 96;
 constexpr int kForkWords = 14;
+// Queued paths are taken up when this many lanes wait (a few loads each).
+constexpr int kPathResume = 8;
+// Shadow records are reserved per warp in chunks, one grid-wide atomic each; a
+// warp takes a new chunk when fewer than kShadowLow are left, and marks what
+// it leaves unused.  Records past the chunk are reserved one by one.
+constexpr int kShadowChunk = 128, kShadowLow = 32;
 
 struct PathWarp {
     float w[12][32];                     // XYZ weights of each lane's path
     uint32_t fork[kForkWords][kForkStack];  // pending sub-paths
     int pending;
+    int shadow_next, shadow_end;         // the warp's chunk of shadow records
 };
 
 constexpr size_t kPathSmem = (kPathBlock / 32) * sizeof(PathWarp);
@@ -70,7 +83,7 @@ __global__ void k_one_request(EngineView E, DRequest r, long long first, int n)
     E.path_base[0] = 0;
     E.give_start[0] = first;
     C->path_n = n;
-    C->path_next = 0;
+    C->next[0] = 0;
     C->paths += (unsigned long long)n;
     if (first == 0) {
         unsigned long long t;
@@ -104,10 +117,34 @@ __device__ __forceinline__ void single_lane_weights(PathWarp& P, int lane, float
     for (int k = 3; k < 12; k++) P.w[k][lane] = 0.f;
 }
 
-// Work of one launch: Counters::path_n paths, numbered over the active list;
-// position r's paths start at path_base[r] and are the request's paths
-// give_start[r], give_start[r] + 1, ...
-__global__ void __launch_bounds__(kPathBlock, PCR_PATH_MIN_BLOCKS) k_paths(const __grid_constant__ EngineView E, float xyz_scale)
+// BVH walk of a shadow ray in place, for a full shadow queue.
+__device__ __noinline__ bool walk_blocked(const DScene& S, float3 o, float3 d, float bound, float d2)
+{
+    float u, v;
+    return bvh4_closest<false, true>(S, o, d, bound, u, v, nullptr, (double)d2 - 1e-3) == -2;
+}
+
+// Reserves shadow records: the first one, or shadow_cap when none is left.
+// (Past the cap the count grows by what is in flight at most, and shadow_cap
+// stays far enough below 2^31 for that.)
+__device__ __forceinline__ int shadow_slots(const EngineView& E, int count)
+{
+    int* next = &E.cnt->shadow_n;
+    return __ldcg(next) < E.shadow_cap ? min(atomicAdd(next, count), E.shadow_cap) : E.shadow_cap;
+}
+
+// Marks the rest of the warp's chunk as unused.
+__device__ __forceinline__ void close_shadow_chunk(const EngineView& E, const PathWarp& P, int lane)
+{
+    for (int k = P.shadow_next + lane; k < P.shadow_end; k += 32) E.sq.o[k] = make_float4(0.f, 0.f, 0.f, -1.f);
+}
+
+// Work of one launch: the paths of queue `cur` (kMesh), then the camera paths
+// numbered over the active list: position r's start at base[r] and are the
+// request's paths give_start[r], give_start[r] + 1, ...
+template <bool kMesh>
+__global__ void __launch_bounds__(kPathBlock, PCR_PATH_MIN_BLOCKS)
+k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
 {
     extern __shared__ __align__(16) unsigned char s_paths[];
     PathWarp& P = reinterpret_cast<PathWarp*>(s_paths)[threadIdx.x >> 5];
@@ -115,8 +152,12 @@ __global__ void __launch_bounds__(kPathBlock, PCR_PATH_MIN_BLOCKS) k_paths(const
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     Counters* C = E.cnt;
-    const int n = C->path_n, n_act = *E.n_active;
-    if (lane == 0) P.pending = 0;
+    const int* base = kMesh ? E.give_base : E.path_base;
+    int* counter = &C->next[kMesh ? 1 : 0];
+    const int queued = kMesh ? min(C->queue_n[cur], E.queue_cap) : 0;
+    const int n = queued + (kMesh ? C->new_n : C->path_n), n_act = *E.n_active;
+    int refill = queued > 0 ? kPathResume : kPathRefill;
+    if (lane == 0) P.pending = P.shadow_next = P.shadow_end = 0;
     __syncwarp();
 
     bool alive = false, more = n > 0;
@@ -125,8 +166,20 @@ __global__ void __launch_bounds__(kPathBlock, PCR_PATH_MIN_BLOCKS) k_paths(const
     float lambda0 = 0.f;
     int meta = 0, slot = 0;
     uint32_t pixel = 0, sample = 0;
+    bool traced = false;               // the ray's hit is known:
+    uint32_t prim = kPrimNone;
+    float t = 0.f, hu = 0.f, hv = 0.f;
     double ax = 0.0, ay = 0.0, az = 0.0;
     unsigned rays = 0, shadows = 0;
+    auto flush = [&]() {
+        if (ax != 0.0 || ay != 0.0 || az != 0.0) {
+            double* acc = E.reqs[slot].accum + (size_t)pixel * 3;
+            red_add(acc + 0, ax);
+            red_add(acc + 1, ay);
+            red_add(acc + 2, az);
+            ax = ay = az = 0.0;
+        }
+    };
 
     while (true) {
         // ---- refill
@@ -154,22 +207,45 @@ __global__ void __launch_bounds__(kPathBlock, PCR_PATH_MIN_BLOCKS) k_paths(const
                 __syncwarp();
                 dead = __ballot_sync(kAll, !alive);
             }
-            if (more && __popc(dead) >= kPathRefill) {
+            if (more && __popc(dead) >= refill) {
                 int first = 0;
-                if (lane == 0) first = atomicAdd(&C->path_next, __popc(dead));
+                if (lane == 0) first = atomicAdd(counter, __popc(dead));
                 first = __shfl_sync(kAll, first, 0);
                 more = first + __popc(dead) < n;
-                const int i = first + __popc(dead & below);
-                if (!alive && i < n) {
+                int i = first + __popc(dead & below);
+                if (kMesh) {
+                    if (!alive && i < queued) {
+                        const PathQueue& Q = E.q[cur];
+                        const int4 id = Q.id[i];
+                        const float4 o4 = Q.o[i], d4 = Q.d[i], h = Q.hit[i];
+                        tp = Q.tp[i];
+                        slot = id.x;
+                        pixel = (uint32_t)id.y;
+                        sample = (uint32_t)id.z;
+                        o = xyz(o4);
+                        d = xyz(d4);
+                        lambda0 = o4.w;
+                        meta = __float_as_int(d4.w);
+                        t = h.x;
+                        prim = __float_as_uint(h.y);
+                        hu = h.z;
+                        hv = h.w;
+                        set_lane_weights(P, lane, (E.reqs[slot].flags & kReqSpectral) ? load_weights(Q, i) : rgb_weights());
+                        alive = traced = true;
+                    }
+                    if (first + __popc(dead) >= queued) refill = kPathRefill;
+                    i -= queued;
+                }
+                if (!alive && i < n - queued) {
                     int lo = 0, hi = n_act - 1;
-                    while (lo < hi) {  // last r with path_base[r] <= i: it has paths in this launch
+                    while (lo < hi) {  // last r with base[r] <= i: it has paths in this launch
                         const int mid = (lo + hi + 1) >> 1;
-                        if (E.path_base[mid] <= i) lo = mid; else hi = mid - 1;
+                        if (base[mid] <= i) lo = mid; else hi = mid - 1;
                     }
                     slot = E.active[lo];
                     const DRequest& R = E.reqs[slot];
                     XyzWeights W = rgb_weights();
-                    const CameraPath p = camera_path(E, R, E.give_start[lo] + (i - E.path_base[lo]), xyz_scale, W);
+                    const CameraPath p = camera_path(E, R, E.give_start[lo] + (i - base[lo]), xyz_scale, W);
                     set_lane_weights(P, lane, W);
                     pixel = p.pixel;
                     sample = p.sample;
@@ -187,19 +263,60 @@ __global__ void __launch_bounds__(kPathBlock, PCR_PATH_MIN_BLOCKS) k_paths(const
             }
         }
 
+        // ---- trace
+        bool wait = false;
+        if (alive && !traced) {
+            const DScene& S = E.scenes[E.reqs[slot].scene];
+            rays++;
+            t = FLT_MAX;
+            prim = scene_analytic(S, o, d, t);
+            if (kMesh) wait = mesh_may_hit(S, o, d, t);
+        }
+        if (kMesh) {
+            const unsigned m = __ballot_sync(kAll, wait);
+            if (m) {
+                int at = 0;
+                if (lane == 0) at = atomicAdd(&C->queue_n[cur ^ 1], __popc(m));
+                at = __shfl_sync(kAll, at, 0) + __popc(m & below);
+                if (wait) {
+                    flush();
+                    alive = false;
+                    if (at < E.queue_cap) {
+                        const PathQueue& Q = E.q[cur ^ 1];
+                        const DRequest& R = E.reqs[slot];
+                        Q.o[at] = make_float4(o.x, o.y, o.z, lambda0);
+                        Q.d[at] = make_float4(d.x, d.y, d.z, __int_as_float(meta));
+                        Q.tp[at] = tp;
+                        Q.id[at] = make_int4(slot, (int)pixel, (int)sample, R.scene);
+                        Q.hit[at] = make_float4(t, __uint_as_float(prim), 0.f, 0.f);
+                        if (R.flags & kReqSpectral) store_weights(Q, at, lane_weights(P, lane));
+                    } else {
+                        atomicOr(&C->status, 2);
+                    }
+                }
+            }
+            if (P.shadow_end - P.shadow_next < kShadowLow) {  // shadow_next may lie past the end
+                close_shadow_chunk(E, P, lane);
+                __syncwarp();
+                if (lane == 0) {
+                    const int at = shadow_slots(E, kShadowChunk);
+                    P.shadow_next = at;
+                    P.shadow_end = min(at + kShadowChunk, E.shadow_cap);
+                }
+                __syncwarp();
+            }
+        }
+
         // ---- one vertex of each live path
         if (alive) {
             const DRequest& R = E.reqs[slot];
             const DScene& S = E.scenes[R.scene];
-            alive = false;
-            rays++;
-            float t = FLT_MAX;
-            const uint32_t prim = scene_analytic(S, o, d, t);
+            alive = traced = false;
             if (prim != kPrimNone) {
                 const int bounce = meta & 0xFF, fork = (meta >> 8) & 7, single = (meta >> 11) & 1, nHero = (meta >> 12) & 7;
                 const bool spectral = (R.flags & kReqSpectral) != 0;
                 const float4 lam4 = spectral ? path_wavelengths(lambda0, single, nHero) : make_float4(0.f, 0.f, 0.f, 0.f);
-                const Surface sf = surface_at<false>(S, prim, t, 0.f, 0.f, o, d);
+                const Surface sf = surface_at<kMesh>(S, prim, t, hu, hv, o, d);
                 const float3 hit = sf.hit;
                 float3 N = sf.N;
                 const bool entering = f3dot(d, N) < 0.f;
@@ -312,7 +429,8 @@ __global__ void __launch_bounds__(kPathBlock, PCR_PATH_MIN_BLOCKS) k_paths(const
                             if (!(g.G > 0.f)) continue;
                             shadows++;
                             float bound;
-                            if (scene_blocked_analytic<false>(S, E.mats, g.so, g.wi, g.d2, bound) == kShadowBlocked) continue;
+                            const int query = scene_blocked_analytic<kMesh>(S, E.mats, g.so, g.wi, g.d2, bound);
+                            if (query == kShadowBlocked) continue;
                             if (L.mat != cached) {
                                 // product of this light material, once per vertex
                                 const DMaterial& lmat = E.mats[S.mat_base + L.mat];
@@ -321,9 +439,22 @@ __global__ void __launch_bounds__(kPathBlock, PCR_PATH_MIN_BLOCKS) k_paths(const
                                 cached = L.mat;
                             }
                             const float f = shadow_factor(S, R, g);
-                            ax += (double)(V.x * f);
-                            ay += (double)(V.y * f);
-                            az += (double)(V.z * f);
+                            const float3 c = make_float3(V.x * f, V.y * f, V.z * f);
+                            if (kMesh && query == kShadowWalk && mesh_may_hit(S, g.so, g.wi, bound)) {
+                                int at = atomicAdd(&P.shadow_next, 1);
+                                if (at >= P.shadow_end) at = shadow_slots(E, 1);
+                                if (at < E.shadow_cap) {
+                                    E.sq.o[at] = make_float4(g.so.x, g.so.y, g.so.z, g.d2);
+                                    E.sq.d[at] = make_float4(g.wi.x, g.wi.y, g.wi.z, __int_as_float((int)pixel));
+                                    E.sq.c[at] = make_float4(c.x, c.y, c.z, __int_as_float(slot | (R.scene << 16)));
+                                    E.sq.bound[at] = bound;
+                                    continue;
+                                }
+                                if (walk_blocked(S, g.so, g.wi, bound, g.d2)) continue;
+                            }
+                            ax += (double)c.x;
+                            ay += (double)c.y;
+                            az += (double)c.z;
                         }
                     }
                     float3 nd;
@@ -337,16 +468,11 @@ __global__ void __launch_bounds__(kPathBlock, PCR_PATH_MIN_BLOCKS) k_paths(const
                     }
                 }
             }
-            if (!alive && (ax != 0.0 || ay != 0.0 || az != 0.0)) {
-                double* acc = R.accum + (size_t)pixel * 3;
-                red_add(acc + 0, ax);
-                red_add(acc + 1, ay);
-                red_add(acc + 2, az);
-                ax = ay = az = 0.0;
-            }
+            if (!alive) flush();
         }
         __syncwarp();
     }
+    if (kMesh) close_shadow_chunk(E, P, lane);
     rays = __reduce_add_sync(kAll, rays);
     shadows = __reduce_add_sync(kAll, shadows);
     if (lane == 0 && rays) {
