@@ -710,11 +710,9 @@ inline unsigned blocks(long long n, int per) { return (unsigned)((n + per - 1) /
 
 }  // namespace
 
-void device_build_bvh_raw(int device, cudaStream_t st, cudaMemPool_t pool, const float* verts9, int n,
-                          std::vector<pcr_bvh_node>& nodes, std::vector<int32_t>& order)
+void device_build_bvh(int device, cudaStream_t st, cudaMemPool_t pool, int n, const std::function<void(float*)>& put,
+                      const std::function<void(const pcr_bvh_node*, int, const int*)>& take)
 {
-    nodes.clear();
-    order.clear();
     if (n <= 0) return;
     if (n > (1 << 28)) throw PcrError(PCR_ERR_INVALID, "BVH build: more than 2^28 triangles");
     BK(cudaSetDevice(device));
@@ -757,7 +755,7 @@ void device_build_bvh_raw(int device, cudaStream_t st, cudaMemPool_t pool, const
     int* bcnt = reinterpret_cast<int*>(base + o_bcnt);
     BuildCounters* ctr = reinterpret_cast<BuildCounters*>(base + o_ctr);
 
-    BK(cudaMemcpyAsync(d_verts, verts9, N * 9 * sizeof(float), cudaMemcpyHostToDevice, st));
+    put(d_verts);
     k_bvh_prep<<<blocks(n, 256), 256, 0, st>>>(d_verts, n, T, perm);
     BK(cudaGetLastError());
 
@@ -851,40 +849,8 @@ void device_build_bvh_raw(int device, cudaStream_t st, cudaMemPool_t pool, const
     k_bvh_emit_top<<<blocks(ntop, 128), 128, 0, st>>>(top, ntop, pre, out);
     if (nsmall) k_bvh_emit_small<<<blocks((long long)nsmall * 32, 256), 256, 0, st>>>(small, nsmall, pre, region, out, (int)total);
     BK(cudaGetLastError());
-    nodes.resize((size_t)total);
-    order.resize(N);
-    BK(cudaMemcpyAsync(nodes.data(), out, (size_t)total * sizeof(pcr_bvh_node), cudaMemcpyDeviceToHost, st));
-    BK(cudaMemcpyAsync(order.data(), perm, N * 4, cudaMemcpyDeviceToHost, st));
+    take(out, (int)total, perm);
     BK(cudaStreamSynchronize(st));
-}
-
-std::vector<pcr_bvh_node> device_build_bvh(int device, cudaStream_t st, cudaMemPool_t pool,
-                                           std::vector<pcr_triangle>& tris, std::vector<int32_t>* ids)
-{
-    std::vector<pcr_bvh_node> nodes;
-    std::vector<int32_t> order;
-    const int n = (int)tris.size();
-    std::vector<float> v((size_t)n * 9);
-    parallel_for(n, [&](int lo, int hi) {
-        for (int i = lo; i < hi; i++)
-            for (int a = 0; a < 3; a++) {
-                v[(size_t)i * 9 + a] = tris[i].v0[a];
-                v[(size_t)i * 9 + 3 + a] = tris[i].v1[a];
-                v[(size_t)i * 9 + 6 + a] = tris[i].v2[a];
-            }
-    });
-    device_build_bvh_raw(device, st, pool, v.data(), n, nodes, order);
-    std::vector<pcr_triangle> t2(tris.size());
-    std::vector<int32_t> i2(ids ? ids->size() : 0);
-    parallel_for(n, [&](int lo, int hi) {
-        for (int i = lo; i < hi; i++) {
-            t2[i] = tris[order[i]];
-            if (ids) i2[i] = (*ids)[order[i]];
-        }
-    });
-    tris.swap(t2);
-    if (ids) ids->swap(i2);
-    return nodes;
 }
 
 }  // namespace pcr

@@ -4,22 +4,19 @@
 
 #include <cuda_runtime.h>
 
-#include <cstdint>
-#include <vector>
+#include <functional>
 
 #include "../../include/pcr_cuda.h"
 
 namespace pcr {
 
-// verts9: n triangles as v0 v1 v2 (9 floats each).  Returns the nodes in
-// depth-first preorder and order[i] = input index of the triangle at leaf
-// position i.  Synchronous on `st`; the workspace (about 360 bytes per
-// triangle) comes from `pool` (null: the device's default pool).
-void device_build_bvh_raw(int device, cudaStream_t st, cudaMemPool_t pool, const float* verts9, int n,
-                          std::vector<pcr_bvh_node>& nodes, std::vector<int32_t>& order);
-
-// As build_bvh: permutes tris (and ids) into leaf order and returns the nodes.
-std::vector<pcr_bvh_node> device_build_bvh(int device, cudaStream_t st, cudaMemPool_t pool,
-                                           std::vector<pcr_triangle>& tris, std::vector<int32_t>* ids);
+// put(d_verts) uploads the n triangles as v0 v1 v2 (9 floats each), ordered on
+// `st`; take(d_nodes, count, d_order) receives the nodes in depth-first preorder
+// and, per leaf position, the input index of its triangle, on the device,
+// ordered on `st` and valid until it returns.  Synchronous; the workspace
+// (about 360 bytes per triangle) comes from `pool` (null: the device's default
+// pool).
+void device_build_bvh(int device, cudaStream_t st, cudaMemPool_t pool, int n, const std::function<void(float*)>& put,
+                      const std::function<void(const pcr_bvh_node*, int, const int*)>& take);
 
 }  // namespace pcr

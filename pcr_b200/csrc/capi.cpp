@@ -87,7 +87,11 @@ void device_bvh(pcr::Engine& e, pcr::HostScene& s)
     const int n = (int)s.triangles.size();
     if (n == 0) return;
     std::vector<int32_t> order;
-    e.build_bvh(s.triangles.data(), n, s.bvh, order);
+    order.resize(n);
+    e.build_bvh(s.triangles.data(), n, [&](int count) {
+        s.bvh.resize(count);
+        return s.bvh.data();
+    }, order.data());
     std::vector<pcr_triangle> t(n);
     std::vector<int32_t> ids(n);
     pcr::parallel_for(n, [&](int lo, int hi) {
@@ -475,13 +479,13 @@ pcr_status pcr_bvh_build(pcr_ctx* ctx, const pcr_triangle* tris, int32_t n, pcr_
     return guard([&] {
         if (n < 0 || max_nodes < 0) throw pcr::PcrError(PCR_ERR_INVALID, "negative count");
         if (!n_nodes || (n > 0 && (!tris || !order_out || !nodes_out))) throw pcr::PcrError(PCR_ERR_INVALID, "null argument");
-        std::vector<pcr_bvh_node> nodes;
-        std::vector<int32_t> order;
-        E(ctx).build_bvh(tris, n, nodes, order);
-        if ((int64_t)nodes.size() > max_nodes) throw pcr::PcrError(PCR_ERR_INVALID, "nodes_out too small");
-        std::copy(nodes.begin(), nodes.end(), nodes_out);
-        std::copy(order.begin(), order.end(), order_out);
-        *n_nodes = (int32_t)nodes.size();
+        int total = 0;
+        E(ctx).build_bvh(tris, n, [&](int count) {
+            if (count > max_nodes) throw pcr::PcrError(PCR_ERR_INVALID, "nodes_out too small");
+            total = count;
+            return nodes_out;
+        }, order_out);
+        *n_nodes = total;
     });
 }
 

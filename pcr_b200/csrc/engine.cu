@@ -157,7 +157,6 @@ Engine::~Engine()
             if (r.act[k]) cudaFreeAsync(r.act[k], stream_);
         if (r.welford) cudaFreeAsync(r.welford, stream_);
         if (r.d_hdr) cudaFreeAsync(r.d_hdr, stream_);
-        if (r.d_rgb) cudaFreeAsync(r.d_rgb, stream_);
         if (r.ev_ready) cudaEventDestroy(r.ev_ready);
     }
     cudaStreamSynchronize(stream_);
@@ -165,6 +164,7 @@ Engine::~Engine()
     for (Staging& st : staging_idle_) {
         cudaStreamSynchronize(st.stream);
         if (st.buf) cudaFreeHost(st.buf);
+        for (cudaEvent_t& e : st.piece) cudaEventDestroy(e);
         cudaStreamDestroy(st.stream);
     }
     for (auto& s : scenes_)
@@ -609,10 +609,19 @@ int Engine::upload_scene(const pcr_scene_desc& d)
         if (d.n_bvh_nodes > 0 && d.bvh_nodes) {
             bvh.assign(d.bvh_nodes, d.bvh_nodes + d.n_bvh_nodes);
         } else {
-            own_tris.assign(d.triangles, d.triangles + d.n_triangles);
+            std::vector<int32_t> order(d.n_triangles);
+            build_bvh_locked(d.triangles, d.n_triangles, [&](int count) {
+                bvh.resize(count);
+                return bvh.data();
+            }, order.data());
+            own_tris.resize(d.n_triangles);
             own_ids.resize(d.n_triangles);
-            for (int i = 0; i < d.n_triangles; i++) own_ids[i] = d.triangle_ids ? d.triangle_ids[i] : i;
-            bvh = device_build_bvh(device_, stream_, pool_, own_tris, &own_ids);
+            parallel_for(d.n_triangles, [&](int lo, int hi) {
+                for (int i = lo; i < hi; i++) {
+                    own_tris[i] = d.triangles[order[i]];
+                    own_ids[i] = d.triangle_ids ? d.triangle_ids[order[i]] : order[i];
+                }
+            });
             tris = own_tris.data();
             ids = own_ids.data();
         }
@@ -984,8 +993,8 @@ void Engine::alloc_request(Request& r)
     const int64_t px = (int64_t)r.desc.width * r.desc.height;
     CK(cudaMallocFromPoolAsync(&r.accum, px * 3 * sizeof(double), pool_, stream_));
     CK(cudaMemsetAsync(r.accum, 0, px * 3 * sizeof(double), stream_));
-    CK(cudaMallocFromPoolAsync(&r.d_hdr, px * 3 * sizeof(float), pool_, stream_));
-    CK(cudaMallocFromPoolAsync(&r.d_rgb, px * 3, pool_, stream_));
+    CK(cudaMallocFromPoolAsync(&r.d_hdr, px * 3 * (sizeof(float) + 1), pool_, stream_));
+    r.d_rgb = reinterpret_cast<uint8_t*>(r.d_hdr + px * 3);  // one block: fetched in one transfer
 }
 
 void Engine::activate(Request& r, int slot)
@@ -1205,17 +1214,19 @@ void Engine::finish_request(Request& r, cudaStream_t rs)
 // and releases it.
 void Engine::release_cancelled(Request& r)
 {
-    for (void** p : {(void**)&r.accum, (void**)&r.d_hdr, (void**)&r.d_rgb, (void**)&r.act[0], (void**)&r.act[1],
-                     (void**)&r.welford})
+    for (void** p : {(void**)&r.accum, (void**)&r.d_hdr, (void**)&r.act[0], (void**)&r.act[1], (void**)&r.welford})
         if (*p) { CK(cudaFreeAsync(*p, stream_)); *p = nullptr; }
+    r.d_rgb = nullptr;
     r.state = ReqState::Cancelled;
     r.t_ready = std::chrono::steady_clock::now();
 }
 
-// A pinned staging buffer of at least `bytes` with its copy stream: an idle
-// one when one is large enough, else an idle one grown, else a new one.
+// A pinned staging buffer of at least min(bytes, kStagingBytes) with its copy
+// stream: an idle one when one is large enough, else an idle one grown, else
+// a new one.
 Engine::Staging Engine::take_staging(size_t bytes)
 {
+    bytes = std::min(bytes, kStagingBytes);
     Staging st;
     {
         std::lock_guard<std::mutex> g(staging_mu_);
@@ -1230,7 +1241,10 @@ Engine::Staging Engine::take_staging(size_t bytes)
             staging_idle_.erase(staging_idle_.begin() + pick);
         }
     }
-    if (!st.stream) CK(cudaStreamCreateWithFlags(&st.stream, cudaStreamNonBlocking));
+    if (!st.stream) {
+        CK(cudaStreamCreateWithFlags(&st.stream, cudaStreamNonBlocking));
+        for (cudaEvent_t& e : st.piece) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
     if (st.bytes < bytes) {
         if (st.buf) CK(cudaFreeHost(st.buf));
         st.buf = nullptr;
@@ -1247,31 +1261,78 @@ void Engine::give_staging(const Staging& st)
     staging_idle_.push_back(st);
 }
 
-// Copies a resolved request's images to caller host buffers through a
-// pinned staging buffer on its own copy stream (ordered after the resolve by
-// the request's event), then frees its device images.
+void Engine::upload_items(void* dev, size_t items, size_t item_bytes, const Fill& fill, cudaStream_t after)
+{
+    if (!items) return;
+    StagingHold hold{this, take_staging(items * item_bytes)};
+    const Staging& st = hold.st;
+    CK(cudaEventRecord(st.piece[0], after));  // earlier work on the target
+    CK(cudaStreamWaitEvent(st.stream, st.piece[0], 0));
+    const size_t round = std::max<size_t>(1, st.bytes / item_bytes);
+    for (size_t first = 0; first < items; first += round) {
+        const size_t count = std::min(round, items - first);
+        fill(st.buf, first, count);
+        CK(cudaMemcpyAsync((uint8_t*)dev + first * item_bytes, st.buf, count * item_bytes, cudaMemcpyHostToDevice, st.stream));
+        CK(cudaStreamSynchronize(st.stream));  // the buffer is filled again, or handed back
+    }
+}
+
+// The bus carries the later pieces while an earlier one is copied on to the
+// caller's memory, on one thread: with the pieces spread over workers, fresh
+// result arrays (whose pages are mapped as they are written) took 1.3 to 1.7
+// times as long.
+void Engine::download_parts(const void* dev, std::initializer_list<HostPart> parts, cudaStream_t after, cudaEvent_t ready)
+{
+    // the wanted range
+    size_t total = 0, begin = SIZE_MAX, end = 0;
+    for (const HostPart& p : parts) {
+        if (p.host && p.bytes) {
+            begin = std::min(begin, total);
+            end = total + p.bytes;
+        }
+        total += p.bytes;
+    }
+    if (begin >= end) return;
+    StagingHold hold{this, take_staging(end - begin)};
+    const Staging& st = hold.st;
+    if (!ready) {
+        CK(cudaEventRecord(st.piece[0], after));
+        ready = st.piece[0];
+    }
+    CK(cudaStreamWaitEvent(st.stream, ready, 0));
+    constexpr size_t kPieceBytes = 1u << 20;
+    for (size_t first = begin; first < end; first += st.bytes) {
+        const size_t count = std::min(st.bytes, end - first);
+        const int pieces = (int)std::min<size_t>(kPieces, (count + kPieceBytes - 1) / kPieceBytes);
+        for (int k = 0; k < pieces; k++) {
+            const size_t lo = count * k / pieces, hi = count * (k + 1) / pieces;
+            CK(cudaMemcpyAsync(st.buf + lo, (const uint8_t*)dev + first + lo, hi - lo, cudaMemcpyDeviceToHost, st.stream));
+            CK(cudaEventRecord(st.piece[k], st.stream));
+        }
+        for (int k = 0; k < pieces; k++) {
+            const size_t lo = first + count * k / pieces, hi = first + count * (k + 1) / pieces;
+            CK(cudaEventSynchronize(st.piece[k]));
+            size_t at = 0;
+            for (const HostPart& p : parts) {
+                const size_t a = std::max(lo, at), z = std::min(hi, at + p.bytes);
+                if (p.host && a < z) std::memcpy((uint8_t*)p.host + (a - at), st.buf + (a - first), z - a);
+                at += p.bytes;
+            }
+        }
+    }
+}
+
+// Copies a resolved request's images (ordered after the resolve by the
+// request's event) to caller host buffers, then frees them on the device.
 void Engine::copy_out(Request& r, float* hdr, uint8_t* rgb)
 {
-    const int64_t px = (int64_t)r.desc.width * r.desc.height;
-    const size_t need = (hdr || rgb) ? (size_t)px * 3 * (sizeof(float) + 1) : 0;
-    struct Hold {  // hands the buffer back on every exit path
-        Engine* e;
-        Staging st;
-        ~Hold() { e->give_staging(st); }
-    } hold{this, take_staging(need)};
-    const Staging& st = hold.st;
-    CK(cudaStreamWaitEvent(st.stream, r.ev_ready, 0));
-    float* sh = reinterpret_cast<float*>(st.buf);
-    uint8_t* sr = st.buf ? st.buf + px * 3 * sizeof(float) : nullptr;
-    if (hdr) CK(cudaMemcpyAsync(sh, r.d_hdr, px * 3 * sizeof(float), cudaMemcpyDeviceToHost, st.stream));
-    if (rgb) CK(cudaMemcpyAsync(sr, r.d_rgb, px * 3, cudaMemcpyDeviceToHost, st.stream));
-    CK(cudaFreeAsync(r.d_hdr, st.stream));
-    CK(cudaFreeAsync(r.d_rgb, st.stream));
+    const size_t px = (size_t)r.desc.width * r.desc.height;
+    if (hdr || rgb) download_parts(r.d_hdr, {{hdr, px * 3 * sizeof(float)}, {rgb, px * 3}}, nullptr, r.ev_ready);
+    else CK(cudaEventSynchronize(r.ev_ready));
+    // (not on stream_, which the serving thread may be capturing)
+    CK(cudaFreeAsync(r.d_hdr, resolve_stream_));
     r.d_hdr = nullptr;
     r.d_rgb = nullptr;
-    CK(cudaStreamSynchronize(st.stream));
-    if (hdr) std::memcpy(hdr, sh, px * 3 * sizeof(float));
-    if (rgb) std::memcpy(rgb, sr, px * 3);
 }
 
 void Engine::harvest(bool)
@@ -1943,30 +2004,23 @@ void Engine::trace(int scene, const float* rays, int64_t n, int32_t* mat, int32_
     CK(cudaSetDevice(device_));
     if (scene < 0 || scene >= (int)scenes_.size() || !scenes_[scene].live) throw PcrError(PCR_ERR_NOT_FOUND, "unknown scene");
     if (n <= 0) return;
+    // outputs one after another: material, primitive, t, counts
+    const size_t N = (size_t)n;
     float* d_rays = nullptr;
-    int *d_mat = nullptr, *d_prim = nullptr, *d_cnt = nullptr;
-    float* d_t = nullptr;
-    CK(cudaMallocFromPoolAsync(&d_rays, n * 6 * sizeof(float), pool_, stream_));
-    CK(cudaMallocFromPoolAsync(&d_mat, n * sizeof(int), pool_, stream_));
-    CK(cudaMallocFromPoolAsync(&d_prim, n * sizeof(int), pool_, stream_));
-    CK(cudaMallocFromPoolAsync(&d_t, n * sizeof(float), pool_, stream_));
-    if (counts) CK(cudaMallocFromPoolAsync(&d_cnt, n * 2 * sizeof(int), pool_, stream_));
-    CK(cudaMemcpyAsync(d_rays, rays, n * 6 * sizeof(float), cudaMemcpyHostToDevice, stream_));
+    int* d_out = nullptr;
+    CK(cudaMallocFromPoolAsync(&d_rays, N * 6 * sizeof(float), pool_, stream_));
+    CK(cudaMallocFromPoolAsync(&d_out, N * (counts ? 5 : 3) * sizeof(int), pool_, stream_));
+    CK(cudaMemcpyAsync(d_rays, rays, N * 6 * sizeof(float), cudaMemcpyHostToDevice, stream_));
     int grid = 0;
     grid_for((const void*)k_trace_rays, 128, 0, &grid);
     if (profile_) CK(cudaEventRecord(prof_ev_[0], stream_));
-    k_trace_rays<<<grid, 128, 0, stream_>>>(d_scenes_ + scene, d_mats_, d_rays, n, d_mat, d_prim, d_t, bvh_only, d_cnt);
+    k_trace_rays<<<grid, 128, 0, stream_>>>(d_scenes_ + scene, d_mats_, d_rays, n, d_out, d_out + N, (float*)(d_out + 2 * N),
+                                            bvh_only, counts ? d_out + 3 * N : nullptr);
     CK(cudaGetLastError());
     if (profile_) record_other(prof_ev_[0], prof_ev_[1]);
-    if (mat) CK(cudaMemcpyAsync(mat, d_mat, n * sizeof(int), cudaMemcpyDeviceToHost, stream_));
-    if (prim) CK(cudaMemcpyAsync(prim, d_prim, n * sizeof(int), cudaMemcpyDeviceToHost, stream_));
-    if (t) CK(cudaMemcpyAsync(t, d_t, n * sizeof(float), cudaMemcpyDeviceToHost, stream_));
-    if (counts) CK(cudaMemcpyAsync(counts, d_cnt, n * 2 * sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    download_parts(d_out, {{mat, N * 4}, {prim, N * 4}, {t, N * 4}, {counts, counts ? N * 8 : 0}}, stream_);
     CK(cudaFreeAsync(d_rays, stream_));
-    CK(cudaFreeAsync(d_mat, stream_));
-    CK(cudaFreeAsync(d_prim, stream_));
-    CK(cudaFreeAsync(d_t, stream_));
-    if (d_cnt) CK(cudaFreeAsync(d_cnt, stream_));
+    CK(cudaFreeAsync(d_out, stream_));
     CK(cudaStreamSynchronize(stream_));
 }
 
@@ -1981,19 +2035,37 @@ void Engine::record_other(cudaEvent_t a, cudaEvent_t z)
     stage_launches_[7]++;
 }
 
-void Engine::build_bvh(const pcr_triangle* tris, int n, std::vector<pcr_bvh_node>& nodes, std::vector<int32_t>& order)
+void Engine::build_bvh(const pcr_triangle* tris, int n, const std::function<pcr_bvh_node*(int)>& nodes, int32_t* order)
 {
     std::lock_guard<std::mutex> g(run_mu_);
-    std::vector<float> v((size_t)n * 9);
-    parallel_for(n, [&](int lo, int hi) {
-        for (int i = lo; i < hi; i++)
-            for (int a = 0; a < 3; a++) {
-                v[(size_t)i * 9 + a] = tris[i].v0[a];
-                v[(size_t)i * 9 + 3 + a] = tris[i].v1[a];
-                v[(size_t)i * 9 + 6 + a] = tris[i].v2[a];
-            }
-    });
-    device_build_bvh_raw(device_, stream_, pool_, v.data(), n, nodes, order);
+    build_bvh_locked(tris, n, nodes, order);
+}
+
+void Engine::build_bvh_locked(const pcr_triangle* tris, int n, const std::function<pcr_bvh_node*(int)>& nodes, int32_t* order)
+{
+    device_build_bvh(
+        device_, stream_, pool_, n,
+        [&](float* d_verts) {
+            upload_items(d_verts, n, 9 * sizeof(float), [&](uint8_t* dst, size_t first, size_t count) {
+                auto pack = [&](int lo, int hi) {
+                    for (int i = lo; i < hi; i++) {
+                        float* v = reinterpret_cast<float*>(dst) + (size_t)i * 9;
+                        const pcr_triangle& t = tris[first + i];
+                        std::memcpy(v, t.v0, 12);
+                        std::memcpy(v + 3, t.v1, 12);
+                        std::memcpy(v + 6, t.v2, 12);
+                    }
+                };
+                // starting threads costs more than packing a few 100,000
+                if (count < (256u << 10)) pack(0, (int)count);
+                else parallel_for((int)count, pack);
+            }, stream_);
+        },
+        [&](const pcr_bvh_node* d_nodes, int count, const int* d_order) {
+            pcr_bvh_node* to = nodes(count);
+            download_parts(d_nodes, {{to, (size_t)count * sizeof(pcr_bvh_node)}}, stream_);
+            download_parts(d_order, {{order, (size_t)n * sizeof(int32_t)}}, stream_);
+        });
 }
 
 void Engine::trace_shadow(int scene, const float* rays, const float* dist2, int64_t n, int32_t* blocked)
@@ -2015,7 +2087,7 @@ void Engine::trace_shadow(int scene, const float* rays, const float* dist2, int6
     k_trace_shadow<<<grid, 128, 0, stream_>>>(d_scenes_ + scene, d_mats_, d_rays, d_d2, n, d_b);
     CK(cudaGetLastError());
     if (profile_) record_other(prof_ev_[0], prof_ev_[1]);
-    CK(cudaMemcpyAsync(blocked, d_b, n * sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    download_parts(d_b, {{blocked, n * sizeof(int)}}, stream_);
     CK(cudaFreeAsync(d_rays, stream_));
     CK(cudaFreeAsync(d_d2, stream_));
     CK(cudaFreeAsync(d_b, stream_));
@@ -2041,7 +2113,7 @@ void Engine::tonemap(const float* hdr, int width, int height, int aces_tm, int d
         k_bilateral<<<grid, 256, 0, stream_>>>(d_tmp, d_rgb, width, height);
     }
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(rgb8, d_rgb, px * 3, cudaMemcpyDeviceToHost, stream_));
+    download_parts(d_rgb, {{rgb8, (size_t)px * 3}}, stream_);
     CK(cudaFreeAsync(d_hdr, stream_));
     CK(cudaFreeAsync(d_rgb, stream_));
     if (d_tmp) CK(cudaFreeAsync(d_tmp, stream_));

@@ -8,6 +8,8 @@
 #include <condition_variable>
 #include <cstdint>
 #include <deque>
+#include <functional>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -94,7 +96,8 @@ public:
                int32_t* counts);
     void record_other(cudaEvent_t a, cudaEvent_t z);
     void trace_shadow(int scene, const float* rays, const float* dist2, int64_t n, int32_t* blocked);
-    void build_bvh(const pcr_triangle* tris, int n, std::vector<pcr_bvh_node>& nodes, std::vector<int32_t>& order);
+    // Device BVH build; `nodes(count)` returns where the nodes go.
+    void build_bvh(const pcr_triangle* tris, int n, const std::function<pcr_bvh_node*(int)>& nodes, int32_t* order);
     void tonemap(const float* hdr, int width, int height, int aces_tm, int denoise, uint8_t* rgb8);
     void eval_stage(int what, const float* params, const float* in, int64_t n, float* out);
     double l2_bandwidth(int64_t bytes, int reps);
@@ -108,6 +111,7 @@ public:
     cudaStream_t stream() const { return stream_; }
 
 private:
+    void build_bvh_locked(const pcr_triangle* tris, int n, const std::function<pcr_bvh_node*(int)>& nodes, int32_t* order);
     void ensure_shadow_capacity(int shadow_samples);
     void alloc_buffers();
     void free_buffers();
@@ -148,18 +152,45 @@ private:
     // queued on stream_: a request is harvested from the device state copied
     // after the block it finished in, by which point its accumulator is final.
     cudaStream_t resolve_stream_ = nullptr;
-    // Result copies: pinned staging buffers, each with its own copy stream,
-    // kept idle between fetches.  A fetch takes one (or makes one), so
-    // fetches from several threads copy at the same time.
+    // Pinned staging buffers, each with its own copy stream and an event per
+    // piece, kept idle between transfers.  A transfer takes one (or makes
+    // one), so fetches from several threads copy at the same time.  A buffer
+    // holds at most kStagingBytes: longer transfers pass through it in rounds.
+    static constexpr size_t kStagingBytes = 32u << 20;
+    static constexpr int kPieces = 16;
     struct Staging {
         uint8_t* buf = nullptr;
         size_t bytes = 0;
         cudaStream_t stream = nullptr;
+        cudaEvent_t piece[kPieces] = {};
     };
     std::mutex staging_mu_;
     std::vector<Staging> staging_idle_;
     Staging take_staging(size_t bytes);
     void give_staging(const Staging& s);
+    struct StagingHold {  // hands the buffer back on every exit path, its copies done
+        Engine* e;
+        Staging st;
+        ~StagingHold()
+        {
+            cudaStreamSynchronize(st.stream);
+            e->give_staging(st);
+        }
+    };
+    // Uploads `items` items that fill(dst, first, count) writes into pinned
+    // memory.  Ordered after the work on `after`; returns when they are on the
+    // device.
+    typedef std::function<void(uint8_t*, size_t, size_t)> Fill;
+    void upload_items(void* dev, size_t items, size_t item_bytes, const Fill& fill, cudaStream_t after);
+    // Downloads a device range that holds the parts one after another (a null
+    // host pointer: not wanted), ordered after `ready`, or after the work on
+    // `after` when that is null.
+    struct HostPart {
+        void* host;
+        size_t bytes;
+    };
+    void download_parts(const void* dev, std::initializer_list<HostPart> parts, cudaStream_t after,
+                        cudaEvent_t ready = nullptr);
     EngineTuning tune_;
     bool use_graph_ = true, profile_ = false;
     int64_t budget_ = 40ll << 30;
