@@ -153,6 +153,30 @@ __device__ void sah_axis(const float (*bmn)[3], const float (*bmx)[3], const int
     }
 }
 
+// Four threads share a node: threads 0 to 2 sweep an axis each, and all four
+// take the best of the three in axis order, as the sequential loop's strict
+// `<` does.
+struct Quad {
+    unsigned mask;
+    int lane, base;
+    __device__ __forceinline__ Quad() : lane(threadIdx.x & 3), base(threadIdx.x & 28) { mask = 0xfu << base; }
+    __device__ __forceinline__ void best(float& cost, int& axis, int& bin, int& lc) const
+    {
+        float c0 = FLT_MAX;
+        int a0 = -1, b0 = 0, l0 = 0;
+        for (int a = 0; a < 3; a++) {
+            const float c = __shfl_sync(mask, cost, base + a);
+            const int x = __shfl_sync(mask, axis, base + a), b = __shfl_sync(mask, bin, base + a),
+                      l = __shfl_sync(mask, lc, base + a);
+            if (x >= 0 && c < c0) { c0 = c; a0 = x; b0 = b; l0 = l; }
+        }
+        cost = c0;
+        axis = a0;
+        bin = b0;
+        lc = l0;
+    }
+};
+
 __global__ void k_bvh_prep(const float* __restrict__ verts, int n, BTri* __restrict__ T, int* __restrict__ perm)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -319,7 +343,7 @@ struct LevelOut {
     int2* chunks;
 };
 
-// The SAH decision of every large node (one thread per node); writes the
+// The SAH decision of every large node (four threads per node); writes the
 // node, allocates its children and queues them for the next level or for a
 // thread of their own.
 __global__ void k_bvh_split(const BTri* __restrict__ T, const int* __restrict__ perm, BTask* __restrict__ tasks,
@@ -327,7 +351,8 @@ __global__ void k_bvh_split(const BTri* __restrict__ T, const int* __restrict__ 
                             TopNode* __restrict__ top, SmallTask* __restrict__ small, LevelOut next,
                             BuildCounters* __restrict__ ctr, Caps cap)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const Quad quad;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
     if (i >= ntasks) return;
     BTask& t = tasks[i];
     TopNode& N = top[t.slot];
@@ -337,17 +362,18 @@ __global__ void k_bvh_split(const BTri* __restrict__ T, const int* __restrict__ 
         const unsigned smax = 0xffffffffu - (unsigned)(t.kmax[a] & 0xffffffffu);
         box_mn[a] = getc(T[perm[smin / 3]].lo, a);
         box_mx[a] = getc(T[perm[smax / 3]].hi, a);
-        N.bmin[a] = box_mn[a];
-        N.bmax[a] = box_mx[a];
+        if (quad.lane == 0) {
+            N.bmin[a] = box_mn[a];
+            N.bmax[a] = box_mx[a];
+        }
     }
     const int count = t.count;
     int best_axis = -1, best_bin = -1, best_lc = 0;
     float best_cost = FLT_MAX;
     const float parent = box_area(box_mn, box_mx);
     if (parent > 0.f) {
-        for (int a = 0; a < 3; a++) {
-            const AxisBin ab = axis_bin(t, a);
-            if (!ab.use) continue;
+        const int a = quad.lane;
+        if (a < 3 && axis_bin(t, a).use) {
             float bmn[kBins][3], bmx[kBins][3];
             int cnt[kBins];
             for (int b = 0; b < kBins; b++) {
@@ -361,6 +387,8 @@ __global__ void k_bvh_split(const BTri* __restrict__ T, const int* __restrict__ 
             sah_axis(bmn, bmx, cnt, parent, a, best_cost, best_axis, best_bin, best_lc);
         }
     }
+    quad.best(best_cost, best_axis, best_bin, best_lc);
+    if (quad.lane != 0) return;
     t.axis = -1;
     const int mid = t.begin + best_lc;
     if (best_axis < 0 || best_cost >= __fmul_rn((float)count, 2.f) || mid == t.begin || mid == t.begin + count) {
@@ -442,28 +470,41 @@ __global__ void __launch_bounds__(kLevelBlock) k_bvh_classify(const BTri* __rest
 }
 
 // Per splitting node: chunk offsets of the left-flag prefix count, and r =
-// the number of right-side triangles before the split point (= swaps).
+// the number of right-side triangles before the split point (= swaps).  One
+// warp per node: at the root of 200,000 triangles one thread read 200 counts
+// and up to 1024 flags one after another (18 us a level).
 __global__ void k_bvh_scan(BTask* __restrict__ tasks, int ntasks, const unsigned char* __restrict__ side,
                            const int* __restrict__ cleft, int* __restrict__ coff, BuildCounters* __restrict__ ctr)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr unsigned kAll = 0xffffffffu;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= ntasks) return;
     BTask& t = tasks[i];
     if (t.axis < 0) return;
-    int off = 0;
-    for (int k = 0; k < t.nchunks; k++) {
-        coff[t.cbase + k] = off;
-        off += cleft[t.cbase + k];
+    const int begin = t.begin, mid = t.mid, cbase = t.cbase, nchunks = t.nchunks;
+    const int km = (mid - begin) / kChunk;
+    int off = 0, lp = 0;
+    for (int k0 = 0; k0 < nchunks; k0 += 32) {
+        const int k = k0 + lane, v = k < nchunks ? cleft[cbase + k] : 0;
+        int inc = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int w = __shfl_up_sync(kAll, inc, o);
+            if (lane >= o) inc += w;
+        }
+        if (k < nchunks) coff[cbase + k] = off + inc - v;
+        if (k == km) lp = off + inc - v;
+        off += __shfl_sync(kAll, inc, 31);
     }
-    if (off != t.mid - t.begin) {   // the flags must agree with the bin counts
-        ctr->error = 4;
-        t.r = 0;
-        return;
+    for (int p = begin + km * kChunk + lane; p < mid; p += 32) lp += side[p];
+    lp = __reduce_add_sync(kAll, lp);
+    if (lane == 0) {
+        if (off != mid - begin) {   // the flags must agree with the bin counts
+            ctr->error = 4;
+            t.r = 0;
+        } else {
+            t.r = (mid - begin) - lp;
+        }
     }
-    const int km = (t.mid - t.begin) / kChunk;
-    int lp = coff[t.cbase + km];
-    for (int p = t.begin + km * kChunk; p < t.mid; p++) lp += side[p];
-    t.r = (t.mid - t.begin) - lp;
 }
 
 // Ranks of the misplaced triangles: R[k] = position of the k-th right-side
@@ -535,13 +576,16 @@ __global__ void __launch_bounds__(kLevelBlock) k_bvh_swap(const BTask* __restric
     }
 }
 
-// The host recursion over one small node, run by one thread: nodes go to
+// The host recursion over one small node, run by four threads in step (the
+// axes' bins and sweeps split among them; one of them writes): nodes go to
 // out[0 ..) in depth-first preorder with indices local to the subtree.
-__global__ void __launch_bounds__(128) k_bvh_small(const BTri* __restrict__ T, int* __restrict__ perm,
+__global__ void __launch_bounds__(64) k_bvh_small(const BTri* __restrict__ T, int* __restrict__ perm,
                                                    SmallTask* __restrict__ small, int nsmall,
                                                    pcr_bvh_node* __restrict__ region)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const Quad quad;
+    const bool writer = quad.lane == 0;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
     if (i >= nsmall) return;
     SmallTask st = small[i];
     pcr_bvh_node* out = region + 2 * (size_t)st.begin;
@@ -550,7 +594,7 @@ __global__ void __launch_bounds__(128) k_bvh_small(const BTri* __restrict__ T, i
     int b = st.begin, e = st.begin + st.count, par = -1;
     for (;;) {
         const int idx = n++;
-        if (par >= 0) out[par].right_child = idx;
+        if (writer && par >= 0) out[par].right_child = idx;
         float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
         float cmn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, cmx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
         for (int p = b; p < e; p++) {
@@ -564,16 +608,18 @@ __global__ void __launch_bounds__(128) k_bvh_small(const BTri* __restrict__ T, i
             }
         }
         pcr_bvh_node& N = out[idx];
-        for (int a = 0; a < 3; a++) { N.bmin[a] = mn[a]; N.bmax[a] = mx[a]; }
+        if (writer)
+            for (int a = 0; a < 3; a++) { N.bmin[a] = mn[a]; N.bmax[a] = mx[a]; }
         const int count = e - b;
         int best_axis = -1, best_bin = -1, best_lc = 0;
         if (count > 4) {
             float best_cost = FLT_MAX;
             const float parent = box_area(mn, mx);
             if (parent > 0.f) {
-                for (int a = 0; a < 3; a++) {
-                    const float lo = cmn[a], ext = __fsub_rn(cmx[a], lo);
-                    if (ext < 1e-6f) continue;
+                const int a = quad.lane;
+                const float lo = a == 0 ? cmn[0] : (a == 1 ? cmn[1] : cmn[2]);
+                const float ext = __fsub_rn(a == 0 ? cmx[0] : (a == 1 ? cmx[1] : cmx[2]), lo);
+                if (a < 3 && !(ext < 1e-6f)) {
                     const float scale = __fdiv_rn((float)kBins, ext);
                     float bmn[kBins][3], bmx[kBins][3];
                     int cnt[kBins];
@@ -594,6 +640,7 @@ __global__ void __launch_bounds__(128) k_bvh_small(const BTri* __restrict__ T, i
                     sah_axis(bmn, bmx, cnt, parent, a, best_cost, best_axis, best_bin, best_lc);
                 }
             }
+            quad.best(best_cost, best_axis, best_bin, best_lc);
             if (best_axis >= 0 && best_cost >= __fmul_rn((float)count, 2.f)) best_axis = -1;
         }
         int mid = b;
@@ -602,7 +649,7 @@ __global__ void __launch_bounds__(128) k_bvh_small(const BTri* __restrict__ T, i
             // std::partition, bidirectional form: two cursors swapping
             // misplaced triangles
             int first = b, last = e;
-            for (;;) {
+            for (; writer;) {
                 while (first != last && bin_of(getc(T[perm[first]].c, best_axis), lo, scale) <= best_bin) first++;
                 if (first == last) break;
                 last--;
@@ -613,21 +660,26 @@ __global__ void __launch_bounds__(128) k_bvh_small(const BTri* __restrict__ T, i
                 perm[last] = x;
                 first++;
             }
-            mid = first;
+            mid = __shfl_sync(quad.mask, first, quad.base);  // (and perm is seen by all four)
+            __syncwarp(quad.mask);
         }
         if (best_axis < 0 || mid == b || mid == e) {
-            N.left_or_first = b;
-            N.right_child = 0;
-            N.count = count;
+            if (writer) {
+                N.left_or_first = b;
+                N.right_child = 0;
+                N.count = count;
+            }
             if (sp == 0) break;
             sp--;
             b = stk_b[sp];
             e = stk_e[sp];
             par = stk_p[sp];
         } else {
-            N.left_or_first = idx + 1;
-            N.right_child = -1;
-            N.count = 0;
+            if (writer) {
+                N.left_or_first = idx + 1;
+                N.right_child = -1;
+                N.count = 0;
+            }
             stk_b[sp] = mid;
             stk_e[sp] = e;
             stk_p[sp] = idx;
@@ -636,7 +688,7 @@ __global__ void __launch_bounds__(128) k_bvh_small(const BTri* __restrict__ T, i
             par = -1;
         }
     }
-    small[i].nnodes = n;
+    if (writer) small[i].nnodes = n;
 }
 
 // Renumbering into depth-first preorder: pre[slot] for the level-built
@@ -798,10 +850,10 @@ void device_build_bvh(int device, cudaStream_t st, cudaMemPool_t pool, int n, co
         k_bvh_bounds<<<nchunks, kLevelBlock, 0, st>>>(T, perm, tasks[cur], chunks[cur]);
         k_bvh_bins<<<nchunks, kLevelBlock, 0, st>>>(T, perm, tasks[cur], chunks[cur], bins, bcnt);
         BK(cudaMemsetAsync(&ctr->ntasks, 0, 2 * sizeof(int), st));
-        k_bvh_split<<<blocks(ntasks, 128), 128, 0, st>>>(T, perm, tasks[cur], ntasks, bins, bcnt, top, small,
+        k_bvh_split<<<blocks((long long)ntasks * 4, 64), 64, 0, st>>>(T, perm, tasks[cur], ntasks, bins, bcnt, top, small,
                                                          LevelOut{tasks[nxt], chunks[nxt]}, ctr, cap);
         k_bvh_classify<<<nchunks, kLevelBlock, 0, st>>>(T, perm, tasks[cur], chunks[cur], side, cleft);
-        k_bvh_scan<<<blocks(ntasks, 128), 128, 0, st>>>(tasks[cur], ntasks, side, cleft, coff, ctr);
+        k_bvh_scan<<<blocks((long long)ntasks * 32, 128), 128, 0, st>>>(tasks[cur], ntasks, side, cleft, coff, ctr);
         k_bvh_ranks<<<nchunks, kLevelBlock, 0, st>>>(tasks[cur], chunks[cur], side, coff, R, L);
         k_bvh_swap<<<nchunks, kLevelBlock, 0, st>>>(tasks[cur], chunks[cur], R, L, perm, ctr);
         BK(cudaGetLastError());
@@ -813,7 +865,7 @@ void device_build_bvh(int device, cudaStream_t st, cudaMemPool_t pool, int n, co
         cur = nxt;
     }
     const int ntop = hc.ntop, nsmall = hc.nsmall;
-    if (nsmall > 0) k_bvh_small<<<blocks(nsmall, 128), 128, 0, st>>>(T, perm, small, nsmall, region);
+    if (nsmall > 0) k_bvh_small<<<blocks((long long)nsmall * 4, 64), 64, 0, st>>>(T, perm, small, nsmall, region);
     BK(cudaGetLastError());
 
     // preorder numbering of the level-built part (children always have
