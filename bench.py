@@ -49,24 +49,24 @@ sys.path.insert(0, REPO)
 METRIC = "paths/s, batched+served wavefront (64 uneven spectral renders); plain per-request alongside"
 UNIT = "paths/s"
 HBM_FALLBACK = 6650.0
-# Variants with a triangle mesh: they run in the queue stages (k_extend,
-# k_shade, k_shadow), the others in the whole-path kernel (k_paths).
+# Variants with a triangle mesh: k_paths with the BVH walks (k_extend,
+# k_shadow) beside it; the others run in k_paths alone.
 MESH_VARIANTS = ("cornell-bunny",)
 # DRAM bytes (read + write) per unit of each kernel, measured with ncu
 # (dram__bytes_read.sum + dram__bytes_write.sum, each launch replayed alone
 # with a cold L2; the summaries and commands are kept in the profiles
 # directory).  Units: rays (path vertices); shadow rays for k_shadow.
-NCU_DRAM_PER_UNIT = {"k_paths": 0.9, "k_extend": 61.0, "k_shade": 548.7, "k_shadow": 83.2}
+NCU_DRAM_PER_UNIT = {"k_paths": 0.43, "k_paths_mesh": 19.0, "k_extend": 10.9, "k_shadow": 10.4}
 # Warp instructions per unit (smsp__inst_executed.sum over the same launches,
 # divided by the same units), for the issue-rate roofline below.
-NCU_INST_PER_UNIT = {"k_paths": 139.6, "k_extend": 48.25, "k_shade": 69.57, "k_shadow": 43.90}
+NCU_INST_PER_UNIT = {"k_paths": 135.5, "k_paths_mesh": 69.1, "k_extend": 28.0, "k_shadow": 16.7}
 # Issue-rate side of the same kernels (ncu --set full, one launch each): the
 # share of issue slots used and the share of a warp's 32 lanes active per
 # instruction.
-NCU_ISSUE = {"k_paths": {"issue_slots_busy": 0.503, "lanes_active": 22.8 / 32},
-             "k_extend": {"issue_slots_busy": 0.638, "lanes_active": 16.2 / 32},
-             "k_shade": {"issue_slots_busy": 0.382, "lanes_active": 23.2 / 32},
-             "k_shadow": {"issue_slots_busy": 0.573, "lanes_active": 17.6 / 32, "l1_busy": 0.649}}
+NCU_ISSUE = {"k_paths": {"issue_slots_busy": 0.497, "lanes_active": 23.8 / 32},
+             "k_paths_mesh": {"issue_slots_busy": 0.341, "lanes_active": 14.6 / 32},
+             "k_extend": {"issue_slots_busy": 0.654, "lanes_active": 11.9 / 32},
+             "k_shadow": {"issue_slots_busy": 0.653, "lanes_active": 8.1 / 32, "l1_busy": 0.556}}
 # Algorithmic BVH-fetch bytes per ray of the batched-mesh workload's two
 # scenes: 2 x 24 B of child boxes per internal node processed plus 36 B per
 # leaf triangle tested, counted by the reference's own traversal order
@@ -632,8 +632,8 @@ def main():
     # ---- per-stage events (profiled pass) for the roofline
     roofline = None
     if not a.no_profile:
-        # Requests on scenes without a mesh run in k_paths, the others in the
-        # queue stages; each kind is profiled by itself.
+        # Requests on scenes without a mesh run in k_paths alone, the others with
+        # the BVH walks beside it; each kind is profiled by itself.
         tune = {k: st[k] for k in ("queue_capacity", "block_size", "chunk_paths", "regen_every")}
         prof = {}
         for kind, mesh in (("paths", False), ("queue", True)):
@@ -652,35 +652,31 @@ def main():
         mhz = clk.summary().get("sm_mhz") or 1965.0
         sms = torch.cuda.get_device_properties(local).multi_processor_count
         issue_peak = sms * 4 * mhz * 1e6
-        # algorithmic bytes per unit (queue records, 16-byte words):
-        #   extend: ray in (origin, dir, id: 48 B) + hit out (16 B)
-        #   shadow: shadow record in (48 B)
-        #   shade : spectral path in (o, d, tp, id, XYZ weights: 112 B) + hit in (16 B)
-        #           + path out (112 B) + shadow out (48 B each)
-        #   paths : the FP64 accumulator read and written once per path (48 B)
+        # units: path vertices (shadow rays for k_shadow).  Algorithmic bytes of
+        # k_paths without a mesh: a path's FP64 accumulator, read and written
+        # (48 B).  The queue records of the mesh kernels depend on how many
+        # rays meet the mesh's box: their traffic is given, as ncu counts it.
         per_kernel = {}
-        for kind_, stage, name, unit_b in (("paths", "other", "k_paths", None), ("queue", "extend", "k_extend", 64.0),
-                                           ("queue", "shade", "k_shade", 240.0), ("queue", "shadow", "k_shadow", 48.0)):
+        for kind_, stage, name in (("paths", "other", "k_paths"), ("queue", "shade", "k_paths_mesh"),
+                                   ("queue", "extend", "k_extend"), ("queue", "shadow", "k_shadow")):
             ps = prof.get(kind_)
             if not ps or ps["stage_ms"][stage] <= 0:
                 continue
             t, n_l = ps["stage_ms"][stage] / 1e3, max(1, ps["stage_launches"][stage])
             units = ps["shadow_rays"] if stage == "shadow" else ps["rays"]
-            nbytes = (48.0 * ps["paths"] if name == "k_paths" else unit_b * units +
-                      (48.0 * ps["shadow_rays"] if stage == "shade" else 0.0))
+            traffic = NCU_DRAM_PER_UNIT[name] * units
+            nbytes = 48.0 * ps["paths"] if name == "k_paths" else traffic
             inst = NCU_INST_PER_UNIT[name] * units
-            per_kernel[name] = {"ms": t * 1e3, "rays": ps["rays"], "shadow_rays": ps["shadow_rays"],
+            per_kernel[name] = {"ms": t * 1e3, "launches": n_l, "rays": ps["rays"], "shadow_rays": ps["shadow_rays"],
                                 "achieved_gbs": nbytes / t / 1e9, "frac_hbm": nbytes / t / 1e9 / peak,
-                                "algorithmic_bytes_per_launch": nbytes / n_l,
-                                "ncu_traffic_per_launch": NCU_DRAM_PER_UNIT[name] * units / n_l,
+                                "bytes": "algorithmic" if name == "k_paths" else "ncu traffic",
+                                "bytes_per_launch": nbytes / n_l, "ncu_traffic_per_launch": traffic / n_l,
                                 "issue_roofline": {"achieved": inst / t, "peak": issue_peak, "unit": "warp instructions/s",
                                                    "frac": inst / t / issue_peak,
                                                    "warp_inst_per_unit": NCU_INST_PER_UNIT[name], "sm_mhz": mhz,
                                                    "sms": sms}}
         dom = max(per_kernel, key=lambda k: per_kernel[k]["ms"])
         dk = per_kernel[dom]
-        dps = prof["paths" if dom == "k_paths" else "queue"]
-        n_l = max(1, dps["stage_launches"]["other" if dom == "k_paths" else dom[2:]])
         # HBM as the base bound of every kernel; the bound that applies is
         # instruction issue (issue_roofline: ncu warp instructions per unit x
         # units over the CUDA-event time, against one warp instruction per
@@ -688,7 +684,7 @@ def main():
         roofline = {"bound": "hbm", "kernel": dom, "achieved": dk["achieved_gbs"], "peak": peak, "unit": "GB/s",
                     "frac": dk["frac_hbm"], "peak_kind": kind, "traffic": dk["ncu_traffic_per_launch"],
                     "traffic_note": "ncu DRAM bytes per unit (8-render capture) x units per launch",
-                    "bytes_per_launch": dk["algorithmic_bytes_per_launch"], "ms_per_launch": dk["ms"] / n_l,
+                    "bytes_per_launch": dk["bytes_per_launch"], "ms_per_launch": dk["ms"] / dk["launches"],
                     "issue": dict(NCU_ISSUE.get(dom, {}), note="ncu, one launch per kernel"),
                     "stage_ms": {k: v["stage_ms"] for k, v in prof.items()}, "per_kernel": per_kernel,
                     "issue_roofline": dk["issue_roofline"]}

@@ -6,10 +6,10 @@
 // * Nodes over more than kSmall triangles are processed level by level, all
 //   nodes of a level at once, by blocks that each own a chunk of 1024
 //   positions of one node: node bounds, centroid bounds, 3 x 16 bins, the SAH
-//   decision (one thread per node), and the reference's two-cursor partition
+//   decision (four threads per node), and the reference's two-cursor partition
 //   restated in parallel (below).
-// * A node of kSmall or fewer triangles is built to the end by one thread,
-//   sequentially, exactly as the host recursion does.
+// * A node of kSmall or fewer triangles is built to the end by four threads
+//   that follow the host recursion.
 // * The finished pieces are renumbered into depth-first preorder.
 //
 // Why the result is bit-equal to the sequential build:
@@ -45,7 +45,7 @@ namespace {
 
 constexpr int kChunk = 1024;      // positions per block in the level passes
 constexpr int kLevelBlock = 256;  // threads per block in the level passes
-constexpr int kSmall = 32;        // nodes at or below this size go to one thread
+constexpr int kSmall = 32;        // nodes at or below this size go to four threads
 constexpr int kBins = 16;
 
 // Per triangle, in input order: lo / hi = the triangle's per-axis min / max

@@ -1769,7 +1769,7 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
 constexpr int kNoAllocFill = 8192;                       // paths per pass
 constexpr int kNoAllocQueue = kNoAllocFill * 4;          // room for 4-way forks
 constexpr int kNoAllocShadowPerVertex = 8;
-constexpr int kNoAllocShadow = kNoAllocQueue * kNoAllocShadowPerVertex;
+constexpr int kNoAllocShadow = kNoAllocQueue * 6;         // past it, shadow rays walk the mesh in place
 constexpr int64_t kNoAllocMaxPixels = 256 * 256;
 constexpr size_t kNoAllocAlign = 256;
 constexpr size_t align_up(size_t x) { return (x + kNoAllocAlign - 1) / kNoAllocAlign * kNoAllocAlign; }
