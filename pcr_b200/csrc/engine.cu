@@ -202,6 +202,8 @@ void Engine::alloc_buffers()
     d_params_ = dalloc<EngineParams>(1, T);
     d_cmf_ = dalloc<float4>(kCmfEntries, T);
     k_cmf_table<<<(kCmfEntries + 255) / 256, 256, 0, stream_>>>(d_cmf_);
+    d_bilateral_ = dalloc<float>(kBilateralEntries, T);
+    k_bilateral_table<<<sms_, 256, 0, stream_>>>(d_bilateral_);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(stream_));
     CK(cudaMemset(d_issued_, 0, 8 * kMaxActive));
@@ -1193,8 +1195,8 @@ void Engine::finish_request(Request& r, cudaStream_t rs)
     if (d.denoise) {
         // two bilateral passes on the 8-bit image, the accumulator as scratch
         unsigned char* tmp = reinterpret_cast<unsigned char*>(r.accum);
-        k_bilateral<<<std::max(1, grid), 256, 0, rs>>>(r.d_rgb, tmp, d.width, d.height);
-        k_bilateral<<<std::max(1, grid), 256, 0, rs>>>(tmp, r.d_rgb, d.width, d.height);
+        k_bilateral<<<std::max(1, grid), 256, 0, rs>>>(r.d_rgb, tmp, d.width, d.height, d_bilateral_);
+        k_bilateral<<<std::max(1, grid), 256, 0, rs>>>(tmp, r.d_rgb, d.width, d.height, d_bilateral_);
         CK(cudaGetLastError());
     }
     // the resolved images stay on the device until fetch copies them out
@@ -1989,8 +1991,8 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     if (desc.denoise && rgb_dev) {
         // two bilateral passes; the accumulator region (24 B a pixel) is free now
         unsigned char* tmp = reinterpret_cast<unsigned char*>(accum);
-        k_bilateral<<<std::max(1, grid), 256, 0, stream_>>>(rgb_dev, tmp, desc.width, desc.height);
-        k_bilateral<<<std::max(1, grid), 256, 0, stream_>>>(tmp, rgb_dev, desc.width, desc.height);
+        k_bilateral<<<std::max(1, grid), 256, 0, stream_>>>(rgb_dev, tmp, desc.width, desc.height, d_bilateral_);
+        k_bilateral<<<std::max(1, grid), 256, 0, stream_>>>(tmp, rgb_dev, desc.width, desc.height, d_bilateral_);
         CK(cudaGetLastError());
     }
     CK(cudaStreamSynchronize(stream_));
@@ -2109,8 +2111,8 @@ void Engine::tonemap(const float* hdr, int width, int height, int aces_tm, int d
     k_tonemap<<<grid, 256, 0, stream_>>>(d_hdr, (int)px, aces_tm, d_rgb);
     if (denoise) {
         CK(cudaMallocFromPoolAsync(&d_tmp, px * 3, pool_, stream_));
-        k_bilateral<<<grid, 256, 0, stream_>>>(d_rgb, d_tmp, width, height);
-        k_bilateral<<<grid, 256, 0, stream_>>>(d_tmp, d_rgb, width, height);
+        k_bilateral<<<grid, 256, 0, stream_>>>(d_rgb, d_tmp, width, height, d_bilateral_);
+        k_bilateral<<<grid, 256, 0, stream_>>>(d_tmp, d_rgb, width, height, d_bilateral_);
     }
     CK(cudaGetLastError());
     download_parts(d_rgb, {{rgb8, (size_t)px * 3}}, stream_);

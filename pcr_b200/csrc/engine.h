@@ -212,6 +212,7 @@ private:
     int *d_give_base_ = nullptr, *d_path_base_ = nullptr, *d_active_ = nullptr, *d_nactive_ = nullptr, *d_done_ = nullptr;
     int *d_round_state_ = nullptr, *d_round_cnt_ = nullptr, *d_round_list_ = nullptr;
     float4* d_cmf_ = nullptr;  // colour-matching table for raygen
+    float* d_bilateral_ = nullptr;  // weights of the bilateral filter
     int* h_active_ = nullptr;     // pinned: [0] = n, then slots
     Counters* d_cnt_ = nullptr;
     struct HostSnap {
