@@ -509,7 +509,9 @@ __device__ __forceinline__ SphereSpan sphere_span(float4 c, const FlatRay& r)
     const float b = f3dot(r.d, cp), cc = f3dot(cp, cp), out = cc - c.w * c.w, disc = fmaf(b, b, -out);
     const float pad = 2e-6f * cc + 2e-6f * c.w * c.w;
     const float far = sqrt_approx(fmaxf(disc + pad, 0.f)) * (1.f + 4e-6f), near = sqrt_approx(fmaxf(disc - pad, 0.f)) * (1.f - 4e-6f);
-    const bool inside = out < 0.f;
+    // On the sphere the sign of `out` is in doubt: the exact test may answer
+    // either root, and the lower bound has to hold for both.
+    const bool inside = out < -pad;
     SphereSpan s;
     // outside with the centre behind: both roots are negative
     s.may = disc > -pad && !(out > pad && b <= 0.f);
