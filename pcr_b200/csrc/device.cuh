@@ -507,7 +507,8 @@ __device__ __forceinline__ SphereSpan sphere_span(float4 c, const FlatRay& r)
 {
     const float3 cp = make_float3(c.x - r.o.x, c.y - r.o.y, c.z - r.o.z);
     const float b = f3dot(r.d, cp), cc = f3dot(cp, cp), out = cc - c.w * c.w, disc = fmaf(b, b, -out);
-    const float pad = 2e-6f * cc + 2e-6f * c.w * c.w;
+    // (1e-36: a point sphere's terms may all be zero, or too small for a relative error)
+    const float pad = 2e-6f * cc + 2e-6f * c.w * c.w + 1e-36f;
     const float far = sqrt_approx(fmaxf(disc + pad, 0.f)) * (1.f + 4e-6f), near = sqrt_approx(fmaxf(disc - pad, 0.f)) * (1.f - 4e-6f);
     // On the sphere the sign of `out` is in doubt: the exact test may answer
     // either root, and the lower bound has to hold for both.
@@ -516,7 +517,7 @@ __device__ __forceinline__ SphereSpan sphere_span(float4 c, const FlatRay& r)
     // outside with the centre behind: both roots are negative
     s.may = disc > -pad && !(out > pad && b <= 0.f);
     s.sure = disc > pad && fabsf(out) > pad;
-    const float e = 1e-6f * (fabsf(b) + c.w);
+    const float e = 1e-6f * (fabsf(b) + fabsf(c.w));  // a negative radius counts as its magnitude
     s.lo = (inside ? b + near : b - far) - e;
     s.hi = (inside ? b + far : b - near) + e;
     return s;

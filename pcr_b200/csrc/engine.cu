@@ -420,7 +420,7 @@ static FlatScene flat_scene(const pcr_scene_desc& d, const std::vector<DPlane>& 
     }
     for (int i = 0; i < d.n_spheres; i++) {
         V c = vec(d.spheres[i].center);
-        for (double& x : c) x = std::fabs(x) + d.spheres[i].radius;
+        for (double& x : c) x = std::fabs(x) + std::fabs(d.spheres[i].radius);
         reach(c);
     }
     if (!(big < 1e6) || d.n_planes + d.n_spheres > 6 * kMaxFlatPrims) return F;  // also NaN
@@ -536,7 +536,7 @@ static FlatScene flat_scene(const pcr_scene_desc& d, const std::vector<DPlane>& 
             const V o = vec(d.planes[i].origin), u = vec(d.planes[i].u), v = vec(d.planes[i].v);
             for (const V& c : {o, add(o, u), add(o, v), add(add(o, u), v)}) hold(c, 0.0);
         }
-    for (int i = 0; i < d.n_spheres; i++) hold(vec(d.spheres[i].center), d.spheres[i].radius);
+    for (int i = 0; i < d.n_spheres; i++) hold(vec(d.spheres[i].center), std::fabs(d.spheres[i].radius));
     for (const DRect& q : F.rects)
         if (__float_as_int_host(q.b.z) & kRectEmissive) {
             const pcr_plane& p = d.planes[__float_as_int_host(q.a.w)];

@@ -111,3 +111,12 @@ def ctx():
 @pytest.mark.parametrize("kind", list(ROOMS))
 def test_rays_that_start_on_a_sphere(ctx, tmp_path, kind):
     _agree(ctx, tmp_path, ROOMS[kind], 7)
+
+
+@pytest.mark.parametrize("radii", [(0.0, 1e-5, 1.99), (-0.5, -1.4, 0.3), (-300.0, 0.5, 0.0)])
+def test_spheres_of_zero_and_negative_radius(ctx, tmp_path, radii):
+    """The intersection only uses the radius's square: a point sphere is met
+    from its centre, a negative radius counts as its magnitude."""
+    a, b, c = radii
+    _agree(ctx, tmp_path, _room([((0.2, -1.9, -3.2), a, "grey"), ((1.1, -0.6, -4.5), b, "red"),
+                                 ((0.0, 0.0, -3.0), c, "grey")]), 11)
