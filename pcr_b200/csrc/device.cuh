@@ -327,8 +327,10 @@ __device__ __forceinline__ int bvh4_closest(const DScene& S, float3 o, float3 d,
 // host by well over the rounding error of a hit point, the segment end by
 // 1e-4 relative; direction components below 1e-30 count as zero (the ray
 // then moves less than the padding along that axis), the others enter as
-// their 1-ulp rcp_approx, whose error the padding also covers.  A false
-// answer means no plane of the group can be hit in (0, closest].
+// their rcp_approx, which leaves each t within 2^-21 of the exact quotient
+// (more than the padding where the origin is far from the box, so the
+// interval's ends are compared with a relative margin).  A false answer means
+// no plane of the group can be hit in (0, closest].
 __device__ __forceinline__ bool group_axis(float lo, float hi, float o, float d, float r, float& tmin, float& tmax)
 {
     if (fabsf(d) < 1e-30f) return o >= lo && o <= hi;
@@ -343,7 +345,7 @@ __device__ __forceinline__ bool group_may_hit(float4 lo, float4 hi, float3 o, fl
     if (!group_axis(lo.x, hi.x, o.x, d.x, rd.x, tmin, tmax)) return false;
     if (!group_axis(lo.y, hi.y, o.y, d.y, rd.y, tmin, tmax)) return false;
     if (!group_axis(lo.z, hi.z, o.z, d.z, rd.z, tmin, tmax)) return false;
-    return tmin <= tmax;
+    return tmin <= tmax * (1.f + 1.9073486328125e-06f);  // 1 + 2^-19
 }
 
 // The analytic part of Renderer::sceneIntersect (code/Renderer.cpp:891-949):
