@@ -475,7 +475,7 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
     if (kMesh) close_shadow_chunk(E, P, lane);
     rays = __reduce_add_sync(kAll, rays);
     shadows = __reduce_add_sync(kAll, shadows);
-    if (lane == 0 && rays) {
+    if (lane == 0 && (rays | shadows)) {  // a resumed path that ends at its vertex traced no ray
         atomicAdd(&C->rays, (unsigned long long)rays);
         atomicAdd(&C->shadow_rays, (unsigned long long)shadows);
     }
