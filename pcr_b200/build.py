@@ -23,7 +23,7 @@ CLI = os.path.join(LIBDIR, "pcr-render")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 SOURCES = ["engine.cu", "bvh_build.cu", "scene.cpp", "capi.cpp"]
-HEADERS = ["layout.h", "device.cuh", "kernels.cuh", "paths.cuh", "engine.h", "scene.h", "bvh_build.h"]
+HEADERS = ["layout.h", "device.cuh", "kernels.cuh", "paths.cuh", "flat_scene.h", "engine.h", "scene.h", "bvh_build.h"]
 
 
 def _newer(target: str, deps) -> bool:
