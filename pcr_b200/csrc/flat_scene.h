@@ -14,10 +14,10 @@ namespace pcr {
 
 // The estimate pass's form of the quads and spheres (device.cuh,
 // flat_closest): boxes, i.e. six consecutive non-emissive quads that bound a
-// rectangular box, and axis-aligned rectangles.  The scene takes the pass
-// only when every quad is one of these and there are at most
-// kMaxFlatPrims primitives: the pass tests them all, while past that number
-// the exact tests' grouped culling skips more than it costs.
+// rectangular box other than the room, and axis-aligned rectangles.  The
+// scene takes the pass only when every quad is one of these and there are at
+// most kMaxFlatPrims primitives: the pass tests them all, while past that
+// number the exact tests' grouped culling skips more than it costs.
 constexpr int kMaxFlatPrims = 64;
 struct FlatScene {
     std::vector<DRect> rects, srects;
@@ -107,15 +107,8 @@ inline FlatScene flat_scene(const pcr_scene_desc& d, const std::vector<DPlane>& 
         B.hi = make_int4(face[0][1 - low(0)], face[1][1 - low(1)], face[2][1 - low(2)], 0);
         return true;
     };
-    // by normal axis, plane coordinate, and order in the scene
-    std::vector<std::tuple<int, float, int>> flat;
-    for (int i = 0; i < d.n_planes;) {
-        DBox B;
-        if (as_box(i, B)) {
-            F.boxes.push_back(B);
-            i += 6;
-            continue;
-        }
+    // the axis an axis-aligned rectangle is normal to, -1 for another quad
+    auto rect_axis = [&](int i) {
         const pcr_plane& p = d.planes[i];
         int axis = -1, along_u = -1, along_v = -1;
         for (int k = 0; k < 3; k++) {
@@ -124,8 +117,50 @@ inline FlatScene flat_scene(const pcr_scene_desc& d, const std::vector<DPlane>& 
             if (p.u[k] != 0.f && p.u[a] == 0.f && p.u[b] == 0.f) along_u = k;
             if (p.v[k] != 0.f && p.v[a] == 0.f && p.v[b] == 0.f) along_v = k;
         }
-        if (axis < 0 || along_u < 0 || along_v < 0 || along_u == along_v || along_u == axis || along_v == axis) return F;
-        flat.push_back({axis, p.origin[axis] + 0.f, i});  // + 0.f: -0 and +0 are one plane
+        return along_u < 0 || along_v < 0 || along_u == along_v || along_u == axis || along_v == axis ? -1 : axis;
+    };
+    // Whether the box of quads i .. i + 5 is a room.  A ray that starts in a
+    // box is in doubt, so a box that holds the camera or a light is none, and
+    // where its quads are rectangles anyway it holds nothing else either
+    // (a closed 4 x 4 x 6 room with a sphere, as a box, by the exact tests
+    // alone, and as rectangles: 1 M closest hits 70, 48 and 40 us, six batched
+    // renders 25.7, 22.0 and 12.4 ms).
+    auto is_room = [&](int i, const DBox& B) {
+        const float half[3] = {B.h.x, B.h.y, B.h.z};
+        auto in = [&](const V& c) {
+            for (int a = 0; a < 3; a++)
+                if (!(std::fabs(dot(V{B.nc[a].x, B.nc[a].y, B.nc[a].z}, c) - B.nc[a].w) < half[a] - B.h.w)) return false;
+            return true;
+        };
+        if (in(vec(d.cam_pos))) return true;
+        bool rects = true;
+        for (int k = i; k < i + 6; k++) rects = rects && rect_axis(k) >= 0;
+        for (int k = 0; k < d.n_planes; k++) {
+            if ((k >= i && k < i + 6) || (planes[k].n_emit.w == 0.f && !rects)) continue;
+            const V o = vec(d.planes[k].origin), u = vec(d.planes[k].u), v = vec(d.planes[k].v);
+            for (const V& c : {o, add(o, u), add(o, v), add(add(o, u), v)})
+                if (in(c)) return true;
+        }
+        for (int k = 0; k < d.n_spheres && rects; k++)
+            if (in(vec(d.spheres[k].center))) return true;
+        return false;
+    };
+    // by normal axis, plane coordinate, and order in the scene
+    std::vector<std::tuple<int, float, int>> flat;
+    int no_box = 0;  // quads before this one are a room's
+    for (int i = 0; i < d.n_planes;) {
+        DBox B;
+        if (i >= no_box && as_box(i, B)) {
+            if (!is_room(i, B)) {
+                F.boxes.push_back(B);
+                i += 6;
+                continue;
+            }
+            no_box = i + 6;
+        }
+        const int axis = rect_axis(i);
+        if (axis < 0) return F;
+        flat.push_back({axis, d.planes[i].origin[axis] + 0.f, i});  // + 0.f: -0 and +0 are one plane
         i++;
     }
     if ((int)(flat.size() + F.boxes.size()) + d.n_spheres > kMaxFlatPrims) return F;
