@@ -352,7 +352,12 @@ __device__ __forceinline__ bool group_may_hit(float4 lo, float4 hi, float3 o, fl
 // spheres, then planes (light planes first); first-tested wins ties.
 // Returns the primitive code (kPrimNone on a miss) with `closest` lowered to
 // its t.
-__device__ __noinline__ uint32_t scene_analytic_exact(const DScene& S, float3 o, float3 d, float& closest)
+//
+// Inlined into the kernels that only trace rays, and one function in k_paths,
+// whose speed depends on its code's size (1 M rays through 88 quads, inlined
+// and called: 332 and 363 us).  The loops stay loops in both: unrolled, 0 to 5 %
+// slower.
+__device__ __forceinline__ uint32_t analytic_tests(const DScene& S, float3 o, float3 d, float& closest)
 {
     uint32_t prim = kPrimNone;
 #pragma unroll 1
@@ -381,6 +386,10 @@ __device__ __noinline__ uint32_t scene_analytic_exact(const DScene& S, float3 o,
         }
     }
     return prim;
+}
+__device__ __noinline__ uint32_t scene_analytic_exact(const DScene& S, float3 o, float3 d, float& closest)
+{
+    return analytic_tests(S, o, d, closest);
 }
 
 // ----------------------------------------------------------------- estimates
@@ -593,11 +602,17 @@ __device__ __forceinline__ bool flat_closest(const DScene& S, float3 o, float3 d
     return true;
 }
 
+// kTrace: in a kernel that only traces rays.
+template <bool kTrace>
 __device__ __forceinline__ uint32_t scene_analytic(const DScene& S, float3 o, float3 d, float& closest)
 {
     uint32_t prim;
-    if (S.flat_ok && flat_closest(S, o, d, closest, prim)) return prim;
-    return scene_analytic_exact(S, o, d, closest);
+    if (!kTrace) return S.flat_ok && flat_closest(S, o, d, closest, prim) ? prim : scene_analytic_exact(S, o, d, closest);
+    float t = FLT_MAX;
+    if (!S.flat_ok || !flat_closest(S, o, d, t, prim)) return analytic_tests(S, o, d, closest);
+    if (!(t < closest)) return kPrimNone;  // the first hit lies past the ray's end
+    closest = t;
+    return prim;
 }
 
 // Whether the mesh can hold a hit closer than `closest`: the padded box test
@@ -611,11 +626,12 @@ __device__ __forceinline__ bool mesh_may_hit(const DScene& S, float3 o, float3 d
 
 // Renderer::sceneIntersect: the analytic primitives, then the triangle BVH.
 // Returns the primitive code; t and barycentrics through refs.
+template <bool kTrace>
 __device__ __forceinline__ uint32_t scene_closest(const DScene& S, float3 o, float3 d, float tmax, float& t, float& hu,
                                                   float& hv)
 {
     float closest = tmax;
-    uint32_t prim = scene_analytic(S, o, d, closest);
+    uint32_t prim = scene_analytic<kTrace>(S, o, d, closest);
     int tri = bvh4_closest<false>(S, o, d, closest, hu, hv, nullptr);
     if (tri >= 0) prim = kPrimTri | (uint32_t)tri;
     t = closest;
@@ -638,13 +654,13 @@ __device__ __forceinline__ uint32_t scene_closest(const DScene& S, float3 o, flo
 // with emissive triangles is decided here in full), else kShadowWalk with
 // `bound` set for an any-hit walk of the BVH.
 constexpr int kShadowLit = 0, kShadowBlocked = 1, kShadowWalk = 2;
-template <bool kMesh>
-__device__ __noinline__ int scene_blocked_exact(const DScene& S, const DMaterial* mats, float3 o, float3 d,
-                                                      float tmax, double lim, float& bound)
+template <bool kMesh, bool kTrace>
+__device__ __forceinline__ int blocked_tests(const DScene& S, const DMaterial* mats, float3 o, float3 d, float tmax,
+                                             double lim, float& bound)
 {
     if ((kMesh && S.emissive_tris) || S.n_emit_spheres < 0 || S.n_emit_planes < 0) {
         float t = tmax, hu, hv;
-        const uint32_t prim = kMesh ? scene_closest(S, o, d, tmax, t, hu, hv) : scene_analytic(S, o, d, t);
+        const uint32_t prim = kMesh ? scene_closest<kTrace>(S, o, d, tmax, t, hu, hv) : scene_analytic<kTrace>(S, o, d, t);
         if ((prim & kPrimKindMask) == kPrimNone) return kShadowLit;
         const uint32_t kind = prim & kPrimKindMask, pidx = prim & kPrimIndexMask;
         int mi;
@@ -686,6 +702,12 @@ __device__ __noinline__ int scene_blocked_exact(const DScene& S, const DMaterial
         }
     }
     return kMesh && S.n_nodes > 0 ? kShadowWalk : kShadowLit;
+}
+template <bool kMesh>
+__device__ __noinline__ int scene_blocked_exact(const DScene& S, const DMaterial* mats, float3 o, float3 d,
+                                                float tmax, double lim, float& bound)
+{
+    return blocked_tests<kMesh, false>(S, mats, o, d, tmax, lim, bound);
 }
 
 // The analytic shadow query where the estimates decide it, else -1.  `light`
@@ -769,7 +791,7 @@ __device__ __forceinline__ float shadow_end(float d2) { return sqrtf(d2) * 1.000
 
 // The part of the shadow query before the triangle BVH (see
 // scene_blocked_exact).
-template <bool kMesh>
+template <bool kMesh, bool kTrace>
 __device__ __forceinline__ int scene_blocked_analytic(const DScene& S, const DMaterial* mats, float3 o, float3 d,
                                                       float d2, float& bound)
 {
@@ -787,13 +809,15 @@ __device__ __forceinline__ int scene_blocked_analytic(const DScene& S, const DMa
             return kShadowWalk;
         }
     }
-    return scene_blocked_exact<kMesh>(S, mats, o, d, shadow_end(d2), (double)d2 - 1e-3, bound);
+    return kTrace ? blocked_tests<kMesh, true>(S, mats, o, d, shadow_end(d2), (double)d2 - 1e-3, bound)
+                  : scene_blocked_exact<kMesh>(S, mats, o, d, shadow_end(d2), (double)d2 - 1e-3, bound);
 }
 
+// In a kernel that only traces rays.
 __device__ __forceinline__ bool scene_blocked(const DScene& S, const DMaterial* mats, float3 o, float3 d, float d2)
 {
     float bound, hu, hv;
-    const int r = scene_blocked_analytic<true>(S, mats, o, d, d2, bound);
+    const int r = scene_blocked_analytic<true, true>(S, mats, o, d, d2, bound);
     if (r != kShadowWalk) return r == kShadowBlocked;
     return bvh4_closest<false, true>(S, o, d, bound, hu, hv, nullptr, (double)d2 - 1e-3) == -2;
 }

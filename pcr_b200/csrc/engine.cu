@@ -634,6 +634,7 @@ int Engine::upload_scene(const pcr_scene_desc& d)
     S.flat_pad = flat.pad;
     S.flat_reach = flat.reach;
     S.emissive_tris = emissive_tris;
+    S.staged = !flat.ok || emissive_tris;
     {
         int only = -1, n_emit = 0;
         for (int i = 0; i < d.n_materials; i++)
@@ -885,7 +886,7 @@ int Engine::active_stages() const
     int m = 0;
     for (int slot : active_slots_) {
         auto it = reqs_.find(slot_owner_[slot]);
-        if (it != reqs_.end()) m |= flat(it->second->scene) ? kStagesFlat : kStagesMesh;
+        if (it != reqs_.end()) m |= flat(it->second->scene) ? kStagesFlat : queue_stages(it->second->scene);
     }
     return m ? m : kStagesMesh;
 }
@@ -893,9 +894,8 @@ int Engine::active_stages() const
 void Engine::launch_iteration(int cur, int stages, bool prof)
 {
     const EngineView E = view();
-    const int B = trace_block();
-    // stage index: 1 extend 2 shade (k_paths on mesh scenes) 3 shadow 5 schedule 6 status (and k_round)
-    // 7 other (k_paths on scenes without a mesh)
+    // stage index: 1 extend 2 shade (k_paths on scenes whose paths can wait) 3 shadow 5 schedule
+    // 6 status (and k_round) 7 other (k_paths on the other scenes)
     int done = 0;
     int stage_of[8];
     auto mark = [&](int stage) {  // the stage just launched ends here
@@ -907,16 +907,13 @@ void Engine::launch_iteration(int cur, int stages, bool prof)
     if (prof) CK(cudaEventRecord(prof_ev_[0], stream_));
     k_schedule<<<1, kSchedThreads, 0, stream_>>>(E, (const EngineParams*)d_params_, cur);
     mark(5);
-    if (stages & kStagesMesh) {
-        k_paths<true><<<grid_mesh_, kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
-        mark(2);
-        k_extend<<<grid_extend_, B, 0, stream_>>>(E, cur ^ 1);
-        mark(1);
-        k_shadow<<<grid_shadow_, B, 0, stream_>>>(E);
-        mark(3);
-    }
+    if (stages & (kStagesMesh | kStagesStaged))
+        for (int stage : {2, 1, 3}) {
+            launch_queue_stage(E, grids_, cur, stages, stage);
+            mark(stage);
+        }
     if (stages & kStagesFlat) {
-        k_paths<false><<<grid_flat_, kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
+        k_paths<kFlatScenes><<<grids_.paths[kFlatScenes], kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
         mark(7);
     }
     k_status<<<1, 1024, 0, stream_>>>(E, cur ^ 1);
@@ -935,13 +932,41 @@ void Engine::launch_iteration(int cur, int stages, bool prof)
     iterations_++;
 }
 
+Engine::Grids Engine::launch_grids()
+{
+    Grids g;
+    const int B = trace_block();
+    grid_for((const void*)k_paths<kFlatScenes>, kPathBlock, kPathSmem, &g.paths[kFlatScenes]);
+    grid_for((const void*)k_paths<kMeshScenes>, kPathBlock, kPathSmem, &g.paths[kMeshScenes]);
+    grid_for((const void*)k_paths<kStagedScenes>, kPathBlock, kPathSmem, &g.paths[kStagedScenes]);
+    grid_for((const void*)k_extend<false>, B, 0, &g.extend[0]);
+    grid_for((const void*)k_extend<true>, B, 0, &g.extend[1]);
+    grid_for((const void*)k_shadow<false>, B, 0, &g.shadow[0]);
+    grid_for((const void*)k_shadow<true>, B, 0, &g.shadow[1]);
+    return g;
+}
+
+// Stage 2 (k_paths), 1 (k_extend) or 3 (k_shadow) of an iteration.
+void Engine::launch_queue_stage(const EngineView& E, const Grids& g, int cur, int stages, int stage)
+{
+    const int B = trace_block(), staged = stages & kStagesStaged ? 1 : 0;
+    if (stage == 2) {
+        // staged first: its shadow records always find room
+        if (staged) k_paths<kStagedScenes><<<g.paths[kStagedScenes], kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
+        if (stages & kStagesMesh)
+            k_paths<kMeshScenes><<<g.paths[kMeshScenes], kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
+    } else if (stage == 1) {
+        if (staged) k_extend<true><<<g.extend[1], B, 0, stream_>>>(E, cur ^ 1);
+        else k_extend<false><<<g.extend[0], B, 0, stream_>>>(E, cur ^ 1);
+    } else {
+        if (staged) k_shadow<true><<<g.shadow[1], B, 0, stream_>>>(E);
+        else k_shadow<false><<<g.shadow[0], B, 0, stream_>>>(E);
+    }
+}
+
 void Engine::launch_shapes()
 {
-    const int B = trace_block();
-    grid_for((const void*)k_extend, B, 0, &grid_extend_);
-    grid_for((const void*)k_shadow, B, 0, &grid_shadow_);
-    grid_for((const void*)k_paths<false>, kPathBlock, kPathSmem, &grid_flat_);
-    grid_for((const void*)k_paths<true>, kPathBlock, kPathSmem, &grid_mesh_);
+    grids_ = launch_grids();
     grid_round_ = sms_ * 2;  // a round's per-pixel step is light; an idle launch reads one word
     drop_graphs();
     graph_dirty_ = false;
@@ -978,7 +1003,7 @@ void Engine::launch_block(int stages)
         CK(cudaGraphLaunch(graphs_[stages], stream_));
         stage_launches_[5] += tune_.iters_per_launch;
         stage_launches_[6] += 2 * tune_.iters_per_launch;
-        if (stages & kStagesMesh)
+        if (stages & (kStagesMesh | kStagesStaged))
             for (int k : {1, 2, 3}) stage_launches_[k] += tune_.iters_per_launch;
         if (stages & kStagesFlat) stage_launches_[7] += tune_.iters_per_launch;
         iterations_ += tune_.iters_per_launch;
@@ -1456,7 +1481,7 @@ void Engine::trace_flat(const EngineView& E, const DRequest& R, int grid)
         const int n = (int)std::min<int64_t>(kPathsPerLaunch, R.total - at);
         k_one_request<<<1, 1, 0, stream_>>>(E, R, at, n);
         if (profile_) CK(cudaEventRecord(prof_ev_[0], stream_));
-        k_paths<false><<<std::min(grid, (n + kPathBlock - 1) / kPathBlock), kPathBlock, kPathSmem, stream_>>>(E, 0, xyz_scale_);
+        k_paths<kFlatScenes><<<std::min(grid, (n + kPathBlock - 1) / kPathBlock), kPathBlock, kPathSmem, stream_>>>(E, 0, xyz_scale_);
         CK(cudaGetLastError());
         if (profile_) record_other(prof_ev_[0], prof_ev_[1]);
         else stage_launches_[7]++;
@@ -1469,7 +1494,7 @@ void Engine::render_flat(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats*
 {
     alloc_request(r);
     const DRequest R = make_request(r.desc, r.scene, r.accum);
-    trace_flat(view(), R, grid_flat_);
+    trace_flat(view(), R, grids_.paths[kFlatScenes]);
     active_dirty_ = true;  // the active list holds slot 0
     CK(cudaMemcpyAsync(h_cnt_, d_cnt_, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
     finish_request(r, stream_);
@@ -1528,10 +1553,11 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     upload_active();
     const int64_t total = px * local_spp(desc) * std::max(1, desc.aa_samples);
     const int64_t fills = (total + tune_.queue_capacity - 1) / tune_.queue_capacity;
+    const int stages = queue_stages(scene);
     int cur = 0;
-    // a path waits for the mesh at most `depth` times
+    // a path waits at most `depth` times
     for (int64_t it = 0; it < fills + desc.depth; it++) {
-        launch_iteration(cur, kStagesMesh, profile_);
+        launch_iteration(cur, stages, profile_);
         cur ^= 1;
     }
     int64_t extra = 0;
@@ -1544,12 +1570,12 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
         if (c.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "device reported queue overflow");
         if (done) break;
         if (++extra > fills * (4 * (int64_t)desc.depth + 8)) throw PcrError(PCR_ERR_TIMEOUT, "plain render did not finish");
-        launch_iteration(cur, kStagesMesh, profile_);
+        launch_iteration(cur, stages, profile_);
         cur ^= 1;
     }
     // a plain render always ends on queue parity 0 for the next user
     if (cur != 0) {
-        launch_iteration(cur, kStagesMesh, false);
+        launch_iteration(cur, stages, false);
         cur ^= 1;
     }
     unsigned long long tf = 0, td = 0;
@@ -1638,7 +1664,7 @@ DRequest Engine::make_request(const pcr_render_desc& d, int scene, double* accum
     R.shadow = d.shadow_samples;
     R.flags = (d.spectral ? kReqSpectral : 0) | (d.mis ? kReqMIS : 0) | (d.russian ? kReqRussian : 0) |
               (d.stratified ? kReqStratified : 0) | (d.spectral_terminate ? kReqTerminate : 0) |
-              (flat(scene) ? kReqFlat : 0);
+              (flat(scene) ? kReqFlat : 0) | (S.dev.staged ? kReqStaged : 0);
     R.hero = std::min(4, std::max(1, d.hero_samples <= 0 ? 4 : d.hero_samples));
     R.strata = d.stratified ? std::max(1, (int)std::lround(std::sqrt((float)d.samples))) : 0;
     R.cam_x = S.cam[0];
@@ -1751,9 +1777,9 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     E.queue_cap = kNoAllocQueue;
 
     const DRequest R = make_request(desc, scene, accum);
-    if (flat(scene)) {
+    if (scenes_[scene].dev.n_nodes == 0) {
         int g_paths;
-        grid_for((const void*)k_paths<false>, kPathBlock, kPathSmem, &g_paths);
+        grid_for((const void*)k_paths<kFlatScenes>, kPathBlock, kPathSmem, &g_paths);
         trace_flat(E, R, g_paths);
     } else {
         k_admit<<<1, 1, 0, stream_>>>(E, R, 0);
@@ -1761,22 +1787,19 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
         L.n = 1;
         L.slots[0] = 0;
         k_set_active<<<1, 32, 0, stream_>>>(E, L);
-        const int pass = (int)std::min<int64_t>(px, kNoAllocFill);
+        // (a staged scene's shadow records have no way past a full queue)
+        int fill = kNoAllocFill;
+        if (scenes_[scene].dev.staged) fill = std::min(fill, kNoAllocShadow / (4 * desc.shadow_samples));
+        const int pass = (int)std::min<int64_t>(px, fill);
         k_set_params<<<1, 1, 0, stream_>>>(params, EngineParams{pass, pass, 1});
         CK(cudaGetLastError());
 
         // launch shapes from the occupancy calculator (no allocation involved)
-        const int B = trace_block();
-        int g_paths, g_extend, g_shadow;
-        grid_for((const void*)k_paths<true>, kPathBlock, kPathSmem, &g_paths);
-        grid_for((const void*)k_extend, B, 0, &g_extend);
-        grid_for((const void*)k_shadow, B, 0, &g_shadow);
+        const Grids g = launch_grids();
         int cur = 0;
         auto iteration = [&]() {
             k_schedule<<<1, kSchedThreads, 0, stream_>>>(E, params, cur);
-            k_paths<true><<<g_paths, kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
-            k_extend<<<g_extend, B, 0, stream_>>>(E, cur ^ 1);
-            k_shadow<<<g_shadow, B, 0, stream_>>>(E);
+            for (int stage : {2, 1, 3}) launch_queue_stage(E, g, cur, queue_stages(scene), stage);
             k_status<<<1, 1024, 0, stream_>>>(E, cur ^ 1);
             CK(cudaGetLastError());
             cur ^= 1;

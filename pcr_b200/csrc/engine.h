@@ -121,10 +121,16 @@ private:
     void alloc_request(Request& r);
     void activate(Request& r, int slot);
     void upload_active();
-    // Which kernels an iteration runs: k_paths and the BVH walks for requests
-    // on mesh scenes, the mesh-free k_paths for the others (bits of the active
-    // requests).
-    static constexpr int kStagesMesh = 1, kStagesFlat = 2;
+    // Which kernels an iteration runs (bits of the active requests): k_paths by
+    // kind of scene, the walks for those whose paths can wait, in the form
+    // that traces in full where a staged scene is among them.
+    static constexpr int kStagesMesh = 1, kStagesFlat = 2, kStagesStaged = 4;
+    int queue_stages(int scene) const { return scenes_[scene].dev.staged ? kStagesStaged : kStagesMesh; }
+    struct Grids {
+        int paths[3], extend[2], shadow[2];
+    };
+    Grids launch_grids();
+    void launch_queue_stage(const EngineView& E, const Grids& g, int cur, int stages, int stage);
     int active_stages() const;
     void launch_iteration(int cur, int stages, bool profile);
     void launch_block(int stages);
@@ -138,7 +144,8 @@ private:
     void release_cancelled(Request& r);
     void copy_out(Request& r, float* hdr, uint8_t* rgb);
     DRequest make_request(const pcr_render_desc& d, int scene, double* accum) const;
-    bool flat(int scene) const { return scenes_[scene].dev.n_nodes == 0; }
+    // Whether the scene's paths never wait.
+    bool flat(int scene) const { return scenes_[scene].dev.n_nodes == 0 && !scenes_[scene].dev.staged; }
     void check_status();
     bool engine_step();
     void serve_loop();
@@ -246,9 +253,10 @@ private:
     std::vector<void*> qallocs_;
 
     // graph
-    cudaGraphExec_t graphs_[4] = {};   // by stages, captured when first launched
+    cudaGraphExec_t graphs_[8] = {};   // by stages, captured when first launched
     bool graph_dirty_ = true;
-    int grid_extend_ = 0, grid_shadow_ = 0, grid_round_ = 0, grid_flat_ = 0, grid_mesh_ = 0;
+    int grid_round_ = 0;
+    Grids grids_{};
 
     // requests
     std::mutex mu_;

@@ -4,9 +4,10 @@
 // new camera paths, and follows each until it ends or its next ray has a
 // triangle mesh to walk: then the path waits in the other queue, where
 // k_extend walks it, as k_shadow does the shadow rays that meet the mesh.
-// Paths on scenes without a mesh never wait.  Every kernel loops over a
-// device-side count, so a whole iteration (and several in a row) can be
-// captured in one CUDA graph with no host round trip.  No kernel waits on another block or on
+// Paths on scenes without a mesh never wait, those on staged scenes
+// (DScene::staged) after every vertex.  Every kernel loops over a device-side
+// count, so a whole iteration (and several in a row) can be captured in one
+// CUDA graph with no host round trip.  No kernel waits on another block or on
 // the host: there is no spin anywhere.
 #pragma once
 
@@ -25,7 +26,7 @@ struct EngineParams {
 // ------------------------------------------------------------------ schedule
 // One block.  Decides how many new camera paths each active request gets
 // this iteration: first up to `chunk` each (round-robin fairness), then the
-// remaining free slots oldest-first.  Requests on scenes without a mesh
+// remaining free slots oldest-first.  Requests whose paths never wait
 // (kReqFlat) share `fill` paths per iteration; the others share what the
 // waiting paths leave of `fill`.
 constexpr int kSchedThreads = 1024;
@@ -394,8 +395,10 @@ constexpr int kTraceMaxBlock = 256, kTraceMinBlocks = PCR_TRACE_MIN_BLOCKS, kSha
 
 // Closest hit of the paths that wait in queue q: the BVH walk, bounded by the
 // analytic hit.  Every ray here meets the mesh's box (others never wait), so
-// warps walk with all lanes from the start.  Also counts each request's
-// waiting paths.
+// warps walk with all lanes from the start.  kStaged: some of them are on
+// staged scenes, for which the analytic part is found here too.  Also counts
+// each request's waiting paths.
+template <bool kStaged>
 __global__ void __launch_bounds__(kTraceMaxBlock, kTraceMinBlocks) k_extend(EngineView E, int q)
 {
     constexpr unsigned kAll = 0xffffffffu;
@@ -410,9 +413,15 @@ __global__ void __launch_bounds__(kTraceMaxBlock, kTraceMinBlocks) k_extend(Engi
         if (i < n) {
             const int4 id = Q.id[i];
             slot = id.x;
-            float t = Q.hit[i].x, u = 0.f, v = 0.f;
-            const int tri = bvh4_closest<false>(E.scenes[id.w], xyz(Q.o[i]), xyz(Q.d[i]), t, u, v, nullptr);
-            if (tri >= 0) Q.hit[i] = make_float4(t, __uint_as_float(kPrimTri | (uint32_t)tri), u, v);
+            const DScene& S = E.scenes[id.w];
+            const float3 o = xyz(Q.o[i]), d = xyz(Q.d[i]);
+            const bool full = kStaged && S.staged;
+            float t = full ? FLT_MAX : Q.hit[i].x, u = 0.f, v = 0.f;
+            uint32_t prim = kPrimNone;
+            if (full) prim = scene_analytic<true>(S, o, d, t);
+            const int tri = bvh4_closest<false>(S, o, d, t, u, v, nullptr);
+            if (tri >= 0) prim = kPrimTri | (uint32_t)tri;
+            if (full || tri >= 0) Q.hit[i] = make_float4(t, __uint_as_float(prim), u, v);
         }
         const unsigned same = __match_any_sync(kAll, slot);
         if (slot >= 0 && lane == __ffs(same) - 1)
@@ -651,7 +660,9 @@ __device__ __forceinline__ bool diffuse_bounce(const DRequest& R, uint32_t pixel
 // rays that meet the mesh's box and that k_paths found lit otherwise: blocked
 // by a hit in front of the bound and closer than lightDist2 - 1e-3 (compared
 // in double, as the reference's double literal promotes it).  Lit samples add
-// their XYZ contribution to the pixel's FP64 accumulator.
+// their XYZ contribution to the pixel's FP64 accumulator.  kStaged: some are
+// on staged scenes, which have the whole test here.
+template <bool kStaged>
 __global__ void __launch_bounds__(kTraceMaxBlock, kShadowMinBlocks) k_shadow(EngineView E)
 {
     const int n = min(E.cnt->shadow_n, E.shadow_cap);
@@ -659,12 +670,18 @@ __global__ void __launch_bounds__(kTraceMaxBlock, kShadowMinBlocks) k_shadow(Eng
     const int stride = gridDim.x * blockDim.x;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const int nx = i + stride;
-        if (nx < n) { prefetch_l2(SQ.o + nx); prefetch_l2(SQ.d + nx); prefetch_l2(SQ.c + nx); prefetch_l2(SQ.bound + nx); }
+        if (nx < n) { prefetch_l2(SQ.o + nx); prefetch_l2(SQ.d + nx); prefetch_l2(SQ.c + nx); if (!kStaged) prefetch_l2(SQ.bound + nx); }
         const float4 o = SQ.o[i];
         if (o.w >= 0.f) {
             const DScene& S = E.scenes[__float_as_int(SQ.c[i].w) >> 16];
-            float t = SQ.bound[i], u, v;
-            if (bvh4_closest<false, true>(S, xyz(o), xyz(SQ.d[i]), t, u, v, nullptr, (double)o.w - 1e-3) != -2) {
+            const float3 d = xyz(SQ.d[i]);
+            float t, u, v;
+            int query = kShadowWalk;
+            if (kStaged && S.staged) query = blocked_tests<true, true>(S, E.mats, xyz(o), d, shadow_end(o.w), (double)o.w - 1e-3, t);
+            else t = SQ.bound[i];
+            if (query == kShadowWalk && bvh4_closest<false, true>(S, xyz(o), d, t, u, v, nullptr, (double)o.w - 1e-3) == -2)
+                query = kShadowBlocked;
+            if (query != kShadowBlocked) {
                 // read after the walk, so that it holds no registers across it
                 const float4 c = SQ.c[i];
                 const int pixel = __float_as_int(SQ.d[i].w);
@@ -886,7 +903,7 @@ __global__ void k_trace_rays(const DScene* scene, const DMaterial* mats, const f
             t_out[i] = tri >= 0 ? t : 0.f;
             if (counts) { counts[i * 2] = tc.nodes; counts[i * 2 + 1] = tc.tris; }
         } else {
-            const uint32_t prim = scene_closest(S, o, d, FLT_MAX, t, u, v);
+            const uint32_t prim = scene_closest<true>(S, o, d, FLT_MAX, t, u, v);
             const uint32_t kind = prim & kPrimKindMask, pidx = prim & kPrimIndexMask;
             int mi = -1;
             uint32_t code = 0;

@@ -115,6 +115,8 @@ struct DScene {
     int n_planes, n_spheres, n_nodes, n_tris, n_lights, mat_base, n_mats, n_pgroups;
     int n_sgroups;
     int emissive_tris;        // 1 when any triangle's material is emissive
+    // 1: k_extend and k_shadow trace the scene's rays in full (paths.cuh)
+    int staged;
     // The scene's only emissive material (scene-local index) when it has
     // exactly one and every light uses it, else -1.  Spectral paths of such
     // a scene carry emission x XYZ weight per wavelength instead of the
@@ -141,7 +143,8 @@ struct DScene {
 // Request flags
 constexpr int kReqSpectral = 1, kReqMIS = 2, kReqRussian = 4, kReqStratified = 8, kReqAdaptive = 16,
               kReqTerminate = 32, kReqCancelled = 64,
-              kReqFlat = 128;       // on a scene without a mesh: its paths never wait in the queues
+              kReqFlat = 128,       // on a scene whose paths never wait in the queues (no mesh, not staged)
+              kReqStaged = 256;     // on a staged scene
 
 struct DRequest {
     int scene, width, height, depth;
@@ -165,8 +168,8 @@ struct DRequest {
     int sample0, local_spp;
 };
 
-// Paths whose next ray has a mesh to walk, structure of arrays, one entry per
-// path.
+// Paths whose next ray has a mesh to walk, or all of it to be traced (staged
+// scenes), structure of arrays, one entry per path.
 struct PathQueue {
     float4* o;     // origin, hero lambda
     float4* d;     // direction, meta (bits): bounce | fork<<8 | single<<11 | n<<12
@@ -179,29 +182,33 @@ struct PathQueue {
     // multiplied by that material's emission at the wavelength.
     float4* w[3];
     // The ray's analytic hit (t, primitive), which k_extend replaces by a
-    // triangle's (t, primitive, u, v) where the mesh is hit first.
+    // triangle's (t, primitive, u, v) where the mesh is hit first; on staged
+    // scenes k_extend writes either.
     float4* hit;
 };
 
-// Shadow rays that have a mesh to walk.
+// Shadow rays that have a mesh to walk, or all of it to be traced.
 struct ShadowQueue {
     float4* o;     // origin, lightDist2 (below zero: an unused record)
     float4* d;     // direction, pixel (bits)
     float4* c;     // contribution (XYZ or RGB), request slot | scene << 16 (bits)
-    float* bound;  // no hit at or past it matters
+    float* bound;  // no hit at or past it matters (not set on staged scenes)
 };
 
 struct Counters {
-    int queue_n[2];
-    int shadow_n;
-    int new_n;            // mesh scenes: new paths of this iteration
+    // What every warp of k_paths adds to, each in an L2 line of its own:
+    // additions to one line are done one after another (six staged renders of
+    // 65 M vertices: 8.5 ms in k_paths, 10.1 ms with all three in one line).
+    alignas(256) int queue_n[2];
+    alignas(256) int shadow_n;
+    alignas(256) int next[3];  // k_paths: paths taken, by kind of scene
+    alignas(256) int new_n;    // requests whose paths can wait: new paths of this iteration
+    int path_n;                // the other requests: paths of this iteration
     int iter;
     int status;           // non-zero: a kernel reported an error
     int idle;             // 1 when no request has work left
     int n_rounds;         // adaptive requests whose round ended this iteration (k_status -> k_round)
     unsigned long long rays, shadow_rays, paths;
-    int path_n;                   // scenes without a mesh: paths of this iteration
-    int next[3];                  // k_paths: paths taken without / with a mesh, queued paths taken up
     unsigned long long path_begin, path_end;  // plain k_paths: globaltimer at its setup and its last block's end
 };
 

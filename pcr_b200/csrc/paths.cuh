@@ -7,7 +7,7 @@ namespace pcr {
 
 // k_paths follows each path in one thread, vertex after vertex, with its state
 // in registers: closest hit, shading, shadow rays, next direction.  On a scene
-// without a mesh (kMesh = false) it goes on to the path's end.  Where a ray
+// without a mesh it goes on to the path's end.  Where a ray
 // meets the mesh's box, the path waits in the queue for k_extend's walk and is
 // taken up again in the next iteration; a shadow ray that would be lit but
 // meets the box becomes a record for k_shadow.
@@ -43,9 +43,29 @@ namespace pcr {
 // With a mesh, against queue stages of one vertex each: bunny 320x320, 8 paths
 // a pixel 4.97 -> 2.01 ms, 24 uneven renders 80.8 -> 75.6 ms; six renders half
 // of them through a glass mesh, where most vertices wait, 22.4 -> 26.0 ms.
+//
+// Staged scenes are those whose rays this kernel would trace by the exact
+// tests (the estimates do not take the scene's quads), or whose shadow rays
+// have to find the closest of the mesh's emissive triangles.  Such traces are
+// long and leave lanes idle, which costs more at 16 warps per SM and inside
+// this code than the stages' memory traffic.  So a path is followed for one
+// vertex and waits: k_extend traces its next ray in full, and each of its
+// shadow samples is a record for k_shadow.  Six batched renders with 4 (16)
+// shadow rays, by stages of one vertex alone / traced here / staged: a Cornell
+// box with a tilted quad 24.9 (63.7) / 32.7 (79.5) / 26.4 (66.3) ms, with 88 quads
+// 71 (206) / 102 (316) / 76 (217) ms, with a mesh light 61 (197) / 112 (330) / 58
+// (193) ms; 256x256, 16 paths a pixel, 4 shadow rays: 4.6 / 1.9 / 1.8, 9.4 / 6.5 /
+// 4.8 and 7.5 / 7.2 / 3.8 ms.  The rest of the difference in the first two: a warp
+// appends its own paths, so neighbours lose each other sooner than where a
+// block appends together (which takes k_shadow 3 % less and k_paths 3 to 8 % more).
 constexpr int kPathBlock = 128;
 #ifndef PCR_PATH_MIN_BLOCKS
 #define PCR_PATH_MIN_BLOCKS 4
+#endif
+// (staged: 4, 5, 6, 7 blocks 8.8, 8.5, 8.4, 8.9 ms of the first batch above, 17.7,
+// 17.1, 17.7, 19.8 ms with 16 shadow rays)
+#ifndef PCR_STAGED_MIN_BLOCKS
+#define PCR_STAGED_MIN_BLOCKS 5
 #endif
 #ifndef PCR_PATH_REFILL
 #define PCR_PATH_REFILL 24
@@ -139,24 +159,64 @@ __device__ __forceinline__ void close_shadow_chunk(const EngineView& E, const Pa
     for (int k = P.shadow_next + lane; k < P.shadow_end; k += 32) E.sq.o[k] = make_float4(0.f, 0.f, 0.f, -1.f);
 }
 
+// Shadow records of a vertex on a staged scene: one per sample, those that add
+// nothing marked as unused.  The lanes that come here together reserve them
+// with one grid-wide atomic.  They find room: a staged path has one vertex an
+// iteration, the shadow queue holds every path's samples, and the launch that
+// may fill it further (mesh scenes) comes after.  Without a mesh the lanes'
+// records of a sample lie side by side (one contiguous run a store), over a
+// BVH those of a vertex, which walk mostly the same nodes.
+struct StagedRecords {
+    int first, step, most;
+    __device__ __forceinline__ int at(int s) const { return first + s * step; }
+    __device__ __forceinline__ void skip(const EngineView& E, int s) const
+    {
+        if (at(s) < E.shadow_cap) E.sq.o[at(s)] = make_float4(0.f, 0.f, 0.f, -1.f);
+    }
+};
+__device__ __forceinline__ StagedRecords staged_records(const EngineView& E, int samples, bool mesh)
+{
+    const unsigned m = __activemask();
+    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1, casters = __popc(m);
+    StagedRecords r;
+    r.most = (int)__reduce_max_sync(m, (unsigned)samples);
+    int at = 0;
+    if (lane == leader) at = shadow_slots(E, r.most * casters);
+    at = __shfl_sync(m, at, leader);
+    const int rank = __popc(m & ((1u << lane) - 1u));
+    const bool rows = __any_sync(m, mesh);
+    r.first = at + (rows ? rank * r.most : rank);
+    r.step = rows ? 1 : casters;
+    return r;
+}
+
+// The scenes whose paths a launch of k_paths follows.
+constexpr int kFlatScenes = 0, kMeshScenes = 1, kStagedScenes = 2;
+
 // Work of one launch: the paths of queue `cur` (kMesh), then the camera paths
 // numbered over the active list: position r's start at base[r] and are the
 // request's paths give_start[r], give_start[r] + 1, ...
-template <bool kMesh>
-__global__ void __launch_bounds__(kPathBlock, PCR_PATH_MIN_BLOCKS)
+template <int kScenes>
+__global__ void __launch_bounds__(kPathBlock, kScenes == kStagedScenes ? PCR_STAGED_MIN_BLOCKS : PCR_PATH_MIN_BLOCKS)
 k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
 {
     extern __shared__ __align__(16) unsigned char s_paths[];
     PathWarp& P = reinterpret_cast<PathWarp*>(s_paths)[threadIdx.x >> 5];
+    constexpr bool kMesh = kScenes != kFlatScenes, kStaged = kScenes == kStagedScenes;
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     Counters* C = E.cnt;
     const int* base = kMesh ? E.give_base : E.path_base;
-    int* counter = &C->next[kMesh ? 1 : 0];
+    int* counter = &C->next[kScenes];
+    // queued and camera paths of the other kind are left to its launch
+    auto mine = [&](const DRequest& R) { return !kMesh || ((R.flags & kReqStaged) != 0) == kStaged; };
     const int queued = kMesh ? min(C->queue_n[cur], E.queue_cap) : 0;
     const int n = queued + (kMesh ? C->new_n : C->path_n), n_act = *E.n_active;
-    int refill = queued > 0 ? kPathResume : kPathRefill;
+    // staged: all lanes at a time, from ranges of a few warps' worth each
+    int refill = kStaged ? 32 : queued > 0 ? kPathResume : kPathRefill;
+    const int take = n / (int)(gridDim.x * (kPathBlock / 32)) >= 512 ? 128 : 32;
+    int own = 0, left = 0;
     if (lane == 0) P.pending = P.shadow_next = P.shadow_end = 0;
     __syncwarp();
 
@@ -181,7 +241,48 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
         }
     };
 
+    // Next rays; a path whose ray waits for k_extend goes to the queue.
+    auto trace = [&]() {
+        bool wait = false;
+        if (alive && !traced) {
+            const DScene& S = E.scenes[E.reqs[slot].scene];
+            rays++;
+            t = FLT_MAX;
+            if (kStaged) {
+                wait = true;  // k_extend finds the hit
+            } else {
+                prim = scene_analytic<false>(S, o, d, t);
+                if (kMesh) wait = mesh_may_hit(S, o, d, t);
+            }
+        }
+        if (kMesh) {
+            const unsigned m = __ballot_sync(kAll, wait);
+            if (m) {
+                int at = 0;
+                if (lane == 0) at = atomicAdd(&C->queue_n[cur ^ 1], __popc(m));
+                at = __shfl_sync(kAll, at, 0) + __popc(m & below);
+                if (wait) {
+                    flush();
+                    alive = false;
+                    if (at < E.queue_cap) {
+                        const PathQueue& Q = E.q[cur ^ 1];
+                        const DRequest& R = E.reqs[slot];
+                        Q.o[at] = make_float4(o.x, o.y, o.z, lambda0);
+                        Q.d[at] = make_float4(d.x, d.y, d.z, __int_as_float(meta));
+                        Q.tp[at] = tp;
+                        Q.id[at] = make_int4(slot, (int)pixel, (int)sample, R.scene);
+                        if (!kStaged) Q.hit[at] = make_float4(t, __uint_as_float(prim), 0.f, 0.f);
+                        if (R.flags & kReqSpectral) store_weights(Q, at, lane_weights(P, lane));
+                    } else {
+                        atomicOr(&C->status, 2);
+                    }
+                }
+            }
+        }
+    };
+
     while (true) {
+        if (kStaged) trace();
         // ---- refill
         unsigned dead = __ballot_sync(kAll, !alive);
         if (dead) {
@@ -209,34 +310,55 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
             }
             if (more && __popc(dead) >= refill) {
                 int first = 0;
-                if (lane == 0) first = atomicAdd(counter, __popc(dead));
-                first = __shfl_sync(kAll, first, 0);
-                more = first + __popc(dead) < n;
+                if (kStaged) {
+                    if (left == 0) {
+                        if (lane == 0) own = atomicAdd(counter, take);
+                        own = __shfl_sync(kAll, own, 0);
+                        left = take;
+                    }
+                    first = own;
+                    own += 32;
+                    left -= 32;
+                    more = own < n;
+                } else {
+                    if (lane == 0) first = atomicAdd(counter, __popc(dead));
+                    first = __shfl_sync(kAll, first, 0);
+                    more = first + __popc(dead) < n;
+                }
                 int i = first + __popc(dead & below);
                 if (kMesh) {
-                    if (!alive && i < queued) {
-                        const PathQueue& Q = E.q[cur];
-                        const int4 id = Q.id[i];
-                        const float4 o4 = Q.o[i], d4 = Q.d[i], h = Q.hit[i];
-                        tp = Q.tp[i];
-                        slot = id.x;
-                        pixel = (uint32_t)id.y;
-                        sample = (uint32_t)id.z;
-                        o = xyz(o4);
-                        d = xyz(d4);
-                        lambda0 = o4.w;
-                        meta = __float_as_int(d4.w);
-                        t = h.x;
-                        prim = __float_as_uint(h.y);
-                        hu = h.z;
-                        hv = h.w;
-                        set_lane_weights(P, lane, (E.reqs[slot].flags & kReqSpectral) ? load_weights(Q, i) : rgb_weights());
-                        alive = traced = true;
+                    const PathQueue& Q = E.q[cur];
+                    if (kStaged && left > 0 && i + 32 < queued) {  // the warp's next paths
+                        const int nx = i + 32;
+                        prefetch_l2(Q.id + nx); prefetch_l2(Q.o + nx); prefetch_l2(Q.d + nx); prefetch_l2(Q.tp + nx);
+                        prefetch_l2(Q.hit + nx);
+                        prefetch_l2(Q.w[0] + nx); prefetch_l2(Q.w[1] + nx); prefetch_l2(Q.w[2] + nx);
                     }
-                    if (first + __popc(dead) >= queued) refill = kPathRefill;
+                    if (!alive && i < queued) {
+                        const int4 id = Q.id[i];
+                        const DRequest& R = E.reqs[id.x];
+                        if (mine(R)) {
+                            const float4 o4 = Q.o[i], d4 = Q.d[i], h = Q.hit[i];
+                            tp = Q.tp[i];
+                            slot = id.x;
+                            pixel = (uint32_t)id.y;
+                            sample = (uint32_t)id.z;
+                            o = xyz(o4);
+                            d = xyz(d4);
+                            lambda0 = o4.w;
+                            meta = __float_as_int(d4.w);
+                            t = h.x;
+                            prim = __float_as_uint(h.y);
+                            hu = h.z;
+                            hv = h.w;
+                            set_lane_weights(P, lane, (R.flags & kReqSpectral) ? load_weights(Q, i) : rgb_weights());
+                            alive = traced = true;
+                        }
+                    }
+                    if (!kStaged && first + __popc(dead) >= queued) refill = kPathRefill;
                     i -= queued;
                 }
-                if (!alive && i < n - queued) {
+                if (!alive && i >= 0 && i < n - queued) {  // (negative: a queued path, perhaps of the other kind)
                     int lo = 0, hi = n_act - 1;
                     while (lo < hi) {  // last r with base[r] <= i: it has paths in this launch
                         const int mid = (lo + hi + 1) >> 1;
@@ -244,17 +366,19 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
                     }
                     slot = E.active[lo];
                     const DRequest& R = E.reqs[slot];
-                    XyzWeights W = rgb_weights();
-                    const CameraPath p = camera_path(E, R, E.give_start[lo] + (i - base[lo]), xyz_scale, W);
-                    set_lane_weights(P, lane, W);
-                    pixel = p.pixel;
-                    sample = p.sample;
-                    o = make_float3(R.cam_x, R.cam_y, R.cam_z);
-                    d = p.d;
-                    lambda0 = p.lambda0;
-                    tp = make_float4(1.f, 1.f, 1.f, 1.f);
-                    meta = ((R.flags & kReqSpectral) ? R.hero : 4) << 12;
-                    alive = true;
+                    if (mine(R)) {
+                        XyzWeights W = rgb_weights();
+                        const CameraPath p = camera_path(E, R, E.give_start[lo] + (i - base[lo]), xyz_scale, W);
+                        set_lane_weights(P, lane, W);
+                        pixel = p.pixel;
+                        sample = p.sample;
+                        o = make_float3(R.cam_x, R.cam_y, R.cam_z);
+                        d = p.d;
+                        lambda0 = p.lambda0;
+                        tp = make_float4(1.f, 1.f, 1.f, 1.f);
+                        meta = ((R.flags & kReqSpectral) ? R.hero : 4) << 12;
+                        alive = true;
+                    }
                 }
             }
             if (!__any_sync(kAll, alive)) {
@@ -263,52 +387,22 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
             }
         }
 
-        // ---- trace
-        bool wait = false;
-        if (alive && !traced) {
-            const DScene& S = E.scenes[E.reqs[slot].scene];
-            rays++;
-            t = FLT_MAX;
-            prim = scene_analytic(S, o, d, t);
-            if (kMesh) wait = mesh_may_hit(S, o, d, t);
-        }
-        if (kMesh) {
-            const unsigned m = __ballot_sync(kAll, wait);
-            if (m) {
-                int at = 0;
-                if (lane == 0) at = atomicAdd(&C->queue_n[cur ^ 1], __popc(m));
-                at = __shfl_sync(kAll, at, 0) + __popc(m & below);
-                if (wait) {
-                    flush();
-                    alive = false;
-                    if (at < E.queue_cap) {
-                        const PathQueue& Q = E.q[cur ^ 1];
-                        const DRequest& R = E.reqs[slot];
-                        Q.o[at] = make_float4(o.x, o.y, o.z, lambda0);
-                        Q.d[at] = make_float4(d.x, d.y, d.z, __int_as_float(meta));
-                        Q.tp[at] = tp;
-                        Q.id[at] = make_int4(slot, (int)pixel, (int)sample, R.scene);
-                        Q.hit[at] = make_float4(t, __uint_as_float(prim), 0.f, 0.f);
-                        if (R.flags & kReqSpectral) store_weights(Q, at, lane_weights(P, lane));
-                    } else {
-                        atomicOr(&C->status, 2);
-                    }
-                }
+        // ---- trace (staged: above, so that the lanes of paths that wait are
+        // filled before the next vertex)
+        if (!kStaged) trace();
+        if (kScenes == kMeshScenes && P.shadow_end - P.shadow_next < kShadowLow) {  // shadow_next may lie past the end
+            close_shadow_chunk(E, P, lane);
+            __syncwarp();
+            if (lane == 0) {
+                const int at = shadow_slots(E, kShadowChunk);
+                P.shadow_next = at;
+                P.shadow_end = min(at + kShadowChunk, E.shadow_cap);
             }
-            if (P.shadow_end - P.shadow_next < kShadowLow) {  // shadow_next may lie past the end
-                close_shadow_chunk(E, P, lane);
-                __syncwarp();
-                if (lane == 0) {
-                    const int at = shadow_slots(E, kShadowChunk);
-                    P.shadow_next = at;
-                    P.shadow_end = min(at + kShadowChunk, E.shadow_cap);
-                }
-                __syncwarp();
-            }
+            __syncwarp();
         }
 
-        // ---- one vertex of each live path
-        if (alive) {
+        // ---- one vertex of each live path (staged: of those whose hit is known)
+        if (alive && (!kStaged || traced)) {
             const DRequest& R = E.reqs[slot];
             const DScene& S = E.scenes[R.scene];
             alive = traced = false;
@@ -423,14 +517,22 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
                             V = f3mul(apply_xyz(lane_weights(P, lane), tpal), scaleS);
                             cached = S.emit_mat;
                         }
+                        StagedRecords rec;
+                        if (kStaged) rec = staged_records(E, R.shadow, S.n_nodes > 0);
                         for (int s = 0; s < R.shadow; s++) {
                             const LightSample L = sample_light(S, R, pixel, sample, (uint32_t)fork, (uint32_t)bounce, (uint32_t)s);
                             const ShadowSegment g = shadow_segment(L, N, hc);
-                            if (!(g.G > 0.f)) continue;
+                            if (!(g.G > 0.f)) {
+                                if (kStaged) rec.skip(E, s);
+                                continue;
+                            }
                             shadows++;
-                            float bound;
-                            const int query = scene_blocked_analytic<kMesh>(S, E.mats, g.so, g.wi, g.d2, bound);
-                            if (query == kShadowBlocked) continue;
+                            float bound = 0.f;
+                            int query = kShadowWalk;
+                            if (!kStaged) {
+                                query = scene_blocked_analytic<kMesh, false>(S, E.mats, g.so, g.wi, g.d2, bound);
+                                if (query == kShadowBlocked) continue;
+                            }
                             if (L.mat != cached) {
                                 // product of this light material, once per vertex
                                 const DMaterial& lmat = E.mats[S.mat_base + L.mat];
@@ -440,14 +542,23 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
                             }
                             const float f = shadow_factor(S, R, g);
                             const float3 c = make_float3(V.x * f, V.y * f, V.z * f);
-                            if (kMesh && query == kShadowWalk && mesh_may_hit(S, g.so, g.wi, bound)) {
-                                int at = atomicAdd(&P.shadow_next, 1);
-                                if (at >= P.shadow_end) at = shadow_slots(E, 1);
+                            if (kMesh && query == kShadowWalk && (kStaged || mesh_may_hit(S, g.so, g.wi, bound))) {
+                                int at;
+                                if (kStaged) {
+                                    at = rec.at(s);
+                                } else {
+                                    at = atomicAdd(&P.shadow_next, 1);
+                                    if (at >= P.shadow_end) at = shadow_slots(E, 1);
+                                }
                                 if (at < E.shadow_cap) {
                                     E.sq.o[at] = make_float4(g.so.x, g.so.y, g.so.z, g.d2);
                                     E.sq.d[at] = make_float4(g.wi.x, g.wi.y, g.wi.z, __int_as_float((int)pixel));
                                     E.sq.c[at] = make_float4(c.x, c.y, c.z, __int_as_float(slot | (R.scene << 16)));
-                                    E.sq.bound[at] = bound;
+                                    if (!kStaged) E.sq.bound[at] = bound;
+                                    continue;
+                                }
+                                if (kStaged) {
+                                    atomicOr(&C->status, 1);  // never expected, see staged_records
                                     continue;
                                 }
                                 if (walk_blocked(S, g.so, g.wi, bound, g.d2)) continue;
@@ -456,6 +567,8 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
                             ay += (double)c.y;
                             az += (double)c.z;
                         }
+                        if (kStaged)
+                            for (int s = R.shadow; s < rec.most; s++) rec.skip(E, s);
                     }
                     float3 nd;
                     float rr_scale;
@@ -472,7 +585,7 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
         }
         __syncwarp();
     }
-    if (kMesh) close_shadow_chunk(E, P, lane);
+    if (kScenes == kMeshScenes) close_shadow_chunk(E, P, lane);
     rays = __reduce_add_sync(kAll, rays);
     shadows = __reduce_add_sync(kAll, shadows);
     if (lane == 0 && (rays | shadows)) {  // a resumed path that ends at its vertex traced no ray

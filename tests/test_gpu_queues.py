@@ -26,7 +26,7 @@ def _boxed(tmp_path, scene):
     from pcr_b200 import workloads
     sc = workloads.read_scene_json(scene_path(scene))
     root = tmp_path / scene
-    root.mkdir()
+    root.mkdir(parents=True)
     (root / "corners.obj").write_text(OBJ)
     if os.path.isdir(os.path.join(GOLDEN, "spd")):
         shutil.copytree(os.path.join(GOLDEN, "spd"), root / "spd")
@@ -58,3 +58,68 @@ def test_ray_counts_do_not_depend_on_the_queue(tmp_path, capacity, scene, kw):
     d = capi.render_desc(70, 41, seed=23, **kw)
     assert _counts(ctx, b, d)[1] == _counts(ctx, a, d)[1]
     ctx.close()
+
+
+def _slanted(tmp_path, scene):
+    """The scene's file with a tiny slanted quad far behind the camera: the
+    estimates do not take it, so its rays are traced in full by the stages."""
+    from pcr_b200 import workloads
+    sc = workloads.read_scene_json(scene_path(scene))
+    sc["primitives"].append({"type": "plane", "origin": [0, 0, 900.0], "u": [1e-3, 1e-3, 0], "v": [0, 1e-3, 1e-3],
+                             "material": next(k for k, m in sc["materials"].items() if "emissive" not in m)})
+    path = tmp_path / f"{scene}-slanted.json"
+    path.write_text(json.dumps(sc))
+    return str(path), GOLDEN
+
+
+@pytest.mark.parametrize("scene,kw", [
+    ("cornell", dict(depth=1, samples=1, shadow=1, spectral=False)),
+    ("cornell", dict(depth=5, samples=4, shadow=3, russian=True)),
+    ("cornell-spheres", dict(depth=4, samples=4, shadow=9, spectral=False, mis=True, stratified=True, aa=2)),
+    ("cornell-glass", dict(depth=8, samples=3, shadow=2, hero=3)),
+    ("cornell-glass", dict(depth=8, samples=3, shadow=2, terminate=True)),
+    ("closed-cornell-glass", dict(depth=8, samples=2, shadow=8)),
+    ("cornell-large-light", dict(depth=3, samples=2, shadow=2, aa=9, adaptive=True)),
+])
+@pytest.mark.parametrize("size", [(1, 1), (33, 7), (128, 96)])
+def test_staged_scenes_give_the_same_images(tmp_path, scene, kw, size):
+    """Scenes that the estimates do not take: the same images and counts, with
+    the rays traced by the extend and shadow stages and not by the path kernel
+    of mesh-free scenes."""
+    from pcr_b200 import capi
+    d = capi.render_desc(*size, seed=11, **kw)
+    for capacity in (1 << 9, 1 << 17):
+        ctx = capi.Context(device=0, queue_capacity=capacity)
+        a, b = ctx.load_scene_json(scene_path(scene), GOLDEN), ctx.load_scene_json(*_slanted(tmp_path, scene))
+        whole, counts, _ = _counts(ctx, a, d)
+        staged, staged_counts, st = _counts(ctx, b, d)
+        if not kw.get("adaptive"):  # (a converged pixel's last bits may decide its number of rounds)
+            assert staged_counts == counts
+            assert np.allclose(staged[0], whole[0], rtol=1e-6, atol=1e-7)
+        else:
+            assert np.allclose(staged[0], whole[0], rtol=1e-4, atol=1e-5)
+        assert st["stage_launches"]["extend"] > 0 and st["stage_launches"]["shadow"] > 0, st["stage_launches"]
+        assert st["stage_launches"]["other"] == 0, st["stage_launches"]
+        ctx.close()
+
+
+def test_one_batch_of_all_kinds_of_scenes(tmp_path):
+    """Requests on scenes without a mesh, with one, and staged (the last two
+    share the queues), in one wavefront: each as if alone."""
+    from pcr_b200 import capi
+    for capacity in (1 << 12, 1 << 18):
+        ctx = capi.Context(device=0, queue_capacity=capacity)
+        sids = [ctx.load_scene_json(*x) for x in (
+            (scene_path("cornell"), GOLDEN), _boxed(tmp_path / str(capacity), "cornell-glass"),
+            _slanted(tmp_path, "cornell-spheres"), (scene_path("cornell-mesh-light"), GOLDEN),
+            _boxed(tmp_path / str(capacity), "cornell"), _slanted(tmp_path, "cornell-glass"))]
+        descs = [capi.render_desc(w, h, depth=depth, samples=spp, shadow=s, seed=60 + k, spectral=spectral)
+                 for k, (w, h, depth, spp, s, spectral) in enumerate([
+                     (64, 48, 4, 4, 2, True), (50, 31, 7, 3, 3, True), (71, 40, 3, 5, 1, False),
+                     (48, 48, 4, 4, 4, True), (33, 90, 5, 2, 10, True), (40, 40, 6, 6, 2, True)])]
+        alone = [ctx.render(s, d)[0] for s, d in zip(sids, descs)]
+        ids = [ctx.submit(s, d) for s, d in zip(sids, descs)]
+        ctx.run_until_idle()
+        for rid, image in zip(ids, alone):
+            assert np.allclose(ctx.fetch(rid)[0], image, rtol=1e-6, atol=1e-7)
+        ctx.close()
