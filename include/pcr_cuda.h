@@ -223,8 +223,9 @@ pcr_status pcr_fetch(pcr_ctx *ctx, pcr_request_id id, float *hdr_out, uint8_t *r
  * cancelRequested flag (code/Renderer.cpp:170-181,
  * code/Gpu/Opengl/OpenglRenderer.cpp:2170-2175).  A request waiting for
  * admission is dropped at once; a running one stops issuing paths at the
- * next block of iterations and ends when the paths in flight retire (within
- * its depth in iterations), its partial result discarded; a finished one
+ * next block of iterations and ends when the paths in flight retire (on
+ * scenes without a mesh, with the iteration they started in; otherwise within
+ * its depth + 1 iterations), its partial result discarded; a finished one
  * keeps its result (the call is then a no-op).  pcr_wait on a cancelled
  * request returns PCR_ERR_CANCELLED; pcr_fetch returns PCR_ERR_CANCELLED
  * and releases it. */

@@ -54,7 +54,8 @@ __global__ void k_set_params(EngineParams* P, EngineParams p) { *P = p; }
 
 // Cancels a running request: no path of it is issued after this point
 // (its total becomes what was issued so far), so it finishes once the paths
-// already in flight retire, within `depth` iterations.  Launched between
+// already in flight retire: those of a flat request with the iteration they
+// started in, others within depth + 1 iterations.  Launched between
 // blocks of iterations on the engine stream, so no kernel reads the entry
 // while it changes.
 __global__ void k_cancel(EngineView E, int slot)
@@ -176,6 +177,12 @@ Engine::~Engine()
     cudaStreamDestroy(stream_);
 }
 
+// What a batched or served iteration may take on.
+static EngineParams batch_params(const EngineTuning& t, int sms)
+{
+    return {t.queue_capacity, t.chunk_paths, t.regen_every, 2 * sms * PCR_PATH_MIN_BLOCKS * kPathBlock};
+}
+
 void Engine::alloc_buffers()
 {
     std::vector<void*>& T = qallocs_;
@@ -237,7 +244,7 @@ void Engine::alloc_buffers()
     sq_.d = dalloc<float4>(shadow_cap_, T);
     sq_.c = dalloc<float4>(shadow_cap_, T);
     sq_.bound = dalloc<float>(shadow_cap_, T);
-    EngineParams p{fill, tune_.chunk_paths, tune_.regen_every};
+    const EngineParams p = batch_params(tune_, sms_);
     CK(cudaMemcpy(d_params_, &p, sizeof(p), cudaMemcpyHostToDevice));
     graph_dirty_ = true;
 }
@@ -988,10 +995,14 @@ void Engine::launch_block(int stages)
     int64_t launches[8];
     std::copy(stage_launches_, stage_launches_ + 8, launches);
     const bool graph = use_graph_ && !profile_;
+    // Flat requests' paths run to their end within the iteration, which lasts
+    // accordingly: its blocks are short, so that what happens between them (a
+    // cancel, an admission, a result) waits for a few iterations only.
+    const int iters = stages & kStagesFlat ? 2 : tune_.iters_per_launch;
     if (graph && !graphs_[stages]) {
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-        for (int it = 0; it < tune_.iters_per_launch; it++) launch_iteration(it & 1, stages, false);
+        for (int it = 0; it < iters; it++) launch_iteration(it & 1, stages, false);
         CK(cudaStreamEndCapture(stream_, &g));
         CK(cudaGraphInstantiate(&graphs_[stages], g, 0));
         CK(cudaGraphDestroy(g));
@@ -1001,14 +1012,14 @@ void Engine::launch_block(int stages)
     }
     if (graph) {
         CK(cudaGraphLaunch(graphs_[stages], stream_));
-        stage_launches_[5] += tune_.iters_per_launch;
-        stage_launches_[6] += 2 * tune_.iters_per_launch;
+        stage_launches_[5] += iters;
+        stage_launches_[6] += 2 * iters;
         if (stages & (kStagesMesh | kStagesStaged))
-            for (int k : {1, 2, 3}) stage_launches_[k] += tune_.iters_per_launch;
-        if (stages & kStagesFlat) stage_launches_[7] += tune_.iters_per_launch;
-        iterations_ += tune_.iters_per_launch;
+            for (int k : {1, 2, 3}) stage_launches_[k] += iters;
+        if (stages & kStagesFlat) stage_launches_[7] += iters;
+        iterations_ += iters;
     } else {
-        for (int it = 0; it < tune_.iters_per_launch; it++) launch_iteration(it & 1, stages, profile_);
+        for (int it = 0; it < iters; it++) launch_iteration(it & 1, stages, profile_);
     }
 }
 
@@ -1471,14 +1482,16 @@ double Engine::progress(int64_t id)
 }
 
 // ---------------------------------------------------------------- plain method
-// Traces every path of R, the only request of E, with k_paths: launches of
-// at most kPathsPerLaunch paths, so that other work of the device gets its
-// turn within about a tenth of a second.
-constexpr int64_t kPathsPerLaunch = 1 << 26;
+// Traces every path of R, the only request of E, with k_paths: launches of as
+// many paths as may take kRaysPerLaunch rays (a Cornell box's in about a tenth
+// of a second, longer where the exact tests trace them), at least what fills
+// the GPU, so that other work of the device gets its turn.
+constexpr int64_t kRaysPerLaunch = 1 << 30, kPathsPerLaunch = 1 << 26;
 void Engine::trace_flat(const EngineView& E, const DRequest& R, int grid)
 {
-    for (int64_t at = 0; at < R.total; at += kPathsPerLaunch) {
-        const int n = (int)std::min<int64_t>(kPathsPerLaunch, R.total - at);
+    const int64_t per = std::min<int64_t>(kPathsPerLaunch, std::max<int64_t>((int64_t)grid * kPathBlock, kRaysPerLaunch / ((int64_t)R.depth * (1 + R.shadow))));
+    for (int64_t at = 0; at < R.total; at += per) {
+        const int n = (int)std::min<int64_t>(per, R.total - at);
         k_one_request<<<1, 1, 0, stream_>>>(E, R, at, n);
         if (profile_) CK(cudaEventRecord(prof_ev_[0], stream_));
         k_paths<kFlatScenes><<<std::min(grid, (n + kPathBlock - 1) / kPathBlock), kPathBlock, kPathSmem, stream_>>>(E, 0, xyz_scale_);
@@ -1546,7 +1559,7 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     ensure_shadow_capacity(desc.shadow_samples);
     if (graph_dirty_) launch_shapes();
     const int64_t px = (int64_t)desc.width * desc.height;
-    EngineParams p{tune_.queue_capacity, tune_.queue_capacity, 1};
+    EngineParams p{tune_.queue_capacity, tune_.queue_capacity, 1, 0};
     k_set_params<<<1, 1, 0, stream_>>>((EngineParams*)d_params_, p);
     activate(r, 0);
     slot_owner_[0] = -1;  // the plain request is not in the request map
@@ -1586,8 +1599,7 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     active_dirty_ = true;
     bytes_in_use_ -= r.bytes;
     upload_active();
-    EngineParams q{tune_.queue_capacity, tune_.chunk_paths, tune_.regen_every};
-    k_set_params<<<1, 1, 0, stream_>>>((EngineParams*)d_params_, q);
+    k_set_params<<<1, 1, 0, stream_>>>((EngineParams*)d_params_, batch_params(tune_, sms_));
     copy_out(r, hdr, rgb);
     cudaEventDestroy(r.ev_ready);
     if (st) {
@@ -1791,7 +1803,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
         int fill = kNoAllocFill;
         if (scenes_[scene].dev.staged) fill = std::min(fill, kNoAllocShadow / (4 * desc.shadow_samples));
         const int pass = (int)std::min<int64_t>(px, fill);
-        k_set_params<<<1, 1, 0, stream_>>>(params, EngineParams{pass, pass, 1});
+        k_set_params<<<1, 1, 0, stream_>>>(params, EngineParams{pass, pass, 1, 0});
         CK(cudaGetLastError());
 
         // launch shapes from the occupancy calculator (no allocation involved)

@@ -21,6 +21,7 @@ struct EngineParams {
     int fill;          // refill target (paths in flight)
     int chunk;         // per-request issue chunk per refill
     int regen_every;   // refill cadence in iterations
+    int wave;          // paths worth an iteration however long they are (0: no bound but `fill`)
 };
 
 // ------------------------------------------------------------------ schedule
@@ -60,6 +61,38 @@ __device__ __forceinline__ Share share_slots(typename Scan::TempStorage& tmp, lo
     return s;
 }
 
+// Paths are followed to their end, or to the mesh, within the iteration they
+// start in, so their number alone does not bound an iteration, and cancels,
+// admissions and results are seen between blocks of iterations.  The new paths
+// of an iteration are cut to kVerticesPerSlot possible vertices per place of
+// `fill`, with p.wave paths at least; where that cuts, every request gets an
+// equal share first.  64: an iteration that is cut is mostly the tail of its
+// few longest paths (1 M places, 6.3 M paths of depth 64 in a closed room,
+// 16 shadow rays, with 16 / 32 / 64 vertices per place: 182 / 152 / 133 ms, a
+// cancel seen after 24 / 52 / 123 ms; 290 ms when an iteration was one vertex).
+constexpr long long kVerticesPerSlot = 64;
+template <typename Scan>
+__device__ __forceinline__ void limit_work(typename Scan::TempStorage& tmp, Share& s, long long cost, const EngineParams& p)
+{
+    __shared__ int s_most;
+    if (p.wave <= 0) return;
+    if (threadIdx.x == 0) s_most = 0;
+    __syncthreads();
+    const long long work = s.mine * cost;
+    if (work > 0) atomicMax(&s_most, (int)cost);
+    long long before, all;
+    Scan(tmp).ExclusiveSum(work, before, all);
+    __syncthreads();
+    const long long wave = p.wave < p.fill ? p.wave : p.fill, least = wave * s_most;
+    const long long budget = least > kVerticesPerSlot * p.fill ? least : kVerticesPerSlot * p.fill;
+    if (all <= budget) return;
+    const int n = __syncthreads_count(work > 0);
+    const Share part = share_slots<Scan>(tmp, work, budget / n, budget);
+    if (work > 0) s.mine = part.mine / cost;
+    Scan(tmp).ExclusiveSum(s.mine, s.before, s.all);
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(kSchedThreads) k_schedule(EngineView E, const EngineParams* P, int cur)
 {
     typedef cub::BlockScan<long long, kSchedThreads, cub::BLOCK_SCAN_WARP_SCANS> Scan;
@@ -79,7 +112,7 @@ __global__ void __launch_bounds__(kSchedThreads) k_schedule(EngineView E, const 
 
     int slot = -1;
     bool flat = false;
-    long long rem = 0;
+    long long rem = 0, cost = 0;  // vertices that a path may have in the iteration, where that is more than one
     if (tid < n_act) {
         slot = E.active[tid];
         if (E.round_state[slot] == 1) {
@@ -103,10 +136,17 @@ __global__ void __launch_bounds__(kSchedThreads) k_schedule(EngineView E, const 
         rem = E.reqs[slot].total - (long long)E.issued[slot];
         if (rem < 0) rem = 0;
         flat = (E.reqs[slot].flags & kReqFlat) != 0;
+        if (!(E.reqs[slot].flags & kReqStaged)) cost = E.reqs[slot].depth;
     }
     Share q = {0, 0, 0}, w = {0, 0, 0};
-    if (__syncthreads_or(!flat && rem > 0)) q = share_slots<Scan>(tmp, flat ? 0 : rem, p.chunk, free_slots);
-    if (__syncthreads_or(flat && rem > 0)) w = share_slots<Scan>(tmp, flat ? rem : 0, p.chunk, p.fill);
+    if (__syncthreads_or(!flat && rem > 0)) {
+        q = share_slots<Scan>(tmp, flat ? 0 : rem, p.chunk, free_slots);
+        limit_work<Scan>(tmp, q, cost, p);
+    }
+    if (__syncthreads_or(flat && rem > 0)) {
+        w = share_slots<Scan>(tmp, flat ? rem : 0, p.chunk, p.fill);
+        limit_work<Scan>(tmp, w, cost, p);
+    }
     if (tid < n_act) {
         const long long g = q.mine + w.mine;
         E.give_base[tid] = (int)q.before;
