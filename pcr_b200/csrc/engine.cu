@@ -227,7 +227,7 @@ void Engine::alloc_buffers()
     snap_next_ = 0;
     snap_inflight_ = 0;
     CK(cudaMallocHost(&h_params_, sizeof(EngineParams)));
-    CK(cudaMallocHost(&h_cnt_, sizeof(Counters)));
+    CK(cudaMallocHost(&h_plain_, sizeof(HostSnap)));
 
     const int fill = tune_.queue_capacity;
     queue_cap_ = fill * 4;   // a dispersive-glass fork turns one path into up to four
@@ -258,8 +258,8 @@ void Engine::free_buffers()
         h = nullptr;
     }
     if (h_params_) cudaFreeHost(h_params_);
-    if (h_cnt_) cudaFreeHost(h_cnt_);
-    h_cnt_ = nullptr;
+    if (h_plain_) cudaFreeHost(h_plain_);
+    h_plain_ = nullptr;
     h_snap_ = nullptr;
     h_params_ = nullptr;
 }
@@ -825,7 +825,7 @@ void Engine::activate(Request& r, int slot)
     const pcr_render_desc& d = r.desc;
     const int64_t px = (int64_t)d.width * d.height;
     alloc_request(r);
-    DRequest R = make_request(d, r.scene, r.accum);
+    DRequest R = make_request(d, r.scene, r.accum, r.staged);
     if (adaptive_rounds(d)) {
         R.flags |= kReqAdaptive;
         CK(cudaMallocFromPoolAsync(&r.act[0], px * sizeof(int), pool_, stream_));
@@ -898,7 +898,7 @@ int Engine::active_stages() const
     return m ? m : kStagesMesh;
 }
 
-void Engine::launch_iteration(int cur, int stages, bool prof)
+void Engine::launch_iteration(int cur, int stages, bool prof, bool rounds)
 {
     const EngineView E = view();
     // stage index: 1 extend 2 shade (k_paths on scenes whose paths can wait) 3 shadow 5 schedule
@@ -924,9 +924,11 @@ void Engine::launch_iteration(int cur, int stages, bool prof)
         mark(7);
     }
     k_status<<<1, 1024, 0, stream_>>>(E, cur ^ 1);
-    k_round<<<grid_round_, 256, 0, stream_>>>(E);
+    if (rounds) {
+        k_round<<<grid_round_, 256, 0, stream_>>>(E);
+        stage_launches_[6]++;
+    }
     mark(6);
-    stage_launches_[6]++;
     CK(cudaGetLastError());
     if (prof) {
         CK(cudaEventSynchronize(prof_ev_[done]));
@@ -1509,11 +1511,11 @@ void Engine::render_flat(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats*
     const DRequest R = make_request(r.desc, r.scene, r.accum);
     trace_flat(view(), R, grids_.paths[kFlatScenes]);
     active_dirty_ = true;  // the active list holds slot 0
-    CK(cudaMemcpyAsync(h_cnt_, d_cnt_, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
+    CK(cudaMemcpyAsync(&h_plain_->cnt, d_cnt_, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
     finish_request(r, stream_);
     copy_out(r, hdr, rgb);  // waits for the resolve, and so for the counters
     cudaEventDestroy(r.ev_ready);
-    const Counters& c = *h_cnt_;
+    const Counters& c = h_plain_->cnt;
     if (c.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "device reported queue overflow");
     if (st) {
         st->device_ms = c.path_end > c.path_begin ? (double)(c.path_end - c.path_begin) * 1e-6 : 0.0;
@@ -1523,6 +1525,14 @@ void Engine::render_flat(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats*
         st->shadow_rays = 0;
     }
 }
+
+// A plain render of at most this many paths on a mesh scene is staged: few warps
+// take long over vertices whose shadow rays follow one another in a lane, as
+// records they run side by side.  Bunny, 4 vertices, 8 shadow rays, stages of
+// before / paths followed to the mesh / staged: 16x16 490 / 603 / 410 us, 64x64
+// 600 / 790 / 515 us, 65,536 paths 2.2 / 1.0 / 0.82 ms, 196,566 paths - / 1.33 /
+// 1.30 ms, 262,144 paths - / 1.45 / 1.56 ms.
+constexpr int64_t kStagedPaths = 1 << 16;
 
 void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, uint8_t* rgb, pcr_render_stats* st)
 {
@@ -1561,39 +1571,36 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     const int64_t px = (int64_t)desc.width * desc.height;
     EngineParams p{tune_.queue_capacity, tune_.queue_capacity, 1, 0};
     k_set_params<<<1, 1, 0, stream_>>>((EngineParams*)d_params_, p);
+    r.staged = px * local_spp(desc) * std::max(1, desc.aa_samples) <= kStagedPaths;
     activate(r, 0);
     slot_owner_[0] = -1;  // the plain request is not in the request map
     upload_active();
     const int64_t total = px * local_spp(desc) * std::max(1, desc.aa_samples);
     const int64_t fills = (total + tune_.queue_capacity - 1) / tune_.queue_capacity;
-    const int stages = queue_stages(scene);
+    const int stages = r.staged ? kStagesStaged : queue_stages(scene);
     int cur = 0;
     // a path waits at most `depth` times
     for (int64_t it = 0; it < fills + desc.depth; it++) {
-        launch_iteration(cur, stages, profile_);
+        launch_iteration(cur, stages, profile_, false);
         cur ^= 1;
     }
     int64_t extra = 0;
+    HostSnap& end = *h_plain_;
     while (true) {
-        int done = 0;
-        CK(cudaMemcpyAsync(&done, d_done_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+        CK(cudaMemcpyAsync(&end.cnt, d_cnt_, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
+        CK(cudaMemcpyAsync(end.done, d_done_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+        CK(cudaMemcpyAsync(end.tf, d_tfirst_, 8, cudaMemcpyDeviceToHost, stream_));
+        CK(cudaMemcpyAsync(end.td, d_tdone_, 8, cudaMemcpyDeviceToHost, stream_));
         CK(cudaStreamSynchronize(stream_));
-        Counters c;
-        CK(cudaMemcpy(&c, d_cnt_, sizeof(c), cudaMemcpyDeviceToHost));
-        if (c.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "device reported queue overflow");
-        if (done) break;
+        if (end.cnt.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "device reported queue overflow");
+        if (end.done[0]) break;
         if (++extra > fills * (4 * (int64_t)desc.depth + 8)) throw PcrError(PCR_ERR_TIMEOUT, "plain render did not finish");
-        launch_iteration(cur, stages, profile_);
+        launch_iteration(cur, stages, profile_, false);
         cur ^= 1;
     }
-    // a plain render always ends on queue parity 0 for the next user
-    if (cur != 0) {
-        launch_iteration(cur, stages, false);
-        cur ^= 1;
-    }
-    unsigned long long tf = 0, td = 0;
-    CK(cudaMemcpy(&tf, d_tfirst_, 8, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(&td, d_tdone_, 8, cudaMemcpyDeviceToHost));
+    // the next user starts with queue 0: both are empty
+    CK(cudaMemsetAsync(d_cnt_->queue_n, 0, sizeof(d_cnt_->queue_n), stream_));
+    const unsigned long long tf = end.tf[0], td = end.td[0];
     finish_request(r, stream_);
     active_slots_.clear();
     active_dirty_ = true;
@@ -1660,7 +1667,7 @@ static void* noalloc_scratch(int device)
 }
 
 // The request entry of a render (Engine::activate adds the adaptive fields).
-DRequest Engine::make_request(const pcr_render_desc& d, int scene, double* accum) const
+DRequest Engine::make_request(const pcr_render_desc& d, int scene, double* accum, bool staged) const
 {
     const SceneEntry& S = scenes_[scene];
     DRequest R{};
@@ -1676,7 +1683,7 @@ DRequest Engine::make_request(const pcr_render_desc& d, int scene, double* accum
     R.shadow = d.shadow_samples;
     R.flags = (d.spectral ? kReqSpectral : 0) | (d.mis ? kReqMIS : 0) | (d.russian ? kReqRussian : 0) |
               (d.stratified ? kReqStratified : 0) | (d.spectral_terminate ? kReqTerminate : 0) |
-              (flat(scene) ? kReqFlat : 0) | (S.dev.staged ? kReqStaged : 0);
+              (flat(scene) ? kReqFlat : 0) | (S.dev.staged || staged ? kReqStaged : 0);
     R.hero = std::min(4, std::max(1, d.hero_samples <= 0 ? 4 : d.hero_samples));
     R.strata = d.stratified ? std::max(1, (int)std::lround(std::sqrt((float)d.samples))) : 0;
     R.cam_x = S.cam[0];

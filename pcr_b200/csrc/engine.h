@@ -57,6 +57,7 @@ struct Request {
     uint64_t admit_block = 0;  // blocks launched before this request's slot was (re)set
     bool cancel_running = false;        // cancel asked while Active
     bool cancel_sent = false;           // k_cancel launched for it
+    bool staged = false;                // traced as on a staged scene
     int* act[2] = {nullptr, nullptr};   // adaptive: pixel lists of alternate rounds
     float4* welford = nullptr;          // adaptive: per-pixel mean / M2
 };
@@ -132,7 +133,7 @@ private:
     Grids launch_grids();
     void launch_queue_stage(const EngineView& E, const Grids& g, int cur, int stages, int stage);
     int active_stages() const;
-    void launch_iteration(int cur, int stages, bool profile);
+    void launch_iteration(int cur, int stages, bool profile, bool rounds = true);  // rounds: for adaptive requests
     void launch_block(int stages);
     void launch_shapes();
     int trace_block() const { return (tune_.block_size + 31) / 32 * 32; }  // whole warps
@@ -143,7 +144,7 @@ private:
     void finish_request(Request& r, cudaStream_t rs);
     void release_cancelled(Request& r);
     void copy_out(Request& r, float* hdr, uint8_t* rgb);
-    DRequest make_request(const pcr_render_desc& d, int scene, double* accum) const;
+    DRequest make_request(const pcr_render_desc& d, int scene, double* accum, bool staged = false) const;
     // Whether the scene's paths never wait.
     bool flat(int scene) const { return scenes_[scene].dev.n_nodes == 0 && !scenes_[scene].dev.staged; }
     void check_status();
@@ -234,7 +235,7 @@ private:
     // while the host harvests or is briefly descheduled.
     static constexpr int kSnapRing = 4;
     cudaMemPool_t pool_ = nullptr;
-    Counters* h_cnt_ = nullptr;   // pinned: a plain render's counters
+    HostSnap* h_plain_ = nullptr;  // pinned: a plain render's counters, and slot 0's words
     HostSnap* h_snaps_[kSnapRing] = {};
     cudaEvent_t ev_snaps_[kSnapRing] = {};
     HostSnap* h_snap_ = nullptr;  // the snapshot harvest reads (one of h_snaps_)

@@ -435,8 +435,8 @@ constexpr int kTraceMaxBlock = 256, kTraceMinBlocks = PCR_TRACE_MIN_BLOCKS, kSha
 
 // Closest hit of the paths that wait in queue q: the BVH walk, bounded by the
 // analytic hit.  Every ray here meets the mesh's box (others never wait), so
-// warps walk with all lanes from the start.  kStaged: some of them are on
-// staged scenes, for which the analytic part is found here too.  Also counts
+// warps walk with all lanes from the start.  kStaged: some of them are of
+// staged requests, for which the analytic part is found here too.  Also counts
 // each request's waiting paths.
 template <bool kStaged>
 __global__ void __launch_bounds__(kTraceMaxBlock, kTraceMinBlocks) k_extend(EngineView E, int q)
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(kTraceMaxBlock, kTraceMinBlocks) k_extend(Engi
             slot = id.x;
             const DScene& S = E.scenes[id.w];
             const float3 o = xyz(Q.o[i]), d = xyz(Q.d[i]);
-            const bool full = kStaged && S.staged;
+            const bool full = kStaged && (E.reqs[slot].flags & kReqStaged);
             float t = full ? FLT_MAX : Q.hit[i].x, u = 0.f, v = 0.f;
             uint32_t prim = kPrimNone;
             if (full) prim = scene_analytic<true>(S, o, d, t);
@@ -700,8 +700,8 @@ __device__ __forceinline__ bool diffuse_bounce(const DRequest& R, uint32_t pixel
 // rays that meet the mesh's box and that k_paths found lit otherwise: blocked
 // by a hit in front of the bound and closer than lightDist2 - 1e-3 (compared
 // in double, as the reference's double literal promotes it).  Lit samples add
-// their XYZ contribution to the pixel's FP64 accumulator.  kStaged: some are
-// on staged scenes, which have the whole test here.
+// their XYZ contribution to the pixel's FP64 accumulator.  kStaged: some are of
+// staged requests, which have the whole test here.
 template <bool kStaged>
 __global__ void __launch_bounds__(kTraceMaxBlock, kShadowMinBlocks) k_shadow(EngineView E)
 {
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(kTraceMaxBlock, kShadowMinBlocks) k_shadow(Eng
             const float3 d = xyz(SQ.d[i]);
             float t, u, v;
             int query = kShadowWalk;
-            if (kStaged && S.staged) query = blocked_tests<true, true>(S, E.mats, xyz(o), d, shadow_end(o.w), (double)o.w - 1e-3, t);
+            if (kStaged && (E.reqs[__float_as_int(SQ.c[i].w) & 0xFFFF].flags & kReqStaged)) query = scene_blocked_analytic<true, true>(S, E.mats, xyz(o), d, o.w, t);
             else t = SQ.bound[i];
             if (query == kShadowWalk && bvh4_closest<false, true>(S, xyz(o), d, t, u, v, nullptr, (double)o.w - 1e-3) == -2)
                 query = kShadowBlocked;

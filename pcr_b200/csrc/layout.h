@@ -115,7 +115,7 @@ struct DScene {
     int n_planes, n_spheres, n_nodes, n_tris, n_lights, mat_base, n_mats, n_pgroups;
     int n_sgroups;
     int emissive_tris;        // 1 when any triangle's material is emissive
-    // 1: k_extend and k_shadow trace the scene's rays in full (paths.cuh)
+    // 1: its requests are kReqStaged (paths.cuh)
     int staged;
     // The scene's only emissive material (scene-local index) when it has
     // exactly one and every light uses it, else -1.  Spectral paths of such
@@ -144,7 +144,7 @@ struct DScene {
 constexpr int kReqSpectral = 1, kReqMIS = 2, kReqRussian = 4, kReqStratified = 8, kReqAdaptive = 16,
               kReqTerminate = 32, kReqCancelled = 64,
               kReqFlat = 128,       // on a scene whose paths never wait in the queues (no mesh, not staged)
-              kReqStaged = 256;     // on a staged scene
+              kReqStaged = 256;     // on a staged scene, or few paths on a mesh scene: k_extend and k_shadow trace its rays in full
 
 struct DRequest {
     int scene, width, height, depth;

@@ -37,9 +37,14 @@ def _boxed(tmp_path, scene):
     return str(path), str(root)
 
 
-def _counts(ctx, sid, desc):
+def _counts(ctx, sid, desc, batch=False):
     ctx.reset_stats()
-    images = ctx.render(sid, desc)[:2]
+    if batch:
+        rid = ctx.submit(sid, desc)
+        ctx.run_until_idle()
+        images = ctx.fetch(rid)[:2]
+    else:
+        images = ctx.render(sid, desc)[:2]
     st = ctx.stats()
     return images, (st["paths"], st["rays"], st["shadow_rays"]), st
 
@@ -56,7 +61,24 @@ def test_ray_counts_do_not_depend_on_the_queue(tmp_path, capacity, scene, kw):
     a = ctx.load_scene_json(scene_path(scene), GOLDEN)
     b = ctx.load_scene_json(*_boxed(tmp_path, scene))
     d = capi.render_desc(70, 41, seed=23, **kw)
-    assert _counts(ctx, b, d)[1] == _counts(ctx, a, d)[1]
+    counts = _counts(ctx, a, d)[1]
+    # (a plain render of few paths is staged, a batched one is not)
+    assert _counts(ctx, b, d)[1] == counts
+    assert _counts(ctx, b, d, batch=True)[1] == counts
+    ctx.close()
+
+
+@pytest.mark.parametrize("depth", [1, 4, 5])
+def test_a_small_plain_render_launches_what_it_needs(tmp_path, depth):
+    """A plain render of few paths on a mesh scene: `depth` iterations after
+    the camera rays', no kernel for adaptive rounds, none to restore the
+    queues' order."""
+    from pcr_b200 import capi
+    ctx = capi.Context(device=0)
+    sid = ctx.load_scene_json(*_boxed(tmp_path, "cornell"))
+    st = _counts(ctx, sid, capi.render_desc(64, depth=depth, samples=1, shadow=2, seed=5))[2]
+    assert st["iterations"] == 1 + depth
+    assert st["stage_launches"]["status"] == st["iterations"], st["stage_launches"]
     ctx.close()
 
 
