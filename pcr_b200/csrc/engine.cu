@@ -473,6 +473,7 @@ int Engine::upload_scene(const pcr_scene_desc& d)
             M.tabE[k] = m.tab_emissive[k];
         }
         e.mats.push_back(M);
+        e.disperses = e.disperses || ((M.flags & kMatTransparent) && M.cauchyB != 0.f);
     }
     auto check_mat = [&](int m, const char* what) {
         if (m < 0 || m >= d.n_materials) throw PcrError(PCR_ERR_INVALID, std::string(what) + ": material index out of range");
@@ -1626,10 +1627,15 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
 // callers that may not allocate device memory during a render.  Inputs are
 // a scene already uploaded to the context; outputs are caller-owned device
 // buffers.  Every GPU that loads the library holds the array until exit.
-constexpr int kNoAllocFill = 8192;                       // paths per pass
+// Mesh scenes: paths in flight (staged, see kStagedPaths).  Four times as many
+// where no path can fork; the more, the fewer iterations of launches and of
+// waits for the longest walk.  Bunny 256x256, 8 vertices, 4 paths a pixel, 4
+// shadow rays, 8192 in flight and paths followed to the mesh / staged 40960:
+// 13.1 / 7.0 ms; half glass 128x128, 4 vertices: 5.3 / 4.4 ms.
+constexpr int kNoAllocFill = 10240;
 constexpr int kNoAllocQueue = kNoAllocFill * 4;          // room for 4-way forks
 constexpr int kNoAllocShadowPerVertex = 8;
-constexpr int kNoAllocShadow = kNoAllocQueue * 6;         // past it, shadow rays walk the mesh in place
+constexpr int kNoAllocShadow = kNoAllocQueue * 4;         // past it, vertices wait for the next iteration
 constexpr int64_t kNoAllocMaxPixels = 256 * 256;
 constexpr size_t kNoAllocAlign = 256;
 constexpr size_t align_up(size_t x) { return (x + kNoAllocAlign - 1) / kNoAllocAlign * kNoAllocAlign; }
@@ -1795,38 +1801,34 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     E.cmf_table = d_cmf_;
     E.queue_cap = kNoAllocQueue;
 
-    const DRequest R = make_request(desc, scene, accum);
+    const DRequest R = make_request(desc, scene, accum, true);
     if (scenes_[scene].dev.n_nodes == 0) {
-        int g_paths;
-        grid_for((const void*)k_paths<kFlatScenes>, kPathBlock, kPathSmem, &g_paths);
-        trace_flat(E, R, g_paths);
+        trace_flat(E, R, graph_dirty_ ? launch_grids().paths[kFlatScenes] : grids_.paths[kFlatScenes]);
     } else {
         k_admit<<<1, 1, 0, stream_>>>(E, R, 0);
         ActiveList L;
         L.n = 1;
         L.slots[0] = 0;
         k_set_active<<<1, 32, 0, stream_>>>(E, L);
-        // (a staged scene's shadow records have no way past a full queue)
-        int fill = kNoAllocFill;
-        if (scenes_[scene].dev.staged) fill = std::min(fill, kNoAllocShadow / (4 * desc.shadow_samples));
-        const int pass = (int)std::min<int64_t>(px, fill);
-        k_set_params<<<1, 1, 0, stream_>>>(params, EngineParams{pass, pass, 1, 0});
+        const bool forks = (R.flags & kReqSpectral) && !(R.flags & kReqTerminate) && R.hero > 1 && scenes_[scene].disperses;
+        const int fill = forks ? kNoAllocFill : std::min(kNoAllocQueue, kNoAllocShadow / desc.shadow_samples);
+        k_set_params<<<1, 1, 0, stream_>>>(params, EngineParams{fill, fill, 1, 0});
         CK(cudaGetLastError());
 
-        // launch shapes from the occupancy calculator (no allocation involved)
-        const Grids g = launch_grids();
+        // (launch shapes: kept, or from the occupancy calculator, which allocates nothing)
+        const Grids g = graph_dirty_ ? launch_grids() : grids_;
         int cur = 0;
         auto iteration = [&]() {
             k_schedule<<<1, kSchedThreads, 0, stream_>>>(E, params, cur);
-            for (int stage : {2, 1, 3}) launch_queue_stage(E, g, cur, queue_stages(scene), stage);
+            for (int stage : {2, 1, 3}) launch_queue_stage(E, g, cur, kStagesStaged, stage);
             k_status<<<1, 1024, 0, stream_>>>(E, cur ^ 1);
             CK(cudaGetLastError());
             cur ^= 1;
         };
         const int64_t total = px * local_spp(desc) * std::max(1, desc.aa_samples);
-        const int64_t fills = (total + pass - 1) / pass;
+        const int64_t fills = (total + fill - 1) / fill;
         for (int64_t it = 0; it < fills + desc.depth; it++) iteration();
-        for (int64_t extra = 0;; extra++) {
+        for (int64_t extra = 0;;) {
             int flag = 0;
             Counters c;
             CK(cudaMemcpyAsync(&flag, done, sizeof(int), cudaMemcpyDeviceToHost, stream_));
@@ -1835,7 +1837,8 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
             if (c.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "pcr_render_noalloc: device reported queue overflow");
             if (flag) break;
             if (extra > fills * (4 * (int64_t)desc.depth + 8)) throw PcrError(PCR_ERR_TIMEOUT, "pcr_render_noalloc did not finish");
-            iteration();
+            // an iteration starts at most `fill` paths, and the last ones need another
+            for (int64_t left = (total - (int64_t)c.paths) / fill; left >= 0; left--, extra++) iteration();
         }
     }
     const double inv = 1.0 / ((double)desc.samples * std::max(1, desc.aa_samples));

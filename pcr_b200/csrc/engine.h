@@ -35,6 +35,7 @@ struct SceneEntry {
     std::string name, version;
     float cam[3] = {0, 0, 0}, fov = 65.f;
     std::vector<DMaterial> mats;
+    bool disperses = false;    // has a dispersive transparent material
     bool live = false;
 };
 

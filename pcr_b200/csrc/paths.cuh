@@ -161,13 +161,13 @@ __device__ __forceinline__ void close_shadow_chunk(const EngineView& E, const Pa
 
 // Shadow records of a vertex on a staged scene: one per sample, those that add
 // nothing marked as unused.  The lanes that come here together reserve them
-// with one grid-wide atomic.  They find room: a staged path has one vertex an
-// iteration, the shadow queue holds every path's samples, and the launch that
-// may fill it further (mesh scenes) comes after.  Without a mesh the lanes'
-// records of a sample lie side by side (one contiguous run a store), over a
-// BVH those of a vertex, which walk mostly the same nodes.
+// with one grid-wide atomic; where they do not fit (the fixed queue of
+// pcr_render_noalloc), the vertices wait for the next iteration.  Without a
+// mesh the lanes' records of a sample lie side by side (one contiguous run a
+// store), over a BVH those of a vertex, which walk mostly the same nodes.
 struct StagedRecords {
     int first, step, most;
+    bool fit;
     __device__ __forceinline__ int at(int s) const { return first + s * step; }
     __device__ __forceinline__ void skip(const EngineView& E, int s) const
     {
@@ -183,6 +183,7 @@ __device__ __forceinline__ StagedRecords staged_records(const EngineView& E, int
     int at = 0;
     if (lane == leader) at = shadow_slots(E, r.most * casters);
     at = __shfl_sync(m, at, leader);
+    r.fit = at + r.most * casters <= E.shadow_cap;
     const int rank = __popc(m & ((1u << lane) - 1u));
     const bool rows = __any_sync(m, mesh);
     r.first = at + (rows ? rank * r.most : rank);
@@ -504,80 +505,88 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
                     // code/Renderer.cpp:782 with samples = 1)
                     const float4 al = spectral ? spec4(m, 0, lam4) : rgb4(m.albedo);
                     float3 hc = f3add(hit, f3mul(N, 1e-3f));
-                    o = hc;
-                    if (S.total_light_area > 0.f) {
-                        const float inv_pi = 1.f / 3.14159274f;
-                        const float scaleS = S.total_light_area * inv_pi / (float)R.shadow;
-                        const float4 tpal = mul4(tp, al);
-                        int cached = -1;
-                        float3 V = make_float3(0.f, 0.f, 0.f);
-                        if (spectral && S.emit_mat >= 0) {
-                            // every light has the one emissive material, whose
-                            // emission the weights already hold
-                            V = f3mul(apply_xyz(lane_weights(P, lane), tpal), scaleS);
-                            cached = S.emit_mat;
+                    StagedRecords rec;
+                    bool postponed = false;
+                    if (kStaged && S.total_light_area > 0.f) {
+                        rec = staged_records(E, R.shadow, S.n_nodes > 0);
+                        if (!rec.fit) {
+                            // the path waits as it came, and its ray is traced again
+                            for (int s = 0; s < rec.most; s++) rec.skip(E, s);
+                            postponed = alive = true;
+                            rays--;
                         }
-                        StagedRecords rec;
-                        if (kStaged) rec = staged_records(E, R.shadow, S.n_nodes > 0);
-                        for (int s = 0; s < R.shadow; s++) {
-                            const LightSample L = sample_light(S, R, pixel, sample, (uint32_t)fork, (uint32_t)bounce, (uint32_t)s);
-                            const ShadowSegment g = shadow_segment(L, N, hc);
-                            if (!(g.G > 0.f)) {
-                                if (kStaged) rec.skip(E, s);
-                                continue;
-                            }
-                            shadows++;
-                            float bound = 0.f;
-                            int query = kShadowWalk;
-                            if (!kStaged) {
-                                query = scene_blocked_analytic<kMesh, false>(S, E.mats, g.so, g.wi, g.d2, bound);
-                                if (query == kShadowBlocked) continue;
-                            }
-                            if (L.mat != cached) {
-                                // product of this light material, once per vertex
-                                const DMaterial& lmat = E.mats[S.mat_base + L.mat];
-                                const float4 c = spectral ? mul4(tpal, spec4(lmat, 1, lam4)) : mul4(tpal, rgb4(lmat.emissive));
-                                V = f3mul(apply_xyz(lane_weights(P, lane), c), scaleS);
-                                cached = L.mat;
-                            }
-                            const float f = shadow_factor(S, R, g);
-                            const float3 c = make_float3(V.x * f, V.y * f, V.z * f);
-                            if (kMesh && query == kShadowWalk && (kStaged || mesh_may_hit(S, g.so, g.wi, bound))) {
-                                int at;
-                                if (kStaged) {
-                                    at = rec.at(s);
-                                } else {
-                                    at = atomicAdd(&P.shadow_next, 1);
-                                    if (at >= P.shadow_end) at = shadow_slots(E, 1);
-                                }
-                                if (at < E.shadow_cap) {
-                                    E.sq.o[at] = make_float4(g.so.x, g.so.y, g.so.z, g.d2);
-                                    E.sq.d[at] = make_float4(g.wi.x, g.wi.y, g.wi.z, __int_as_float((int)pixel));
-                                    E.sq.c[at] = make_float4(c.x, c.y, c.z, __int_as_float(slot | (R.scene << 16)));
-                                    if (!kStaged) E.sq.bound[at] = bound;
-                                    continue;
-                                }
-                                if (kStaged) {
-                                    atomicOr(&C->status, 1);  // never expected, see staged_records
-                                    continue;
-                                }
-                                if (walk_blocked(S, g.so, g.wi, bound, g.d2)) continue;
-                            }
-                            ax += (double)c.x;
-                            ay += (double)c.y;
-                            az += (double)c.z;
-                        }
-                        if (kStaged)
-                            for (int s = R.shadow; s < rec.most; s++) rec.skip(E, s);
                     }
-                    float3 nd;
-                    float rr_scale;
-                    if (diffuse_bounce(R, pixel, sample, (uint32_t)fork, bounce, last, spectral, al, N, nd, rr_scale)) {
-                        d = nd;
-                        tp = make_float4(tp.x * al.x * rr_scale, tp.y * al.y * rr_scale, tp.z * al.z * rr_scale,
-                                         tp.w * al.w * rr_scale);
-                        meta++;
-                        alive = true;
+                    if (!postponed) {
+                        o = hc;
+                        if (S.total_light_area > 0.f) {
+                            const float inv_pi = 1.f / 3.14159274f;
+                            const float scaleS = S.total_light_area * inv_pi / (float)R.shadow;
+                            const float4 tpal = mul4(tp, al);
+                            int cached = -1;
+                            float3 V = make_float3(0.f, 0.f, 0.f);
+                            if (spectral && S.emit_mat >= 0) {
+                                // every light has the one emissive material, whose
+                                // emission the weights already hold
+                                V = f3mul(apply_xyz(lane_weights(P, lane), tpal), scaleS);
+                                cached = S.emit_mat;
+                            }
+                            for (int s = 0; s < R.shadow; s++) {
+                                const LightSample L = sample_light(S, R, pixel, sample, (uint32_t)fork, (uint32_t)bounce, (uint32_t)s);
+                                const ShadowSegment g = shadow_segment(L, N, hc);
+                                if (!(g.G > 0.f)) {
+                                    if (kStaged) rec.skip(E, s);
+                                    continue;
+                                }
+                                shadows++;
+                                float bound = 0.f;
+                                int query = kShadowWalk;
+                                if (!kStaged) {
+                                    query = scene_blocked_analytic<kMesh, false>(S, E.mats, g.so, g.wi, g.d2, bound);
+                                    if (query == kShadowBlocked) continue;
+                                }
+                                if (L.mat != cached) {
+                                    // product of this light material, once per vertex
+                                    const DMaterial& lmat = E.mats[S.mat_base + L.mat];
+                                    const float4 c = spectral ? mul4(tpal, spec4(lmat, 1, lam4)) : mul4(tpal, rgb4(lmat.emissive));
+                                    V = f3mul(apply_xyz(lane_weights(P, lane), c), scaleS);
+                                    cached = L.mat;
+                                }
+                                const float f = shadow_factor(S, R, g);
+                                const float3 c = make_float3(V.x * f, V.y * f, V.z * f);
+                                if (kMesh && query == kShadowWalk && (kStaged || mesh_may_hit(S, g.so, g.wi, bound))) {
+                                    int at;
+                                    if (kStaged) {
+                                        at = rec.at(s);
+                                    } else {
+                                        at = atomicAdd(&P.shadow_next, 1);
+                                        if (at >= P.shadow_end) at = shadow_slots(E, 1);
+                                    }
+                                    if (at < E.shadow_cap) {
+                                        E.sq.o[at] = make_float4(g.so.x, g.so.y, g.so.z, g.d2);
+                                        E.sq.d[at] = make_float4(g.wi.x, g.wi.y, g.wi.z, __int_as_float((int)pixel));
+                                        E.sq.c[at] = make_float4(c.x, c.y, c.z, __int_as_float(slot | (R.scene << 16)));
+                                        if (!kStaged) E.sq.bound[at] = bound;
+                                        continue;
+                                    }
+                                    if (kStaged) continue;  // (they fit)
+                                    if (walk_blocked(S, g.so, g.wi, bound, g.d2)) continue;
+                                }
+                                ax += (double)c.x;
+                                ay += (double)c.y;
+                                az += (double)c.z;
+                            }
+                            if (kStaged)
+                                for (int s = R.shadow; s < rec.most; s++) rec.skip(E, s);
+                        }
+                        float3 nd;
+                        float rr_scale;
+                        if (diffuse_bounce(R, pixel, sample, (uint32_t)fork, bounce, last, spectral, al, N, nd, rr_scale)) {
+                            d = nd;
+                            tp = make_float4(tp.x * al.x * rr_scale, tp.y * al.y * rr_scale, tp.z * al.z * rr_scale,
+                                             tp.w * al.w * rr_scale);
+                            meta++;
+                            alive = true;
+                        }
                     }
                 }
             }
