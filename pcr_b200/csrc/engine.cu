@@ -1804,6 +1804,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     const DRequest R = make_request(desc, scene, accum, true);
     if (scenes_[scene].dev.n_nodes == 0) {
         trace_flat(E, R, graph_dirty_ ? launch_grids().paths[kFlatScenes] : grids_.paths[kFlatScenes]);
+        CK(cudaMemcpyAsync(&h_plain_->cnt, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
     } else {
         k_admit<<<1, 1, 0, stream_>>>(E, R, 0);
         ActiveList L;
@@ -1854,6 +1855,8 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
         CK(cudaGetLastError());
     }
     CK(cudaStreamSynchronize(stream_));
+    if (scenes_[scene].dev.n_nodes == 0 && h_plain_->cnt.status)
+        throw PcrError(PCR_ERR_DEVICE_STATUS, "pcr_render_noalloc: device reported queue overflow");
 }
 
 // ---------------------------------------------------------------- parity entry points
