@@ -979,8 +979,14 @@ __global__ void k_eval_stage(int what, const float* __restrict__ params, const f
 {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         switch (what) {
-        case 0: out[i] = sigmoid_fit<false>(make_float4(params[0], params[1], params[2], params[3]), in[i]); break;
-        case 1: out[i] = spectrum_lerp<false>(params, in[i]); break;
+        // (the form that renders use, over the wavelengths they carry)
+        case 0: {
+            const float4 fit = make_float4(params[0], params[1], params[2], params[3]);
+            out[i] = in[i] >= 400.f && in[i] <= 700.f ? sigmoid_fit<true>(fit, in[i]) : sigmoid_fit<false>(fit, in[i]);
+        } break;
+        case 1:
+            out[i] = in[i] >= 400.f && in[i] <= 700.f ? spectrum_lerp<true>(params, in[i]) : spectrum_lerp<false>(params, in[i]);
+            break;
         case 2: { float3 c = cmf(in[i]); out[i * 3] = c.x; out[i * 3 + 1] = c.y; out[i * 3 + 2] = c.z; } break;
         case 3: {
             float3 c = cmf(in[i * 2]);
