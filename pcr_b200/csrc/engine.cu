@@ -1137,23 +1137,35 @@ void Engine::upload_items(void* dev, size_t items, size_t item_bytes, const Fill
 // times as long.
 void Engine::download_parts(const void* dev, std::initializer_list<HostPart> parts, cudaStream_t after, cudaEvent_t ready)
 {
-    // the wanted range
+    // The wanted range.  (A result in device memory, which this thread cannot
+    // write, is copied by itself.)
+    struct DevicePart { void* to; size_t at, bytes; };
+    std::vector<HostPart> wanted(parts);
+    std::vector<DevicePart> on_device;
     size_t total = 0, begin = SIZE_MAX, end = 0;
-    for (const HostPart& p : parts) {
+    for (HostPart& p : wanted) {
+        cudaPointerAttributes a{};
+        if (p.host) CK(cudaPointerGetAttributes(&a, p.host));
+        if (p.host && a.type == cudaMemoryTypeDevice) {
+            on_device.push_back({p.host, total, p.bytes});
+            p.host = nullptr;
+        }
         if (p.host && p.bytes) {
             begin = std::min(begin, total);
             end = total + p.bytes;
         }
         total += p.bytes;
     }
-    if (begin >= end) return;
-    StagingHold hold{this, take_staging(end - begin)};
+    if (begin >= end && on_device.empty()) return;
+    StagingHold hold{this, take_staging(begin < end ? end - begin : 0)};
     const Staging& st = hold.st;
     if (!ready) {
         CK(cudaEventRecord(st.piece[0], after));
         ready = st.piece[0];
     }
     CK(cudaStreamWaitEvent(st.stream, ready, 0));
+    for (const DevicePart& p : on_device)
+        CK(cudaMemcpyAsync(p.to, (const uint8_t*)dev + p.at, p.bytes, cudaMemcpyDeviceToDevice, st.stream));
     constexpr size_t kPieceBytes = 1u << 20;
     for (size_t first = begin; first < end; first += st.bytes) {
         const size_t count = std::min(st.bytes, end - first);
@@ -1167,7 +1179,7 @@ void Engine::download_parts(const void* dev, std::initializer_list<HostPart> par
             const size_t lo = first + count * k / pieces, hi = first + count * (k + 1) / pieces;
             CK(cudaEventSynchronize(st.piece[k]));
             size_t at = 0;
-            for (const HostPart& p : parts) {
+            for (const HostPart& p : wanted) {
                 const size_t a = std::max(lo, at), z = std::min(hi, at + p.bytes);
                 if (p.host && a < z) std::memcpy((uint8_t*)p.host + (a - at), st.buf + (a - first), z - a);
                 at += p.bytes;
