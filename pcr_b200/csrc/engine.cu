@@ -123,6 +123,7 @@ Engine::Engine(const pcr_ctx_opts* o)
     CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_));
     CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&resolve_stream_, cudaStreamNonBlocking));
+    CK(cudaStreamCreateWithFlags(&capture_stream_, cudaStreamNonBlocking));
     xyz_scale_ = (700.f - 400.f) / host_ybar_integral();
     slot_owner_.assign(kMaxActive, -1);
     scenes_.reserve(256);
@@ -161,6 +162,7 @@ Engine::~Engine()
     }
     cudaStreamSynchronize(stream_);
     cudaStreamDestroy(resolve_stream_);
+    cudaStreamDestroy(capture_stream_);
     for (Staging& st : staging_idle_) {
         cudaStreamSynchronize(st.stream);
         if (st.buf) cudaFreeHost(st.buf);
@@ -899,7 +901,7 @@ int Engine::active_stages() const
     return m ? m : kStagesMesh;
 }
 
-void Engine::launch_iteration(int cur, int stages, bool prof, bool rounds)
+void Engine::launch_iteration(int cur, int stages, bool prof, bool rounds, cudaStream_t st)
 {
     const EngineView E = view();
     // stage index: 1 extend 2 shade (k_paths on scenes whose paths can wait) 3 shadow 5 schedule
@@ -910,23 +912,23 @@ void Engine::launch_iteration(int cur, int stages, bool prof, bool rounds)
         stage_launches_[stage]++;
         if (!prof) return;
         stage_of[done++] = stage;
-        CK(cudaEventRecord(prof_ev_[done], stream_));
+        CK(cudaEventRecord(prof_ev_[done], st));
     };
-    if (prof) CK(cudaEventRecord(prof_ev_[0], stream_));
-    k_schedule<<<1, kSchedThreads, 0, stream_>>>(E, (const EngineParams*)d_params_, cur);
+    if (prof) CK(cudaEventRecord(prof_ev_[0], st));
+    k_schedule<<<1, kSchedThreads, 0, st>>>(E, (const EngineParams*)d_params_, cur);
     mark(5);
     if (stages & (kStagesMesh | kStagesStaged))
         for (int stage : {2, 1, 3}) {
-            launch_queue_stage(E, grids_, cur, stages, stage);
+            launch_queue_stage(E, grids_, cur, stages, stage, st);
             mark(stage);
         }
     if (stages & kStagesFlat) {
-        k_paths<kFlatScenes><<<grids_.paths[kFlatScenes], kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
+        k_paths<kFlatScenes><<<grids_.paths[kFlatScenes], kPathBlock, kPathSmem, st>>>(E, cur, xyz_scale_);
         mark(7);
     }
-    k_status<<<1, 1024, 0, stream_>>>(E, cur ^ 1);
+    k_status<<<1, 1024, 0, st>>>(E, cur ^ 1);
     if (rounds) {
-        k_round<<<grid_round_, 256, 0, stream_>>>(E);
+        k_round<<<grid_round_, 256, 0, st>>>(E);
         stage_launches_[6]++;
     }
     mark(6);
@@ -957,20 +959,20 @@ Engine::Grids Engine::launch_grids()
 }
 
 // Stage 2 (k_paths), 1 (k_extend) or 3 (k_shadow) of an iteration.
-void Engine::launch_queue_stage(const EngineView& E, const Grids& g, int cur, int stages, int stage)
+void Engine::launch_queue_stage(const EngineView& E, const Grids& g, int cur, int stages, int stage, cudaStream_t st)
 {
     const int B = trace_block(), staged = stages & kStagesStaged ? 1 : 0;
     if (stage == 2) {
         // staged first: its shadow records always find room
-        if (staged) k_paths<kStagedScenes><<<g.paths[kStagedScenes], kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
+        if (staged) k_paths<kStagedScenes><<<g.paths[kStagedScenes], kPathBlock, kPathSmem, st>>>(E, cur, xyz_scale_);
         if (stages & kStagesMesh)
-            k_paths<kMeshScenes><<<g.paths[kMeshScenes], kPathBlock, kPathSmem, stream_>>>(E, cur, xyz_scale_);
+            k_paths<kMeshScenes><<<g.paths[kMeshScenes], kPathBlock, kPathSmem, st>>>(E, cur, xyz_scale_);
     } else if (stage == 1) {
-        if (staged) k_extend<true><<<g.extend[1], B, 0, stream_>>>(E, cur ^ 1);
-        else k_extend<false><<<g.extend[0], B, 0, stream_>>>(E, cur ^ 1);
+        if (staged) k_extend<true><<<g.extend[1], B, 0, st>>>(E, cur ^ 1);
+        else k_extend<false><<<g.extend[0], B, 0, st>>>(E, cur ^ 1);
     } else {
-        if (staged) k_shadow<true><<<g.shadow[1], B, 0, stream_>>>(E);
-        else k_shadow<false><<<g.shadow[0], B, 0, stream_>>>(E);
+        if (staged) k_shadow<true><<<g.shadow[1], B, 0, st>>>(E);
+        else k_shadow<false><<<g.shadow[0], B, 0, st>>>(E);
     }
 }
 
@@ -1004,9 +1006,10 @@ void Engine::launch_block(int stages)
     const int iters = stages & kStagesFlat ? 2 : tune_.iters_per_launch;
     if (graph && !graphs_[stages]) {
         cudaGraph_t g;
-        CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-        for (int it = 0; it < iters; it++) launch_iteration(it & 1, stages, false);
-        CK(cudaStreamEndCapture(stream_, &g));
+        // (on a stream that no one else knows: a caller may use stream_ meanwhile)
+        CK(cudaStreamBeginCapture(capture_stream_, cudaStreamCaptureModeThreadLocal));
+        for (int it = 0; it < iters; it++) launch_iteration(it & 1, stages, false, true, capture_stream_);
+        CK(cudaStreamEndCapture(capture_stream_, &g));
         CK(cudaGraphInstantiate(&graphs_[stages], g, 0));
         CK(cudaGraphDestroy(g));
         // capture counted launches that did not run
@@ -1022,7 +1025,7 @@ void Engine::launch_block(int stages)
         if (stages & kStagesFlat) stage_launches_[7] += iters;
         iterations_ += iters;
     } else {
-        for (int it = 0; it < iters; it++) launch_iteration(it & 1, stages, profile_);
+        for (int it = 0; it < iters; it++) launch_iteration(it & 1, stages, profile_, true, stream_);
     }
 }
 
@@ -1195,7 +1198,6 @@ void Engine::copy_out(Request& r, float* hdr, uint8_t* rgb)
     const size_t px = (size_t)r.desc.width * r.desc.height;
     if (hdr || rgb) download_parts(r.d_hdr, {{hdr, px * 3 * sizeof(float)}, {rgb, px * 3}}, nullptr, r.ev_ready);
     else CK(cudaEventSynchronize(r.ev_ready));
-    // (not on stream_, which the serving thread may be capturing)
     CK(cudaFreeAsync(r.d_hdr, resolve_stream_));
     r.d_hdr = nullptr;
     r.d_rgb = nullptr;
@@ -1594,7 +1596,7 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     int cur = 0;
     // a path waits at most `depth` times
     for (int64_t it = 0; it < fills + desc.depth; it++) {
-        launch_iteration(cur, stages, profile_, false);
+        launch_iteration(cur, stages, profile_, false, stream_);
         cur ^= 1;
     }
     int64_t extra = 0;
@@ -1608,7 +1610,7 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
         if (end.cnt.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "device reported queue overflow");
         if (end.done[0]) break;
         if (++extra > fills * (4 * (int64_t)desc.depth + 8)) throw PcrError(PCR_ERR_TIMEOUT, "plain render did not finish");
-        launch_iteration(cur, stages, profile_, false);
+        launch_iteration(cur, stages, profile_, false, stream_);
         cur ^= 1;
     }
     // the next user starts with queue 0: both are empty
@@ -1833,7 +1835,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
         int cur = 0;
         auto iteration = [&]() {
             k_schedule<<<1, kSchedThreads, 0, stream_>>>(E, params, cur);
-            for (int stage : {2, 1, 3}) launch_queue_stage(E, g, cur, kStagesStaged, stage);
+            for (int stage : {2, 1, 3}) launch_queue_stage(E, g, cur, kStagesStaged, stage, stream_);
             k_status<<<1, 1024, 0, stream_>>>(E, cur ^ 1);
             CK(cudaGetLastError());
             cur ^= 1;

@@ -132,9 +132,9 @@ private:
         int paths[3], extend[2], shadow[2];
     };
     Grids launch_grids();
-    void launch_queue_stage(const EngineView& E, const Grids& g, int cur, int stages, int stage);
+    void launch_queue_stage(const EngineView& E, const Grids& g, int cur, int stages, int stage, cudaStream_t st);
     int active_stages() const;
-    void launch_iteration(int cur, int stages, bool profile, bool rounds = true);  // rounds: for adaptive requests
+    void launch_iteration(int cur, int stages, bool profile, bool rounds, cudaStream_t st);  // rounds: for adaptive requests
     void launch_block(int stages);
     void launch_shapes();
     int trace_block() const { return (tune_.block_size + 31) / 32 * 32; }  // whole warps
@@ -161,6 +161,7 @@ private:
     // queued on stream_: a request is harvested from the device state copied
     // after the block it finished in, by which point its accumulator is final.
     cudaStream_t resolve_stream_ = nullptr;
+    cudaStream_t capture_stream_ = nullptr;  // graphs are captured on it; nothing runs there
     // Pinned staging buffers, each with its own copy stream and an event per
     // piece, kept idle between transfers.  A transfer takes one (or makes
     // one), so fetches from several threads copy at the same time.  A buffer
