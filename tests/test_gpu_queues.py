@@ -145,3 +145,65 @@ def test_one_batch_of_all_kinds_of_scenes(tmp_path):
         for rid, image in zip(ids, alone):
             assert np.allclose(ctx.fetch(rid)[0], image, rtol=1e-6, atol=1e-7)
         ctx.close()
+
+
+@pytest.mark.parametrize("capacity", [1 << 9, 1 << 17])
+@pytest.mark.parametrize("scene,kw", [
+    ("cornell", dict(depth=1, samples=1, shadow=1, spectral=False)),
+    ("cornell", dict(depth=6, samples=5, shadow=20, hero=1)),
+    ("cornell-spheres", dict(depth=4, samples=4, shadow=2, spectral=False, mis=True, russian=True, stratified=True, aa=2)),
+    ("cornell-glass", dict(depth=8, samples=3, shadow=2, hero=2)),
+    ("cornell-glass", dict(depth=8, samples=3, shadow=2, hero=3)),
+    ("cornell-glass", dict(depth=8, samples=3, shadow=2, terminate=True)),
+    ("closed-cornell-glass", dict(depth=8, samples=2, shadow=8)),
+])
+@pytest.mark.parametrize("size", [(1, 1), (33, 7), (128, 96)])
+def test_waiting_paths_give_the_same_images(tmp_path, capacity, scene, kw, size):
+    """Batched, so that the path kernel of mesh scenes follows the paths: they
+    are resumed after every vertex, with their weights, hits and pending forks.
+    The queue of the small context holds fewer shadow records than its warps
+    reserve, so that shadow rays are also walked in place."""
+    from pcr_b200 import capi
+    ctx = capi.Context(device=0, queue_capacity=capacity)
+    a, b = ctx.load_scene_json(scene_path(scene), GOLDEN), ctx.load_scene_json(*_boxed(tmp_path, scene))
+    d = capi.render_desc(*size, seed=11, **kw)
+    whole, counts, _ = _counts(ctx, a, d)
+    waited, waited_counts, st = _counts(ctx, b, d, batch=True)
+    assert waited_counts == counts
+    assert st["stage_launches"]["extend"] > 0 and st["stage_launches"]["other"] == 0
+    assert np.allclose(waited[0], whole[0], rtol=1e-6, atol=1e-7)
+    ctx.close()
+
+
+def test_a_large_plain_render_waits_too(tmp_path):
+    """A plain render of more paths than are staged, in several fills of the
+    queue."""
+    from pcr_b200 import capi
+    ctx = capi.Context(device=0, queue_capacity=1 << 14)
+    a, b = ctx.load_scene_json(scene_path("cornell-glass"), GOLDEN), ctx.load_scene_json(*_boxed(tmp_path, "cornell-glass"))
+    d = capi.render_desc(160, 120, depth=6, samples=7, shadow=3, seed=12)
+    whole, counts, _ = _counts(ctx, a, d)
+    waited, waited_counts, _ = _counts(ctx, b, d)
+    assert waited_counts == counts and counts[0] > 1 << 16
+    assert np.allclose(waited[0], whole[0], rtol=1e-6, atol=1e-7)
+    ctx.close()
+
+
+def test_many_shadow_samples_grow_the_queue_of_a_mesh_scene(tmp_path):
+    """More than 8 shadow samples per hit on a scene whose shadow rays become
+    records: the queue grows, plain, batched and between the two."""
+    from pcr_b200 import capi
+    ctx = capi.Context(device=0, queue_capacity=1 << 12)
+    a, b = ctx.load_scene_json(scene_path("cornell"), GOLDEN), ctx.load_scene_json(*_boxed(tmp_path, "cornell"))
+    before = ctx.stats()["device_bytes"]
+    for shadow, w in ((40, 48), (64, 300), (3, 48)):
+        d = capi.render_desc(w, 48, depth=3, samples=8, shadow=shadow, seed=91)
+        want = ctx.render(a, d)[0]
+        rid = ctx.submit(b, d)
+        ctx.run_until_idle()
+        assert np.allclose(ctx.fetch(rid)[0], want, rtol=1e-6, atol=1e-7)
+        assert np.allclose(ctx.render(b, d)[0], want, rtol=1e-6, atol=1e-7)
+    assert ctx.stats()["device_bytes"] >= before
+    with pytest.raises(capi.PcrError):
+        ctx.render(b, capi.render_desc(16, samples=1, shadow=65))
+    ctx.close()
