@@ -743,6 +743,22 @@ static int local_spp(const pcr_render_desc& d)
     return d.sample_end > 0 ? d.sample_end - d.sample_begin : d.samples;
 }
 
+// A render's paths (an adaptive one's at most).
+static int64_t path_count(const pcr_render_desc& d)
+{
+    return (int64_t)d.width * d.height * local_spp(d) * std::max(1, d.aa_samples);
+}
+
+// A plain render of at most this many paths on a mesh scene is staged, and so
+// are requests admitted while no more than these are there in all: few warps
+// take long over vertices whose shadow rays follow one another in a lane, as
+// records they run side by side.  Bunny, 4 vertices, 8 shadow rays, stages of
+// one vertex alone / paths followed to the mesh / staged: 16x16 490 / 603 / 410 us,
+// 64x64 600 / 790 / 515 us, 65,536 paths 2.2 / 1.0 / 0.82 ms, 196,566 paths - /
+// 1.33 / 1.30 ms, 262,144 paths - / 1.45 / 1.56 ms; one served request of 8192
+// paths, 8 vertices: 1.46 / 2.07 / 1.42 ms.
+constexpr int64_t kStagedPaths = 1 << 16;
+
 int64_t Engine::request_bytes(const pcr_render_desc& d) const
 {
     const int64_t px = (int64_t)d.width * d.height;
@@ -858,6 +874,12 @@ void Engine::activate(Request& r, int slot)
 
 void Engine::admit_locked()
 {
+    // few paths in all on scenes whose paths can wait: staged (kStagedPaths)
+    int64_t waiting = 0;
+    if (!pending_.empty())
+        for (auto& kv : reqs_)
+            if ((kv.second->state == ReqState::Pending || kv.second->state == ReqState::Active) && !flat(kv.second->scene))
+                waiting += path_count(kv.second->desc);
     // first fit under the slot limit and the memory budget, in submit order
     for (auto it = pending_.begin(); it != pending_.end();) {
         Request& r = *reqs_[*it];
@@ -868,6 +890,7 @@ void Engine::admit_locked()
         for (int s = 0; s < kMaxActive; s++)
             if (slot_owner_[s] < 0) { slot = s; break; }
         if (slot < 0) break;
+        r.staged = !flat(r.scene) && waiting <= kStagedPaths;
         activate(r, slot);
         it = pending_.erase(it);
     }
@@ -896,7 +919,7 @@ int Engine::active_stages() const
     int m = 0;
     for (int slot : active_slots_) {
         auto it = reqs_.find(slot_owner_[slot]);
-        if (it != reqs_.end()) m |= flat(it->second->scene) ? kStagesFlat : queue_stages(it->second->scene);
+        if (it != reqs_.end()) m |= flat(it->second->scene) ? kStagesFlat : queue_stages(*it->second);
     }
     return m ? m : kStagesMesh;
 }
@@ -1541,14 +1564,6 @@ void Engine::render_flat(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats*
     }
 }
 
-// A plain render of at most this many paths on a mesh scene is staged: few warps
-// take long over vertices whose shadow rays follow one another in a lane, as
-// records they run side by side.  Bunny, 4 vertices, 8 shadow rays, stages of
-// before / paths followed to the mesh / staged: 16x16 490 / 603 / 410 us, 64x64
-// 600 / 790 / 515 us, 65,536 paths 2.2 / 1.0 / 0.82 ms, 196,566 paths - / 1.33 /
-// 1.30 ms, 262,144 paths - / 1.45 / 1.56 ms.
-constexpr int64_t kStagedPaths = 1 << 16;
-
 void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, uint8_t* rgb, pcr_render_stats* st)
 {
     if (adaptive_rounds(desc)) {
@@ -1583,16 +1598,15 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     }
     ensure_shadow_capacity(desc.shadow_samples);
     if (graph_dirty_) launch_shapes();
-    const int64_t px = (int64_t)desc.width * desc.height;
     EngineParams p{tune_.queue_capacity, tune_.queue_capacity, 1, 0};
     k_set_params<<<1, 1, 0, stream_>>>((EngineParams*)d_params_, p);
-    r.staged = px * local_spp(desc) * std::max(1, desc.aa_samples) <= kStagedPaths;
+    r.staged = path_count(desc) <= kStagedPaths;
     activate(r, 0);
     slot_owner_[0] = -1;  // the plain request is not in the request map
     upload_active();
-    const int64_t total = px * local_spp(desc) * std::max(1, desc.aa_samples);
+    const int64_t total = path_count(desc);
     const int64_t fills = (total + tune_.queue_capacity - 1) / tune_.queue_capacity;
-    const int stages = r.staged ? kStagesStaged : queue_stages(scene);
+    const int stages = queue_stages(r);
     int cur = 0;
     // a path waits at most `depth` times
     for (int64_t it = 0; it < fills + desc.depth; it++) {
@@ -1840,7 +1854,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
             CK(cudaGetLastError());
             cur ^= 1;
         };
-        const int64_t total = px * local_spp(desc) * std::max(1, desc.aa_samples);
+        const int64_t total = path_count(desc);
         const int64_t fills = (total + fill - 1) / fill;
         for (int64_t it = 0; it < fills + desc.depth; it++) iteration();
         for (int64_t extra = 0;;) {

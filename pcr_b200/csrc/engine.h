@@ -127,7 +127,7 @@ private:
     // kind of scene, the walks for those whose paths can wait, in the form
     // that traces in full where a staged scene is among them.
     static constexpr int kStagesMesh = 1, kStagesFlat = 2, kStagesStaged = 4;
-    int queue_stages(int scene) const { return scenes_[scene].dev.staged ? kStagesStaged : kStagesMesh; }
+    int queue_stages(const Request& r) const { return r.staged || scenes_[r.scene].dev.staged ? kStagesStaged : kStagesMesh; }
     struct Grids {
         int paths[3], extend[2], shadow[2];
     };

@@ -38,15 +38,25 @@ def _boxed(tmp_path, scene):
 
 
 def _counts(ctx, sid, desc, batch=False):
+    """A render's images, its path and ray counts, and the stats.  batch: in
+    one with a request of more paths than are staged (on the scene alone, so
+    that the path kernel of mesh scenes follows both); its counts are left
+    out."""
+    from pcr_b200 import capi
+    if batch:
+        big = capi.render_desc(300, 250, depth=1, samples=1, shadow=1, seed=77, spectral=False)
+        alone = _counts(ctx, sid, big)[1]
     ctx.reset_stats()
     if batch:
-        rid = ctx.submit(sid, desc)
+        rid, other = ctx.submit(sid, desc), ctx.submit(sid, big)
         ctx.run_until_idle()
         images = ctx.fetch(rid)[:2]
+        ctx.fetch(other)
     else:
         images = ctx.render(sid, desc)[:2]
     st = ctx.stats()
-    return images, (st["paths"], st["rays"], st["shadow_rays"]), st
+    counts = (st["paths"], st["rays"], st["shadow_rays"])
+    return images, tuple(x - y for x, y in zip(counts, alone)) if batch else counts, st
 
 
 @pytest.mark.parametrize("capacity", [1 << 10, 1 << 17])
@@ -62,7 +72,7 @@ def test_ray_counts_do_not_depend_on_the_queue(tmp_path, capacity, scene, kw):
     b = ctx.load_scene_json(*_boxed(tmp_path, scene))
     d = capi.render_desc(70, 41, seed=23, **kw)
     counts = _counts(ctx, a, d)[1]
-    # (a plain render of few paths is staged, a batched one is not)
+    # (few paths are staged; in the batch they are not)
     assert _counts(ctx, b, d)[1] == counts
     assert _counts(ctx, b, d, batch=True)[1] == counts
     ctx.close()
@@ -206,4 +216,30 @@ def test_many_shadow_samples_grow_the_queue_of_a_mesh_scene(tmp_path):
     assert ctx.stats()["device_bytes"] >= before
     with pytest.raises(capi.PcrError):
         ctx.render(b, capi.render_desc(16, samples=1, shadow=65))
+    ctx.close()
+
+
+def test_few_paths_are_staged_in_a_batch_too(tmp_path):
+    """One small request on a mesh scene: the staged form, as in a plain
+    render, and the same image beside requests that are not."""
+    from pcr_b200 import capi
+    ctx = capi.Context(device=0, queue_capacity=1 << 14)
+    a, b = ctx.load_scene_json(scene_path("cornell-glass"), GOLDEN), ctx.load_scene_json(*_boxed(tmp_path, "cornell-glass"))
+    d = capi.render_desc(61, 47, depth=7, samples=3, shadow=5, seed=31)
+    want = ctx.render(a, d)[0]
+    for n in (1, 3):
+        ids = [ctx.submit(b, d) for _ in range(n)]
+        ctx.run_until_idle()
+        for i in ids:
+            assert np.allclose(ctx.fetch(i)[0], want, rtol=1e-6, atol=1e-7)
+    # staged ones first, others join them while they run
+    ctx.serve_start()
+    ids = [ctx.submit(b, d)]
+    ids += [ctx.submit(b, capi.render_desc(300, 200, depth=4, samples=4, shadow=3, seed=k)) for k in range(3)]
+    ids += [ctx.submit(a, d), ctx.submit(b, d)]
+    for i in ids:
+        ctx.wait(i, 30000)
+    for i in (ids[0], ids[4], ids[5]):
+        assert np.allclose(ctx.fetch(i)[0], want, rtol=1e-6, atol=1e-7)
+    ctx.serve_stop()
     ctx.close()
