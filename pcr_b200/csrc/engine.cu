@@ -749,15 +749,32 @@ static int64_t path_count(const pcr_render_desc& d)
     return (int64_t)d.width * d.height * local_spp(d) * std::max(1, d.aa_samples);
 }
 
-// A plain render of at most this many paths on a mesh scene is staged, and so
-// are requests admitted while no more than these are there in all: few warps
-// take long over vertices whose shadow rays follow one another in a lane, as
-// records they run side by side.  Bunny, 4 vertices, 8 shadow rays, stages of
-// one vertex alone / paths followed to the mesh / staged: 16x16 490 / 603 / 410 us,
-// 64x64 600 / 790 / 515 us, 65,536 paths 2.2 / 1.0 / 0.82 ms, 196,566 paths - /
-// 1.33 / 1.30 ms, 262,144 paths - / 1.45 / 1.56 ms; one served request of 8192
-// paths, 8 vertices: 1.46 / 2.07 / 1.42 ms.
-constexpr int64_t kStagedPaths = 1 << 16;
+// How a request is traced, by its scene and by `paths`, all that are there on
+// scenes like its own: followed to the end (kStagesFlat) or to the mesh
+// (kStagesMesh) in k_paths, or staged.
+//
+// Meshes: few warps take long over vertices whose shadow rays follow one
+// another in a lane; as records they run side by side.  Bunny, 4 vertices, 8
+// shadow rays, stages of one vertex alone / paths followed to the mesh / staged:
+// 16x16 490 / 603 / 410 us, 64x64 600 / 790 / 515 us, 65,536 paths 2.2 / 1.0 /
+// 0.82 ms, 196,566 paths - / 1.33 / 1.30 ms, 262,144 paths - / 1.45 / 1.56 ms; one
+// served request of 8192 paths, 8 vertices: 1.46 / 2.07 / 1.42 ms.
+//
+// Exact tests without a mesh: the whole path in one launch saves the stages'
+// launches and waits, but tests S x primitives in a lane one after another.
+// Whole / staged: Cornell box with a tilted quad (19 primitives), 4096 paths of
+// 3 vertices and 1 shadow ray 115 / 268 us, 2 M paths 1.43 / 1.85 ms; 4 vertices
+// and 4 shadow rays 184 / 312 us, 262,144 paths 625 / 677 us, 2 M 3.6 / 3.5 ms;
+// 16 shadow rays 438 / 334 us; 88 quads and 1 shadow ray 238 / 444 us, 262,144
+// paths 724 / 733 us, 4 shadow rays 563 / 589 us and 2.0 / 1.5 ms.
+int Engine::route(int scene, const pcr_render_desc& d, int64_t paths) const
+{
+    const DScene& S = scenes_[scene].dev;
+    if (S.n_nodes > 0) return S.staged || paths <= (1 << 16) ? kStagesStaged : kStagesMesh;
+    const int64_t tests = (int64_t)(S.n_planes + S.n_spheres) * d.shadow_samples;
+    const bool whole = !S.staged || tests <= 24 || (tests <= 96 && paths <= 1 << 18);
+    return whole ? kStagesFlat : kStagesStaged;
+}
 
 int64_t Engine::request_bytes(const pcr_render_desc& d) const
 {
@@ -799,7 +816,7 @@ void Engine::ensure_shadow_capacity(int shadow_samples)
 int64_t Engine::submit(int scene, const pcr_render_desc& desc)
 {
     validate(scene, desc);
-    if (!flat(scene) && (int64_t)queue_cap_ * desc.shadow_samples > shadow_cap_) {
+    if (!never_waits(scene) && (int64_t)queue_cap_ * desc.shadow_samples > shadow_cap_) {
         std::lock_guard<std::mutex> g(run_mu_);
         ensure_shadow_capacity(desc.shadow_samples);
     }
@@ -844,7 +861,7 @@ void Engine::activate(Request& r, int slot)
     const pcr_render_desc& d = r.desc;
     const int64_t px = (int64_t)d.width * d.height;
     alloc_request(r);
-    DRequest R = make_request(d, r.scene, r.accum, r.staged);
+    DRequest R = make_request(d, r.scene, r.accum, r.route);
     if (adaptive_rounds(d)) {
         R.flags |= kReqAdaptive;
         CK(cudaMallocFromPoolAsync(&r.act[0], px * sizeof(int), pool_, stream_));
@@ -874,12 +891,12 @@ void Engine::activate(Request& r, int slot)
 
 void Engine::admit_locked()
 {
-    // few paths in all on scenes whose paths can wait: staged (kStagedPaths)
-    int64_t waiting = 0;
+    // paths on scenes without / with a mesh, for their routes
+    int64_t paths[2] = {0, 0};
     if (!pending_.empty())
         for (auto& kv : reqs_)
-            if ((kv.second->state == ReqState::Pending || kv.second->state == ReqState::Active) && !flat(kv.second->scene))
-                waiting += path_count(kv.second->desc);
+            if (kv.second->state == ReqState::Pending || kv.second->state == ReqState::Active)
+                paths[scenes_[kv.second->scene].dev.n_nodes > 0] += path_count(kv.second->desc);
     // first fit under the slot limit and the memory budget, in submit order
     for (auto it = pending_.begin(); it != pending_.end();) {
         Request& r = *reqs_[*it];
@@ -890,7 +907,7 @@ void Engine::admit_locked()
         for (int s = 0; s < kMaxActive; s++)
             if (slot_owner_[s] < 0) { slot = s; break; }
         if (slot < 0) break;
-        r.staged = !flat(r.scene) && waiting <= kStagedPaths;
+        r.route = route(r.scene, r.desc, paths[scenes_[r.scene].dev.n_nodes > 0]);
         activate(r, slot);
         it = pending_.erase(it);
     }
@@ -919,7 +936,7 @@ int Engine::active_stages() const
     int m = 0;
     for (int slot : active_slots_) {
         auto it = reqs_.find(slot_owner_[slot]);
-        if (it != reqs_.end()) m |= flat(it->second->scene) ? kStagesFlat : queue_stages(*it->second);
+        if (it != reqs_.end()) m |= it->second->route;
     }
     return m ? m : kStagesMesh;
 }
@@ -946,7 +963,7 @@ void Engine::launch_iteration(int cur, int stages, bool prof, bool rounds, cudaS
             mark(stage);
         }
     if (stages & kStagesFlat) {
-        k_paths<kFlatScenes><<<grids_.paths[kFlatScenes], kPathBlock, kPathSmem, st>>>(E, cur, xyz_scale_);
+        k_paths<kFlatPaths><<<grids_.paths[kFlatPaths], kPathBlock, kPathSmem, st>>>(E, cur, xyz_scale_);
         mark(7);
     }
     k_status<<<1, 1024, 0, st>>>(E, cur ^ 1);
@@ -971,9 +988,9 @@ Engine::Grids Engine::launch_grids()
 {
     Grids g;
     const int B = trace_block();
-    grid_for((const void*)k_paths<kFlatScenes>, kPathBlock, kPathSmem, &g.paths[kFlatScenes]);
-    grid_for((const void*)k_paths<kMeshScenes>, kPathBlock, kPathSmem, &g.paths[kMeshScenes]);
-    grid_for((const void*)k_paths<kStagedScenes>, kPathBlock, kPathSmem, &g.paths[kStagedScenes]);
+    grid_for((const void*)k_paths<kFlatPaths>, kPathBlock, kPathSmem, &g.paths[kFlatPaths]);
+    grid_for((const void*)k_paths<kMeshPaths>, kPathBlock, kPathSmem, &g.paths[kMeshPaths]);
+    grid_for((const void*)k_paths<kStagedPaths>, kPathBlock, kPathSmem, &g.paths[kStagedPaths]);
     grid_for((const void*)k_extend<false>, B, 0, &g.extend[0]);
     grid_for((const void*)k_extend<true>, B, 0, &g.extend[1]);
     grid_for((const void*)k_shadow<false>, B, 0, &g.shadow[0]);
@@ -987,9 +1004,9 @@ void Engine::launch_queue_stage(const EngineView& E, const Grids& g, int cur, in
     const int B = trace_block(), staged = stages & kStagesStaged ? 1 : 0;
     if (stage == 2) {
         // staged first: its shadow records always find room
-        if (staged) k_paths<kStagedScenes><<<g.paths[kStagedScenes], kPathBlock, kPathSmem, st>>>(E, cur, xyz_scale_);
+        if (staged) k_paths<kStagedPaths><<<g.paths[kStagedPaths], kPathBlock, kPathSmem, st>>>(E, cur, xyz_scale_);
         if (stages & kStagesMesh)
-            k_paths<kMeshScenes><<<g.paths[kMeshScenes], kPathBlock, kPathSmem, st>>>(E, cur, xyz_scale_);
+            k_paths<kMeshPaths><<<g.paths[kMeshPaths], kPathBlock, kPathSmem, st>>>(E, cur, xyz_scale_);
     } else if (stage == 1) {
         if (staged) k_extend<true><<<g.extend[1], B, 0, st>>>(E, cur ^ 1);
         else k_extend<false><<<g.extend[0], B, 0, st>>>(E, cur ^ 1);
@@ -1534,7 +1551,7 @@ void Engine::trace_flat(const EngineView& E, const DRequest& R, int grid)
         const int n = (int)std::min<int64_t>(per, R.total - at);
         k_one_request<<<1, 1, 0, stream_>>>(E, R, at, n);
         if (profile_) CK(cudaEventRecord(prof_ev_[0], stream_));
-        k_paths<kFlatScenes><<<std::min(grid, (n + kPathBlock - 1) / kPathBlock), kPathBlock, kPathSmem, stream_>>>(E, 0, xyz_scale_);
+        k_paths<kFlatPaths><<<std::min(grid, (n + kPathBlock - 1) / kPathBlock), kPathBlock, kPathSmem, stream_>>>(E, 0, xyz_scale_);
         CK(cudaGetLastError());
         if (profile_) record_other(prof_ev_[0], prof_ev_[1]);
         else stage_launches_[7]++;
@@ -1546,8 +1563,8 @@ void Engine::trace_flat(const EngineView& E, const DRequest& R, int grid)
 void Engine::render_flat(Request& r, float* hdr, uint8_t* rgb, pcr_render_stats* st)
 {
     alloc_request(r);
-    const DRequest R = make_request(r.desc, r.scene, r.accum);
-    trace_flat(view(), R, grids_.paths[kFlatScenes]);
+    const DRequest R = make_request(r.desc, r.scene, r.accum, r.route);
+    trace_flat(view(), R, grids_.paths[kFlatPaths]);
     active_dirty_ = true;  // the active list holds slot 0
     CK(cudaMemcpyAsync(&h_plain_->cnt, d_cnt_, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
     finish_request(r, stream_);
@@ -1591,7 +1608,8 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     r.bytes = request_bytes(desc);
     if (r.bytes > budget_) throw PcrError(PCR_ERR_NO_MEMORY, "request larger than the device memory budget");
     if (graph_dirty_) launch_shapes();
-    if (flat(scene)) {
+    r.route = route(scene, desc, path_count(desc));
+    if (r.route == kStagesFlat) {
         render_flat(r, hdr, rgb, st);
         if (st) st->latency_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         return;
@@ -1600,17 +1618,15 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
     if (graph_dirty_) launch_shapes();
     EngineParams p{tune_.queue_capacity, tune_.queue_capacity, 1, 0};
     k_set_params<<<1, 1, 0, stream_>>>((EngineParams*)d_params_, p);
-    r.staged = path_count(desc) <= kStagedPaths;
     activate(r, 0);
     slot_owner_[0] = -1;  // the plain request is not in the request map
     upload_active();
     const int64_t total = path_count(desc);
     const int64_t fills = (total + tune_.queue_capacity - 1) / tune_.queue_capacity;
-    const int stages = queue_stages(r);
     int cur = 0;
     // a path waits at most `depth` times
     for (int64_t it = 0; it < fills + desc.depth; it++) {
-        launch_iteration(cur, stages, profile_, false, stream_);
+        launch_iteration(cur, r.route, profile_, false, stream_);
         cur ^= 1;
     }
     int64_t extra = 0;
@@ -1624,7 +1640,7 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
         if (end.cnt.status) throw PcrError(PCR_ERR_DEVICE_STATUS, "device reported queue overflow");
         if (end.done[0]) break;
         if (++extra > fills * (4 * (int64_t)desc.depth + 8)) throw PcrError(PCR_ERR_TIMEOUT, "plain render did not finish");
-        launch_iteration(cur, stages, profile_, false, stream_);
+        launch_iteration(cur, r.route, profile_, false, stream_);
         cur ^= 1;
     }
     // the next user starts with queue 0: both are empty
@@ -1655,7 +1671,7 @@ void Engine::render_plain(int scene, const pcr_render_desc& desc, float* hdr, ui
 // callers that may not allocate device memory during a render.  Inputs are
 // a scene already uploaded to the context; outputs are caller-owned device
 // buffers.  Every GPU that loads the library holds the array until exit.
-// Mesh scenes: paths in flight (staged, see kStagedPaths).  Four times as many
+// Mesh scenes: paths in flight (staged: they are few, see Engine::route).  Four times as many
 // where no path can fork; the more, the fewer iterations of launches and of
 // waits for the longest walk.  Bunny 256x256, 8 vertices, 4 paths a pixel, 4
 // shadow rays, 8192 in flight and paths followed to the mesh / staged 40960:
@@ -1701,7 +1717,7 @@ static void* noalloc_scratch(int device)
 }
 
 // The request entry of a render (Engine::activate adds the adaptive fields).
-DRequest Engine::make_request(const pcr_render_desc& d, int scene, double* accum, bool staged) const
+DRequest Engine::make_request(const pcr_render_desc& d, int scene, double* accum, int route) const
 {
     const SceneEntry& S = scenes_[scene];
     DRequest R{};
@@ -1717,7 +1733,7 @@ DRequest Engine::make_request(const pcr_render_desc& d, int scene, double* accum
     R.shadow = d.shadow_samples;
     R.flags = (d.spectral ? kReqSpectral : 0) | (d.mis ? kReqMIS : 0) | (d.russian ? kReqRussian : 0) |
               (d.stratified ? kReqStratified : 0) | (d.spectral_terminate ? kReqTerminate : 0) |
-              (flat(scene) ? kReqFlat : 0) | (S.dev.staged || staged ? kReqStaged : 0);
+              (route == kStagesFlat ? kReqFlat : 0) | (route == kStagesStaged ? kReqStaged : 0);
     R.hero = std::min(4, std::max(1, d.hero_samples <= 0 ? 4 : d.hero_samples));
     R.strata = d.stratified ? std::max(1, (int)std::lround(std::sqrt((float)d.samples))) : 0;
     R.cam_x = S.cam[0];
@@ -1829,9 +1845,10 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     E.cmf_table = d_cmf_;
     E.queue_cap = kNoAllocQueue;
 
-    const DRequest R = make_request(desc, scene, accum, true);
-    if (scenes_[scene].dev.n_nodes == 0) {
-        trace_flat(E, R, graph_dirty_ ? launch_grids().paths[kFlatScenes] : grids_.paths[kFlatScenes]);
+    const bool mesh = scenes_[scene].dev.n_nodes > 0;
+    const DRequest R = make_request(desc, scene, accum, mesh ? kStagesStaged : kStagesFlat);
+    if (!mesh) {
+        trace_flat(E, R, graph_dirty_ ? launch_grids().paths[kFlatPaths] : grids_.paths[kFlatPaths]);
         CK(cudaMemcpyAsync(&h_plain_->cnt, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
     } else {
         k_admit<<<1, 1, 0, stream_>>>(E, R, 0);
@@ -1883,7 +1900,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
         CK(cudaGetLastError());
     }
     CK(cudaStreamSynchronize(stream_));
-    if (scenes_[scene].dev.n_nodes == 0 && h_plain_->cnt.status)
+    if (!mesh && h_plain_->cnt.status)
         throw PcrError(PCR_ERR_DEVICE_STATUS, "pcr_render_noalloc: device reported queue overflow");
 }
 

@@ -58,7 +58,7 @@ struct Request {
     uint64_t admit_block = 0;  // blocks launched before this request's slot was (re)set
     bool cancel_running = false;        // cancel asked while Active
     bool cancel_sent = false;           // k_cancel launched for it
-    bool staged = false;                // traced as on a staged scene
+    int route = 0;                      // Engine::kStages* bit: how it is traced
     int* act[2] = {nullptr, nullptr};   // adaptive: pixel lists of alternate rounds
     float4* welford = nullptr;          // adaptive: per-pixel mean / M2
 };
@@ -123,11 +123,11 @@ private:
     void alloc_request(Request& r);
     void activate(Request& r, int slot);
     void upload_active();
-    // Which kernels an iteration runs (bits of the active requests): k_paths by
-    // kind of scene, the walks for those whose paths can wait, in the form
-    // that traces in full where a staged scene is among them.
+    // Which kernels an iteration runs (the active requests' routes): k_paths by
+    // route, the walks for those whose paths can wait, in the form that traces
+    // in full where a staged request is among them.
     static constexpr int kStagesMesh = 1, kStagesFlat = 2, kStagesStaged = 4;
-    int queue_stages(const Request& r) const { return r.staged || scenes_[r.scene].dev.staged ? kStagesStaged : kStagesMesh; }
+    int route(int scene, const pcr_render_desc& d, int64_t paths) const;
     struct Grids {
         int paths[3], extend[2], shadow[2];
     };
@@ -145,9 +145,9 @@ private:
     void finish_request(Request& r, cudaStream_t rs);
     void release_cancelled(Request& r);
     void copy_out(Request& r, float* hdr, uint8_t* rgb);
-    DRequest make_request(const pcr_render_desc& d, int scene, double* accum, bool staged = false) const;
-    // Whether the scene's paths never wait.
-    bool flat(int scene) const { return scenes_[scene].dev.n_nodes == 0 && !scenes_[scene].dev.staged; }
+    DRequest make_request(const pcr_render_desc& d, int scene, double* accum, int route) const;
+    // Whether no request's paths on the scene ever wait.
+    bool never_waits(int scene) const { return scenes_[scene].dev.n_nodes == 0 && !scenes_[scene].dev.staged; }
     void check_status();
     bool engine_step();
     void serve_loop();

@@ -4,8 +4,8 @@
 // new camera paths, and follows each until it ends or its next ray has a
 // triangle mesh to walk: then the path waits in the other queue, where
 // k_extend walks it, as k_shadow does the shadow rays that meet the mesh.
-// Paths on scenes without a mesh never wait, those on staged scenes
-// (DScene::staged) after every vertex.  Every kernel loops over a device-side
+// Paths on scenes without a mesh never wait, those of staged requests
+// (Engine::route) after every vertex.  Every kernel loops over a device-side
 // count, so a whole iteration (and several in a row) can be captured in one
 // CUDA graph with no host round trip.  No kernel waits on another block or on
 // the host: there is no spin anywhere.

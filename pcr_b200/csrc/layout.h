@@ -115,7 +115,8 @@ struct DScene {
     int n_planes, n_spheres, n_nodes, n_tris, n_lights, mat_base, n_mats, n_pgroups;
     int n_sgroups;
     int emissive_tris;        // 1 when any triangle's material is emissive
-    // 1: its requests are kReqStaged (paths.cuh)
+    // 1: the estimates do not decide its rays (a quad that is neither, too many
+    // primitives), or shadow rays have to find the closest emissive triangle
     int staged;
     // The scene's only emissive material (scene-local index) when it has
     // exactly one and every light uses it, else -1.  Spectral paths of such
@@ -143,8 +144,8 @@ struct DScene {
 // Request flags
 constexpr int kReqSpectral = 1, kReqMIS = 2, kReqRussian = 4, kReqStratified = 8, kReqAdaptive = 16,
               kReqTerminate = 32, kReqCancelled = 64,
-              kReqFlat = 128,       // on a scene whose paths never wait in the queues (no mesh, not staged)
-              kReqStaged = 256;     // on a staged scene, or few paths on a mesh scene: k_extend and k_shadow trace its rays in full
+              kReqFlat = 128,       // its paths never wait in the queues (Engine::route)
+              kReqStaged = 256;     // k_extend and k_shadow trace its rays in full
 
 struct DRequest {
     int scene, width, height, depth;
@@ -168,8 +169,8 @@ struct DRequest {
     int sample0, local_spp;
 };
 
-// Paths whose next ray has a mesh to walk, or all of it to be traced (staged
-// scenes), structure of arrays, one entry per path.
+// Paths whose next ray has a mesh to walk, or is to be traced in full (staged
+// requests), structure of arrays, one entry per path.
 struct PathQueue {
     float4* o;     // origin, hero lambda
     float4* d;     // direction, meta (bits): bounce | fork<<8 | single<<11 | n<<12
@@ -182,17 +183,17 @@ struct PathQueue {
     // multiplied by that material's emission at the wavelength.
     float4* w[3];
     // The ray's analytic hit (t, primitive), which k_extend replaces by a
-    // triangle's (t, primitive, u, v) where the mesh is hit first; on staged
-    // scenes k_extend writes either.
+    // triangle's (t, primitive, u, v) where the mesh is hit first; for staged
+    // requests k_extend writes either.
     float4* hit;
 };
 
-// Shadow rays that have a mesh to walk, or all of it to be traced.
+// Shadow rays that have a mesh to walk, or are to be traced in full.
 struct ShadowQueue {
     float4* o;     // origin, lightDist2 (below zero: an unused record)
     float4* d;     // direction, pixel (bits)
     float4* c;     // contribution (XYZ or RGB), request slot | scene << 16 (bits)
-    float* bound;  // no hit at or past it matters (not set on staged scenes)
+    float* bound;  // no hit at or past it matters (not set for staged requests)
 };
 
 struct Counters {

@@ -44,11 +44,12 @@ namespace pcr {
 // a pixel 4.97 -> 2.01 ms, 24 uneven renders 80.8 -> 75.6 ms; six renders half
 // of them through a glass mesh, where most vertices wait, 22.4 -> 26.0 ms.
 //
-// Staged scenes are those whose rays this kernel would trace by the exact
-// tests (the estimates do not take the scene's quads), or whose shadow rays
-// have to find the closest of the mesh's emissive triangles.  Such traces are
-// long and leave lanes idle, which costs more at 16 warps per SM and inside
-// this code than the stages' memory traffic.  So a path is followed for one
+// Staged requests are those on scenes whose rays this kernel would trace by the
+// exact tests (the estimates do not take the scene's quads), or whose shadow
+// rays have to find the closest of the mesh's emissive triangles (and requests
+// of few paths on mesh scenes, see Engine::route).  Such traces are long and
+// leave lanes idle, which costs more at 16 warps per SM and inside this code
+// than the stages' memory traffic.  So a path is followed for one
 // vertex and waits: k_extend traces its next ray in full, and each of its
 // shadow samples is a record for k_shadow.  Six batched renders with 4 (16)
 // shadow rays, by stages of one vertex alone / traced here / staged: a Cornell
@@ -159,7 +160,7 @@ __device__ __forceinline__ void close_shadow_chunk(const EngineView& E, const Pa
     for (int k = P.shadow_next + lane; k < P.shadow_end; k += 32) E.sq.o[k] = make_float4(0.f, 0.f, 0.f, -1.f);
 }
 
-// Shadow records of a vertex on a staged scene: one per sample, those that add
+// Shadow records of a staged request's vertex: one per sample, those that add
 // nothing marked as unused.  The lanes that come here together reserve them
 // with one grid-wide atomic; where they do not fit (the fixed queue of
 // pcr_render_noalloc), the vertices wait for the next iteration.  Without a
@@ -191,25 +192,26 @@ __device__ __forceinline__ StagedRecords staged_records(const EngineView& E, int
     return r;
 }
 
-// The scenes whose paths a launch of k_paths follows.
-constexpr int kFlatScenes = 0, kMeshScenes = 1, kStagedScenes = 2;
+// Whose paths a launch of k_paths follows (Engine::route): to their end, to the
+// mesh, or staged.
+constexpr int kFlatPaths = 0, kMeshPaths = 1, kStagedPaths = 2;
 
 // Work of one launch: the paths of queue `cur` (kMesh), then the camera paths
 // numbered over the active list: position r's start at base[r] and are the
 // request's paths give_start[r], give_start[r] + 1, ...
-template <int kScenes>
-__global__ void __launch_bounds__(kPathBlock, kScenes == kStagedScenes ? PCR_STAGED_MIN_BLOCKS : PCR_PATH_MIN_BLOCKS)
+template <int kPaths>
+__global__ void __launch_bounds__(kPathBlock, kPaths == kStagedPaths ? PCR_STAGED_MIN_BLOCKS : PCR_PATH_MIN_BLOCKS)
 k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
 {
     extern __shared__ __align__(16) unsigned char s_paths[];
     PathWarp& P = reinterpret_cast<PathWarp*>(s_paths)[threadIdx.x >> 5];
-    constexpr bool kMesh = kScenes != kFlatScenes, kStaged = kScenes == kStagedScenes;
+    constexpr bool kMesh = kPaths != kFlatPaths, kStaged = kPaths == kStagedPaths;
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     Counters* C = E.cnt;
     const int* base = kMesh ? E.give_base : E.path_base;
-    int* counter = &C->next[kScenes];
+    int* counter = &C->next[kPaths];
     // queued and camera paths of the other kind are left to its launch
     auto mine = [&](const DRequest& R) { return !kMesh || ((R.flags & kReqStaged) != 0) == kStaged; };
     const int queued = kMesh ? min(C->queue_n[cur], E.queue_cap) : 0;
@@ -391,7 +393,7 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
         // ---- trace (staged: above, so that the lanes of paths that wait are
         // filled before the next vertex)
         if (!kStaged) trace();
-        if (kScenes == kMeshScenes && P.shadow_end - P.shadow_next < kShadowLow) {  // shadow_next may lie past the end
+        if (kPaths == kMeshPaths && P.shadow_end - P.shadow_next < kShadowLow) {  // shadow_next may lie past the end
             close_shadow_chunk(E, P, lane);
             __syncwarp();
             if (lane == 0) {
@@ -594,7 +596,7 @@ k_paths(const __grid_constant__ EngineView E, int cur, float xyz_scale)
         }
         __syncwarp();
     }
-    if (kScenes == kMeshScenes) close_shadow_chunk(E, P, lane);
+    if (kPaths == kMeshPaths) close_shadow_chunk(E, P, lane);
     rays = __reduce_add_sync(kAll, rays);
     shadows = __reduce_add_sync(kAll, shadows);
     if (lane == 0 && (rays | shadows)) {  // a resumed path that ends at its vertex traced no ray

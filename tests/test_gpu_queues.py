@@ -92,14 +92,15 @@ def test_a_small_plain_render_launches_what_it_needs(tmp_path, depth):
     ctx.close()
 
 
-def _slanted(tmp_path, scene):
-    """The scene's file with a tiny slanted quad far behind the camera: the
-    estimates do not take it, so its rays are traced in full by the stages."""
+def _slanted(tmp_path, scene, n=100):
+    """The scene's file with tiny slanted quads far behind the camera: the
+    estimates do not take them, and with many its rays are traced in full by
+    the stages."""
     from pcr_b200 import workloads
     sc = workloads.read_scene_json(scene_path(scene))
-    sc["primitives"].append({"type": "plane", "origin": [0, 0, 900.0], "u": [1e-3, 1e-3, 0], "v": [0, 1e-3, 1e-3],
-                             "material": next(k for k, m in sc["materials"].items() if "emissive" not in m)})
-    path = tmp_path / f"{scene}-slanted.json"
+    sc["primitives"] += [{"type": "plane", "origin": [0, k, 900.0], "u": [1e-3, 1e-3, 0], "v": [0, 1e-3, 1e-3],
+                          "material": next(k for k, m in sc["materials"].items() if "emissive" not in m)} for k in range(n)]
+    path = tmp_path / f"{scene}-slanted{n}.json"
     path.write_text(json.dumps(sc))
     return str(path), GOLDEN
 
@@ -133,6 +134,24 @@ def test_staged_scenes_give_the_same_images(tmp_path, scene, kw, size):
         assert st["stage_launches"]["extend"] > 0 and st["stage_launches"]["shadow"] > 0, st["stage_launches"]
         assert st["stage_launches"]["other"] == 0, st["stage_launches"]
         ctx.close()
+
+
+def test_few_exact_tests_stay_in_one_launch(tmp_path):
+    """One slanted quad, few shadow rays, few paths: the whole path in one
+    launch, plain and batched; more shadow rays are staged.  Same images."""
+    from pcr_b200 import capi
+    ctx = capi.Context(device=0, queue_capacity=1 << 14)
+    a, b = ctx.load_scene_json(scene_path("cornell"), GOLDEN), ctx.load_scene_json(*_slanted(tmp_path, "cornell", 1))
+    for shadow, whole in ((1, True), (4, True), (16, False)):
+        d = capi.render_desc(61, 47, depth=5, samples=3, shadow=shadow, seed=41)
+        want, counts, _ = _counts(ctx, a, d)
+        got, got_counts, st = _counts(ctx, b, d)
+        assert got_counts == counts and np.allclose(got[0], want[0], rtol=1e-6, atol=1e-7)
+        assert (st["stage_launches"]["other"] > 0) == whole and (st["stage_launches"]["extend"] == 0) == whole
+        rid = ctx.submit(b, d)
+        ctx.run_until_idle()
+        assert np.allclose(ctx.fetch(rid)[0], want[0], rtol=1e-6, atol=1e-7)
+    ctx.close()
 
 
 def test_one_batch_of_all_kinds_of_scenes(tmp_path):
