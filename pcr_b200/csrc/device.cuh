@@ -413,8 +413,8 @@ __device__ __noinline__ uint32_t scene_analytic_exact(const DScene& S, float3 o,
 // What bounds it: instruction issue.  About 30 instructions a rectangle and 90
 // a box for all lanes of a warp; the exact tests' early rejects left half of
 // the lanes idle (16 to 18 of 32 active) through about 1500 (Cornell box, 18
-// quads).  0.1 % of the rays are in doubt.  24 uneven renders batched, three of
-// them on a mesh: 114.9 -> 108.8 ms.
+// quads).  0.1 % of the rays are in doubt (more where many start on spheres).
+// 24 uneven renders batched, three of them on a mesh: 114.9 -> 108.8 ms.
 struct FlatRay {
     float3 o, d, rd;
     bool sure;

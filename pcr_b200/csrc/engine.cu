@@ -1849,7 +1849,6 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     const DRequest R = make_request(desc, scene, accum, mesh ? kStagesStaged : kStagesFlat);
     if (!mesh) {
         trace_flat(E, R, graph_dirty_ ? launch_grids().paths[kFlatPaths] : grids_.paths[kFlatPaths]);
-        CK(cudaMemcpyAsync(&h_plain_->cnt, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
     } else {
         k_admit<<<1, 1, 0, stream_>>>(E, R, 0);
         ActiveList L;
@@ -1890,7 +1889,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     const double inv = 1.0 / ((double)desc.samples * std::max(1, desc.aa_samples));
     const int grid = (int)std::min<int64_t>((px + 255) / 256, (int64_t)sms_ * 8);
     k_resolve<<<std::max(1, grid), 256, 0, stream_>>>(accum, (int)px, inv, desc.spectral ? 1 : 0, desc.aces ? 1 : 0,
-                                                       hdr_dev, rgb_dev);
+                                                       hdr_dev, rgb_dev, &cnt->status, &h_plain_->cnt.status);
     CK(cudaGetLastError());
     if (desc.denoise && rgb_dev) {
         // two bilateral passes; the accumulator region (24 B a pixel) is free now
@@ -1900,7 +1899,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
         CK(cudaGetLastError());
     }
     CK(cudaStreamSynchronize(stream_));
-    if (!mesh && h_plain_->cnt.status)
+    if (h_plain_->cnt.status)
         throw PcrError(PCR_ERR_DEVICE_STATUS, "pcr_render_noalloc: device reported queue overflow");
 }
 

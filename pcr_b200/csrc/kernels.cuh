@@ -660,13 +660,6 @@ __device__ __forceinline__ float shadow_factor(const DScene& S, const DRequest& 
     return g.G * w;
 }
 
-// What every sample of a vertex is scaled by: light area / (pi S).
-__device__ __forceinline__ float light_scale(const DScene& S, const DRequest& R)
-{
-    const float inv_pi = 1.f / 3.14159274f;
-    return S.total_light_area * inv_pi / (float)R.shadow;
-}
-
 // Continuation of a diffuse vertex: Russian roulette and the cosine
 // hemisphere.  Returns whether the path goes on; nd its direction and
 // rr_scale its throughput factor.
@@ -829,8 +822,11 @@ __global__ void k_round(EngineView E)
 // Per-pixel mean -> linear sRGB (code/Renderer.cpp:300-302), then tone map
 // and 8-bit quantise (code/Renderer.cpp:365-382) on the device.
 __global__ void k_resolve(const double* __restrict__ acc, int npix, double inv_n, int spectral, int aces_tm,
-                          float* __restrict__ hdr, unsigned char* __restrict__ rgb8)
+                          float* __restrict__ hdr, unsigned char* __restrict__ rgb8, const int* status = nullptr,
+                          int* status_host = nullptr)
 {
+    // (a copy of this one word would cost the call 9 us)
+    if (status_host && blockIdx.x == 0 && threadIdx.x == 0) *status_host = *status;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
         float3 c = make_float3((float)(acc[i * 3] * inv_n), (float)(acc[i * 3 + 1] * inv_n), (float)(acc[i * 3 + 2] * inv_n));
         if (spectral) c = xyz_to_srgb(c);
