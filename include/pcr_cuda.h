@@ -125,7 +125,7 @@ typedef struct {
     int32_t device;          /* CUDA ordinal */
     int64_t memory_budget;   /* bytes the context may hold for requests (0: 40 GiB) */
     int32_t queue_capacity;  /* paths in flight (0: autotuned / default) */
-    int32_t block_size;      /* threads per block for the trace/shade kernels (0: default) */
+    int32_t block_size;      /* threads per block of the extend and shadow kernels (0: default) */
     int32_t chunk_paths;     /* per-request issue chunk per iteration (0: default) */
     int32_t regen_every;     /* refill cadence in iterations (0: 1) */
     int32_t use_graph;       /* capture the iteration loop in a CUDA graph (default 1) */
@@ -239,7 +239,10 @@ pcr_status pcr_progress(pcr_ctx *ctx, pcr_request_id id, double *fraction);
 
 /* ------------------------------------------------------------- engine info */
 typedef struct {
-    double stage_ms[8];      /* regen, extend, shade, shadow, resolve, schedule, status, other */
+    /* By stage: [0] none (camera rays are part of the path kernel), [1] extend, [2] shade: the
+     * path kernel for requests whose paths can wait, [3] shadow, [4] none, [5] schedule,
+     * [6] status and adaptive rounds, [7] other: the path kernel of whole paths, ray queries */
+    double stage_ms[8];
     int64_t stage_launches[8];
     int64_t iterations, paths, rays, shadow_rays;
     int64_t device_bytes;
