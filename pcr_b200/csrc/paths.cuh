@@ -7,10 +7,10 @@ namespace pcr {
 
 // k_paths follows each path in one thread, vertex after vertex, with its state
 // in registers: closest hit, shading, shadow rays, next direction.  On a scene
-// without a mesh it goes on to the path's end.  Where a ray
-// meets the mesh's box, the path waits in the queue for k_extend's walk and is
-// taken up again in the next iteration; a shadow ray that would be lit but
-// meets the box becomes a record for k_shadow.
+// without a mesh it goes on to the path's end.  Where a ray meets the mesh's
+// box, the path waits in the queue for k_extend's walk and is taken up again in
+// the next iteration; a shadow ray that would be lit but meets the box becomes
+// a record for k_shadow.
 //
 // Why one kernel and not one per stage: a ray meets at most a few dozen quads
 // and spheres outside the mesh, so that part of its trace is short, and what
@@ -49,16 +49,16 @@ namespace pcr {
 // rays have to find the closest of the mesh's emissive triangles (and requests
 // of few paths on mesh scenes, see Engine::route).  Such traces are long and
 // leave lanes idle, which costs more at 16 warps per SM and inside this code
-// than the stages' memory traffic.  So a path is followed for one
-// vertex and waits: k_extend traces its next ray in full, and each of its
-// shadow samples is a record for k_shadow.  Six batched renders with 4 (16)
-// shadow rays, by stages of one vertex alone / traced here / staged: a Cornell
-// box with a tilted quad 24.9 (63.7) / 32.7 (79.5) / 26.4 (66.3) ms, with 88 quads
-// 71 (206) / 102 (316) / 76 (217) ms, with a mesh light 61 (197) / 112 (330) / 58
-// (193) ms; 256x256, 16 paths a pixel, 4 shadow rays: 4.6 / 1.9 / 1.8, 9.4 / 6.5 /
-// 4.8 and 7.5 / 7.2 / 3.8 ms.  The rest of the difference in the first two: a warp
-// appends its own paths, so neighbours lose each other sooner than where a
-// block appends together (which takes k_shadow 3 % less and k_paths 3 to 8 % more).
+// than the stages' memory traffic.  So a path is followed for one vertex and
+// waits: k_extend traces its next ray in full, and each of its shadow samples
+// is a record for k_shadow.  Six batched renders with 4 (16) shadow rays, by
+// stages of one vertex alone / traced here / staged: a Cornell box with a tilted
+// quad 24.9 (63.7) / 32.7 (79.5) / 26.7 (66) ms, with 88 quads 71 (206) / 102 (316)
+// / 75 (217) ms, with a mesh light 61 (197) / 112 (330) / 57 (191) ms; 256x256, 16
+// paths a pixel, 4 shadow rays: 4.6 / 1.9 / 1.8, 9.4 / 6.5 / 4.8 and 7.5 / 7.2 / 3.7
+// ms.  The rest of the difference in the first two: a warp appends its own
+// paths, so neighbours lose each other sooner than where a block appends
+// together (which takes k_shadow 3 % less and k_paths 3 to 8 % more).
 constexpr int kPathBlock = 128;
 #ifndef PCR_PATH_MIN_BLOCKS
 #define PCR_PATH_MIN_BLOCKS 4
