@@ -1770,7 +1770,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
         throw PcrError(PCR_ERR_INVALID, "pcr_render_noalloc while batched work is active");
 
     unsigned char* base = static_cast<unsigned char*>(noalloc_scratch(device_));
-    // carve the array: header words first, then queues, hits, shadows, accumulator
+    // carve the array: header words first, then accumulator, queues, shadows
     size_t off = 0;
     auto take = [&](size_t bytes) {
         unsigned char* p = base + off;
@@ -1795,6 +1795,7 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     int* round_list = reinterpret_cast<int*>(take(4));
     const size_t header_used = off;
     off = kNoAllocHeader;
+    double* accum = reinterpret_cast<double*>(take(kNoAllocAccumBytes));  // (cleared with the header)
     PathQueue q[2];
     for (int b = 0; b < 2; b++) {
         unsigned char* p = take(kNoAllocQueueBytes);
@@ -1812,13 +1813,11 @@ void Engine::render_noalloc(int scene, const pcr_render_desc& desc, float* hdr_d
     sq.d = sq.o + kNoAllocShadow;
     sq.c = sq.d + kNoAllocShadow;
     sq.bound = reinterpret_cast<float*>(sq.c + kNoAllocShadow);
-    double* accum = reinterpret_cast<double*>(take(kNoAllocAccumBytes));
     if (off > kNoAllocBytes || header_used > kNoAllocHeader)
         throw PcrError(PCR_ERR_INVALID, "pcr_render_noalloc: scratch layout overflow");
 
     // the array keeps the previous call's contents: clear what starts at zero
-    CK(cudaMemsetAsync(base, 0, header_used, stream_));
-    CK(cudaMemsetAsync(accum, 0, (size_t)px * 3 * sizeof(double), stream_));
+    CK(cudaMemsetAsync(base, 0, kNoAllocHeader + (size_t)px * 3 * sizeof(double), stream_));
 
     EngineView E{};
     E.scenes = d_scenes_;
